@@ -282,7 +282,8 @@ __device__ __forceinline__ void wait_rows(const BuildArgs& A, int layer, int lo,
 
 // K1 on one tile (32 cells of layer T and all their actions) by one CTA.
 template <typename CntT, bool UNIT, bool FUSED>
-__device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* smem, const int T, const int tile) {
+__device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* smem, const int T, const int tile,
+                                           const int n_listed = -1) {
   const DevProblem& P = A.P;
   const int nthr = blockDim.x;
   const int tid = threadIdx.x;
@@ -303,7 +304,10 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
   if (!FUSED) {
     if (tid < 32) {
       const int cpw_log2 = 5 - lanes_log2;
-      const int64_t grp = group_of_slot((int64_t)tile * nwarps + (tid >> cpw_log2), g, 1 << cpw_log2);
+      const int slot = tile * nwarps + (tid >> cpw_log2);
+      int64_t grp = A.etiles_per_layer;  // a listed launch's unused warp: cells beyond the layer
+      if (n_listed < 0) grp = group_of_slot(slot, g, 1 << cpw_log2);
+      else if (slot < n_listed) grp = A.defer_list[(int64_t)T * A.etiles_per_layer + slot];
       cell_tab[tid] = (int)((grp << cpw_log2) + (tid & ((1 << cpw_log2) - 1)));
     }
     __syncthreads();
@@ -1000,9 +1004,10 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
   }
   const int total = __shfl_sync(0xffffffffu, incl, 31);
   unsigned long long wbase = 0;
-  if (lane == 0) {
+  const int first = cell_tab[warp << (5 - A.lanes_log2)];
+  if (lane == 0 && first < nc) {
     wbase = atomicAdd(A.counters + CTR_STAGE, (unsigned long long)total);
-    const int64_t wt = (int64_t)T * A.tiles_per_layer * nwarps + (cell_tab[warp << (5 - A.lanes_log2)] >> (5 - A.lanes_log2));
+    const int64_t wt = (int64_t)T * A.etiles_per_layer + (first >> (5 - A.lanes_log2));
     A.tile_base[wt] = (int64_t)wbase;
     A.tile_len[wt] = total;
   }
@@ -1047,11 +1052,32 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
   }
 }
 
-// K1 over a grid of (tile, layer - t0) CTAs.
+// K1 over a grid of (tile, layer - t0) CTAs; or, with a list from the ranked
+// builder, resident CTAs striding over the listed tiles, a CTA's warps taking
+// tiles of one layer.
 template <typename CntT, bool UNIT>
 __global__ void __launch_bounds__(1024) k_build_tiles(BuildArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  build_tile<CntT, UNIT, false>(A, smem, A.t0 + (int)blockIdx.y, (int)blockIdx.x);
+  const bool listed = A.defer_count != nullptr;
+  int T = A.t0 + (int)blockIdx.y, tile = (int)blockIdx.x, n = -1;
+  if (listed && A.counters[CTR_DEFERRED] == 0ull) return;
+  int64_t before = 0;  // items of the layers before T
+  const int nwarps = blockDim.x >> 5;
+  for (int64_t item = blockIdx.x;; item += gridDim.x) {
+    if (listed) {
+      for (; T < A.t1; ++T) {
+        n = (int)A.defer_count[T];
+        const int items = (n + nwarps - 1) / nwarps;
+        if (item < before + items) break;
+        before += items;
+      }
+      if (T >= A.t1) return;
+      tile = (int)(item - before);
+    }
+    build_tile<CntT, UNIT, false>(A, smem, T, tile, n);
+    if (!listed) return;
+    __syncthreads();  // the shared memory is free for the next tile
+  }
 }
 
 // Fused build+backup of all layers in one cooperative launch.  Tiles are
@@ -1266,6 +1292,10 @@ static cudaError_t raise_smem_cap(K kern, size_t sm, int* cap_set, std::mutex& m
 template <typename CntT, bool UNIT>
 static cudaError_t launch_one(const BuildArgs& A, int n_layers, cudaStream_t st) {
   dim3 grid((unsigned)A.tiles_per_layer, (unsigned)n_layers);
+  if (A.defer_count) {  // resident CTAs: about two an SM
+    const int64_t most = (int64_t)A.tiles_per_layer * n_layers;
+    grid = dim3((unsigned)std::min<int64_t>(most, 296));
+  }
   dim3 block((unsigned)(32u << A.lanes_log2));
   const size_t sm = build_smem_bytes(A.P.na, A.P.nm, A.rc, UNIT, A.ybufs);
   static std::mutex mu;
@@ -1304,6 +1334,10 @@ cudaError_t launch_build_tiles(const BuildArgs& A, int count_bits, int n_layers,
   if (count_bits == 16) return unit ? launch_one<uint16_t, true>(A, n_layers, st)
                                     : launch_one<uint16_t, false>(A, n_layers, st);
   return unit ? launch_one<uint32_t, true>(A, n_layers, st) : launch_one<uint32_t, false>(A, n_layers, st);
+}
+
+cudaError_t launch_build_deferred(const BuildArgs& A, int count_bits, cudaStream_t st) {
+  return launch_build_tiles(A, count_bits, A.t1 - A.t0, st);
 }
 
 cudaError_t launch_build_fused(const BuildArgs& A, cudaStream_t st, int* grid) {

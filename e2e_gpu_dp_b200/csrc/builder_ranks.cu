@@ -1,0 +1,802 @@
+// K1 by velocity ranks: the Monte-Carlo transition builder for grids whose
+// spacing is a power of two, up to ten modes and 2 to 32 actions; groups of
+// cells it cannot take (velocities spread too widely for a table, rows with
+// samples outside their 8x8 window) are listed and left to k_build_tiles.
+//
+// transition_calc (src/build_model.cu:483-559) moves every sample of every
+// action.  But along one axis the landing cell is a step function of the
+// velocity alone, and the steps of all actions lie at the same few places of
+// every cell (rank_plan.h).  So a velocity is ranked once among the steps of all
+// actions, one table lookup per axis, a cell's samples are counted by their
+// pair of ranks, and prefix sums over that small table give each action's cell
+// counts as differences of four entries:
+//   per (cell, realisation): the mode sum (20 fused multiply-adds, packed two
+//     realisations at a time) and about 17 more instructions, for all actions
+//     together, against 11-14 per action of the counting loops;
+//   per (cell, action): at most 81 table reads.
+// A sample within the zone of a step (where the reference's float rounding
+// decides) or outside the table's range, about 1 in 2000, goes to the cell's
+// list and takes the reference's full expression for each action.  Counts are
+// the reference's exactly; rewards are folded from the counts as in
+// k_build_tiles.
+//
+// Measured on B200 (whole call): 200x200x120, 16 actions, 5000 realisations
+// 330.6 -> 75.8 ms; 300x300x40, 2000 realisations 102.2 -> 27.8 ms; 137x137x53,
+// 24 actions, 777 realisations 29.6 -> 9.2 ms; 50x50x30, 500 realisations from
+// host fields 2.56 -> 1.65 ms.
+//
+// A CTA (8 warps) takes a run of cells of one layer, 256 rows where the action
+// count allows it.  A warp holds the coefficients of 128 realisations (4 a
+// lane) in registers and walks a subset of the cells, whose modes it reads as
+// broadcasts; the tables of the cells are shared by the CTA's warps (atomic
+// increments, no order needed).
+#include <algorithm>
+#include <mutex>
+#include <vector>
+
+#include "common.cuh"
+#include "kernels.h"
+#include "rank_plan.h"
+
+namespace e2e {
+
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kWarps = kThreads / 32;
+constexpr int kWin = 8;           // window side, as k_build_tiles
+constexpr int kListPool = 768;    // samples on the lists of a CTA's cells
+constexpr int kObsR = 10;         // obstacle bitmap radius around a cell
+constexpr int kObsRows = 2 * kObsR + 1;
+constexpr int kMaxCells = 32;     // cells of a CTA
+
+// A sampled cell's table.  state: 0 counted, 1 nothing to count (terminal or
+// obstacle cell, beyond the layer), 2 left to the general builder
+struct __align__(16) CellTab {
+  float bx, by;        // fixed-point offset of a velocity sum, x and y
+  int qax, qbx;        // the range's ends (bits): the zones of its first and last step
+  int qay, qby;
+  int lxo, lyo;        // word offset of slot 0 of the axis' lookup table
+  uint32_t mul, cst;   // counter index = rank_x + rank_y * stride + cst
+  int bax, bay;        // step index of the range's lower end, in table units
+  int orgx, orgy;      // step index of cell boundary b: b * G + off[action] - org
+  int nx, ny;          // ranks in the table
+  int stride, base;    // row stride and first word of the prefix sums (ny + 1 x nx + 1)
+  int kx, ky;          // table kinds
+  float u1, v1;
+  int state, pad;
+};
+
+// counts of one CTA's cells (see the file's head): 4 realisations of a lane
+// over the cells [c_lo, c_hi)
+template <int NM, bool FULL>
+__device__ __forceinline__ void count_block(const RankArgs& K, const float* yt, int r0, int nrz, const float4* md,
+                                            const CellTab* cells, int c_lo, int c_hi, const uint32_t* lut,
+                                            uint32_t* pool, int* lcnt, float2* list, int lcap) {
+  float2 y01[NM], y23[NM];
+#pragma unroll
+  for (int k = 0; k < NM; ++k) {
+    const float4 y = __ldg(reinterpret_cast<const float4*>(yt + (int64_t)k * K.nrp + r0));
+    y01[k] = make_float2(y.x, y.y);
+    y23[k] = make_float2(y.z, y.w);
+  }
+  const int sh = kRankFrac - K.slots_log2;
+  const uint32_t zm = K.zone_mask;
+  for (int c = c_lo; c < c_hi; ++c) {
+    const CellTab* ct = cells + c;
+    if (ct->state != 0) continue;
+    const float4 h0 = *reinterpret_cast<const float4*>(ct);
+    const int4 h1 = *reinterpret_cast<const int4*>(&ct->qay);
+    const uint2 h2 = *reinterpret_cast<const uint2*>(&ct->mul);
+    float2 sx01 = make_float2(0.f, 0.f), sx23 = sx01, sy01 = sx01, sy23 = sx01;
+    // extract_velocity's mode sums (src/build_model.cu:389-401), a chain of fused
+    // multiply-adds in mode order for each realisation and component
+#pragma unroll
+    for (int k = 0; k < NM; ++k) {
+      const float4 m = md[c * NM + k];
+      const float2 mu = make_float2(m.x, m.y), mv = make_float2(m.z, m.w);
+      sx01 = __ffma2_rn(mu, y01[k], sx01);
+      sx23 = __ffma2_rn(mu, y23[k], sx23);
+      sy01 = __ffma2_rn(mv, y01[k], sy01);
+      sy23 = __ffma2_rn(mv, y23[k], sy23);
+    }
+    const float2 fx = make_float2(K.sx, K.sx), fy = make_float2(K.sy, K.sy);
+    const float2 bx = make_float2(h0.x, h0.x), by = make_float2(h0.y, h0.y);
+    const float2 qx01 = __ffma2_rn(sx01, fx, bx), qx23 = __ffma2_rn(sx23, fx, bx);
+    const float2 qy01 = __ffma2_rn(sy01, fy, by), qy23 = __ffma2_rn(sy23, fy, by);
+    const int qax = __float_as_int(h0.z), qbx = __float_as_int(h0.w);
+    const float qx[4] = {qx01.x, qx01.y, qx23.x, qx23.y}, qy[4] = {qy01.x, qy01.y, qy23.x, qy23.y};
+    bool listed[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      // (a NaN or an overflow has bits beyond an end and is clamped to it)
+      const int x = min(max(__float_as_int(qx[i]), qax), qbx);
+      const int y = min(max(__float_as_int(qy[i]), h1.x), h1.y);
+      const uint32_t s = lut[(x >> sh) + h1.z] + (uint32_t)x;
+      const uint32_t t = lut[(y >> sh) + h1.w] + (uint32_t)y;
+      const bool amb = (s & zm) == 0u || (t & zm) == 0u;
+      const uint32_t at = __dp2a_lo(__byte_perm(s, t, 0x7632), h2.x, h2.y);
+      const bool in = FULL || r0 + i < nrz;
+      listed[i] = amb && in;
+      if (!amb && in) atomicAdd(pool + at, 1u);
+    }
+    if (listed[0] || listed[1] || listed[2] || listed[3]) {
+      const float sx[4] = {sx01.x, sx01.y, sx23.x, sx23.y}, sy[4] = {sy01.x, sy01.y, sy23.x, sy23.y};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (listed[i]) {
+          const int at = atomicAdd(lcnt + c, 1);
+          if (at < lcap) list[c * lcap + at] = make_float2(ct->u1 + sx[i], ct->v1 + sy[i]);
+        }
+      }
+    }
+  }
+}
+
+// the reference's obstacle override of (i1, j1) -> (i1 + di, j1 + dj)
+// (goes_through_obstacle, src/build_model.cu:444-477) from the cell's obstacle
+// bits: the same within_band tests, for the obstacle cells of the box only
+__device__ __forceinline__ bool passes_obstacle(const DevProblem& P, const int32_t* mask, int T, const uint32_t* rows,
+                                                int i1, int j1, int di, int dj) {
+  if (abs(di) > kObsR || abs(dj) > kObsR) return through_obstacle(P, mask, T, i1, j1, i1 + di, j1 + dj);
+  const int a0 = min(di, 0), a1 = max(di, 0), b0 = min(dj, 0), b1 = max(dj, 0);
+  const uint32_t cols = ((2u << (b1 - b0)) - 1u) << (b0 + kObsR);
+  for (int a = a0; a <= a1; ++a) {
+    uint32_t m = rows[a + kObsR] & cols;
+    if (!m) continue;
+    if (di == 0 || dj == 0) return true;  // within_band of an axis-parallel way
+    do {
+      const int b = __ffs(m) - 1 - kObsR;
+      if (within_band(P, i1 + a, j1 + b, i1, j1, i1 + di, j1 + dj)) return true;
+      m &= m - 1;
+    } while (m);
+  }
+  return false;
+}
+
+__device__ __forceinline__ void land_any(const DevProblem& P, float F, float cs, float sn, float vx, float vy, float x,
+                                         float y, int& i2, int& j2) {
+  if (P.unit_step) land_unit(P, F, cs, sn, vx, vy, x, y, i2, j2);
+  else land_general(P, F, cs, sn, vx, vy, x, y, i2, j2);
+}
+
+struct Smem {
+  uint32_t* lut;     // the plan's words
+  float* tab;        // 32 x 8 landing rewards
+  float4* md;        // cells x NM modes: (ui, ui, vi, vi)
+  CellTab* cells;
+  uint32_t* orow;    // cells x kObsRows obstacle bits
+  int* lcnt;         // cells: samples on the list
+  float2* list;      // kListPool
+  uint16_t* wcol;    // warps x 64 bins x 32 rows: counts of the rows a warp finishes
+  uint32_t* pool;    // rank tables
+};
+
+__host__ __device__ inline size_t smem_fixed_bytes(int slots_log2, int nm, int ct) {
+  size_t b = sizeof(uint32_t) * (size_t)rank_plan_words(slots_log2);
+  b += sizeof(float) * 32 * 8;
+  b += sizeof(float4) * (size_t)ct * nm;
+  b += sizeof(CellTab) * (size_t)ct;
+  b += sizeof(uint32_t) * (size_t)((ct * kObsRows + 3) & ~3);
+  b += sizeof(int) * kMaxCells;
+  b += sizeof(float2) * kListPool;
+  b += sizeof(uint16_t) * (size_t)kWarps * 64 * 32;
+  return b;
+}
+
+// the rows of one emission tile (32 / P cells x P action lanes of a warp):
+// window counts from the prefix sums and the lists, rewards, emission
+template <typename Dummy = void>
+__device__ __forceinline__ void finish_tile(const BuildArgs& A, const RankArgs& K, const Smem& S, int T, int64_t c0,
+                                            int tile, int lcap) {
+  const DevProblem& P = A.P;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = P.g;
+  const int64_t nc = (int64_t)g * g;
+  const int cpw_log2 = 5 - A.lanes_log2;
+  const int cl = (tile << cpw_log2) + (lane >> A.lanes_log2);
+  const int a = lane & ((1 << A.lanes_log2) - 1);
+  const int64_t cell = c0 + cl;
+  const int64_t et = (c0 >> cpw_log2) + tile;  // emission tile within the layer
+  if (c0 + ((int64_t)tile << cpw_log2) >= nc) return;  // beyond the layer (whole warp)
+  const CellTab& ct = S.cells[cl];
+  const bool valid = cell < nc && a < P.na;
+  uint16_t* const wcol = S.wcol + warp * 64 * 32 + lane;
+  const int i1 = valid ? (int)(cell / g) : 0;
+  const int j1 = valid ? (int)(cell - (int64_t)i1 * g) : 0;
+  const int aa = a < P.na ? a : 0;
+  const float F = P.ac_speed[aa], cs = P.ac_cos[aa], sn = P.ac_sin[aa];
+  const float x1 = P.xs[j1], y1 = P.ys[g - 1 - i1];
+  const bool late = T > P.nt - 20;
+  const bool rad = P.reward_type == 2 || P.reward_type == 3;
+  const int W = g < kWin ? g : kWin;
+  bool window = valid && ct.state != 1;
+  bool ok = !(valid && ct.state >= 2);
+  const int nlist = window ? S.lcnt[cl] : 0;
+  ok = ok && nlist <= lcap;
+  int wi0 = 0, wj0 = 0, n_cl = 0;
+  uint64_t nz = 0, ovr = 0;
+  if (window && ok) {
+    int ci, cj;  // the window around the mean flow's landing, as k_build_tiles
+    land_any(P, F, cs, sn, ct.u1, ct.v1, x1, y1, ci, cj);
+    wi0 = min(max(ci - (kWin / 2 - 1), i1 - P.del), i1 + P.del - W + 1);
+    wj0 = min(max(cj - (kWin / 2 - 1), j1 - P.del), j1 + P.del - W + 1);
+    wi0 = min(max(wi0, 0), g - W);
+    wj0 = min(max(wj0, 0), g - W);
+    const int* offs = reinterpret_cast<const int*>(S.lut + rank_off_at(K.slots_log2));
+    const int Gx = K.groups[ct.kx], Gy = K.groups[ct.ky];
+    const int nx = ct.nx, ny = ct.ny, stride = ct.stride;
+    const uint32_t* sat = S.pool + ct.base;
+    const int tx = wj0 * Gx + offs[ct.kx * 2 * kRankMaxActions + aa] - ct.orgx;
+    const int ty = wi0 * Gy + offs[ct.ky * 2 * kRankMaxActions + aa] - ct.orgy;
+    // ranks below window column lj; a clamped sample lands in the edge cell, so
+    // the grid's first and last cell have no outer boundary
+    int cx[kWin + 1];
+#pragma unroll
+    for (int lj = 0; lj <= kWin; ++lj) {
+      int t = min(max(tx + lj * Gx, 0), nx);
+      if (wj0 + lj <= 0) t = 0;
+      if (wj0 + lj >= g) t = nx;
+      if (lj > W) t = cx[lj > 0 ? lj - 1 : 0];
+      cx[lj] = t;
+    }
+    auto row_of = [&](int li) -> int {
+      int t = min(max(ty + li * Gy, 0), ny);
+      if (wi0 + li <= 0) t = 0;
+      if (wi0 + li >= g) t = ny;
+      return t;
+    };
+    uint32_t inside = 0;
+    int r0 = row_of(0);
+    for (int li = 0; li < W; ++li) {
+      const int r1 = row_of(li + 1);
+      if (r1 > r0) {
+        const uint32_t* p0 = sat + r0 * stride;
+        const uint32_t* p1 = sat + r1 * stride;
+        uint32_t left = p1[cx[0]] - p0[cx[0]];
+#pragma unroll
+        for (int lj = 0; lj < kWin; ++lj) {
+          if (cx[lj + 1] > cx[lj]) {
+            const uint32_t right = p1[cx[lj + 1]] - p0[cx[lj + 1]];
+            const uint32_t n = right - left;
+            left = right;
+            if (n) {
+              const int b = li * kWin + lj;
+              wcol[b * 32] = (uint16_t)n;
+              nz |= 1ull << b;
+              inside += n;
+            }
+          }
+        }
+      }
+      r0 = r1;
+    }
+    ok = inside == (uint32_t)(P.nrzns - nlist);  // else samples outside the window
+    // the listed samples, by the full expression
+    bool clamped = false;
+    for (int e = 0; e < nlist && ok; ++e) {
+      const float2 v = S.list[cl * lcap + e];
+      int i2, j2;
+      land_any(P, F, cs, sn, v.x, v.y, x1, y1, i2, j2);
+      const int li = i2 - wi0, lj = j2 - wj0;
+      ok = (unsigned)li < (unsigned)W && (unsigned)lj < (unsigned)W;
+      if (ok) {
+        const int b = li * kWin + lj;
+        const uint64_t bit = 1ull << b;
+        wcol[b * 32] = (uint16_t)((nz & bit) ? wcol[b * 32] + 1 : 1);
+        nz |= bit;
+        clamped = clamped || i2 == 0 || j2 == 0 || i2 == g - 1 || j2 == g - 1;
+      }
+    }
+    if (ok) {
+      for (uint64_t m = nz; m; m &= m - 1) {
+        const int b = __ffsll((long long)m) - 1;
+        const int i2 = wi0 + (b >> 3), j2 = wj0 + (b & 7);
+        if (passes_obstacle(P, A.F.mask, T, S.orow + cl * kObsRows, i1, j1, i2 - i1, j2 - j1)) ovr |= 1ull << b;
+      }
+      // domain clamps of the samples in bins that no obstacle overrides: each adds
+      // one r_outbound (move(), src/build_model.cu:291-310)
+      if (clamped) {
+        for (int e = 0; e < nlist; ++e) {
+          const float2 v = S.list[cl * lcap + e];
+          int i2, j2;
+          land_any(P, F, cs, sn, v.x, v.y, x1, y1, i2, j2);
+          const int b = (i2 - wi0) * kWin + j2 - wj0;
+          if ((ovr >> b) & 1ull) continue;
+          float xn, yn;
+          advect(P, F, cs, sn, v.x, v.y, x1, y1, xn, yn);
+          n_cl += (xn > P.xsn || xn < P.xs0) ? 1 : 0;
+          n_cl += (yn > P.ysn || yn < P.ys0) ? 1 : 0;
+        }
+      }
+      auto rect = [&](int ra, int rb, int ca, int cb) -> int {
+        if (rb <= ra || cb <= ca) return 0;
+        return (int)(sat[rb * stride + cb] - sat[ra * stride + cb] - sat[rb * stride + ca] + sat[ra * stride + ca]);
+      };
+      if (ct.kx & 1) {
+        const int te = offs[ct.kx * 2 * kRankMaxActions + kRankMaxActions + aa] - ct.orgx;
+        for (int side = 0; side < 2; ++side) {
+          const int lj = side ? g - 1 - wj0 : -wj0;
+          if (lj < 0 || lj >= W) continue;
+          const int t = min(max(te + (side ? g - 1 : 0) * Gx, 0), nx);
+          const int ca = side ? t : 0, cb = side ? nx : t;
+          for (int li = 0; li < W; ++li)
+            if (!((ovr >> (li * kWin + lj)) & 1ull)) n_cl += rect(row_of(li), row_of(li + 1), ca, cb);
+        }
+      }
+      if (ct.ky & 1) {
+        const int te = offs[ct.ky * 2 * kRankMaxActions + kRankMaxActions + aa] - ct.orgy;
+        for (int side = 0; side < 2; ++side) {
+          const int li = side ? g - 1 - wi0 : -wi0;
+          if (li < 0 || li >= W) continue;
+          const int t = min(max(te + (side ? g - 1 : 0) * Gy, 0), ny);
+          const int ra = side ? t : 0, rb = side ? ny : t;
+#pragma unroll
+          for (int lj = 0; lj < kWin; ++lj)
+            if (!((ovr >> (li * kWin + lj)) & 1ull)) n_cl += rect(ra, rb, cx[lj], cx[lj + 1]);
+        }
+      }
+    }
+  }
+  if (__any_sync(0xffffffffu, !ok)) {  // the tile goes to the general builder
+    if (lane == 0) {
+      const unsigned at = atomicAdd(A.defer_count + T, 1u);
+      A.defer_list[(int64_t)T * K.etiles_per_layer + at] = (int32_t)et;
+      atomicAdd(A.counters + CTR_DEFERRED, 1ull);
+    }
+    return;
+  }
+  float sumR = 0.f;
+  uint32_t n_drop = 0, n_misbin = 0;
+  if (window) {
+    // the rewards folded from the counts, as k_build_tiles' fold_window
+    const float rad1 = rad ? __ldg(A.F.s + (int64_t)T * nc + cell) : 0.f;
+    for (uint64_t m = nz; m; m &= m - 1) {
+      const int b = __ffsll((long long)m) - 1;
+      const uint32_t c = wcol[b * 32];
+      const int i2 = wi0 + (b >> 3), j2 = wj0 + (b & 7);
+      float r;
+      if ((ovr >> b) & 1ull) {
+        r = P.r_out;
+      } else {
+        const int k = (i2 == 0 || i2 == g - 1 || j2 == 0 || j2 == g - 1) ? 1 : 0;
+        const bool tm = is_terminal(P, i2, j2);
+        if (!rad) {
+          r = S.tab[aa * 8 + (tm ? 4 : 0) + k];
+        } else {
+          const float rad2 = __ldg(A.F.s + (int64_t)(T + 1) * nc + (int64_t)i2 * g + j2);
+          r = k ? P.r_out : 0.f;
+          if (tm) r += P.r_term;
+          else if (late) r += 0.05 * P.r_out;
+          r += step_reward(P, F, rad1, rad2);
+        }
+      }
+      sumR = __fmaf_rn((float)c, r, sumR);
+      if (abs(i2 - i1) > P.del || abs(j2 - j1) > P.del) {  // the reference counts its reward only
+        n_drop += c;
+        if (i2 - i1 + P.del < P.m && j2 - j1 + P.del < P.m) n_misbin += c;
+        nz &= ~(1ull << b);
+      }
+    }
+    sumR = __fmaf_rn((float)n_cl, P.r_out, sumR);
+    if (n_drop) atomicAdd(A.counters + CTR_DROPPED, (unsigned long long)n_drop);
+    if (n_misbin) atomicAdd(A.counters + CTR_MISBIN, (unsigned long long)n_misbin);
+  } else if (valid && !is_terminal(P, i1, j1)) {
+    sumR = K.stay_sum;  // obstacle cell: no move, r_outbound per sample (:542-544)
+  }
+  const int nnz = !valid ? 0 : (window ? __popcll(nz) : 1);
+  int incl = nnz;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t2 = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t2;
+  }
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  unsigned long long wbase = 0;
+  if (lane == 0) {
+    wbase = atomicAdd(A.counters + CTR_STAGE, (unsigned long long)total);
+    const int64_t wt = (int64_t)T * K.etiles_per_layer + et;
+    A.tile_base[wt] = (int64_t)wbase;
+    A.tile_len[wt] = total;
+  }
+  wbase = __shfl_sync(0xffffffffu, wbase, 0);
+  if (!valid) return;
+  const int64_t grow = ((int64_t)T * nc + cell) * P.na + a;
+  A.row_off[grow] = (uint32_t)(incl - nnz);
+  A.R[grow] = sumR / P.nrzns;  // compute_mean, src/build_model.cu:567
+  if (A.sumR) A.sumR[grow] = sumR;
+  unsigned long long off = wbase + (unsigned long long)(incl - nnz);
+  if (off + (unsigned long long)nnz > (unsigned long long)A.stage_cap) return;  // host re-runs
+  const int32_t next = (int32_t)((int64_t)(T + 1) * nc);
+  auto put = [&](int32_t col, uint32_t n) {
+    A.stage_col[off] = col;
+    if (K.count_bits == 16) reinterpret_cast<uint16_t*>(A.stage_cnt)[off] = (uint16_t)n;
+    else reinterpret_cast<uint32_t*>(A.stage_cnt)[off] = n;
+    ++off;
+  };
+  if (!window) {
+    put(next + (int32_t)cell, (uint32_t)P.nrzns);
+  } else {
+    for (uint64_t m = nz; m; m &= m - 1) {
+      const int b = __ffsll((long long)m) - 1;
+      put(next + (wi0 + (b >> 3)) * g + wj0 + (b & 7), wcol[b * 32]);
+    }
+  }
+}
+
+// the range of one axis' table: a thread per (cell, axis)
+__device__ __forceinline__ void cell_axis(const RankArgs& K, const uint32_t* plan, CellTab& ct, const float4* md, int nm,
+                                          int axis, float mean_v, int idx, int g, const float* stat) {
+  float centre = mean_v, var = 0.f;
+  for (int k = 0; k < nm; ++k) {
+    const float w = axis ? md[k].z : md[k].x;
+    centre = fmaf(w, __ldg(stat + 2 * k), centre);
+    var = fmaf(w * w, __ldg(stat + 2 * k + 1), var);
+  }
+  RankRange r;
+  if (!rank_range(plan, K.slots_log2, K.groups, axis, axis ? K.sy : K.sx, K.shift, K.a_min[axis], K.a_max[axis], mean_v,
+                  centre, var, idx, g, &r)) {
+    ct.state = 2;  // (both axes' threads write 2)
+    return;
+  }
+  if (axis == 0) {
+    ct.bx = r.bias;
+    ct.qax = r.qa;
+    ct.qbx = r.qb;
+    ct.lxo = r.lut;
+    ct.bax = r.first;
+    ct.orgx = r.org;
+    ct.nx = r.n;
+    ct.kx = r.kind;
+  } else {
+    ct.by = r.bias;
+    ct.qay = r.qa;
+    ct.qby = r.qb;
+    ct.lyo = r.lut;
+    ct.bay = r.first;
+    ct.orgy = r.org;
+    ct.ny = r.n;
+    ct.ky = r.kind;
+  }
+}
+
+template <int NM>
+__global__ void __launch_bounds__(kThreads, 2) k_build_ranks(BuildArgs A, RankArgs K) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const DevProblem& P = A.P;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = P.g, nrz = P.nrzns, CT = K.cells;
+  const int64_t nc = (int64_t)g * g;
+  const int lcap = kListPool / CT;
+  const int cpw_log2 = 5 - A.lanes_log2;
+  const int ntiles = CT >> cpw_log2;
+  Smem S;
+  {
+    unsigned char* p = smem;
+    auto take = [&](size_t b) {
+      unsigned char* q = p;
+      p += b;
+      return q;
+    };
+    S.md = reinterpret_cast<float4*>(take(sizeof(float4) * CT * NM));
+    S.cells = reinterpret_cast<CellTab*>(take(sizeof(CellTab) * CT));
+    S.lut = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * rank_plan_words(K.slots_log2)));
+    S.tab = reinterpret_cast<float*>(take(sizeof(float) * 32 * 8));
+    S.orow = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * ((CT * kObsRows + 3) & ~3)));
+    S.lcnt = reinterpret_cast<int*>(take(sizeof(int) * kMaxCells));
+    S.list = reinterpret_cast<float2*>(take(sizeof(float2) * kListPool));
+    S.wcol = reinterpret_cast<uint16_t*>(take(sizeof(uint16_t) * kWarps * 64 * 32));
+    S.pool = reinterpret_cast<uint32_t*>(p);
+  }
+  __shared__ int pool_used;
+  for (int i = tid; i < rank_plan_words(K.slots_log2); i += kThreads) S.lut[i] = __ldg(K.plan + i);
+  const int tasks_per_layer = (int)((nc + CT - 1) / CT);
+  const int64_t tasks = (int64_t)(K.t1 - K.t0) * tasks_per_layer;
+  int tab_late = -1;
+  for (int64_t task = blockIdx.x; task < tasks; task += gridDim.x) {
+    const int T = K.t0 + (int)(task / tasks_per_layer);
+    const int64_t c0 = (task % tasks_per_layer) * CT;
+    __syncthreads();  // the previous task's tables are consumed
+    // ---- stage the cells -------------------------------------------------------
+    const bool late = T > P.nt - 20;
+    if (tab_late != (late ? 1 : 0)) {
+      tab_late = late ? 1 : 0;
+      if (tid < P.na) {
+        // landing rewards after k r_outbound additions, then terminal or late, then
+        // the step reward: move() + transition_calc (:343-354, :533)
+        const float r_step = step_reward(P, P.ac_speed[tid], 0.f, 0.f);
+        float tk = 0;
+        for (int k = 0; k < 4; ++k) {
+          float r = tk;
+          if (late) r += 0.05 * P.r_out;
+          r += r_step;
+          S.tab[tid * 8 + k] = r;
+          float rt = tk;
+          rt += P.r_term;
+          rt += r_step;
+          S.tab[tid * 8 + 4 + k] = rt;
+          tk += P.r_out;
+        }
+      }
+    }
+    for (int e = tid; e < CT * NM; e += kThreads) {
+      const int k = e / CT, c = e - k * CT;
+      float ui = 0.f, vi = 0.f;
+      if (k < P.nm && c0 + c < nc) {
+        ui = __ldg(A.F.ui + ((int64_t)T * P.nm + k) * nc + c0 + c);
+        vi = __ldg(A.F.vi + ((int64_t)T * P.nm + k) * nc + c0 + c);
+      }
+      S.md[c * NM + k] = make_float4(ui, ui, vi, vi);
+    }
+    for (int e = tid; e < CT * kObsRows; e += kThreads) {
+      const int c = e / kObsRows, a = e - c * kObsRows - kObsR;
+      uint32_t bits = 0;
+      if (c0 + c < nc) {
+        const int i1 = (int)((c0 + c) / g), j1 = (int)(c0 + c - (int64_t)i1 * g), i = i1 + a;
+        if (i >= 0 && i < g) {
+          const uint32_t* row = K.obits + ((int64_t)T * g + i) * K.owords;
+          const int b = j1 - kObsR, w = b >> 5;
+          const uint32_t lo = w >= 0 ? __ldg(row + w) : 0u, hi = w + 1 < K.owords ? __ldg(row + w + 1) : 0u;
+          bits = __funnelshift_r(lo, hi, b & 31) & ((1u << kObsRows) - 1u);
+          if (a == 0) bits &= ~(1u << kObsR);  // the cell itself does not count
+        }
+      }
+      S.orow[e] = bits;
+    }
+    if (tid < CT) {
+      const int64_t cell = c0 + tid;
+      CellTab& ct = S.cells[tid];
+      ct.state = 1;
+      S.lcnt[tid] = 0;
+      if (cell < nc) {
+        const int i1 = (int)(cell / g), j1 = (int)(cell - (int64_t)i1 * g);
+        ct.u1 = __ldg(A.F.u + (int64_t)T * nc + cell);
+        ct.v1 = __ldg(A.F.v + (int64_t)T * nc + cell);
+        if (!is_terminal(P, i1, j1) && __ldg(A.F.mask + (int64_t)T * nc + cell) != 1) ct.state = 0;
+      }
+    }
+    __syncthreads();
+    // ---- ranges and table space ----------------------------------------------
+    if (tid < 2 * CT) {
+      const int c = tid >> 1, axis = tid & 1;
+      CellTab& ct = S.cells[c];
+      if (ct.state != 1) {
+        const int64_t cell = c0 + c;
+        const int i1 = (int)(cell / g), j1 = (int)(cell - (int64_t)i1 * g);
+        cell_axis(K, S.lut, ct, S.md + c * NM, NM, axis, axis ? ct.v1 : ct.u1, axis ? i1 : j1, g,
+                  K.ystat + (int64_t)T * 2 * NM);
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      int words = 0, stride = 0, state = 1;
+      CellTab* ct = S.cells + (lane < CT ? lane : 0);
+      if (lane < CT) {
+        state = ct->state;
+        if (state == 0) {
+          stride = (ct->nx + 1) | 1;
+          words = (ct->ny + 1) * stride;
+          if (stride > 255) {
+            state = 2;
+            words = 0;
+          }
+        }
+      }
+      int end = words;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += v;
+      }
+      if (state == 0 && end > K.pool_words) state = 2;
+      const unsigned out = __ballot_sync(0xffffffffu, state == 2);
+      // a cell beside one that is left to the general builder is not counted either
+      const unsigned mates = (cpw_log2 == 5 ? ~0u : ((1u << (1 << cpw_log2)) - 1u) << ((lane >> cpw_log2) << cpw_log2));
+      if (state == 0 && (out & mates)) state = 2;
+      if (lane < CT) {
+        ct->state = state;
+        if (state == 0) {
+          const int base = end - words;
+          ct->stride = stride;
+          ct->base = base;
+          ct->mul = ((uint32_t)stride << 8) | 1u;
+          ct->cst = (uint32_t)(base - ct->bax - ct->bay * stride);
+        }
+      }
+      const int used = min(__shfl_sync(0xffffffffu, end, 31), K.pool_words);
+      if (lane == 0) pool_used = used;
+    }
+    __syncthreads();
+    {
+      const int n4 = (pool_used + 3) >> 2;
+      for (int i = tid; i < n4; i += kThreads) reinterpret_cast<uint4*>(S.pool)[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    __syncthreads();
+    // ---- count the realisations ------------------------------------------------
+    {
+      const float* yt = K.yt + (int64_t)T * NM * K.nrp;
+      const int per = CT / K.nsub;
+      for (int it = warp; it < K.nblocks * K.nsub; it += kWarps) {
+        const int blk = it / K.nsub, sub = it - blk * K.nsub;
+        const int r0 = blk * 128 + 4 * lane;
+        if (blk * 128 + 128 <= nrz)
+          count_block<NM, true>(K, yt, r0, nrz, S.md, S.cells, sub * per, (sub + 1) * per, S.lut, S.pool, S.lcnt, S.list,
+                                lcap);
+        else
+          count_block<NM, false>(K, yt, r0, nrz, S.md, S.cells, sub * per, (sub + 1) * per, S.lut, S.pool, S.lcnt, S.list,
+                                 lcap);
+      }
+    }
+    __syncthreads();
+    // ---- prefix sums of the tables: along x, then along y -------------------------
+    for (int c = warp; c < CT; c += kWarps) {
+      const CellTab& ct = S.cells[c];
+      if (ct.state != 0) continue;
+      uint32_t* t = S.pool + ct.base;
+      for (int y = 1 + lane; y <= ct.ny; y += 32) {
+        uint32_t* p = t + y * ct.stride + 1;
+        uint32_t run = 0;
+        for (int x = 0; x < ct.nx; ++x) {
+          run += p[x];
+          p[x] = run;
+        }
+      }
+      __syncwarp();
+      for (int x = 1 + lane; x <= ct.nx; x += 32) {
+        uint32_t* p = t + ct.stride + x;
+        uint32_t run = 0;
+        for (int y = 0; y < ct.ny; ++y) {
+          run += *p;
+          *p = run;
+          p += ct.stride;
+        }
+      }
+    }
+    __syncthreads();
+    // ---- the rows ------------------------------------------------------------------
+    for (int tile = warp; tile < ntiles; tile += kWarps) finish_tile(A, K, S, T, c0, tile, lcap);
+  }
+}
+
+// Per layer [t0, t1): the coefficients mode-major with rows padded to nrp (so a
+// lane reads four realisations at once), their mean and variance per mode (the
+// tables' ranges), and a bit per cell for the obstacles at T or T + 1.
+// blockIdx.y == 0: coefficients; others: 32 grid rows each.
+template <int NM>
+__global__ void __launch_bounds__(1024) k_rank_prepare(DevProblem P, DevFields F, RankArgs K, float* yt, float* ystat,
+                                                       uint32_t* obits) {
+  const int T = K.t0 + blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (blockIdx.y == 0) {
+    __shared__ float red[32][2 * NM];
+    const float* y = F.Y + (int64_t)T * P.nrzns * P.nm;
+    float* o = yt + (int64_t)T * NM * K.nrp;
+    float s[NM], q[NM];
+#pragma unroll
+    for (int k = 0; k < NM; ++k) s[k] = q[k] = 0.f;
+    for (int r = tid; r < K.nrp; r += 1024) {
+#pragma unroll
+      for (int k = 0; k < NM; ++k) {
+        const float v = (r < P.nrzns && k < P.nm) ? __ldg(y + (int64_t)r * P.nm + k) : 0.f;
+        o[(int64_t)k * K.nrp + r] = v;
+        s[k] += v;
+        q[k] = fmaf(v, v, q[k]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < NM; ++k) {
+      for (int w = 16; w > 0; w >>= 1) {
+        s[k] += __shfl_xor_sync(0xffffffffu, s[k], w);
+        q[k] += __shfl_xor_sync(0xffffffffu, q[k], w);
+      }
+      if (lane == 0) {
+        red[warp][2 * k] = s[k];
+        red[warp][2 * k + 1] = q[k];
+      }
+    }
+    __syncthreads();
+    if (tid < NM) {
+      float a = 0.f, b = 0.f;
+      for (int w = 0; w < 32; ++w) {
+        a += red[w][2 * tid];
+        b += red[w][2 * tid + 1];
+      }
+      const float m = a / (float)P.nrzns;
+      ystat[(int64_t)T * 2 * NM + 2 * tid] = m;
+      ystat[(int64_t)T * 2 * NM + 2 * tid + 1] = fmaxf(b / (float)P.nrzns - m * m, 0.f);
+    }
+    return;
+  }
+  const int i = ((int)blockIdx.y - 1) * 32 + warp;
+  if (i >= P.g) return;
+  const int64_t nc = (int64_t)P.g * P.g;
+  const int32_t* m0 = F.mask + (int64_t)T * nc + (int64_t)i * P.g;
+  for (int w = 0; w < K.owords; ++w) {
+    const int j = w * 32 + lane;
+    const bool ob = j < P.g && (__ldg(m0 + j) == 1 || __ldg(m0 + nc + j) == 1);
+    const uint32_t bits = __ballot_sync(0xffffffffu, ob);
+    if (lane == 0) obits[((int64_t)T * P.g + i) * K.owords + w] = bits;
+  }
+}
+
+std::mutex g_cap_mu;
+bool g_cap_set[64][8] = {};
+
+// f(integral constant of the padded mode count)
+template <typename F>
+cudaError_t dispatch_nm(int nmp, F&& f) {
+  switch (nmp) {
+    case 2: return f(std::integral_constant<int, 2>{});
+    case 4: return f(std::integral_constant<int, 4>{});
+    case 6: return f(std::integral_constant<int, 6>{});
+    case 8: return f(std::integral_constant<int, 8>{});
+    case 10: return f(std::integral_constant<int, 10>{});
+  }
+  return cudaErrorInvalidValue;
+}
+
+constexpr size_t kSmemPerCta = 112 * 1024;  // two CTAs an SM
+
+}  // namespace
+
+int rank_padded_modes(int nm) { return nm <= 2 ? 2 : (nm + 1) & ~1; }
+
+bool rank_shape(int nm, int slots_log2, int lanes_log2, int nrzns, RankArgs* K) {
+  if (nm > 10) return false;
+  const int nmp = rank_padded_modes(nm);
+  K->slots_log2 = slots_log2;
+  K->cells = std::min(kMaxCells, 256 >> lanes_log2);
+  const size_t fixed = smem_fixed_bytes(slots_log2, nmp, K->cells);
+  if (fixed + 16 * 1024 > kSmemPerCta) return false;
+  K->pool_words = (int)((kSmemPerCta - fixed) / 4) & ~3;
+  K->nrp = (nrzns + 127) / 128 * 128;
+  K->nblocks = K->nrp / 128;
+  // subsets of the cells: a warp's work item is 128 realisations x one subset.
+  // Fewer subsets load the coefficients less often (about a cell's worth of
+  // work), more of them spread few realisation blocks over the warps.
+  double best = 1e30;
+  for (int ns = 2; ns <= 8; ns *= 2) {
+    const double cost = ((K->nblocks * ns + kWarps - 1) / kWarps) * (K->cells / ns + 1.0);
+    if (cost < best) {
+      best = cost;
+      K->nsub = ns;
+    }
+  }
+  return true;
+}
+
+cudaError_t launch_rank_prepare(const DevProblem& P, const DevFields& F, const RankArgs& K, cudaStream_t st) {
+  const dim3 grid((unsigned)(K.t1 - K.t0), (unsigned)(1 + (P.g + 31) / 32));
+  return dispatch_nm(rank_padded_modes(P.nm), [&](auto nm) -> cudaError_t {
+    k_rank_prepare<decltype(nm)::value><<<grid, 1024, 0, st>>>(P, F, K, const_cast<float*>(K.yt),
+                                                                const_cast<float*>(K.ystat),
+                                                                const_cast<uint32_t*>(K.obits));
+    return cudaGetLastError();
+  });
+}
+
+cudaError_t launch_build_ranks(const BuildArgs& A, const RankArgs& K, cudaStream_t st) {
+  const int nmp = rank_padded_modes(A.P.nm);
+  const size_t sm = smem_fixed_bytes(K.slots_log2, nmp, K.cells) + 4 * (size_t)K.pool_words;
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+  const int64_t nc = (int64_t)A.P.g * A.P.g;
+  const int64_t tasks = (int64_t)(K.t1 - K.t0) * ((nc + K.cells - 1) / K.cells);
+  const unsigned grid = (unsigned)std::min<int64_t>(tasks, 2 * (int64_t)sms);
+  if (grid == 0) return cudaSuccess;
+  return dispatch_nm(nmp, [&](auto nm) -> cudaError_t {
+    auto kern = k_build_ranks<decltype(nm)::value>;
+    {
+      std::lock_guard<std::mutex> lk(g_cap_mu);
+      if (dev < 0 || dev >= 64 || !g_cap_set[dev][nmp / 2]) {
+        cudaError_t e2 = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemPerCta);
+        if (e2 != cudaSuccess) return e2;
+        if (dev >= 0 && dev < 64) g_cap_set[dev][nmp / 2] = true;
+      }
+    }
+    kern<<<grid, kThreads, sm, st>>>(A, K);
+    return cudaGetLastError();
+  });
+}
+
+}  // namespace e2e

@@ -17,6 +17,7 @@
 #include "internal.h"
 #include "kernels.h"
 #include "npy_io.h"
+#include "rank_plan.h"
 
 using namespace e2e;
 
@@ -670,6 +671,22 @@ extern "C" e2e_status e2e_build_model(const e2e_problem* p, const e2e_fields* f,
 
 namespace e2e {
 
+// Whether a row's reward sum is the same in any order of its samples: rewards
+// of the time type that are all multiples of one power of two, with sums below
+// 2^24 of it.
+static bool order_free_rewards(const e2e_problem* p) {
+  if (p->reward_type != 0) return false;
+  const double late = (float)(0.05 * p->r_outbound);
+  const double v[4] = {p->r_outbound, p->r_terminal, p->dt, late};
+  double biggest = 3 * std::fabs(v[0]) + std::fabs(v[1]) + std::fabs(v[2]) + std::fabs(v[3]);
+  for (double unit = 1.0; unit > 1e-6; unit /= 2) {
+    bool all = true;
+    for (double x : v) all = all && std::fmod(x, unit) == 0;
+    if (all) return biggest * p->nrzns < 16777216.0 * unit;
+  }
+  return false;
+}
+
 e2e_status plan_build(const e2e_problem* p, int count_bits, int64_t stage_hint, BuildPlan* pl) {
   pl->count_bits = count_bits;
   pl->ncells = (int64_t)p->gsize * p->gsize;
@@ -680,7 +697,7 @@ e2e_status plan_build(const e2e_problem* p, int count_bits, int64_t stage_hint, 
   {
     const int nwarps = 1 << build_lanes_log2(pl->na);  // emission tiles (warps) per CTA
     pl->cells_per_tile = 32 / nwarps;
-    pl->etiles_per_layer = pl->tiles_per_layer * nwarps;
+    pl->etiles_per_layer = (pl->ncells + pl->cells_per_tile - 1) / pl->cells_per_tile;
     pl->n_tiles = pl->etiles_per_layer * (p->nt - 1);
   }
   // realisations per velocity chunk: 128 for unit spacing (no mask table)
@@ -688,8 +705,34 @@ e2e_status plan_build(const e2e_problem* p, int count_bits, int64_t stage_hint, 
   // need exceeds 200 KB
   bool unit;
   {  // the test of make_dev_problem (unit_step) on the same ticks
-    std::vector<float> xs, ys;
+    std::vector<float> xs, ys, speed, angle;
     host_ticks(p, xs, ys);
+    host_actions(p, speed, angle);
+    RankPlan rp;
+    // Unit spacing: the general builder folds its rewards from the counts too.
+    // Other spacings: it adds them sample by sample, so only sums that do not
+    // depend on the order come from the counts.
+    const bool unit_step = std::fabs(xs[1] - xs[0]) == 1.0f && std::fabs(ys[1] - ys[0]) == 1.0f;
+    if ((unit_step || order_free_rewards(p)) &&
+        make_rank_plan(p->gsize, pl->na, p->dt, speed, angle, xs, ys, &rp) &&
+        rank_shape(p->nmodes, rp.slots_log2, build_lanes_log2(pl->na), p->nrzns, &pl->rank)) {
+      pl->ranked = true;
+      pl->rank_words.swap(rp.words);
+      RankArgs& K = pl->rank;
+      K.zone_mask = rp.zone_mask;
+      K.shift = rp.shift;
+      K.sx = rp.sx;
+      K.sy = rp.sy;
+      for (int k = 0; k < 4; ++k) K.groups[k] = rp.groups[k];
+      for (int k = 0; k < 2; ++k) {
+        K.a_min[k] = (float)rp.a_min[k];
+        K.a_max[k] = (float)rp.a_max[k];
+      }
+      K.owords = (p->gsize + 31) / 32;
+      for (int r = 0; r < p->nrzns; ++r) K.stay_sum += p->r_outbound;
+      K.count_bits = count_bits;
+      K.etiles_per_layer = pl->etiles_per_layer;
+    }
     unit = std::fabs(xs[1] - xs[0]) == 1.0f && std::fabs(ys[1] - ys[0]) == 1.0f;
   }
   pl->rc = unit ? 128 : 64;
@@ -801,6 +844,34 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
   CK(dalloc((void**)&ctr, sizeof(unsigned long long) * CTR_COUNT, st));
   scratch->add(ctr);
 
+  // the ranked builder's inputs, filled on the device per range of layers
+  RankArgs K = pl.rank;
+  unsigned int* defer_count = nullptr;
+  int32_t* defer_list = nullptr;
+  if (pl.ranked) {
+    const size_t nmp = (size_t)rank_padded_modes(p->nmodes), layers = (size_t)(p->nt - 1);
+    uint32_t *plan = nullptr, *obits = nullptr;
+    float *yt = nullptr, *ystat = nullptr;
+    const size_t pb = sizeof(uint32_t) * pl.rank_words.size();
+    CK(dalloc((void**)&plan, pb, st));
+    scratch->add(plan);
+    CK(cudaMemcpyAsync(plan, pl.rank_words.data(), pb, cudaMemcpyHostToDevice, st));
+    CK(dalloc((void**)&yt, sizeof(float) * layers * nmp * (size_t)K.nrp, st));
+    scratch->add(yt);
+    CK(dalloc((void**)&ystat, sizeof(float) * layers * nmp * 2, st));
+    scratch->add(ystat);
+    CK(dalloc((void**)&obits, sizeof(uint32_t) * layers * (size_t)p->gsize * (size_t)K.owords, st));
+    scratch->add(obits);
+    CK(dalloc((void**)&defer_count, sizeof(unsigned int) * layers, st));
+    scratch->add(defer_count);
+    CK(dalloc((void**)&defer_list, sizeof(int32_t) * (size_t)pl.n_tiles, st));
+    scratch->add(defer_list);
+    K.plan = plan;
+    K.yt = yt;
+    K.ystat = ystat;
+    K.obits = obits;
+  }
+
   int64_t cap = pl.stage_cap, pool_units = pl.pool_units;
   int32_t* stage_col = nullptr;
   void* stage_cnt = nullptr;
@@ -822,10 +893,12 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
     }
     if (!pool) CK(dalloc((void**)&pool, sizeof(uint32_t) * (size_t)mm * (size_t)pool_units, st));
     CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * CTR_COUNT, st));
-    BuildArgs A;
+    BuildArgs A{};
     A.P = D;
     A.F = F;
     A.t0 = 0;
+    A.t1 = p->nt - 1;
+    A.etiles_per_layer = pl.etiles_per_layer;
     A.tiles_per_layer = (int)pl.tiles_per_layer;
     A.rc = pl.rc;
     A.ybufs = pl.ybufs;
@@ -841,6 +914,24 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
     A.sumR = m->sumR;
     A.pool = pool;
     A.pool_units = pool_units;
+    if (pl.ranked) {
+      CK(cudaMemsetAsync(defer_count, 0, sizeof(unsigned int) * (size_t)(p->nt - 1), st));
+      A.defer_count = defer_count;
+      A.defer_list = defer_list;
+    }
+    // layers [t0, t1)
+    auto build_layers = [&](int t0, int t1) -> cudaError_t {
+      m->build_launches++;
+      BuildArgs B = A;
+      B.t0 = t0;
+      B.t1 = t1;
+      if (!pl.ranked) return launch_build_tiles(B, pl.count_bits, t1 - t0, st);
+      RankArgs R = K;
+      R.t0 = t0;
+      R.t1 = t1;
+      cudaError_t e = launch_rank_prepare(D, F, R, st);
+      return e != cudaSuccess ? e : launch_build_ranks(B, R, st);
+    };
     CK(cudaEventRecord(ev[0], st));
     trace_mark("buffers");
     if (attempt == 0 && fd.n_deferred) {
@@ -873,21 +964,16 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
         CK(cudaEventRecord(evs[1], cps));
         trace_mark("copies");
       }
-      BuildArgs A0 = A;
-      CK(launch_build_tiles(A0, pl.count_bits, la, st));
-      m->build_launches++;
+      CK(build_layers(0, la));
       trace_mark("first_layers");
       if (la < p->nt - 1) {
         CK(cudaStreamWaitEvent(st, evs[1], 0));
-        BuildArgs A1 = A;
-        A1.t0 = la;
-        CK(launch_build_tiles(A1, pl.count_bits, p->nt - 1 - la, st));
-        m->build_launches++;
+        CK(build_layers(la, p->nt - 1));
       }
     } else {
-      CK(launch_build_tiles(A, pl.count_bits, p->nt - 1, st));
-      m->build_launches++;
+      CK(build_layers(0, p->nt - 1));
     }
+    if (pl.ranked) CK(launch_build_deferred(A, pl.count_bits, st));  // what the tables could not take
     trace_mark("launch");
     CK(cudaEventRecord(ev[1], st));
     trace_mark("record");

@@ -72,13 +72,16 @@ __device__ __forceinline__ float step_reward(const DevProblem& P, float ac_speed
     return 0;
 }
 
-// Advection of move(), src/build_model.cu:284-289: the reference's expressions.
+// Advection of move(), src/build_model.cu:284-289: the reference's expressions
+// F*cos + vx and x + vnet*dt, whose products nvcc contracts there.  The fused
+// multiply-adds are written out: in a loop over samples F*cos is invariant, and
+// hoisted out of it the product would be rounded by itself.
 __device__ __forceinline__ void advect(const DevProblem& P, float F, float cs, float sn, float vx,
                                       float vy, float x, float y, float& xnew, float& ynew) {
-  float vnetx = F * cs + vx;
-  float vnety = F * sn + vy;
-  xnew = x + (vnetx * P.dt);
-  ynew = y + (vnety * P.dt);
+  const float vnetx = __fmaf_rn(F, cs, vx);
+  const float vnety = __fmaf_rn(F, sn, vy);
+  xnew = __fmaf_rn(vnetx, P.dt, x);
+  ynew = __fmaf_rn(vnety, P.dt, y);
 }
 
 // Snapping of move(), src/build_model.cu:313-335: nearest cell centre with

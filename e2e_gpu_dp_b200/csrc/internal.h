@@ -89,6 +89,9 @@ struct BuildPlan {
   int na = 0, rc = 128;
   int ybufs = 1;  // coefficient buffers of the builder's chunk loop (2 when occupancy allows)
   int64_t stage_cap = 0, pool_units = 0;
+  bool ranked = false;     // the builder by velocity ranks takes the problem
+  RankArgs rank{};         // its launch shape (pointers set by run_build)
+  std::vector<uint32_t> rank_words;
   bool keep_sums = false;  // keep per-row reward sums (e2e_build_opts.keep_reward_parts)
 };
 

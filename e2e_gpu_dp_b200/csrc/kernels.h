@@ -18,6 +18,7 @@ enum : int {
   CTR_POOL = 4,           // dense-histogram pool slots requested
   CTR_FLAGS = 5,          // error flags
   CTR_NEXT_TILE = 6,      // fused build+backup: the next tile to take
+  CTR_DEFERRED = 7,       // emission tiles the ranked builder left to the general one
   CTR_COUNT = 8
 };
 // FLAG_WAIT_TIMEOUT: a wait of the fused build+backup for the next layer's
@@ -27,7 +28,12 @@ enum : unsigned int { FLAG_POOL_EXHAUSTED = 1u, FLAG_WAIT_TIMEOUT = 2u };
 struct BuildArgs {
   DevProblem P;
   DevFields F;
-  int t0;               // first layer of this launch (blockIdx.y offset)
+  int t0, t1;           // layers of this launch: t0 + blockIdx.y (t1: end, for listed tiles)
+  int64_t etiles_per_layer;      // emission tiles (warps' groups of cells) per layer
+  // null, or the emission tiles left by the ranked builder: per layer their
+  // number and, from T * etiles_per_layer on, their indices in the layer
+  unsigned int* defer_count;
+  int32_t* defer_list;
   int tiles_per_layer;  // CTAs per layer = ceil(ncells / 32); emission tiles are warps
   int rc;               // realisations per warp-private velocity chunk
   int ybufs;            // chunk coefficient buffers in shared memory: 1, or 2 (one CTA barrier a chunk)
@@ -64,6 +70,36 @@ struct AssembleArgs {
   void* cnt;
 };
 
+// ---- builder by velocity ranks (builder_ranks.cu, rank_plan.h) -----------------
+struct RankArgs {
+  const uint32_t* plan;      // the plan's words (rank_plan.h)
+  int slots_log2;
+  uint32_t zone_mask;
+  double shift;              // the plan's shift
+  float sx, sy;              // ... and its fixed-point units per velocity
+  int groups[4];
+  float a_min[2], a_max[2];  // displacements of the actions in cells, x and y
+  const float* yt;           // per layer: coefficients mode-major, rows of nrp
+  const float* ystat;        // per layer and mode: mean, variance
+  const uint32_t* obits;     // per layer and grid row: a bit per cell, obstacle at T or T + 1
+  int owords;                // words of such a row
+  int nrp;                   // realisations padded to 128
+  int nblocks, nsub;         // 128-realisation blocks; subsets of a CTA's cells
+  int cells;                 // cells of a CTA
+  int pool_words;            // shared words for its rank tables
+  float stay_sum;            // r_outbound added once per realisation: an obstacle cell's reward sum
+  int count_bits;            // staged counts: 16 or 32 bits
+  int t0, t1;                // layers of the launch
+  int64_t etiles_per_layer;
+};
+int rank_padded_modes(int nm);
+// launch shape for nm modes and a plan; false when the kernel does not take it
+bool rank_shape(int nm, int slots_log2, int lanes_log2, int nrzns, RankArgs* K);
+// fills yt, ystat, obits of layers [K.t0, K.t1)
+cudaError_t launch_rank_prepare(const DevProblem& P, const DevFields& F, const RankArgs& K, cudaStream_t st);
+// builds layers [K.t0, K.t1); tiles it does not take go to A.defer_list
+cudaError_t launch_build_ranks(const BuildArgs& A, const RankArgs& K, cudaStream_t st);
+
 int build_lanes_log2(int na);
 size_t build_smem_bytes(int na, int nm, int rc, bool unit, int ybufs);
 // builder CTAs that fit one SM with this dynamic shared memory (the lowest of
@@ -71,6 +107,8 @@ size_t build_smem_bytes(int na, int nm, int rc, bool unit, int ybufs);
 // kernels' registers and static shared memory and the device's limits
 int build_ctas_per_sm(int na, size_t smem, bool unit);
 cudaError_t launch_build_tiles(const BuildArgs& A, int count_bits, int n_layers, cudaStream_t st);
+// the tiles of layers [A.t0, A.t1) that the ranked builder listed
+cudaError_t launch_build_deferred(const BuildArgs& A, int count_bits, cudaStream_t st);
 // The fused build+backup of every layer (uses A.V, A.pi, A.pool, A.counters,
 // A.layer_done; no staging): one cooperative launch whose CTAs take the tiles
 // of layers nt-2 down to 0 in order and back each row up as soon as layer t+1
