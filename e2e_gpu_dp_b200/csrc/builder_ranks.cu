@@ -20,12 +20,17 @@
 // the reference's exactly; rewards are folded from the counts as in
 // k_build_tiles.
 //
-// Measured on B200 (whole call): 200x200x120, 16 actions, 5000 realisations
-// 330.6 -> 75.8 ms; 300x300x40, 2000 realisations 102.2 -> 27.8 ms; 137x137x53,
-// 24 actions, 777 realisations 29.6 -> 9.2 ms; 50x50x30, 500 realisations from
-// host fields 2.56 -> 1.65 ms.
+// Measured on B200 (whole call, counting loops -> ranks): 200x200x120, 16
+// actions, 5000 realisations 330.6 -> 66.2 ms; 300x300x40, 2000 realisations
+// 102.3 -> 24.4 ms; 137x137x53, 24 actions, 777 realisations 29.7 -> 8.8 ms.
+// Of the 14.3 ms of 200x200x30 the counting takes 10.5 ms (shared-memory
+// wavefronts and issue slots both at about half of their peaks), staging 0.9,
+// the prefix sums 0.5, the rows 2.4.  Four CTAs of 4 warps an SM: one CTA's
+// staging and rows run beside the others' counting (two of 8 warps: 16.8 ms);
+// the table reads of a lane's four samples before their increments: 15.5 ->
+// 14.3 ms.
 //
-// A CTA (8 warps) takes a run of cells of one layer, 256 rows where the action
+// A CTA (4 warps) takes a run of cells of one layer, 128 rows where the action
 // count allows it.  A warp holds the coefficients of 128 realisations (4 a
 // lane) in registers and walks a subset of the cells, whose modes it reads as
 // broadcasts; the tables of the cells are shared by the CTA's warps (atomic
@@ -42,37 +47,56 @@ namespace e2e {
 
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 128;     // 4 CTAs an SM: one CTA's set-up and rows overlap the others' counting
 constexpr int kWarps = kThreads / 32;
 constexpr int kWin = 8;           // window side, as k_build_tiles
-constexpr int kListPool = 768;    // samples on the lists of a CTA's cells
+constexpr int kListPool = 384;    // samples on the lists of a CTA's cells
 constexpr int kObsR = 10;         // obstacle bitmap radius around a cell
 constexpr int kObsRows = 2 * kObsR + 1;
 constexpr int kMaxCells = 32;     // cells of a CTA
+constexpr int kMaxTiles = 4;      // emission tiles of a CTA, one a warp
 
-// A sampled cell's table.  state: 0 counted, 1 nothing to count (terminal or
-// obstacle cell, beyond the layer), 2 left to the general builder
+// A cell of the CTA and its table
 struct __align__(16) CellTab {
-  float bx, by;        // fixed-point offset of a velocity sum, x and y
-  int qax, qbx;        // the range's ends (bits): the zones of its first and last step
-  int qay, qby;
-  int lxo, lyo;        // word offset of slot 0 of the axis' lookup table
-  uint32_t mul, cst;   // counter index = rank_x + rank_y * stride + cst
-  int bax, bay;        // step index of the range's lower end, in table units
-  int orgx, orgy;      // step index of cell boundary b: b * G + off[action] - org
-  int nx, ny;          // ranks in the table
-  int stride, base;    // row stride and first word of the prefix sums (ny + 1 x nx + 1)
-  int kx, ky;          // table kinds
+  float bx, bx2, by, by2;  // fixed-point offset of a velocity sum, x and y, each twice
+  int qax, qbx, qay, qby;  // the ranges' ends (bits): the zones of their first and last step
+  uint32_t lx, ly;         // shared address of slot 0 of the axis' lookup table, less q's constant bits
+  uint32_t mul;            // counter index = rank_x + rank_y * stride + cst: 1 | stride << 8;
+  uint32_t cst;            //   mul is 0 while the cell is not counted
+  int bax, bay;            // step index of the range's lower end, in table units
+  int orgx, orgy;          // step index of cell boundary b: b * G + off[action] - org
+  int nx, ny;              // ranks in the table
+  int stride, base;        // row stride and first word of the prefix sums (ny + 1 x nx + 1)
+  int kx, ky;              // table kinds
   float u1, v1;
-  int state, pad;
+  int i1, j1;
+  int state;               // 0 counted, 1 nothing to count (terminal or obstacle cell, beyond the
+                           // layer), 2 left to the general builder
+  int pad;
 };
 
-// counts of one CTA's cells (see the file's head): 4 realisations of a lane
-// over the cells [c_lo, c_hi)
+// a word of the lookup tables, which nothing writes while samples are counted:
+// not volatile, so that the loads of several samples are in flight together
+__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
+  uint32_t v;
+  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+  return v;
+}
+
+__device__ __forceinline__ void reds_inc(uint32_t addr) {
+  asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(addr) : "memory");
+}
+
+// The counts of 4 realisations a lane (rows r0 .. r0 + 3 of the coefficients)
+// over the cells [c_lo, c_hi).  Sums: extract_velocity's (src/build_model.cu:
+// 389-401), for each realisation and component a chain of fused multiply-adds in
+// mode order.  A sample in a step's zone, or clamped into the zone at its
+// range's end (NaN and overflow too: their bits lie beyond an end), counts in the
+// pool's word 0 and goes to the cell's list.
 template <int NM, bool FULL>
 __device__ __forceinline__ void count_block(const RankArgs& K, const float* yt, int r0, int nrz, const float4* md,
-                                            const CellTab* cells, int c_lo, int c_hi, const uint32_t* lut,
-                                            uint32_t* pool, int* lcnt, float2* list, int lcap) {
+                                            const CellTab* cells, int c_lo, int c_hi, uint32_t pool, int* lcnt,
+                                            float2* list, int lcap) {
   float2 y01[NM], y23[NM];
 #pragma unroll
   for (int k = 0; k < NM; ++k) {
@@ -82,17 +106,24 @@ __device__ __forceinline__ void count_block(const RankArgs& K, const float* yt, 
   }
   const int sh = kRankFrac - K.slots_log2;
   const uint32_t zm = K.zone_mask;
+  const float2 fx = make_float2(K.sx, K.sx), fy = make_float2(K.sy, K.sy);
   for (int c = c_lo; c < c_hi; ++c) {
     const CellTab* ct = cells + c;
-    if (ct->state != 0) continue;
+    const uint4 h2 = *reinterpret_cast<const uint4*>(&ct->lx);
+    if (h2.z == 0u) continue;
     const float4 h0 = *reinterpret_cast<const float4*>(ct);
-    const int4 h1 = *reinterpret_cast<const int4*>(&ct->qay);
-    const uint2 h2 = *reinterpret_cast<const uint2*>(&ct->mul);
-    float2 sx01 = make_float2(0.f, 0.f), sx23 = sx01, sy01 = sx01, sy23 = sx01;
-    // extract_velocity's mode sums (src/build_model.cu:389-401), a chain of fused
-    // multiply-adds in mode order for each realisation and component
+    const int4 h1 = *reinterpret_cast<const int4*>(&ct->qax);
+    float2 sx01, sx23, sy01, sy23;
+    {
+      const float4 m = md[c * NM];
+      const float2 mu = make_float2(m.x, m.y), mv = make_float2(m.z, m.w);
+      sx01 = __fmul2_rn(mu, y01[0]);  // fma(m, y, 0) but for the sign of a zero, which no result depends on
+      sx23 = __fmul2_rn(mu, y23[0]);
+      sy01 = __fmul2_rn(mv, y01[0]);
+      sy23 = __fmul2_rn(mv, y23[0]);
+    }
 #pragma unroll
-    for (int k = 0; k < NM; ++k) {
+    for (int k = 1; k < NM; ++k) {
       const float4 m = md[c * NM + k];
       const float2 mu = make_float2(m.x, m.y), mv = make_float2(m.z, m.w);
       sx01 = __ffma2_rn(mu, y01[k], sx01);
@@ -100,25 +131,32 @@ __device__ __forceinline__ void count_block(const RankArgs& K, const float* yt, 
       sy01 = __ffma2_rn(mv, y01[k], sy01);
       sy23 = __ffma2_rn(mv, y23[k], sy23);
     }
-    const float2 fx = make_float2(K.sx, K.sx), fy = make_float2(K.sy, K.sy);
-    const float2 bx = make_float2(h0.x, h0.x), by = make_float2(h0.y, h0.y);
+    const float2 bx = make_float2(h0.x, h0.y), by = make_float2(h0.z, h0.w);
     const float2 qx01 = __ffma2_rn(sx01, fx, bx), qx23 = __ffma2_rn(sx23, fx, bx);
     const float2 qy01 = __ffma2_rn(sy01, fy, by), qy23 = __ffma2_rn(sy23, fy, by);
-    const int qax = __float_as_int(h0.z), qbx = __float_as_int(h0.w);
     const float qx[4] = {qx01.x, qx01.y, qx23.x, qx23.y}, qy[4] = {qy01.x, qy01.y, qy23.x, qy23.y};
+    uint32_t s[4], t[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      s[i] = (uint32_t)min(max(__float_as_int(qx[i]), h1.x), h1.y);
+      t[i] = (uint32_t)min(max(__float_as_int(qy[i]), h1.z), h1.w);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      s[i] += lds_u32(h2.x + ((s[i] >> sh) << 2));
+      t[i] += lds_u32(h2.y + ((t[i] >> sh) << 2));
+    }
     bool listed[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      // (a NaN or an overflow has bits beyond an end and is clamped to it)
-      const int x = min(max(__float_as_int(qx[i]), qax), qbx);
-      const int y = min(max(__float_as_int(qy[i]), h1.x), h1.y);
-      const uint32_t s = lut[(x >> sh) + h1.z] + (uint32_t)x;
-      const uint32_t t = lut[(y >> sh) + h1.w] + (uint32_t)y;
-      const bool amb = (s & zm) == 0u || (t & zm) == 0u;
-      const uint32_t at = __dp2a_lo(__byte_perm(s, t, 0x7632), h2.x, h2.y);
-      const bool in = FULL || r0 + i < nrz;
-      listed[i] = amb && in;
-      if (!amb && in) atomicAdd(pool + at, 1u);
+      uint32_t at = __dp2a_lo(__byte_perm(s[i], t[i], 0x7632), h2.z, h2.w);
+      listed[i] = (s[i] & zm) == 0u || (t[i] & zm) == 0u;
+      if (!FULL && r0 + i >= nrz) {
+        listed[i] = false;
+        at = 0u;
+      }
+      if (listed[i]) at = 0u;
+      reds_inc(pool + (at << 2));
     }
     if (listed[0] || listed[1] || listed[2] || listed[3]) {
       const float sx[4] = {sx01.x, sx01.y, sx23.x, sx23.y}, sy[4] = {sy01.x, sy01.y, sy23.x, sy23.y};
@@ -202,8 +240,7 @@ __device__ __forceinline__ void finish_tile(const BuildArgs& A, const RankArgs& 
   const CellTab& ct = S.cells[cl];
   const bool valid = cell < nc && a < P.na;
   uint16_t* const wcol = S.wcol + warp * 64 * 32 + lane;
-  const int i1 = valid ? (int)(cell / g) : 0;
-  const int j1 = valid ? (int)(cell - (int64_t)i1 * g) : 0;
+  const int i1 = valid ? ct.i1 : 0, j1 = valid ? ct.j1 : 0;
   const int aa = a < P.na ? a : 0;
   const float F = P.ac_speed[aa], cs = P.ac_cos[aa], sn = P.ac_sin[aa];
   const float x1 = P.xs[j1], y1 = P.ys[g - 1 - i1];
@@ -425,34 +462,39 @@ __device__ __forceinline__ void finish_tile(const BuildArgs& A, const RankArgs& 
 }
 
 // the range of one axis' table: a thread per (cell, axis)
-__device__ __forceinline__ void cell_axis(const RankArgs& K, const uint32_t* plan, CellTab& ct, const float4* md, int nm,
-                                          int axis, float mean_v, int idx, int g, const float* stat) {
+template <int NM>
+__device__ __forceinline__ void cell_axis(const RankArgs& K, const uint32_t* plan, CellTab& ct, const float4* md, int axis,
+                                          int g, const float* stat) {
+  const float mean_v = axis ? ct.v1 : ct.u1;
   float centre = mean_v, var = 0.f;
-  for (int k = 0; k < nm; ++k) {
+#pragma unroll
+  for (int k = 0; k < NM; ++k) {
     const float w = axis ? md[k].z : md[k].x;
-    centre = fmaf(w, __ldg(stat + 2 * k), centre);
-    var = fmaf(w * w, __ldg(stat + 2 * k + 1), var);
+    const float2 st = __ldg(reinterpret_cast<const float2*>(stat) + k);
+    centre = fmaf(w, st.x, centre);
+    var = fmaf(w * w, st.y, var);
   }
   RankRange r;
   if (!rank_range(plan, K.slots_log2, K.groups, axis, axis ? K.sy : K.sx, K.shift, K.a_min[axis], K.a_max[axis], mean_v,
-                  centre, var, idx, g, &r)) {
+                  centre, var, axis ? ct.i1 : ct.j1, g, &r)) {
     ct.state = 2;  // (both axes' threads write 2)
     return;
   }
+  const uint32_t lut = (uint32_t)__cvta_generic_to_shared(plan) + ((uint32_t)r.lut << 2);
   if (axis == 0) {
-    ct.bx = r.bias;
+    ct.bx = ct.bx2 = r.bias;
     ct.qax = r.qa;
     ct.qbx = r.qb;
-    ct.lxo = r.lut;
+    ct.lx = lut;
     ct.bax = r.first;
     ct.orgx = r.org;
     ct.nx = r.n;
     ct.kx = r.kind;
   } else {
-    ct.by = r.bias;
+    ct.by = ct.by2 = r.bias;
     ct.qay = r.qa;
     ct.qby = r.qb;
-    ct.lyo = r.lut;
+    ct.ly = lut;
     ct.bay = r.first;
     ct.orgy = r.org;
     ct.ny = r.n;
@@ -461,13 +503,13 @@ __device__ __forceinline__ void cell_axis(const RankArgs& K, const uint32_t* pla
 }
 
 template <int NM>
-__global__ void __launch_bounds__(kThreads, 2) k_build_ranks(BuildArgs A, RankArgs K) {
+__global__ void __launch_bounds__(kThreads, 4) k_build_ranks(BuildArgs A, RankArgs K) {
   extern __shared__ __align__(16) unsigned char smem[];
   const DevProblem& P = A.P;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = P.g, nrz = P.nrzns, CT = K.cells;
-  const int64_t nc = (int64_t)g * g;
-  const int lcap = kListPool / CT;
+  const int g = P.g, nrz = P.nrzns, ct_log2 = K.cells_log2, CT = 1 << ct_log2;
+  const int nc = g * g;  // (states fit 31 bits: validate_problem)
+  const int lcap = kListPool >> ct_log2;
   const int cpw_log2 = 5 - A.lanes_log2;
   const int ntiles = CT >> cpw_log2;
   Smem S;
@@ -488,14 +530,20 @@ __global__ void __launch_bounds__(kThreads, 2) k_build_ranks(BuildArgs A, RankAr
     S.wcol = reinterpret_cast<uint16_t*>(take(sizeof(uint16_t) * kWarps * 64 * 32));
     S.pool = reinterpret_cast<uint32_t*>(p);
   }
-  __shared__ int pool_used;
+  // the tiles in rounds whose tables fit the pool together (one round, but for
+  // cells with wide tables): a tile's round, and the words a round uses
+  __shared__ int tile_round[kMaxTiles], round_words[kMaxTiles], rounds;
   for (int i = tid; i < rank_plan_words(K.slots_log2); i += kThreads) S.lut[i] = __ldg(K.plan + i);
-  const int tasks_per_layer = (int)((nc + CT - 1) / CT);
-  const int64_t tasks = (int64_t)(K.t1 - K.t0) * tasks_per_layer;
+  const int tasks_per_layer = (nc + CT - 1) >> ct_log2;
   int tab_late = -1;
-  for (int64_t task = blockIdx.x; task < tasks; task += gridDim.x) {
-    const int T = K.t0 + (int)(task / tasks_per_layer);
-    const int64_t c0 = (task % tasks_per_layer) * CT;
+  int T = K.t0, chunk = (int)blockIdx.x;
+  for (;; chunk += (int)gridDim.x) {
+    while (chunk >= tasks_per_layer) {
+      chunk -= tasks_per_layer;
+      ++T;
+    }
+    if (T >= K.t1) break;
+    const int c0 = chunk << ct_log2;
     __syncthreads();  // the previous task's tables are consumed
     // ---- stage the cells -------------------------------------------------------
     const bool late = T > P.nt - 20;
@@ -519,8 +567,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_build_ranks(BuildArgs A, RankAr
         }
       }
     }
-    for (int e = tid; e < CT * NM; e += kThreads) {
-      const int k = e / CT, c = e - k * CT;
+    for (int e = tid; e < (NM << ct_log2); e += kThreads) {
+      const int k = e >> ct_log2, c = e & (CT - 1);
       float ui = 0.f, vi = 0.f;
       if (k < P.nm && c0 + c < nc) {
         ui = __ldg(A.F.ui + ((int64_t)T * P.nm + k) * nc + c0 + c);
@@ -528,14 +576,16 @@ __global__ void __launch_bounds__(kThreads, 2) k_build_ranks(BuildArgs A, RankAr
       }
       S.md[c * NM + k] = make_float4(ui, ui, vi, vi);
     }
+    const int i0 = c0 / g, j0 = c0 - i0 * g;
     for (int e = tid; e < CT * kObsRows; e += kThreads) {
       const int c = e / kObsRows, a = e - c * kObsRows - kObsR;
       uint32_t bits = 0;
       if (c0 + c < nc) {
-        const int i1 = (int)((c0 + c) / g), j1 = (int)(c0 + c - (int64_t)i1 * g), i = i1 + a;
+        int i = i0 + a, j = j0 + c;
+        for (; j >= g; j -= g) ++i;
         if (i >= 0 && i < g) {
           const uint32_t* row = K.obits + ((int64_t)T * g + i) * K.owords;
-          const int b = j1 - kObsR, w = b >> 5;
+          const int b = j - kObsR, w = b >> 5;
           const uint32_t lo = w >= 0 ? __ldg(row + w) : 0u, hi = w + 1 < K.owords ? __ldg(row + w + 1) : 0u;
           bits = __funnelshift_r(lo, hi, b & 31) & ((1u << kObsRows) - 1u);
           if (a == 0) bits &= ~(1u << kObsR);  // the cell itself does not count
@@ -544,28 +594,25 @@ __global__ void __launch_bounds__(kThreads, 2) k_build_ranks(BuildArgs A, RankAr
       S.orow[e] = bits;
     }
     if (tid < CT) {
-      const int64_t cell = c0 + tid;
       CellTab& ct = S.cells[tid];
-      ct.state = 1;
+      int state = 1, i = i0, j = j0 + tid;
+      for (; j >= g; j -= g) ++i;
+      ct.i1 = i;
+      ct.j1 = j;
+      ct.mul = 0u;
       S.lcnt[tid] = 0;
-      if (cell < nc) {
-        const int i1 = (int)(cell / g), j1 = (int)(cell - (int64_t)i1 * g);
-        ct.u1 = __ldg(A.F.u + (int64_t)T * nc + cell);
-        ct.v1 = __ldg(A.F.v + (int64_t)T * nc + cell);
-        if (!is_terminal(P, i1, j1) && __ldg(A.F.mask + (int64_t)T * nc + cell) != 1) ct.state = 0;
+      if (c0 + tid < nc) {
+        ct.u1 = __ldg(A.F.u + (int64_t)T * nc + c0 + tid);
+        ct.v1 = __ldg(A.F.v + (int64_t)T * nc + c0 + tid);
+        if (!is_terminal(P, i, j) && __ldg(A.F.mask + (int64_t)T * nc + c0 + tid) != 1) state = 0;
       }
+      ct.state = state;
     }
     __syncthreads();
     // ---- ranges and table space ----------------------------------------------
     if (tid < 2 * CT) {
-      const int c = tid >> 1, axis = tid & 1;
-      CellTab& ct = S.cells[c];
-      if (ct.state != 1) {
-        const int64_t cell = c0 + c;
-        const int i1 = (int)(cell / g), j1 = (int)(cell - (int64_t)i1 * g);
-        cell_axis(K, S.lut, ct, S.md + c * NM, NM, axis, axis ? ct.v1 : ct.u1, axis ? i1 : j1, g,
-                  K.ystat + (int64_t)T * 2 * NM);
-      }
+      CellTab& ct = S.cells[tid >> 1];
+      if (ct.state != 1) cell_axis<NM>(K, S.lut, ct, S.md + (tid >> 1) * NM, tid & 1, g, K.ystat + (int64_t)T * 2 * NM);
     }
     __syncthreads();
     if (warp == 0) {
@@ -576,84 +623,108 @@ __global__ void __launch_bounds__(kThreads, 2) k_build_ranks(BuildArgs A, RankAr
         if (state == 0) {
           stride = (ct->nx + 1) | 1;
           words = (ct->ny + 1) * stride;
-          if (stride > 255) {
-            state = 2;
-            words = 0;
-          }
+          if (stride > 255) state = 2;
         }
       }
-      int end = words;
+      int end = words;  // inclusive prefix sum over the cells
       for (int o = 1; o < 32; o <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, end, o);
         if (lane >= o) end += v;
       }
-      if (state == 0 && end > K.pool_words) state = 2;
       const unsigned out = __ballot_sync(0xffffffffu, state == 2);
-      // a cell beside one that is left to the general builder is not counted either
-      const unsigned mates = (cpw_log2 == 5 ? ~0u : ((1u << (1 << cpw_log2)) - 1u) << ((lane >> cpw_log2) << cpw_log2));
-      if (state == 0 && (out & mates)) state = 2;
-      if (lane < CT) {
-        ct->state = state;
-        if (state == 0) {
-          const int base = end - words;
-          ct->stride = stride;
-          ct->base = base;
-          ct->mul = ((uint32_t)stride << 8) | 1u;
-          ct->cst = (uint32_t)(base - ct->bax - ct->bay * stride);
+      const int first = lane & ~((1 << cpw_log2) - 1), last = first + (1 << cpw_log2) - 1;  // the tile's lanes
+      const unsigned mates = (cpw_log2 == 5 ? ~0u : (1u << (1 << cpw_log2)) - 1u) << first;
+      const int before = __shfl_sync(0xffffffffu, end - words, first);
+      const int need = __shfl_sync(0xffffffffu, end, last & 31) - before;
+      // a cell beside one that is left to the general builder is not counted
+      // either, nor is a tile larger than the pool (word 0 is the listed samples')
+      bool skip = (out & mates) != 0 || need > K.pool_words - 4;
+      int round = 0, used = 4, base = 0;
+      for (int t = 0; t < ntiles; ++t) {
+        const int n = __shfl_sync(0xffffffffu, need, t << cpw_log2);
+        const bool sk = __shfl_sync(0xffffffffu, skip, t << cpw_log2);
+        if (sk) {
+          if (lane == 0) tile_round[t] = 0;
+          continue;
+        }
+        if (used + n > K.pool_words) {
+          if (lane == 0) round_words[round] = used;
+          ++round;
+          used = 4;
+        }
+        if ((lane >> cpw_log2) == t) base = used + (end - words - before);
+        used += n;
+        if (lane == 0) tile_round[t] = round;
+      }
+      if (lane == 0) {
+        round_words[round] = used;
+        rounds = round + 1;
+      }
+      if (lane < CT && state != 1) {
+        ct->state = skip ? 2 : 0;
+        ct->stride = stride;
+        ct->base = base;
+        ct->cst = (uint32_t)(base - ct->bax - ct->bay * stride);
+      }
+    }
+    __syncthreads();
+    for (int round = 0; round < rounds; ++round) {
+      // ---- clear the tables ------------------------------------------------------
+      {
+        const int n4 = (round_words[round] + 3) >> 2;
+        for (int i = tid; i < n4; i += kThreads) reinterpret_cast<uint4*>(S.pool)[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (tid < CT) {
+          CellTab& ct = S.cells[tid];
+          ct.mul = ct.state == 0 && tile_round[tid >> cpw_log2] == round ? ((uint32_t)ct.stride << 8) | 1u : 0u;
         }
       }
-      const int used = min(__shfl_sync(0xffffffffu, end, 31), K.pool_words);
-      if (lane == 0) pool_used = used;
-    }
-    __syncthreads();
-    {
-      const int n4 = (pool_used + 3) >> 2;
-      for (int i = tid; i < n4; i += kThreads) reinterpret_cast<uint4*>(S.pool)[i] = make_uint4(0u, 0u, 0u, 0u);
-    }
-    __syncthreads();
-    // ---- count the realisations ------------------------------------------------
-    {
-      const float* yt = K.yt + (int64_t)T * NM * K.nrp;
-      const int per = CT / K.nsub;
-      for (int it = warp; it < K.nblocks * K.nsub; it += kWarps) {
-        const int blk = it / K.nsub, sub = it - blk * K.nsub;
-        const int r0 = blk * 128 + 4 * lane;
-        if (blk * 128 + 128 <= nrz)
-          count_block<NM, true>(K, yt, r0, nrz, S.md, S.cells, sub * per, (sub + 1) * per, S.lut, S.pool, S.lcnt, S.list,
-                                lcap);
-        else
-          count_block<NM, false>(K, yt, r0, nrz, S.md, S.cells, sub * per, (sub + 1) * per, S.lut, S.pool, S.lcnt, S.list,
-                                 lcap);
-      }
-    }
-    __syncthreads();
-    // ---- prefix sums of the tables: along x, then along y -------------------------
-    for (int c = warp; c < CT; c += kWarps) {
-      const CellTab& ct = S.cells[c];
-      if (ct.state != 0) continue;
-      uint32_t* t = S.pool + ct.base;
-      for (int y = 1 + lane; y <= ct.ny; y += 32) {
-        uint32_t* p = t + y * ct.stride + 1;
-        uint32_t run = 0;
-        for (int x = 0; x < ct.nx; ++x) {
-          run += p[x];
-          p[x] = run;
+      __syncthreads();
+      // ---- count the realisations ------------------------------------------------
+      {
+        const float* yt = K.yt + (int64_t)T * NM * K.nrp;
+        const uint32_t pool = (uint32_t)__cvta_generic_to_shared(S.pool);
+        const int per = CT >> K.nsub_log2;
+        for (int it = warp; it < (K.nblocks << K.nsub_log2); it += kWarps) {
+          const int blk = it >> K.nsub_log2, lo = (it & ((1 << K.nsub_log2) - 1)) * per;
+          const int r0 = blk * 128 + 4 * lane;
+          if (blk * 128 + 128 <= nrz)
+            count_block<NM, true>(K, yt, r0, nrz, S.md, S.cells, lo, lo + per, pool, S.lcnt, S.list, lcap);
+          else
+            count_block<NM, false>(K, yt, r0, nrz, S.md, S.cells, lo, lo + per, pool, S.lcnt, S.list, lcap);
         }
       }
-      __syncwarp();
-      for (int x = 1 + lane; x <= ct.nx; x += 32) {
-        uint32_t* p = t + ct.stride + x;
-        uint32_t run = 0;
-        for (int y = 0; y < ct.ny; ++y) {
-          run += *p;
-          *p = run;
-          p += ct.stride;
+      __syncthreads();
+      // ---- prefix sums of the tables: along x, then along y -------------------------
+      for (int c = warp; c < CT; c += kWarps) {
+        const CellTab& ct = S.cells[c];
+        if (ct.mul == 0u) continue;
+        uint32_t* t = S.pool + ct.base;
+        for (int y = 1 + lane; y <= ct.ny; y += 32) {
+          uint32_t* p = t + y * ct.stride + 1;
+          uint32_t run = 0;
+#pragma unroll 4
+          for (int x = 0; x < ct.nx; ++x) {
+            run += p[x];
+            p[x] = run;
+          }
+        }
+        __syncwarp();
+        for (int x = 1 + lane; x <= ct.nx; x += 32) {
+          uint32_t* p = t + ct.stride + x;
+          uint32_t run = 0;
+#pragma unroll 4
+          for (int y = 0; y < ct.ny; ++y) {
+            run += *p;
+            *p = run;
+            p += ct.stride;
+          }
         }
       }
+      __syncthreads();
+      // ---- the rows ------------------------------------------------------------------
+      if (warp < ntiles && tile_round[warp] == round) finish_tile(A, K, S, T, c0, warp, lcap);
+      if (round + 1 < rounds) __syncthreads();
     }
-    __syncthreads();
-    // ---- the rows ------------------------------------------------------------------
-    for (int tile = warp; tile < ntiles; tile += kWarps) finish_tile(A, K, S, T, c0, tile, lcap);
   }
 }
 
@@ -733,7 +804,7 @@ cudaError_t dispatch_nm(int nmp, F&& f) {
   return cudaErrorInvalidValue;
 }
 
-constexpr size_t kSmemPerCta = 112 * 1024;  // two CTAs an SM
+constexpr size_t kSmemPerCta = 55 * 1024;  // four CTAs an SM
 
 }  // namespace
 
@@ -743,8 +814,10 @@ bool rank_shape(int nm, int slots_log2, int lanes_log2, int nrzns, RankArgs* K) 
   if (nm > 10) return false;
   const int nmp = rank_padded_modes(nm);
   K->slots_log2 = slots_log2;
-  K->cells = std::min(kMaxCells, 256 >> lanes_log2);
-  const size_t fixed = smem_fixed_bytes(slots_log2, nmp, K->cells);
+  // kMaxTiles emission tiles of 32 / P cells (P action lanes)
+  K->cells_log2 = std::min(5, 7 - lanes_log2);
+  const int cells = 1 << K->cells_log2;
+  const size_t fixed = smem_fixed_bytes(slots_log2, nmp, cells);
   if (fixed + 16 * 1024 > kSmemPerCta) return false;
   K->pool_words = (int)((kSmemPerCta - fixed) / 4) & ~3;
   K->nrp = (nrzns + 127) / 128 * 128;
@@ -753,11 +826,11 @@ bool rank_shape(int nm, int slots_log2, int lanes_log2, int nrzns, RankArgs* K) 
   // Fewer subsets load the coefficients less often (about a cell's worth of
   // work), more of them spread few realisation blocks over the warps.
   double best = 1e30;
-  for (int ns = 2; ns <= 8; ns *= 2) {
-    const double cost = ((K->nblocks * ns + kWarps - 1) / kWarps) * (K->cells / ns + 1.0);
+  for (int l = 0; l <= 2; ++l) {
+    const double cost = (((K->nblocks << l) + kWarps - 1) / kWarps) * ((cells >> l) + 1.0);
     if (cost < best) {
       best = cost;
-      K->nsub = ns;
+      K->nsub_log2 = l;
     }
   }
   return true;
@@ -775,14 +848,14 @@ cudaError_t launch_rank_prepare(const DevProblem& P, const DevFields& F, const R
 
 cudaError_t launch_build_ranks(const BuildArgs& A, const RankArgs& K, cudaStream_t st) {
   const int nmp = rank_padded_modes(A.P.nm);
-  const size_t sm = smem_fixed_bytes(K.slots_log2, nmp, K.cells) + 4 * (size_t)K.pool_words;
+  const size_t sm = smem_fixed_bytes(K.slots_log2, nmp, 1 << K.cells_log2) + 4 * (size_t)K.pool_words;
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   const int64_t nc = (int64_t)A.P.g * A.P.g;
-  const int64_t tasks = (int64_t)(K.t1 - K.t0) * ((nc + K.cells - 1) / K.cells);
-  const unsigned grid = (unsigned)std::min<int64_t>(tasks, 2 * (int64_t)sms);
+  const int64_t tasks = (int64_t)(K.t1 - K.t0) * ((nc + (1 << K.cells_log2) - 1) >> K.cells_log2);
+  const unsigned grid = (unsigned)std::min<int64_t>(tasks, 4 * (int64_t)sms);
   if (grid == 0) return cudaSuccess;
   return dispatch_nm(nmp, [&](auto nm) -> cudaError_t {
     auto kern = k_build_ranks<decltype(nm)::value>;

@@ -84,8 +84,8 @@ struct RankArgs {
   const uint32_t* obits;     // per layer and grid row: a bit per cell, obstacle at T or T + 1
   int owords;                // words of such a row
   int nrp;                   // realisations padded to 128
-  int nblocks, nsub;         // 128-realisation blocks; subsets of a CTA's cells
-  int cells;                 // cells of a CTA
+  int nblocks, nsub_log2;    // 128-realisation blocks; subsets of a CTA's cells
+  int cells_log2;            // cells of a CTA
   int pool_words;            // shared words for its rank tables
   float stay_sum;            // r_outbound added once per realisation: an obstacle cell's reward sum
   int count_bits;            // staged counts: 16 or 32 bits

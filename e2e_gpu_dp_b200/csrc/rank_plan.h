@@ -95,9 +95,12 @@ E2E_RANK_FN bool rank_range(const uint32_t* plan, int slots_log2, const int* gro
       kl += (int)gq[k] <= fl ? 1 : 0;
       kh += (int)gq[k] <= fh ? 1 : 0;
     }
-    const int ba = (ql >> kRankFrac) * G + kl - 1;  // last step at or below the range,
-    const int bb = (qh >> kRankFrac) * G + kh;      // first one above it
-    const int qa = ((ba / G) << kRankFrac) + (int)gq[ba % G], qb = ((bb / G) << kRankFrac) + (int)gq[bb % G];
+    // the last step at or below the range and the first one above it
+    int ua = ql >> kRankFrac, ub = qh >> kRankFrac;
+    if (--kl < 0) kl = G - 1, --ua;
+    if (kh == G) kh = 0, ++ub;
+    const int ba = ua * G + kl, bb = ub * G + kh;
+    const int qa = (ua << kRankFrac) + (int)gq[kl], qb = (ub << kRankFrac) + (int)gq[kh];
     if (!(kind & 1)) {  // do samples in the range reach the domain's clamps?
       const float at = (float)(idx + n0) - (float)shift;
       if (!(at + a_min + (float)qa / unit > 0.01f && at + a_max + (float)qb / unit < (float)(g - 1) - 0.01f)) continue;
