@@ -12,7 +12,8 @@
 //    consecutive cells x P action lanes (P = next power of two >= actions),
 //    i.e. a contiguous range of model rows.  Which cell groups a CTA takes is
 //    chosen by group_of_slot (warps that reach the grid edge in CTAs of their
-//    own); the fused build+backup keeps 32 consecutive cells;
+//    own).  Problems that the ranked builder takes (builder_ranks.cu) come here
+//    only for the groups of cells it lists;
 //  * the velocity of every (cell, realisation) is computed once per chunk of
 //    realisations (u + sum_k ui_k*Y_k, reference order) into warp-private
 //    shared memory and reused by all actions (the reference recomputes it per
@@ -79,69 +80,6 @@ __host__ __device__ __forceinline__ int counter_log2_stride(int nthr) {
   return l;
 }
 
-// Backup of the lane's row (cell, action a) of layer T from its counters:
-// Q = R + (sum over entries in column order of fma(count, V[col], acc)) / nrzns
-// with R = sumR / nrzns, the arithmetic of the value-iteration sweeps
-// (solver_do_backup, src/spvi_2.cu:174-260) on the row the staging path would
-// emit; then the first maximum over the cell's action lanes (select_best_action,
-// src/spvi_2.cu:93-122: strict '>', NaN never taken, values at or below -1e6
-// give -1e6 / -1) and one write of V and the policy per cell.  Entries are
-// counted into CTR_STAGE (the model's nnz) per warp.
-__device__ __forceinline__ void fused_backup(const BuildArgs& A, int T, int64_t cell, bool valid, bool cvalid,
-                                             int a, int lane, int lanes_log2, int mode, float sumR,
-                                             const uint16_t* wcol, int log2S, int wi0, int wj0, int i1,
-                                             int j1, const uint32_t* dense) {
-  const DevProblem& P = A.P;
-  const int g = P.g;
-  const int64_t nc = (int64_t)g * g;
-  // the caller waited for the rows of layer T+1 that it reads (wait_rows)
-  const float* Vn = A.V + (int64_t)(T + 1) * nc;
-  float acc = 0.f;
-  int nnz = 0;
-  if (valid) {
-    if (mode == MODE_FIXED) {
-      acc = fmaf((float)P.nrzns, Vn[cell], acc);
-      nnz = 1;
-    } else if (mode == MODE_WINDOW) {
-      for (int wl = 0; wl < kWinBins; ++wl) {
-        const uint32_t c = wcol[wl << log2S] & kCountMask;
-        if (c) {
-          acc = fmaf((float)c, Vn[(int64_t)(wi0 + wl / kWin) * g + wj0 + wl % kWin], acc);
-          ++nnz;
-        }
-      }
-    } else if (mode == MODE_DENSE) {
-      for (int b = 0; b < P.m * P.m; ++b) {
-        const uint32_t c = dense[b];
-        if (c) {
-          acc = fmaf((float)c, Vn[(int64_t)(b / P.m + i1 - P.del) * g + b % P.m + j1 - P.del], acc);
-          ++nnz;
-        }
-      }
-    }
-  }
-  const float R = sumR / P.nrzns;  // compute_mean, src/build_model.cu:567
-  float q = R + acc / (float)P.nrzns;
-  if (!valid || mode == MODE_LOST || isnan(q)) q = -INFINITY;
-  int ba = a;
-  const int per = 1 << lanes_log2;
-  for (int o = per >> 1; o > 0; o >>= 1) {
-    const float oq = __shfl_xor_sync(0xffffffffu, q, o);
-    const int oa = __shfl_xor_sync(0xffffffffu, ba, o);
-    if (oq > q || (oq == q && oa < ba)) {
-      q = oq;
-      ba = oa;
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) nnz += __shfl_xor_sync(0xffffffffu, nnz, o);
-  if (lane == 0 && nnz) atomicAdd(A.counters + CTR_STAGE, (unsigned long long)nnz);
-  if (cvalid && a == 0) {
-    const bool ok = q > -1e6f;
-    A.V[(int64_t)T * nc + cell] = ok ? q : -1e6f;
-    A.pi[(int64_t)T * nc + cell] = ok ? ba : -1;
-  }
-}
-
 // K1.  Template: CntT = staged count type; UNIT = unit cell spacing.
 //
 // A CTA owns 32 cells of one layer and all their actions.  Warp w holds
@@ -165,10 +103,6 @@ __device__ __forceinline__ void fused_backup(const BuildArgs& A, int T, int64_t 
 // the full reference expression for it afterwards, so its reward joins the
 // row's sum after the chunk's in-window rewards.
 //
-// FUSED (k_build_fused, one cooperative launch over all layers): instead of
-// staging the rows, back them up at once against V of layer t+1 (the rows it
-// reads, waited for by wait_rows) and write V, policy of layer t; see
-// fused_backup.
 // Row stride (floats) of the staged coefficients: a lane reads 8-byte pairs
 // of row a + 16r, so an even stride with stride/2 odd (or an odd stride) keeps
 // the 16 rows of a warp's loads on distinct banks.
@@ -240,48 +174,8 @@ __device__ __forceinline__ void vel_pairs4(const float2* md, const float* y0, in
   }
 }
 
-// Fused build+backup: warp 0 waits until every cell of rows lo..hi of layer
-// `layer` is backed up (per (layer, grid row) completion counters, released
-// by the CTAs of those cells), then the CTA passes a barrier, so every
-// thread's later loads of those values are ordered after the writes.  The
-// wait is bounded: past A.wait_ns (or a poll limit) it sets FLAG_WAIT_TIMEOUT
-// and returns, and once the flag is set every later wait returns at once, so
-// the launch drains.  The last layer has no rows: its values are written
-// before the launch.
-__device__ __forceinline__ void wait_rows(const BuildArgs& A, int layer, int lo, int hi) {
-  if (threadIdx.x < 32 && layer <= A.P.nt - 2) {
-    const int lane = threadIdx.x;
-    const unsigned int target = (unsigned int)A.P.g + A.wait_extra;
-    const unsigned int* done = A.layer_done + (int64_t)layer * A.P.g;
-    unsigned int* flags = reinterpret_cast<unsigned int*>(A.counters + CTR_FLAGS);
-    unsigned long long t0;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-    long long it = 0;
-    for (;;) {
-      bool ok = true;
-      for (int r = lo + lane; r <= hi; r += 32) {
-        unsigned int v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(done + r) : "memory");
-        ok = ok && v >= target;
-      }
-      if (__all_sync(0xffffffffu, ok)) break;
-      unsigned int f;
-      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(flags) : "memory");
-      unsigned long long t;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      const bool give_up = (f & FLAG_WAIT_TIMEOUT) || ++it > (1ll << 26) || t - t0 > A.wait_ns;
-      if (__any_sync(0xffffffffu, give_up)) {
-        if (lane == 0) atomicOr(flags, FLAG_WAIT_TIMEOUT);
-        break;
-      }
-      __nanosleep(64);
-    }
-  }
-  __syncthreads();
-}
-
 // K1 on one tile (32 cells of layer T and all their actions) by one CTA.
-template <typename CntT, bool UNIT, bool FUSED>
+template <typename CntT, bool UNIT>
 __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* smem, const int T, const int tile,
                                            const int n_listed = -1) {
   const DevProblem& P = A.P;
@@ -296,12 +190,10 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
   const int cl = warp * (32 >> lanes_log2) + cw; // cell within tile (0..31)
   const int g = P.g;
   const int64_t nc = (int64_t)g * g;
-  const int64_t c0 = (int64_t)tile * 32;
-  // the cells of the tile's warps' groups (group_of_slot), local cell l at
-  // cell_tab[l]; the fused pass keeps the identity (its completion counts are
-  // per grid row of consecutive cells)
+  // the cells of the tile's warps' groups (group_of_slot, or the list), local
+  // cell l at cell_tab[l]
   __shared__ int cell_tab[32];
-  if (!FUSED) {
+  {
     if (tid < 32) {
       const int cpw_log2 = 5 - lanes_log2;
       const int slot = tile * nwarps + (tid >> cpw_log2);
@@ -312,7 +204,7 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
     }
     __syncthreads();
   }
-  auto cell_of = [&](int l) -> int64_t { return FUSED ? c0 + l : (int64_t)cell_tab[l]; };
+  auto cell_of = [&](int l) -> int64_t { return (int64_t)cell_tab[l]; };
   const int64_t cell = cell_of(cl);
   const bool valid = (cell < nc) && (a < P.na);
   const int nm = P.nm;
@@ -662,7 +554,7 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
   const bool two_bufs = A.ybufs == 2;
   const int yalt = two_bufs ? rc * ys : 0;  // offset of the other buffer, toggled by xor
   // velocity bounds of the chunk (plain warps of the unit-spacing staging kernel)
-  const bool track = UNIT && !FUSED && !clamp_warp && P.dt > 0.f;
+  const bool track = UNIT && !clamp_warp && P.dt > 0.f;
   int yoff = 0;
   stage_coeffs(ysm, ys, ylayer, min(rc, P.nrzns), nm, tid, nthr);
   for (int base = 0; base < P.nrzns; base += rc, yoff ^= yalt) {
@@ -855,11 +747,6 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
         if (clamp_warp) {
 #pragma unroll 8
           for (int q = 0; q < clen; ++q) count_sample_clamp(myvel[q]);
-        } else if constexpr (FUSED) {
-          // one realisation a load: the fused instance measured 444 ms with
-          // the pairs below and 419 ms without them (200x200x120)
-#pragma unroll 16
-          for (int q = 0; q < clen; ++q) count_sample(myvel[q]);
         } else if (in_win) {
           // every sample of the chunk is in the window (bounding box above): the
           // bin is the low six bits of (by << 3) + bx (the 0x4B400000 offsets
@@ -963,27 +850,6 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
   if (n_misbin) atomicAdd(A.counters + CTR_MISBIN, (unsigned long long)n_misbin);
   if (mode == MODE_LOST) atomicOr(reinterpret_cast<unsigned int*>(A.counters + CTR_FLAGS), FLAG_POOL_EXHAUSTED);
 
-  if (FUSED) {
-    // the backup reads layer T+1 within the rows' m x m neighbourhoods and
-    // 8 x 8 windows: rows of the tile's cells +- max(del, 7)
-    const int64_t c_last = min(c0 + 31, nc - 1);
-    const int r0 = (int)(c0 / g), r1 = (int)(c_last / g), reach = max(P.del, kWin - 1);
-    wait_rows(A, T + 1, max(r0 - reach, 0), min(r1 + reach, g - 1));
-    fused_backup(A, T, cell, valid, cvalid, a, lane, lanes_log2, mode, sumR, wcol, log2S, wi0, wj0, i1, j1,
-                 dense);
-    __syncthreads();  // every row of the tile is backed up
-    if (tid == 0) {
-      __threadfence();
-      for (int r = r0; r <= r1; ++r) {  // the tile's cells in each grid row it spans
-        const int64_t lo = max(c0, (int64_t)r * g), hi = min(c_last, (int64_t)(r + 1) * g - 1);
-        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(A.layer_done + (int64_t)T * g + r),
-                     "r"((unsigned int)(hi - lo + 1))
-                     : "memory");
-      }
-    }
-    return;
-  }
-
   // ---- per-warp emission: row lengths, warp scan, one atomicAdd -----------
   int nnz = 0;
   if (valid) {
@@ -1074,40 +940,9 @@ __global__ void __launch_bounds__(1024) k_build_tiles(BuildArgs A) {
       if (T >= A.t1) return;
       tile = (int)(item - before);
     }
-    build_tile<CntT, UNIT, false>(A, smem, T, tile, n);
+    build_tile<CntT, UNIT>(A, smem, T, tile, n);
     if (!listed) return;
     __syncthreads();  // the shared memory is free for the next tile
-  }
-}
-
-// Fused build+backup of all layers in one cooperative launch.  Tiles are
-// numbered g = 0, 1, ... with layer nt-2-g/tiles_per_layer, and a CTA that is
-// ready takes the next number from a counter (CTR_NEXT_TILE); a tile samples,
-// waits for the layer after its own (wait_rows), backs its rows up and counts
-// itself done.  Every tile of layer t+1 has a smaller number than every tile
-// of layer t and numbers are taken in increasing order by resident CTAs (a
-// cooperative launch), so by induction over g every awaited tile has been
-// taken and finishes: the waits end.  A tile waits only for the rows of layer
-// t+1 its backup reads (its cells' rows +- max(del, 7)), which were taken
-// about a layer's worth of tiles before it.  Sampling needs no values, so a
-// layer's sampling overlaps the completion of the layer after it, with no
-// launch boundary between layers.  (Fixed assignment, CTA b taking g = b, b + grid,
-// ..., let slow CTAs fall ever further behind and the others wait for them at
-// every layer: 400 ms on c2 against 367 ms with one launch per layer.)
-template <typename CntT, bool UNIT>
-__global__ void __launch_bounds__(1024) k_build_fused(BuildArgs A) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ long long taken;
-  const int64_t tpl = A.tiles_per_layer;
-  const int64_t total = (int64_t)(A.P.nt - 1) * tpl;
-  for (;;) {
-    if (threadIdx.x == 0) taken = (long long)atomicAdd(A.counters + CTR_NEXT_TILE, 1ull);
-    __syncthreads();
-    const int64_t g = taken;
-    if (g >= total) break;
-    const int L = (int)(g / tpl);
-    build_tile<CntT, UNIT, true>(A, smem, A.P.nt - 2 - L, (int)(g - (int64_t)L * tpl));
-    __syncthreads();  // the next tile reuses the shared memory (and `taken`)
   }
 }
 
@@ -1254,16 +1089,13 @@ int build_ctas_per_sm(int na, size_t smem, bool unit) {
     return none();
   const int nthr = 32 << build_lanes_log2(na);
   int best = thr_sm / nthr;
-  // the staging kernel with 16- and 32-bit counts, and the fused kernel
-  cudaFuncAttributes fa[3];
+  // the kernel with 16- and 32-bit counts
+  cudaFuncAttributes fa[2];
   cudaError_t e = unit ? cudaFuncGetAttributes(&fa[0], k_build_tiles<uint16_t, true>)
                        : cudaFuncGetAttributes(&fa[0], k_build_tiles<uint16_t, false>);
   if (e != cudaSuccess) return none();
   e = unit ? cudaFuncGetAttributes(&fa[1], k_build_tiles<uint32_t, true>)
            : cudaFuncGetAttributes(&fa[1], k_build_tiles<uint32_t, false>);
-  if (e != cudaSuccess) return none();
-  e = unit ? cudaFuncGetAttributes(&fa[2], k_build_fused<uint32_t, true>)
-           : cudaFuncGetAttributes(&fa[2], k_build_fused<uint32_t, false>);
   if (e != cudaSuccess) return none();
   for (const cudaFuncAttributes& f : fa) {
     const size_t per_cta = smem + f.sharedSizeBytes + (size_t)reserved;
@@ -1306,42 +1138,12 @@ static cudaError_t launch_one(const BuildArgs& A, int n_layers, cudaStream_t st)
   return cudaGetLastError();
 }
 
-template <bool UNIT>
-static cudaError_t launch_fused(const BuildArgs& A, cudaStream_t st, int* grid_out) {
-  auto kern = k_build_fused<uint32_t, UNIT>;
-  const int threads = 32 << A.lanes_log2;
-  const size_t sm = build_smem_bytes(A.P.na, A.P.nm, A.rc, UNIT, A.ybufs);
-  static std::mutex mu;
-  static int cap_set[64] = {};
-  cudaError_t e = raise_smem_cap(kern, sm, cap_set, mu);
-  if (e != cudaSuccess) return e;
-  int dev = 0, per_sm = 0, sms = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, sm)) != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  const int64_t total = (int64_t)(A.P.nt - 1) * A.tiles_per_layer;
-  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(total, (int64_t)per_sm * sms));
-  if (grid_out) *grid_out = (int)grid;
-  BuildArgs B = A;
-  void* args[] = {&B};
-  return cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3((unsigned)threads), args, sm, st);
-}
-
 cudaError_t launch_build_tiles(const BuildArgs& A, int count_bits, int n_layers,
                                cudaStream_t st) {
   const bool unit = A.P.unit_step != 0;
   if (count_bits == 16) return unit ? launch_one<uint16_t, true>(A, n_layers, st)
                                     : launch_one<uint16_t, false>(A, n_layers, st);
   return unit ? launch_one<uint32_t, true>(A, n_layers, st) : launch_one<uint32_t, false>(A, n_layers, st);
-}
-
-cudaError_t launch_build_deferred(const BuildArgs& A, int count_bits, cudaStream_t st) {
-  return launch_build_tiles(A, count_bits, A.t1 - A.t0, st);
-}
-
-cudaError_t launch_build_fused(const BuildArgs& A, cudaStream_t st, int* grid) {
-  return A.P.unit_step != 0 ? launch_fused<true>(A, st, grid) : launch_fused<false>(A, st, grid);
 }
 
 cudaError_t launch_scan_tiles(const int32_t* tile_len, int64_t n_tiles, int64_t* canon,

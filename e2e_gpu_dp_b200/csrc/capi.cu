@@ -817,6 +817,61 @@ e2e_status copy_field_steps(const FieldsOnDevice& fd, int t0, int t1, cudaStream
   return E2E_OK;
 }
 
+e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, cudaStream_t st, DeviceScratch* scratch,
+                               LayerBuild* L) {
+  if (!pl.ranked) return E2E_OK;
+  const size_t nmp = (size_t)rank_padded_modes(p->nmodes), layers = (size_t)(p->nt - 1);
+  RankArgs& K = L->K;
+  K = pl.rank;
+  auto take = [&](size_t bytes, void** q) -> cudaError_t {
+    cudaError_t e = dalloc(q, bytes, st);
+    if (e == cudaSuccess) scratch->add(*q);
+    return e;
+  };
+  void *plan, *yt, *ystat, *obits, *count, *list;
+  const size_t pb = sizeof(uint32_t) * pl.rank_words.size();
+  CK(take(pb, &plan));
+  CK(cudaMemcpyAsync(plan, pl.rank_words.data(), pb, cudaMemcpyHostToDevice, st));
+  CK(take(sizeof(float) * layers * nmp * (size_t)K.nrp, &yt));
+  CK(take(sizeof(float) * layers * nmp * 2, &ystat));
+  CK(take(sizeof(uint32_t) * layers * (size_t)p->gsize * (size_t)K.owords, &obits));
+  CK(take(sizeof(unsigned int) * layers, &count));
+  CK(take(sizeof(int32_t) * (size_t)pl.n_tiles, &list));
+  K.plan = static_cast<const uint32_t*>(plan);
+  K.yt = static_cast<const float*>(yt);
+  K.ystat = static_cast<const float*>(ystat);
+  K.obits = static_cast<const uint32_t*>(obits);
+  L->defer_count = static_cast<unsigned int*>(count);
+  L->defer_list = static_cast<int32_t*>(list);
+  return E2E_OK;
+}
+
+cudaError_t launch_layers(const BuildArgs& A, const BuildPlan& pl, const LayerBuild& L, int t0, int t1, cudaStream_t st) {
+  BuildArgs B = A;
+  B.t0 = t0;
+  B.t1 = t1;
+  if (!pl.ranked) return launch_build_tiles(B, pl.count_bits, t1 - t0, st);
+  B.defer_count = L.defer_count;
+  B.defer_list = L.defer_list;
+  RankArgs R = L.K;
+  R.t0 = t0;
+  R.t1 = t1;
+  cudaError_t e = cudaMemsetAsync(L.defer_count + t0, 0, sizeof(unsigned int) * (size_t)(t1 - t0), st);
+  if (e == cudaSuccess) e = launch_rank_prepare(A.P, A.F, R, st);
+  return e != cudaSuccess ? e : launch_build_ranks(B, R, st);
+}
+
+cudaError_t launch_leftover(const BuildArgs& A, const BuildPlan& pl, const LayerBuild& L, int t0, int t1,
+                            cudaStream_t st) {
+  if (!pl.ranked) return cudaSuccess;
+  BuildArgs B = A;
+  B.t0 = t0;
+  B.t1 = t1;
+  B.defer_count = L.defer_count;
+  B.defer_list = L.defer_list;
+  return launch_build_tiles(B, pl.count_bits, t1 - t0, st);
+}
+
 e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const BuildPlan& pl,
                      cudaStream_t st, DeviceScratch* scratch, e2e_model* m) {
   const DevFields& F = fd.F;
@@ -844,33 +899,9 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
   CK(dalloc((void**)&ctr, sizeof(unsigned long long) * CTR_COUNT, st));
   scratch->add(ctr);
 
-  // the ranked builder's inputs, filled on the device per range of layers
-  RankArgs K = pl.rank;
-  unsigned int* defer_count = nullptr;
-  int32_t* defer_list = nullptr;
-  if (pl.ranked) {
-    const size_t nmp = (size_t)rank_padded_modes(p->nmodes), layers = (size_t)(p->nt - 1);
-    uint32_t *plan = nullptr, *obits = nullptr;
-    float *yt = nullptr, *ystat = nullptr;
-    const size_t pb = sizeof(uint32_t) * pl.rank_words.size();
-    CK(dalloc((void**)&plan, pb, st));
-    scratch->add(plan);
-    CK(cudaMemcpyAsync(plan, pl.rank_words.data(), pb, cudaMemcpyHostToDevice, st));
-    CK(dalloc((void**)&yt, sizeof(float) * layers * nmp * (size_t)K.nrp, st));
-    scratch->add(yt);
-    CK(dalloc((void**)&ystat, sizeof(float) * layers * nmp * 2, st));
-    scratch->add(ystat);
-    CK(dalloc((void**)&obits, sizeof(uint32_t) * layers * (size_t)p->gsize * (size_t)K.owords, st));
-    scratch->add(obits);
-    CK(dalloc((void**)&defer_count, sizeof(unsigned int) * layers, st));
-    scratch->add(defer_count);
-    CK(dalloc((void**)&defer_list, sizeof(int32_t) * (size_t)pl.n_tiles, st));
-    scratch->add(defer_list);
-    K.plan = plan;
-    K.yt = yt;
-    K.ystat = ystat;
-    K.obits = obits;
-  }
+  LayerBuild L;
+  s = layer_build_buffers(p, pl, st, scratch, &L);
+  if (s != E2E_OK) return s;
 
   int64_t cap = pl.stage_cap, pool_units = pl.pool_units;
   int32_t* stage_col = nullptr;
@@ -914,23 +945,9 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
     A.sumR = m->sumR;
     A.pool = pool;
     A.pool_units = pool_units;
-    if (pl.ranked) {
-      CK(cudaMemsetAsync(defer_count, 0, sizeof(unsigned int) * (size_t)(p->nt - 1), st));
-      A.defer_count = defer_count;
-      A.defer_list = defer_list;
-    }
-    // layers [t0, t1)
     auto build_layers = [&](int t0, int t1) -> cudaError_t {
       m->build_launches++;
-      BuildArgs B = A;
-      B.t0 = t0;
-      B.t1 = t1;
-      if (!pl.ranked) return launch_build_tiles(B, pl.count_bits, t1 - t0, st);
-      RankArgs R = K;
-      R.t0 = t0;
-      R.t1 = t1;
-      cudaError_t e = launch_rank_prepare(D, F, R, st);
-      return e != cudaSuccess ? e : launch_build_ranks(B, R, st);
+      return launch_layers(A, pl, L, t0, t1, st);
     };
     CK(cudaEventRecord(ev[0], st));
     trace_mark("buffers");
@@ -973,7 +990,7 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
     } else {
       CK(build_layers(0, p->nt - 1));
     }
-    if (pl.ranked) CK(launch_build_deferred(A, pl.count_bits, st));  // what the tables could not take
+    CK(launch_leftover(A, pl, L, 0, p->nt - 1, st));
     trace_mark("launch");
     CK(cudaEventRecord(ev[1], st));
     trace_mark("record");
@@ -1176,6 +1193,44 @@ e2e_status ensure_pack(const e2e_model* m, double* pack_ms, cudaStream_t st) {
   return E2E_OK;
 }
 
+// bytes of one sweep in CSR form: row_ptr, col, count, R, V read, V' and policy written
+static int64_t csr_sweep_bytes(const e2e_model* m) {
+  const int64_t pbytes = m->index_bits == 32 ? 4 : 8;
+  const int64_t cbytes = m->count_type == E2E_COUNT_U16 ? 2 : 4;
+  return (m->n_rows + 1) * pbytes + m->nnz * (4 + cbytes) + m->ns * m->na * 4 + m->ns * 12;
+}
+
+// FP64 backward solve on the device against the FP32 values (opts.fp64_check)
+static e2e_status fp64_check(const e2e_model* m, const float* dV, e2e_vi_stats* stats, DeviceScratch* scratch,
+                             cudaStream_t st) {
+  if (!m->layered) return fail(E2E_ERR_UNSUPPORTED, "fp64 check needs a time-layered model");
+  const ViModel M = vi_model(m);
+  const int64_t ns = m->ns;
+  double* Vd = nullptr;
+  unsigned long long* err = nullptr;
+  CK(dalloc((void**)&Vd, sizeof(double) * (size_t)ns, st));
+  scratch->add(Vd);
+  CK(dalloc((void**)&err, sizeof(unsigned long long) * 2, st));
+  scratch->add(err);
+  CK(cudaMemsetAsync(err, 0, sizeof(unsigned long long) * 2, st));
+  const int64_t nc = m->ncells;
+  CK(launch_vi_sweep_f64(M, m->n_row_states, ns, Vd, st));
+  for (int64_t t = (m->n_row_states / nc) - 1; t >= 0; --t)
+    CK(launch_vi_sweep_f64(M, t * nc, (t + 1) * nc, Vd, st));
+  CK(launch_compare_f64(dV, Vd, ns, err, st));
+  unsigned long long h[2];
+  CK(cudaMemcpyAsync(h, err, sizeof(h), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  double ea, er;
+  std::memcpy(&ea, &h[0], 8);
+  std::memcpy(&er, &h[1], 8);
+  if (stats) {
+    stats->fp64_max_abs_err = ea;
+    stats->fp64_max_rel_err = er > 0 ? ea / er : ea;
+  }
+  return E2E_OK;
+}
+
 e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, int32_t* dpi,
                            e2e_vi_stats* stats, cudaStream_t st) {
   const int64_t ns = m->ns;
@@ -1218,9 +1273,7 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
   int iters = 0;
   double last_res = 0.0;
   bool layered_pass = false;
-  const int64_t pbytes = m->index_bits == 32 ? 4 : 8;
-  const int64_t cbytes = m->count_type == E2E_COUNT_U16 ? 2 : 4;
-  int64_t sweep_bytes = (m->n_rows + 1) * pbytes + m->nnz * (4 + cbytes) + ns * m->na * 4 + ns * 12;
+  const int64_t sweep_bytes = csr_sweep_bytes(m);
   CK(cudaEventRecord(e0, st));
   if (o.method == 1) {
     if (!m->layered || m->ncells <= 0 || m->nt <= 0 || P.nlayers < 2)
@@ -1296,32 +1349,7 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
     stats->fp64_max_abs_err = 0;
     stats->fp64_max_rel_err = 0;
   }
-  if (o.fp64_check) {
-    if (!m->layered) return fail(E2E_ERR_UNSUPPORTED, "fp64 check needs a time-layered model");
-    const ViModel M = vi_model(m);
-    double* Vd = nullptr;
-    unsigned long long* err = nullptr;
-    CK(dalloc((void**)&Vd, sizeof(double) * (size_t)ns, st));
-    scratch.add(Vd);
-    CK(dalloc((void**)&err, sizeof(unsigned long long) * 2, st));
-    scratch.add(err);
-    CK(cudaMemsetAsync(err, 0, sizeof(unsigned long long) * 2, st));
-    const int64_t nc = m->ncells;
-    CK(launch_vi_sweep_f64(M, m->n_row_states, ns, Vd, st));
-    for (int64_t t = (m->n_row_states / nc) - 1; t >= 0; --t)
-      CK(launch_vi_sweep_f64(M, t * nc, (t + 1) * nc, Vd, st));
-    CK(launch_compare_f64(dV, Vd, ns, err, st));
-    unsigned long long h[2];
-    CK(cudaMemcpyAsync(h, err, sizeof(h), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    double ea, er;
-    std::memcpy(&ea, &h[0], 8);
-    std::memcpy(&er, &h[1], 8);
-    if (stats) {
-      stats->fp64_max_abs_err = ea;
-      stats->fp64_max_rel_err = er > 0 ? ea / er : ea;
-    }
-  }
+  if (o.fp64_check) return fp64_check(m, dV, stats, &scratch, st);
   return E2E_OK;
 }
 

@@ -5,18 +5,18 @@
 // (src/spvi_2.cu:650-726).  Transitions only go from layer t to t+1
 // (src/build_model.cu:635) and the last layer has no rows (:1173-1176), so the
 // values of layer t are final as soon as layer t+1's are: the layered schedule
-// reaches the Jacobi fixed point in one pass.  Here each layer's rows are built
-// by K1 and backed up in its epilogue from the counters still in shared memory
-// (launch_build_fused): one cooperative launch whose CTAs take the tiles of
-// layers nt-2 down to 0 in order, each tile waiting (bounded) before its
-// backup only for the rows of the layer after its own that the backup reads,
-// so a layer's sampling overlaps the completion of the next one.
+// reaches the Jacobi fixed point in one pass.  Here the builder runs over a few
+// layers at a time, from the last, into a staging area of bounded size, and
+// k_backup_layers backs the rows up from there, layer by layer.  (The pass
+// before this one backed rows up in the builder's epilogue, each tile waiting
+// for the rows of the layer after its own; that tied it to the counting
+// builder: 100x100x60, 1000 realisations 13.0 ms, now 4.1 ms.)
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cstdlib>
 
 #include "e2e_dp.h"
+#include "grid_sync.cuh"
 #include "internal.h"
 #include "kernels.h"
 
@@ -27,6 +27,84 @@ using namespace e2e;
     cudaError_t _e = (call);                            \
     if (_e != cudaSuccess) return cuda_fail(_e, #call); \
   } while (0)
+
+namespace {
+
+constexpr int kThreads = 256;
+constexpr size_t kStageBudget = size_t(256) << 20;  // bytes of a block of layers' staging
+
+struct BackupArgs {
+  int t0, t1, na, lanes_log2, cells_log2, nrzns;  // 1 << cells_log2 cells per emission tile
+  int nc;
+  int64_t etiles_per_layer;
+  const uint32_t* row_off;  // these four and stage_* hold layers [t0, t1): index from layer t0
+  const int64_t* tile_base;
+  const int32_t* tile_len;
+  const float* R;
+  const int32_t* stage_col;
+  const uint16_t* stage_cnt;
+  float* V;
+  int32_t* pi;
+  unsigned int* sync;
+  WaitBound wb;
+};
+
+// Backups of the staged rows of layers t1-1 down to t0, one cooperative launch:
+// P lanes a cell (P = next power of two >= actions).  Q = R + (sum over the
+// row's entries in column order of fma(count, V[next], acc)) / nrzns, the
+// arithmetic of the sweeps over a stored model (solver_do_backup,
+// src/spvi_2.cu:174-260); the first maximum over the cell's lanes
+// (select_best_action, :93-122: strict '>', NaN never taken, values at or below
+// -1e6 give -1e6 / -1).  Bound by the grid barrier between the layers (a layer's
+// rows are some MB): its waits are bounded as the sweeps' are.
+__global__ void __launch_bounds__(kThreads) k_backup_layers(BackupArgs A) {
+  const int64_t n = (int64_t)A.nc << A.lanes_log2, stride = (int64_t)gridDim.x * kThreads;
+  const int a = threadIdx.x & ((1 << A.lanes_log2) - 1);
+  unsigned int gen = 0;
+  for (int t = A.t1 - 1; t >= A.t0; --t) {
+    const float* Vn = A.V;  // written by other CTAs of this launch: plain loads, ordered by the barrier
+    const int64_t layer = t - A.t0;
+    for (int64_t k0 = (int64_t)blockIdx.x * kThreads; k0 < n; k0 += stride) {  // whole warps
+      const int64_t k = k0 + threadIdx.x;
+      const int cell = (int)(k >> A.lanes_log2);
+      const bool valid = k < n && a < A.na;
+      float q = -INFINITY;
+      if (valid) {
+        const int64_t row = (layer * A.nc + cell) * A.na + a;
+        const int64_t tile = layer * A.etiles_per_layer + (cell >> A.cells_log2);
+        const uint32_t off = A.row_off[row];
+        // the tile's last row ends with the tile
+        const bool last = a == A.na - 1 && (((cell + 1) & ((1 << A.cells_log2) - 1)) == 0 || cell + 1 == A.nc);
+        const uint32_t end = last ? (uint32_t)A.tile_len[tile] : A.row_off[row + 1];
+        const int64_t base = A.tile_base[tile];
+        float acc = 0.f;
+        for (int64_t e = base + off; e < base + end; ++e) acc = fmaf((float)A.stage_cnt[e], Vn[A.stage_col[e]], acc);
+        q = finish_row(A.R[row], acc, 0.f, A.nrzns, true);
+        if (isnan(q)) q = -INFINITY;
+      }
+      int ba = a;
+      for (int o = (1 << A.lanes_log2) >> 1; o > 0; o >>= 1) {
+        const float oq = __shfl_xor_sync(0xffffffffu, q, o);
+        const int oa = __shfl_xor_sync(0xffffffffu, ba, o);
+        if (oq > q || (oq == q && oa < ba)) {
+          q = oq;
+          ba = oa;
+        }
+      }
+      if (valid && a == 0) {
+        const bool ok = q > -1e6f;
+        A.V[(int64_t)t * A.nc + cell] = ok ? q : -1e6f;
+        A.pi[(int64_t)t * A.nc + cell] = ok ? ba : -1;
+      }
+    }
+    if (t > A.t0) {
+      ++gen;
+      if (!grid_barrier(A.sync, gen * gridDim.x, A.wb)) return;
+    }
+  }
+}
+
+}  // namespace
 
 extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f, int where,
                                       int32_t* policy_out, float* value_out, int out_where,
@@ -40,7 +118,7 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
   cudaStream_t st = (cudaStream_t)stream;
 
   BuildPlan pl;
-  e2e_status s = plan_build(p, 32, 0, &pl);
+  e2e_status s = plan_build(p, 16, 0, &pl);
   if (s != E2E_OK) return s;
   DeviceScratch scratch(st);
   FieldsOnDevice fd;
@@ -48,6 +126,9 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
   if (s != E2E_OK) return s;
   DevProblem D;
   s = make_dev_problem(p, st, &D, &scratch);
+  if (s != E2E_OK) return s;
+  LayerBuild L;
+  s = layer_build_buffers(p, pl, st, &scratch, &L);
   if (s != E2E_OK) return s;
 
   const int64_t ns = pl.ns, nc = pl.ncells;
@@ -71,91 +152,164 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
   CK(cudaMemsetAsync(dV + last, 0, sizeof(float) * (size_t)nc, st));
   CK(cudaMemsetAsync(dpi + last, 0, sizeof(int32_t) * (size_t)nc, st));
 
+  // blocks of layers, of about equal size within the staging budget
+  const int layers = p->nt - 1;
+  const int64_t rows = nc * pl.na;
+  const size_t per_layer = (size_t)rows * (sizeof(uint32_t) + sizeof(float) + 4 * 6);
+  const int most = (int)std::max<size_t>(1, std::min<size_t>((size_t)layers, kStageBudget / per_layer));
+  const int nblocks = (layers + most - 1) / most, bl = (layers + nblocks - 1) / nblocks;
+  uint32_t* row_off = nullptr;
+  int64_t* tile_base = nullptr;
+  int32_t* tile_len = nullptr;
+  float* R = nullptr;
+  CK(dalloc((void**)&row_off, sizeof(uint32_t) * (size_t)rows * bl, st));
+  scratch.add(row_off);
+  CK(dalloc((void**)&R, sizeof(float) * (size_t)rows * bl, st));
+  scratch.add(R);
+  CK(dalloc((void**)&tile_base, sizeof(int64_t) * (size_t)pl.etiles_per_layer * bl, st));
+  scratch.add(tile_base);
+  CK(dalloc((void**)&tile_len, sizeof(int32_t) * (size_t)pl.etiles_per_layer * bl, st));
+  scratch.add(tile_len);
+  // per block: the builder's counters, then the barrier words of its backup
   unsigned long long* ctr = nullptr;
-  CK(dalloc((void**)&ctr, sizeof(unsigned long long) * CTR_COUNT, st));
+  const size_t ctr_words = CTR_COUNT + 1;
+  CK(dalloc((void**)&ctr, sizeof(unsigned long long) * ctr_words * nblocks, st));
   scratch.add(ctr);
-  unsigned int* done = nullptr;  // per (layer, grid row): cells backed up
-  const size_t n_done = (size_t)p->nt * (size_t)p->gsize;
-  CK(dalloc((void**)&done, sizeof(unsigned int) * n_done, st));
-  scratch.add(done);
-  // bound of one wait for a layer's completion: E2E_WAIT_LIMIT_MS (default
-  // 5000); E2E_TEST_UNREACHABLE_WAIT=1 raises the targets so that none
-  // completes (tests of the bounded waits only)
-  unsigned long long wait_ns = 5000000000ull;
-  if (const char* ms = std::getenv("E2E_WAIT_LIMIT_MS")) {
-    const double v = std::atof(ms);
-    if (v > 0 && v <= 60000) wait_ns = (unsigned long long)(v * 1e6);
-  }
-  const char* unreachable = std::getenv("E2E_TEST_UNREACHABLE_WAIT");
-  const unsigned int wait_extra = (unreachable && unreachable[0] == '1') ? 1u : 0u;
+  CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * ctr_words * nblocks, st));
   const int mm = p->neighb_gsize * p->neighb_gsize;
-  int64_t pool_units = pl.pool_units;
-  uint32_t* pool = nullptr;
-  unsigned long long hc[CTR_COUNT];
+  int64_t pool_units = pl.pool_units, cap = rows * bl * 4 + 4096;
+  struct Growing {  // buffers that a re-run may replace
+    cudaStream_t st;
+    void *pool = nullptr, *col = nullptr, *cnt = nullptr;
+    ~Growing() {
+      dfree(pool, st);
+      dfree(col, st);
+      dfree(cnt, st);
+    }
+  } buf{st};
+  auto take = [&](void** q, size_t bytes) { return *q ? cudaSuccess : dalloc(q, bytes, st); };
+
+  int dev = 0, sms = 0, per_sm = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backup_layers, kThreads, 0));
+  if (per_sm < 1) return fail(E2E_ERR_DEVICE, "the backup kernel does not fit the device");
+
   cudaEvent_t ev[2];
   for (int k = 0; k < 2; ++k) CK(cudaEventCreate(&ev[k]));
   struct EvFree {
     cudaEvent_t* e;
     ~EvFree() { for (int k = 0; k < 2; ++k) cudaEventDestroy(e[k]); }
   } evfree{ev};
+  CK(cudaEventRecord(ev[0], st));
   int launches = 0;
-  for (int attempt = 0; attempt < 3; ++attempt) {
-    if (!pool) CK(dalloc((void**)&pool, sizeof(uint32_t) * (size_t)mm * (size_t)pool_units, st));
-    CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * CTR_COUNT, st));
-    CK(cudaMemsetAsync(done, 0, sizeof(unsigned int) * n_done, st));
-    BuildArgs A{};
-    A.P = D;
-    A.F = fd.F;
-    A.tiles_per_layer = (int)pl.tiles_per_layer;
-    A.rc = pl.rc;
-    A.ybufs = pl.ybufs;
-    A.lanes_log2 = build_lanes_log2(pl.na);
-    A.counters = ctr;
-    A.pool = pool;
-    A.pool_units = pool_units;
-    A.V = dV;
-    A.pi = dpi;
-    A.layer_done = done;
-    A.wait_ns = wait_ns;
-    A.wait_extra = wait_extra;
-    CK(cudaEventRecord(ev[0], st));
-    if (p->nt > 1) {
-      int grid = 0;
-      CK(launch_build_fused(A, st, &grid));
+  unsigned long long sum[CTR_COUNT] = {}, *bc = ctr;
+  for (int b = 0, t1 = layers; t1 > 0; ++b, t1 = std::max(0, t1 - bl)) {
+    const int t0 = std::max(0, t1 - bl);
+    bc = ctr + ctr_words * b;
+    unsigned long long hc[CTR_COUNT + 1];
+    for (int attempt = 0;; ++attempt) {
+      CK(take(&buf.col, sizeof(int32_t) * (size_t)cap));
+      CK(take(&buf.cnt, sizeof(uint16_t) * (size_t)cap));
+      CK(take(&buf.pool, sizeof(uint32_t) * (size_t)mm * (size_t)pool_units));
+      if (attempt) CK(cudaMemsetAsync(bc, 0, sizeof(unsigned long long) * CTR_COUNT, st));
+      BuildArgs A{};
+      A.P = D;
+      A.F = fd.F;
+      A.t0 = t0;
+      A.t1 = t1;
+      A.etiles_per_layer = pl.etiles_per_layer;
+      A.tiles_per_layer = (int)pl.tiles_per_layer;
+      A.rc = pl.rc;
+      A.ybufs = pl.ybufs;
+      A.lanes_log2 = build_lanes_log2(pl.na);
+      A.counters = bc;
+      A.pool = static_cast<uint32_t*>(buf.pool);
+      A.pool_units = pool_units;
+      A.stage_col = static_cast<int32_t*>(buf.col);
+      A.stage_cnt = buf.cnt;
+      A.stage_cap = cap;
+      // the builder indexes by layer: the block's first one at the buffers' start
+      A.row_off = row_off - rows * t0;
+      A.R = R - rows * t0;
+      A.tile_base = tile_base - pl.etiles_per_layer * t0;
+      A.tile_len = tile_len - pl.etiles_per_layer * t0;
+      CK(launch_layers(A, pl, L, t0, t1, st));
+      CK(launch_leftover(A, pl, L, t0, t1, st));
       ++launches;
+      // sleep through the block, then read its counters and the error word of the
+      // backup before it
+      CK(sleep_sync(st));
+      CK(cudaMemcpyAsync(hc, b ? bc - 1 : bc, sizeof(unsigned long long) * (CTR_COUNT + (b ? 1 : 0)),
+                         cudaMemcpyDeviceToHost, st));
+      CK(cudaStreamSynchronize(st));
+      if (b) {
+        if (hc[0] >> 32) return fail(E2E_ERR_DEVICE, "build+solve: a wait for a layer's completion ran out of its bound");
+        std::copy(hc + 1, hc + 1 + CTR_COUNT, hc);
+      }
+      bool again = false;
+      if (hc[CTR_FLAGS] & FLAG_POOL_EXHAUSTED) {
+        dfree(buf.pool, st);
+        buf.pool = nullptr;
+        pool_units = (int64_t)hc[CTR_POOL];
+        if ((double)pool_units * mm * 4 > 32.0 * (1ull << 30))
+          return fail(E2E_ERR_UNSUPPORTED, "transition spread too wide: dense-histogram pool above 32 GiB");
+        again = true;
+      }
+      if ((int64_t)hc[CTR_STAGE] > cap) {
+        dfree(buf.col, st);
+        dfree(buf.cnt, st);
+        buf.col = buf.cnt = nullptr;
+        cap = (int64_t)hc[CTR_STAGE] + (int64_t)hc[CTR_STAGE] / 8;  // (later blocks differ a little)
+        again = true;
+      }
+      if (!again) break;
+      if (attempt == 2) return fail(E2E_ERR_DEVICE, "build did not settle after re-runs");
     }
-    CK(cudaEventRecord(ev[1], st));
-    // sleep through the pass, then read its counters
-    CK(sleep_sync(st));
-    CK(cudaMemcpyAsync(hc, ctr, sizeof(hc), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    if (hc[CTR_FLAGS] & FLAG_WAIT_TIMEOUT)
-      return fail(E2E_ERR_DEVICE, "fused build+backup: a wait for a layer's completion ran out of its bound");
-    if (!(hc[CTR_FLAGS] & FLAG_POOL_EXHAUSTED)) break;
-    // rows that found no dense histogram were not backed up: again with the
-    // pool size the pass asked for
-    dfree(pool, st);
-    pool = nullptr;
-    pool_units = (int64_t)hc[CTR_POOL];
-    if ((double)pool_units * mm * 4 > 32.0 * (1ull << 30))
-      return fail(E2E_ERR_UNSUPPORTED, "transition spread too wide: dense-histogram pool above 32 GiB");
-    if (attempt == 2) return fail(E2E_ERR_DEVICE, "fused build did not settle after re-runs");
+    for (int k = 0; k < CTR_COUNT; ++k) sum[k] += hc[k];
+    BackupArgs B{};
+    B.t0 = t0;
+    B.t1 = t1;
+    B.na = pl.na;
+    B.lanes_log2 = build_lanes_log2(pl.na);
+    B.cells_log2 = 5 - B.lanes_log2;
+    B.nrzns = p->nrzns;
+    B.nc = (int)nc;
+    B.etiles_per_layer = pl.etiles_per_layer;
+    B.row_off = row_off;
+    B.tile_base = tile_base;
+    B.tile_len = tile_len;
+    B.R = R;
+    B.stage_col = static_cast<const int32_t*>(buf.col);
+    B.stage_cnt = static_cast<const uint16_t*>(buf.cnt);
+    B.V = dV;
+    B.pi = dpi;
+    B.sync = reinterpret_cast<unsigned int*>(bc + CTR_COUNT);
+    B.wb = wait_bound_from_env();
+    const int64_t need = ((nc << B.lanes_log2) + kThreads - 1) / kThreads;
+    const unsigned grid = (unsigned)std::min<int64_t>(need, (int64_t)per_sm * sms);
+    void* args[] = {&B};
+    CK(cudaLaunchCooperativeKernel((const void*)k_backup_layers, dim3(grid), dim3(kThreads), args, 0, st));
+    ++launches;
   }
-  scratch.add(pool);
-  float ms = 0.f;
-  CK(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+  CK(cudaEventRecord(ev[1], st));
   if (out_where == E2E_HOST) {
     if (value_out) CK(cudaMemcpyAsync(value_out, dV, sizeof(float) * ns, cudaMemcpyDeviceToHost, st));
     if (policy_out) CK(cudaMemcpyAsync(policy_out, dpi, sizeof(int32_t) * ns, cudaMemcpyDeviceToHost, st));
   }
+  unsigned long long err = 0;
+  CK(cudaMemcpyAsync(&err, bc + CTR_COUNT, sizeof(err), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  if (err >> 32) return fail(E2E_ERR_DEVICE, "build+solve: a wait for a layer's completion ran out of its bound");
+  float ms = 0.f;
+  CK(cudaEventElapsedTime(&ms, ev[0], ev[1]));
   if (stats) {
     stats->seconds = ms * 1e-3;
     stats->n_rows = pl.n_rows;
-    stats->nnz = (int64_t)hc[CTR_STAGE];
-    stats->dropped = hc[CTR_DROPPED];
-    stats->misbinned = hc[CTR_MISBIN];
-    stats->overflow_rows = hc[CTR_OVERFLOW_ROWS];
+    stats->nnz = (int64_t)sum[CTR_STAGE];
+    stats->dropped = sum[CTR_DROPPED];
+    stats->misbinned = sum[CTR_MISBIN];
+    stats->overflow_rows = sum[CTR_OVERFLOW_ROWS];
     stats->launches = launches;
     stats->h2d_bytes = (int64_t)fd.h2d_bytes;
   }

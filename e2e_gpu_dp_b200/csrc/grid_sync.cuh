@@ -1,0 +1,72 @@
+// Bounded device-side waits shared by the persistent kernels: the limits, the
+// acquire loads and the grid barrier of a cooperative launch.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdlib>
+
+namespace e2e {
+
+// A wait gives up after `spins` polls or `timeout_ns`, sets an error bit the
+// host reads (E2E_ERR_DEVICE) and lets the launch drain.  `extra` raises every
+// wait's target so that no wait can complete: the test hook that makes the
+// bounded waits run out on purpose, without any fault.
+struct WaitBound {
+  unsigned long long timeout_ns;
+  long long spins;
+  unsigned int extra;
+};
+
+// Host: E2E_WAIT_LIMIT_MS (default 2000) bounds each wait; with
+// E2E_TEST_UNREACHABLE_WAIT=1 the targets are raised by one (tests only).
+inline WaitBound wait_bound_from_env() {
+  WaitBound w{2000000000ull, 1ll << 22, 0u};
+  if (const char* ms = std::getenv("E2E_WAIT_LIMIT_MS")) {
+    const double v = std::atof(ms);
+    if (v > 0 && v <= 60000) w.timeout_ns = (unsigned long long)(v * 1e6);
+  }
+  if (const char* u = std::getenv("E2E_TEST_UNREACHABLE_WAIT")) w.extra = (u[0] == '1') ? 1u : 0u;
+  return w;
+}
+
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+__device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
+  unsigned int v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Grid-wide barrier of a cooperative launch.  sync[0] counts arrivals (never
+// reset inside a launch); a wait that outlives its limit sets bit 1 of sync[1]
+// and every later barrier returns false at once.
+__device__ __forceinline__ bool grid_barrier(unsigned int* sync, unsigned int target, const WaitBound& wb) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int good = 1;
+    __threadfence();
+    atomicAdd(sync, 1u);
+    const unsigned long long t0 = global_ns();
+    long long it = 0;
+    while (ld_acquire(sync) < target + wb.extra) {
+      if (ld_acquire(sync + 1) != 0u || ++it > wb.spins || global_ns() - t0 > wb.timeout_ns) {
+        atomicOr(sync + 1, 2u);
+        good = 0;
+        break;
+      }
+      __nanosleep(32);
+    }
+    __threadfence();
+    ok = good;
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+}  // namespace e2e

@@ -121,6 +121,20 @@ e2e_status copy_field_steps(const FieldsOnDevice& fd, int t0, int t1, cudaStream
 // first and the rest overlaps the builder's first launch
 e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const BuildPlan& pl,
                      cudaStream_t st, DeviceScratch* scratch, e2e_model* m);
+// Builder launches over ranges of layers.  layer_build_buffers allocates what the
+// ranked builder needs beside the fields (nothing for other problems);
+// launch_layers queues the builder for layers [t0, t1); launch_leftover the
+// general builder for the tiles of [t0, t1) that the ranked one listed.
+struct LayerBuild {
+  RankArgs K{};
+  unsigned int* defer_count = nullptr;
+  int32_t* defer_list = nullptr;
+};
+e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, cudaStream_t st, DeviceScratch* scratch,
+                               LayerBuild* L);
+cudaError_t launch_layers(const BuildArgs& A, const BuildPlan& pl, const LayerBuild& L, int t0, int t1, cudaStream_t st);
+cudaError_t launch_leftover(const BuildArgs& A, const BuildPlan& pl, const LayerBuild& L, int t0, int t1,
+                            cudaStream_t st);
 ViModel vi_model(const e2e_model* m);
 void free_model_buffers(e2e_model* m);
 int64_t model_bytes(const e2e_model* m);

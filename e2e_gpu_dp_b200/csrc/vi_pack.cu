@@ -36,6 +36,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "grid_sync.cuh"
 #include "internal.h"
 
 namespace e2e {
@@ -46,48 +47,10 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int PF_NEXT = VI_TUNE_PF_NEXT;
 constexpr int PF_CURRENT = VI_TUNE_PF_CURRENT;
-constexpr long long kBarrierSpinLimit = 1ll << 22;
-constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;  // 2 s
-
-// Bounds of the device-side waits of the persistent sweeps (grid barriers of
-// the layered sweep, per-layer completion counters of the batched sweep): a
-// wait gives up after `spins` polls or `timeout_ns`, sets an error bit the
-// host reads (E2E_ERR_DEVICE) and lets the launch drain.  `extra` raises every
-// wait's target so that no wait can complete: the test hook that makes the
-// bounded waits run out on purpose, without any fault.
-struct WaitBound {
-  unsigned long long timeout_ns;
-  long long spins;
-  unsigned int extra;
-};
-
-// Host: E2E_WAIT_LIMIT_MS (default 2000) bounds each wait; with
-// E2E_TEST_UNREACHABLE_WAIT=1 the targets are raised by one (tests only).
-WaitBound wait_bound_from_env() {
-  WaitBound w{kBarrierTimeoutNs, kBarrierSpinLimit, 0u};
-  if (const char* ms = std::getenv("E2E_WAIT_LIMIT_MS")) {
-    const double v = std::atof(ms);
-    if (v > 0 && v <= 60000) w.timeout_ns = (unsigned long long)(v * 1e6);
-  }
-  if (const char* u = std::getenv("E2E_TEST_UNREACHABLE_WAIT")) w.extra = (u[0] == '1') ? 1u : 0u;
-  return w;
-}
 
 __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   // bulk prefetch into L2: no shared memory, no completion to wait for
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
-  unsigned int v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
 }
 
 __device__ __forceinline__ int ld_acquire_s32(const int* p) {
@@ -612,33 +575,6 @@ __global__ void __launch_bounds__(kThreads)
       if (mx > 0.0) atomicMax(resid, (unsigned long long)__double_as_longlong(mx));
     }
   }
-}
-
-// Grid-wide barrier of a cooperative launch.  sync[0] counts arrivals (never
-// reset inside a launch); a wait that outlives its limit sets bit 1 of sync[1]
-// and every later barrier returns false at once.
-__device__ __forceinline__ bool grid_barrier(unsigned int* sync, unsigned int target, const WaitBound& wb) {
-  __shared__ int ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int good = 1;
-    __threadfence();
-    atomicAdd(sync, 1u);
-    const unsigned long long t0 = global_ns();
-    long long it = 0;
-    while (ld_acquire(sync) < target + wb.extra) {
-      if (ld_acquire(sync + 1) != 0u || ++it > wb.spins || global_ns() - t0 > wb.timeout_ns) {
-        atomicOr(sync + 1, 2u);
-        good = 0;
-        break;
-      }
-      __nanosleep(32);
-    }
-    __threadfence();
-    ok = good;
-  }
-  __syncthreads();
-  return ok != 0;
 }
 
 // The layered (backward-induction) schedule in one persistent launch: layer
