@@ -469,7 +469,9 @@ def run_ours(args, ws, rank, local):
 
     # the fused VI kernel in the reference's Jacobi schedule (VI SpMV GB/s)
     m = api.build_model(prob, dev, stream=stream)
-    _, _, jst = m.solve(method="jacobi", threshold=0.1, value=V, policy=pi, stream=stream)
+    # (schedule 0x140: one streaming sweep after another, whose bandwidth this measures;
+    # without a schedule the solver takes all sweeps of a layer at once)
+    _, _, jst = m.solve(method="jacobi", threshold=0.1, value=V, policy=pi, stream=stream, schedule=0x140)
     _, _, lst = m.solve(method="layered", fp64_check=True, value=V, policy=pi, stream=stream)
     minf = m.info()
     # parity: the device's rows against the oracle's rows of the CPU baseline's

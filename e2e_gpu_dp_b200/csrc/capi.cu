@@ -1231,6 +1231,82 @@ static e2e_status fp64_check(const e2e_model* m, const float* dV, e2e_vi_stats* 
   return E2E_OK;
 }
 
+// The Jacobi iteration of a layered model without one sweep after another
+// (jacobi.cu).  *done false: not taken (no layers, a wall-clock limit, which is
+// checked between sweeps, or no memory for the history), nothing changed.
+static e2e_status jacobi_by_layers(const e2e_model* m, const e2e_vi_opts& o, float* dV, int32_t* dpi,
+                                   e2e_vi_stats* stats, cudaStream_t st, bool* done) {
+  *done = false;
+  const int64_t ns = m->ns, nc = m->ncells;
+  if (!m->layered || nc <= 0 || ns % nc != 0 || m->na > 32 || o.timeout_s > 0) return E2E_OK;
+  const int64_t L64 = ns / nc;
+  if (L64 < 3 || L64 > 4096 || m->n_row_states > ns - nc) return E2E_OK;
+  const int L = (int)L64, max_iter = o.max_iter > 0 ? o.max_iter : (m->nt > 0 ? m->nt + 2 : 100000);
+  const int J = std::min(max_iter, L);
+  const size_t hist_bytes = sizeof(float) * jacobi_history_floats(nc, L, J);
+  // (a layer's history is indexed with 32 bits)
+  if (hist_bytes > (size_t(8) << 30) || nc * (int64_t)(J + 32) >= ((int64_t)1 << 31)) return E2E_OK;
+  DeviceScratch scratch(st);
+  float* hist = nullptr;
+  if (dalloc((void**)&hist, hist_bytes, st) != cudaSuccess) {
+    cudaGetLastError();
+    return E2E_OK;
+  }
+  scratch.add(hist);
+  float* prev = nullptr;
+  unsigned long long* resid = nullptr;
+  CK(dalloc((void**)&prev, sizeof(float) * (size_t)ns, st));
+  scratch.add(prev);
+  const size_t words = (size_t)J + 2 + (size_t)L;  // residuals, then a flag word per layer
+  CK(dalloc((void**)&resid, sizeof(unsigned long long) * words, st));
+  scratch.add(resid);
+  CK(cudaMemsetAsync(resid, 0, sizeof(unsigned long long) * words, st));
+  int dev = 0, sms = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  cudaEvent_t e0, e1;
+  CK(cudaEventCreate(&e0));
+  CK(cudaEventCreate(&e1));
+  struct EvGuard {
+    cudaEvent_t a, b;
+    ~EvGuard() { cudaEventDestroy(a); cudaEventDestroy(b); }
+  } evg{e0, e1};
+  const ViModel M = vi_model(m);
+  CK(cudaEventRecord(e0, st));
+  CK(launch_jacobi_layers(M, nc, L, J, hist, resid, reinterpret_cast<unsigned int*>(resid + J + 2), sms, st));
+  std::vector<unsigned long long> h((size_t)J + 1);
+  CK(cudaMemcpyAsync(h.data(), resid, sizeof(unsigned long long) * h.size(), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  // the sweep that ends the iteration; sweeps beyond the layers change nothing
+  int iters = 0;
+  double res = 0.0;
+  bool converged = false;
+  while (!converged && iters < max_iter) {
+    ++iters;
+    res = 0.0;
+    if (iters <= J) std::memcpy(&res, &h[iters], sizeof(double));
+    converged = res < (double)o.threshold;
+    if (iters > L && !converged) iters = max_iter;
+  }
+  CK(launch_jacobi_gather(nc, L, J, hist, iters - 1, prev, st));
+  CK(launch_vi_sweep(M, 0, ns, prev, dV, dpi, nullptr, st));
+  CK(cudaEventRecord(e1, st));
+  CK(cudaStreamSynchronize(st));
+  *done = true;
+  if (stats) {
+    float ms = 0.f;
+    CK(cudaEventElapsedTime(&ms, e0, e1));
+    std::memset(stats, 0, sizeof(*stats));
+    stats->iterations = iters;
+    stats->residual = res;
+    stats->seconds = ms * 1e-3;
+    stats->bytes_per_sweep = csr_sweep_bytes(m);
+    stats->stream_bytes_per_sweep = m->pack ? pack_sweep_bytes(m->pack->v) : stats->bytes_per_sweep;
+  }
+  if (!converged) return fail(E2E_ERR_NOT_CONVERGED, "max_iter reached before the threshold");
+  return o.fp64_check ? fp64_check(m, dV, stats, &scratch, st) : E2E_OK;
+}
+
 e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, int32_t* dpi,
                            e2e_vi_stats* stats, cudaStream_t st) {
   const int64_t ns = m->ns;
@@ -1243,6 +1319,11 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
   const bool tune_given = (o.schedule & 0x100) != 0;
   const int tune_layered = tune_given ? (o.schedule >> 4) & 15 : VI_TUNE_PF_NEXT;
   const int tune_jacobi = tune_given ? (o.schedule >> 4) & 15 : VI_TUNE_LEAN;
+  if (o.method == 0 && !tune_given) {
+    bool done = false;
+    e2e_status js = jacobi_by_layers(m, o, dV, dpi, stats, st, &done);
+    if (done || js != E2E_OK) return js;
+  }
   double pack_ms = 0.0;
   {
     e2e_status ps = ensure_pack(m, &pack_ms, st);

@@ -132,6 +132,17 @@ cudaError_t launch_vi_sweep_f64(const ViModel& M, int64_t s_begin, int64_t s_end
 cudaError_t launch_compare_f64(const float* V, const double* Vd, int64_t n,
                                unsigned long long* err, cudaStream_t st);
 
+// ---- Jacobi iteration, all sweeps of a layer at once (jacobi.cu) ----------------
+// History of a layered model of nlayers x nc states over `sweeps` sweeps: floats.
+size_t jacobi_history_floats(int64_t nc, int nlayers, int sweeps);
+// Sweeps 1 .. sweeps of every layer into hist; resid[j] (zeroed): bits of the FP64
+// max |V_j - V_j-1|; odd: nlayers zeroed words.  The last layer must have no rows.
+cudaError_t launch_jacobi_layers(const ViModel& M, int64_t nc, int nlayers, int sweeps, float* hist,
+                                 unsigned long long* resid, unsigned int* odd, int sms, cudaStream_t st);
+// V after j sweeps
+cudaError_t launch_jacobi_gather(int64_t nc, int nlayers, int sweeps, const float* hist, int j, float* V,
+                                 cudaStream_t st);
+
 // ---- sliced copy of a model for value iteration (vi_pack.cu) ------------------
 // entry layouts of the sliced copy
 enum : int {
