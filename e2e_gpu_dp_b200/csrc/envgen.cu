@@ -3,7 +3,9 @@
 // scalar "cloud" field and the obstacle mask
 // (src/data_input/build_environment_DG_with_westward_clouds.py:106-590).
 //
-// Per time step t (one at a time, so memory is one step's matrices):
+// Per time step t, for a batch of steps at once (both fields' matrices of up to
+// about 2 GB of steps: a step alone leaves the device idle, its Gram-Schmidt is
+// one CTA; one matrix after another took 28.0 ms for the reference's parameters):
 //   k_env_realisations  vx, vy, phi of every (sample k, coarse cell) in double,
 //                       the reference's expressions in its evaluation order
 //                       without contraction (:130-147, 20-84 for the cloud)
@@ -39,6 +41,7 @@
 #include <algorithm>
 #include <cmath>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "e2e_dp.h"
@@ -60,11 +63,11 @@ __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, 
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
 
 struct RealArgs {
-  int g, nws, t;
-  double tt;  // ts[t] = t * dt
+  int g, nws, t0;
+  double dt;  // ts[t] = t * dt
   double dxy, A, eps, wlo, whi, wx, wy;
-  double* Xv;  // nws x 2n: vx then vy
-  double* Xp;  // nws x n: phi
+  double* Xv;  // per step: nws x 2n, vx then vy
+  double* Xp;  // per step: nws x n, phi
 };
 
 // DG_velocity_field.vx_vy / phi / sample_w / get_ij_from_xy (:130-166)
@@ -74,12 +77,15 @@ __global__ void k_env_realisations(RealArgs a) {
   if (idx >= (int64_t)a.nws * n) return;
   const int k = (int)(idx / n), c = (int)(idx - (int64_t)k * n);
   const int i = c / a.g, j = c - i * a.g;
+  const double tt = mul((double)(a.t0 + (int)blockIdx.y), a.dt);
+  double* const Xv = a.Xv + (int64_t)blockIdx.y * a.nws * 2 * n;
+  double* const Xp = a.Xp + (int64_t)blockIdx.y * a.nws * n;
   // w = w_i + r (w_f - w_i), r = k / (n_wsamples - 1)
   const double r = a.nws > 1 ? (double)k / (double)(a.nws - 1) : 0.0;
   const double w = add(a.wlo, mul(r, sub(a.whi, a.wlo)));
   const double x = mul(add(0.5, (double)j), a.dxy);
   const double y = mul(add(0.5, (double)(a.g - 1 - i)), a.dxy);
-  const double swt = sin(mul(w, a.tt));
+  const double swt = sin(mul(w, tt));
   // f = eps sin(wt) x^2 + (1 - 2 eps sin(wt)) x;  fx = 2 eps sin(wt) (x - 1) + 1
   const double term1 = mul(mul(a.eps, swt), mul(x, x));
   const double e2s = mul(mul(2.0, a.eps), swt);
@@ -91,48 +97,85 @@ __global__ void k_env_realisations(RealArgs a) {
   const double vx = -mul(mul(mul(mul(0.5, a.A), kPi), swf), cwy);
   const double vy = mul(mul(mul(mul(a.A, kPi), swy), fx), cwf);
   const double ph = mul(mul(a.A, sin(mul(kPi, f))), swy);
-  a.Xv[(int64_t)k * 2 * n + c] = vx;
-  a.Xv[(int64_t)k * 2 * n + n + c] = vy;
-  a.Xp[(int64_t)k * n + c] = ph;
+  Xv[(int64_t)k * 2 * n + c] = vx;
+  Xv[(int64_t)k * 2 * n + n + c] = vy;
+  Xp[(int64_t)k * n + c] = ph;
 }
 
-// column means (sequential sum over samples, then / n_wsamples) and centring
-__global__ void k_env_center(double* X, int nws, int ncols, double* mean) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+// ---- the batch: nb steps' velocity matrices, then their scalar ones ------------
+// Matrix z of a launch (blockIdx.z) is step z of kind 0, or step z - nb of kind 1;
+// its arrays lie z * their size behind the kind's pointers.
+struct RrKind {
+  int ncols, k;        // columns; range-finder columns
+  int nseg, seg_rows;  // row segments of X^T B and of the residual
+  int colblocks;       // 128-column blocks
+  double *X, *mean;                  // nws x ncols, ncols
+  double *Q, *L;                     // nws x k
+  double *Z, *Bt, *Ub;               // ncols x k
+  double *R, *V, *U, *Vs, *S;        // k x k, S: k
+  double *P, *part, *scal;           // nseg x k x ncols; nseg x colblocks; 2
+  double *C, *M;                     // nws x r, r x ncols
+  double* svals;                     // r
+  int* sweeps;
+};
+struct RrBatch {
+  RrKind kind[2];
+  int nb, nws, r;
+  const double* Om;  // test matrix (the same values for every matrix)
+};
+struct RrMat {
+  int m;  // the step
+  const RrKind* K;
+};
+__device__ __forceinline__ RrMat rr_mat(const RrBatch& b, int z) {
+  return z >= b.nb ? RrMat{z - b.nb, &b.kind[1]} : RrMat{z, &b.kind[0]};
+}
+
+// column means: a sequential sum over the samples, then / n_wsamples (the loads of
+// sixteen rows are in flight together, the additions keep their order)
+__global__ void k_env_means(RrBatch b) {
+  const RrMat t = rr_mat(b, blockIdx.z);
+  const int ncols = t.K->ncols, c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncols) return;
-  double s = X[c];
-  for (int k = 1; k < nws; ++k) s = add(s, X[(int64_t)k * ncols + c]);
-  const double m = __ddiv_rn(s, (double)nws);
-  mean[c] = m;
-  for (int k = 0; k < nws; ++k) X[(int64_t)k * ncols + c] = sub(X[(int64_t)k * ncols + c], m);
+  const double* X = t.K->X + (int64_t)t.m * b.nws * ncols + c;
+  double s = X[0];
+  int k = 1;
+  for (; k + 16 <= b.nws; k += 16) {
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v[u] = X[(int64_t)(k + u) * ncols];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) s = add(s, v[u]);
+  }
+  for (; k < b.nws; ++k) s = add(s, X[(int64_t)k * ncols]);
+  t.K->mean[(int64_t)t.m * ncols + c] = __ddiv_rn(s, (double)b.nws);
+}
+
+__global__ void k_env_subtract(RrBatch b) {
+  const RrMat t = rr_mat(b, blockIdx.z);
+  const int ncols = t.K->ncols, c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= ncols) return;
+  const double m = t.K->mean[(int64_t)t.m * ncols + c];
+  double* X = t.K->X + (int64_t)t.m * b.nws * ncols + c;
+  for (int k = blockIdx.y; k < b.nws; k += gridDim.y) X[(int64_t)k * ncols] = sub(X[(int64_t)k * ncols], m);
 }
 
 // From the SVD of the centred matrix X (nws x ncols): coefficients C (nws x r)
 // and modes M (r x ncols), mode q = the q-th largest singular value:
-// C[k][q] = Us[k + q ldu] s_q (the left singular vectors scaled, rank_reduction's
-// u1 diag(s1)), M[q][c] = Vs[c + q ldv] (Vh's rows).  Signs: the
+// C[k][q] = L[k][q] s_q (the left singular vectors scaled, rank_reduction's
+// u1 diag(s1)), M[q][c] = Ub[c][q] (Vh's rows).  Signs: the
 // largest-magnitude coefficient of each mode is made positive.
-struct ModeArgs {
-  int nws, ncols, r;
-  const double* S;   // singular values, descending
-  const double* Us;  // left singular vectors (sample side), column q at Us + q * ldu
-  int ldu;
-  const double* Vs;  // right singular vectors (grid side), column q at Vs + q * ldv
-  int ldv;
-  double* C;         // nws x r
-  double* M;         // r x ncols
-  double* svals;     // r
-};
-
-__global__ void k_env_modes(ModeArgs a) {
+__global__ void k_env_modes(RrBatch a0) {
+  const RrMat t = rr_mat(a0, blockIdx.z);
+  const int nws = a0.nws, ncols = t.K->ncols, r = a0.r, kk = t.K->k;
   const int q = blockIdx.x;  // one block per mode
-  const double s = a.S[q];
+  const double s = t.K->S[(int64_t)t.m * kk + q];
   __shared__ double best_v[32];
   __shared__ int best_k[32];
-  const double* u = a.Us + (int64_t)q * a.ldu;
+  const double* u = t.K->L + ((int64_t)t.m * kk + q) * nws;
   double bv = -1.0;
   int bk = 0x7fffffff;
-  for (int k = threadIdx.x; k < a.nws; k += blockDim.x) {
+  for (int k = threadIdx.x; k < nws; k += blockDim.x) {
     const double v = fabs(u[k] * s);
     if (v > bv || (v == bv && k < bk)) {
       bv = v;
@@ -162,10 +205,10 @@ __global__ void k_env_modes(ModeArgs a) {
   }
   __syncthreads();
   const double sgn = u[best_k[0]] < 0.0 ? -1.0 : 1.0;
-  if (threadIdx.x == 0) a.svals[q] = s;
-  for (int k = threadIdx.x; k < a.nws; k += blockDim.x) a.C[(int64_t)k * a.r + q] = sgn * (u[k] * s);
-  const double* v = a.Vs + (int64_t)q * a.ldv;
-  for (int c = threadIdx.x; c < a.ncols; c += blockDim.x) a.M[(int64_t)q * a.ncols + c] = sgn * v[c];
+  if (threadIdx.x == 0) t.K->svals[(int64_t)t.m * r + q] = s;
+  for (int k = threadIdx.x; k < nws; k += blockDim.x) t.K->C[((int64_t)t.m * nws + k) * r + q] = sgn * (u[k] * s);
+  const double* v = t.K->Ub + ((int64_t)t.m * kk + q) * ncols;
+  for (int c = threadIdx.x; c < ncols; c += blockDim.x) t.K->M[((int64_t)t.m * r + q) * ncols + c] = sgn * v[c];
 }
 
 // test matrix of the range finder: deterministic values in [-1, 1) from a
@@ -185,26 +228,32 @@ __global__ void k_env_test_matrix(double* O, int64_t n) {
 // coarse means and modes in float32 arrays except all_phi_mat, a float64 array
 // (:271), so every value but phi's mean is rounded to float before it is
 // interpolated.
-__global__ void k_env_store(int n, int nws, int r, const double* mv, const double* mp, const double* Mv,
-                            const double* Mp, const double* Cv, const double* Cp, double* coarse, float* yi,
-                            float* phi_yi) {
+__global__ void k_env_store(RrBatch b, int n, double* coarse0, float* yi0, float* phi_yi0) {
+  const int nws = b.nws, r = b.r, t = blockIdx.y;
+  const double* mv = b.kind[0].mean + (int64_t)t * 2 * n;
+  const double* mp = b.kind[1].mean + (int64_t)t * n;
+  const double* Mv = b.kind[0].M + (int64_t)t * r * 2 * n;
+  const double* Mp = b.kind[1].M + (int64_t)t * r * n;
+  const double* Cv = b.kind[0].C + (int64_t)t * nws * r;
+  const double* Cp = b.kind[1].C + (int64_t)t * nws * r;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nb = (int64_t)(3 + 3 * r) * n;
   if (idx < nb) {
-    const int b = (int)(idx / n), c = (int)(idx - (int64_t)b * n);
+    double* coarse = coarse0 + (int64_t)t * nb;
+    const int b2 = (int)(idx / n), c = (int)(idx - (int64_t)b2 * n);
     double v;
-    if (b == 0) v = mv[c];
-    else if (b == 1) v = mv[n + c];
-    else if (b == 2) v = mp[c];
-    else if (b < 3 + r) v = Mv[(int64_t)(b - 3) * 2 * n + c];
-    else if (b < 3 + 2 * r) v = Mv[(int64_t)(b - 3 - r) * 2 * n + n + c];
-    else v = Mp[(int64_t)(b - 3 - 2 * r) * n + c];
-    coarse[idx] = b == 2 ? v : (double)(float)v;
+    if (b2 == 0) v = mv[c];
+    else if (b2 == 1) v = mv[n + c];
+    else if (b2 == 2) v = mp[c];
+    else if (b2 < 3 + r) v = Mv[(int64_t)(b2 - 3) * 2 * n + c];
+    else if (b2 < 3 + 2 * r) v = Mv[(int64_t)(b2 - 3 - r) * 2 * n + n + c];
+    else v = Mp[(int64_t)(b2 - 3 - 2 * r) * n + c];
+    coarse[idx] = b2 == 2 ? v : (double)(float)v;
   }
   const int64_t nc = (int64_t)nws * r;
   if (idx < nc) {
-    yi[idx] = (float)Cv[idx];
-    phi_yi[idx] = (float)Cp[idx];
+    yi0[(int64_t)t * nc + idx] = (float)Cv[idx];
+    phi_yi0[(int64_t)t * nc + idx] = (float)Cp[idx];
   }
 }
 
@@ -320,8 +369,13 @@ constexpr int kRrMaxSweeps = 60;  // Jacobi sweeps at most (convergence is quadr
 // partial products of X^T B over row segments: P[seg][c][j] = sum over the
 // segment's rows i, in order, of X[i][j] B[i][c]; a thread per column j
 template <int K>
-__global__ void __launch_bounds__(128) k_rr_xtb(const double* X, int nws, int ncols, const double* B, int ldb,
-                                                int k, int seg_rows, double* P) {
+__global__ void __launch_bounds__(128) k_rr_xtb(RrBatch b) {
+  const RrMat t = rr_mat(b, blockIdx.z);
+  const int nws = b.nws, ncols = t.K->ncols, k = t.K->k, seg_rows = t.K->seg_rows, ldb = nws;
+  if ((int)blockIdx.x >= t.K->colblocks || (int)blockIdx.y >= t.K->nseg) return;
+  const double* X = t.K->X + (int64_t)t.m * nws * ncols;
+  const double* B = t.K->Q + (int64_t)t.m * nws * k;
+  double* P = t.K->P + (int64_t)t.m * t.K->nseg * k * ncols;
   __shared__ double Bs[32][K];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const int i0 = blockIdx.y * seg_rows, i1 = min(nws, i0 + seg_rows);
@@ -351,8 +405,12 @@ __global__ void __launch_bounds__(128) k_rr_xtb(const double* X, int nws, int nc
   }
 }
 
-// C[j + c ldc] = sum over segments s = 0.. in order of P[s][c][j]
-__global__ void k_rr_sum_segments(const double* P, int nseg, int ncols, int k, double* C, int ldc) {
+// C[j + c ncols] = sum over segments s = 0.. in order of P[s][c][j], C = Bt or Z
+__global__ void k_rr_sum_segments(RrBatch b, bool to_bt) {
+  const RrMat t = rr_mat(b, blockIdx.z);
+  const int nseg = t.K->nseg, ncols = t.K->ncols, k = t.K->k, ldc = ncols;
+  const double* P = t.K->P + (int64_t)t.m * nseg * k * ncols;
+  double* C = (to_bt ? t.K->Bt : t.K->Z) + (int64_t)t.m * ncols * k;
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (int64_t)ncols * k) return;
   const int c = (int)(e / ncols), j = (int)(e - (int64_t)c * ncols);
@@ -361,35 +419,59 @@ __global__ void k_rr_sum_segments(const double* P, int nseg, int ncols, int k, d
   C[(int64_t)c * ldc + j] = s;
 }
 
-// C (nws x k) = X B, B ncols x k: a warp per row of X, lanes over its columns,
-// lane sums reduced by a shuffle tree (lane 0's result is written)
-template <int K>
-__global__ void __launch_bounds__(256) k_rr_xb(const double* X, int nws, int ncols, const double* B, int ldb,
-                                               int k, double* C, int ldc) {
-  const int row = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (row >= nws) return;  // whole warps
-  double acc[K];
+// Q (nws x k) = X B, B ncols x k (Z, or the test matrix): a warp takes ROWS rows
+// of X, lanes over the columns, lane sums reduced by a shuffle tree (lane 0's
+// result is written).  Reading B once for four rows instead of one: 0.68 -> 0.19
+// ms for the 20 matrices of the reference's parameters.
+template <int K, int ROWS>
+__global__ void __launch_bounds__(128) k_rr_xb(RrBatch b, bool test) {
+  const RrMat t = rr_mat(b, blockIdx.z);
+  const int nws = b.nws, ncols = t.K->ncols, k = t.K->k, ldb = ncols, ldc = nws;
+  const double* B = test ? b.Om : t.K->Z + (int64_t)t.m * ncols * k;
+  double* C = t.K->Q + (int64_t)t.m * nws * k;
+  const int row0 = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * ROWS, lane = threadIdx.x & 31;
+  if (row0 >= nws) return;  // whole warps
+  const double* x[ROWS];
 #pragma unroll
-  for (int c = 0; c < K; ++c) acc[c] = 0.0;
-  const double* x = X + (int64_t)row * ncols;
+  for (int r = 0; r < ROWS; ++r) x[r] = t.K->X + ((int64_t)t.m * nws + min(row0 + r, nws - 1)) * ncols;
+  double acc[ROWS][K];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+    for (int c = 0; c < K; ++c) acc[r][c] = 0.0;
   for (int j = lane; j < ncols; j += 32) {
-    const double xv = x[j];
+    double xv[ROWS];
 #pragma unroll
-    for (int c = 0; c < K; ++c)
-      if (c < k) acc[c] = fma(xv, B[(int64_t)c * ldb + j], acc[c]);
+    for (int r = 0; r < ROWS; ++r) xv[r] = x[r][j];
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      if (c < k) {
+        const double bv = B[(int64_t)c * ldb + j];
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) acc[r][c] = fma(xv[r], bv, acc[r][c]);
+      }
+    }
   }
 #pragma unroll
-  for (int c = 0; c < K; ++c) {
-    if (c < k) {
-      double v = acc[c];
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) C[(int64_t)c * ldc + row] = v;
+  for (int r = 0; r < ROWS; ++r) {
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      if (c < k) {
+        double v = acc[r][c];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0 && row0 + r < nws) C[(int64_t)c * ldc + row0 + r] = v;
+      }
     }
   }
 }
 
-// C (rows x k) = A (rows x k) W (k x k, ld k): a thread per entry, sum in order
-__global__ void k_rr_small(const double* A, int lda, int rows, int k, const double* W, double* C, int ldc) {
+// Ub = Bt U (ncols x k), or L = Q Vs (nws x k): a thread per entry, sum in order
+__global__ void k_rr_small(RrBatch b, bool left) {
+  const RrMat t = rr_mat(b, blockIdx.z);
+  const int k = t.K->k, rows = left ? b.nws : t.K->ncols, lda = rows, ldc = rows;
+  const double* A = (left ? t.K->Q : t.K->Bt) + (int64_t)t.m * rows * k;
+  const double* W = (left ? t.K->Vs : t.K->U) + (int64_t)t.m * k * k;
+  double* C = (left ? t.K->L : t.K->Ub) + (int64_t)t.m * rows * k;
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (int64_t)rows * k) return;
   const int c = (int)(e / rows), i = (int)(e - (int64_t)c * rows);
@@ -421,9 +503,15 @@ __device__ double rr_block_sum(double v, double* red) {
 // coefficients and the norms.  A column that the second pass shrinks below
 // half its length lies in the span of the earlier ones to working precision
 // (what is left is rounding, which no further pass makes orthogonal): it
-// becomes zero, as does a zero column (R's diagonal 0).  One CTA.
+// becomes zero, as does a zero column (R's diagonal 0).  One CTA a matrix: Q, Z,
+// or Bt with R kept.
+enum : int { RR_Q = 0, RR_Z = 1, RR_BT = 2 };
 template <int K>
-__global__ void __launch_bounds__(256) k_rr_cgs2(double* A, int rows, int k, int lda, double* R) {
+__global__ void __launch_bounds__(256) k_rr_cgs2(RrBatch b, int which) {
+  const RrMat t = rr_mat(b, blockIdx.z);
+  const int k = t.K->k, rows = which == RR_Q ? b.nws : t.K->ncols, lda = rows;
+  double* A = (which == RR_Q ? t.K->Q : which == RR_Z ? t.K->Z : t.K->Bt) + (int64_t)t.m * rows * k;
+  double* R = which == RR_BT ? t.K->R + (int64_t)t.m * k * k : nullptr;
   __shared__ double red[33];
   __shared__ double wsum[8][K];
   __shared__ double d[K];
@@ -488,9 +576,16 @@ __global__ void __launch_bounds__(256) k_rr_cgs2(double* A, int rows, int k, int
 // descending singular value (ties: lower column first): S (k), U and Vs (k x k,
 // ld k; a zero singular value gives a zero U column).  Rounds of disjoint
 // pairs (a round-robin tournament over the columns), a warp per pair, each
-// warp's reductions broadcast from lane 0 so all lanes rotate alike.  One CTA.
-__global__ void __launch_bounds__(256) k_rr_jacobi(double* W, double* V, int k, double* S, double* U, double* Vs,
-                                                   int* sweeps) {
+// warp's reductions broadcast from lane 0 so all lanes rotate alike.  One CTA a matrix.
+__global__ void __launch_bounds__(256) k_rr_jacobi(RrBatch b) {
+  const RrMat t = rr_mat(b, blockIdx.z);
+  const int k = t.K->k;
+  double* W = t.K->R + (int64_t)t.m * k * k;
+  double* V = t.K->V + (int64_t)t.m * k * k;
+  double* U = t.K->U + (int64_t)t.m * k * k;
+  double* Vs = t.K->Vs + (int64_t)t.m * k * k;
+  double* S = t.K->S + (int64_t)t.m * k;
+  int* sweeps = t.K->sweeps + t.m;
   __shared__ int rotated;
   __shared__ double sv[kRrMaxK];
   __shared__ int order[kRrMaxK];
@@ -580,8 +675,14 @@ __global__ void __launch_bounds__(256) k_rr_jacobi(double* W, double* V, int k, 
 // partial sums of squares of the residual X - Q Bt^T (Q nws x k, Bt ncols x
 // k): a thread per column j over a row segment, one partial per CTA
 template <int K>
-__global__ void __launch_bounds__(128) k_rr_resid(const double* X, int nws, int ncols, const double* Q,
-                                                  const double* Bt, int k, int seg_rows, double* part) {
+__global__ void __launch_bounds__(128) k_rr_resid(RrBatch bt) {
+  const RrMat t = rr_mat(bt, blockIdx.z);
+  const int nws = bt.nws, ncols = t.K->ncols, k = t.K->k, seg_rows = t.K->seg_rows;
+  if ((int)blockIdx.x >= t.K->colblocks || (int)blockIdx.y >= t.K->nseg) return;  // whole CTAs
+  const double* X = t.K->X + (int64_t)t.m * nws * ncols;
+  const double* Q = t.K->Q + (int64_t)t.m * nws * k;
+  const double* Bt = t.K->Bt + (int64_t)t.m * ncols * k;
+  double* part = t.K->part + (int64_t)t.m * t.K->nseg * t.K->colblocks;
   __shared__ double Qs[32][K];
   __shared__ double red[33];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -608,44 +709,44 @@ __global__ void __launch_bounds__(128) k_rr_resid(const double* X, int nws, int 
     }
   }
   const double s = rr_block_sum(ssq, red);
-  if (threadIdx.x == 0) part[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = s;
+  if (threadIdx.x == 0) part[(int64_t)blockIdx.y * t.K->colblocks + blockIdx.x] = s;
 }
 
-// out[slot] = sum of v[0..n) in order (one thread: a few hundred partials)
-__global__ void k_rr_sum_serial(const double* v, int n, double* out, int slot) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// scal[0] = sum of the residual's partials in order (one thread: a few hundred)
+__global__ void k_rr_sum_serial(RrBatch b) {
+  if (threadIdx.x != 0) return;
+  const RrMat t = rr_mat(b, blockIdx.z);
+  const int n = t.K->nseg * t.K->colblocks;
+  const double* v = t.K->part + (int64_t)t.m * n;
   double s = 0.0;
-  for (int i = 0; i < n; ++i) s += v[i];
-  out[slot] = s;
+  int i = 0;
+  for (; i + 8 <= n; i += 8) {
+    double x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = v[i + u];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += x[u];
+  }
+  for (; i < n; ++i) s += v[i];
+  t.K->scal[2 * t.m] = s;
 }
 
-// out[slot] = sum of squares of v[0..n), one CTA, fixed order
-__global__ void __launch_bounds__(256) k_rr_sumsq(const double* v, int n, double* out, int slot) {
+// scal[1] = sum of squares of the mean, one CTA a matrix, fixed order
+__global__ void __launch_bounds__(256) k_rr_sumsq(RrBatch b) {
   __shared__ double red[33];
+  const RrMat t = rr_mat(b, blockIdx.z);
+  const int n = t.K->ncols;
+  const double* v = t.K->mean + (int64_t)t.m * n;
   double s = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s = fma(v[i], v[i], s);
   s = rr_block_sum(s, red);
-  if (threadIdx.x == 0) out[slot] = s;
+  if (threadIdx.x == 0) t.K->scal[2 * t.m + 1] = s;
 }
-
-struct SvdWork {
-  int kmax = 0;      // columns the buffers hold
-  int ncols_max = 0;
-  double *Om = nullptr, *Q = nullptr, *Z = nullptr, *Bt = nullptr, *L = nullptr, *Ub = nullptr;
-  double *R = nullptr, *V = nullptr, *U = nullptr, *Vs = nullptr, *S = nullptr;
-  double* P = nullptr;     // segment partials: kRrSegs x ncols_max x kmax
-  double* part = nullptr;  // residual partials
-  int part_cap = 0;
-  double* scal = nullptr;  // device: [0] residual^2, [1] |mean|^2
-  double hscal[3] = {0.0, 0.0, 0.0};  // host copy of scal and S[0]
-  int* sweeps = nullptr;
-};
 
 constexpr int kRrSegs = 16;  // row segments of the X^T B products at most
 
-int rr_bucket(int k) { return k <= 16 ? 16 : (k <= 32 ? 32 : 64); }
-
-// row segments for X^T B / the residual: enough CTAs to cover the SMs
+// row segments for X^T B / the residual: enough CTAs to cover the SMs for one
+// matrix (the sums' order is part of the result: it does not depend on the batch)
 void rr_segments(int nws, int ncols, int* nseg, int* seg_rows) {
   const int colblocks = (ncols + 127) / 128;
   int s = std::max(1, std::min(kRrSegs, (296 + colblocks - 1) / colblocks));
@@ -656,145 +757,136 @@ void rr_segments(int nws, int ncols, int* nseg, int* seg_rows) {
   *nseg = (nws + rows - 1) / rows;
 }
 
-// C (ncols x k, ld ncols) = X^T B (B nws x k, ld nws)
-e2e_status rr_xtb(SvdWork& w, const double* X, int nws, int ncols, const double* B, int k, double* C,
-                  cudaStream_t st) {
-  int nseg, seg_rows;
-  rr_segments(nws, ncols, &nseg, &seg_rows);
-  const dim3 grid((unsigned)((ncols + 127) / 128), (unsigned)nseg);
-  switch (rr_bucket(k)) {
-    case 16: k_rr_xtb<16><<<grid, 128, 0, st>>>(X, nws, ncols, B, nws, k, seg_rows, w.P); break;
-    case 32: k_rr_xtb<32><<<grid, 128, 0, st>>>(X, nws, ncols, B, nws, k, seg_rows, w.P); break;
-    default: k_rr_xtb<64><<<grid, 128, 0, st>>>(X, nws, ncols, B, nws, k, seg_rows, w.P); break;
-  }
-  CK(cudaGetLastError());
-  const int64_t ne = (int64_t)ncols * k;
-  k_rr_sum_segments<<<(unsigned)((ne + 255) / 256), 256, 0, st>>>(w.P, nseg, ncols, k, C, ncols);
+// f(bucket of the range-finder columns)
+template <typename F>
+void rr_bucket(int k, F&& f) {
+  if (k <= 16) f(std::integral_constant<int, 16>{});
+  else if (k <= 32) f(std::integral_constant<int, 32>{});
+  else f(std::integral_constant<int, 64>{});
+}
+
+// doubles of one matrix' work arrays (RrKind from Q on, but mean, C, M, svals)
+size_t rr_work_doubles(int nws, int ncols, int k) {
+  int nseg, rows;
+  rr_segments(nws, ncols, &nseg, &rows);
+  return (size_t)2 * nws * k + (size_t)3 * ncols * k + (size_t)4 * k * k + k + (size_t)nseg * k * ncols +
+         (size_t)nseg * ((ncols + 127) / 128) + 2 + 1;
+}
+
+// carve the work arrays of nb matrices from p
+double* rr_carve(RrKind* K, int nws, int ncols, int k, int nb, double* p) {
+  K->ncols = ncols;
+  K->k = k;
+  K->colblocks = (ncols + 127) / 128;
+  rr_segments(nws, ncols, &K->nseg, &K->seg_rows);
+  auto take = [&](size_t each) {
+    double* q = p;
+    p += each * nb;
+    return q;
+  };
+  K->Q = take((size_t)nws * k);
+  K->L = take((size_t)nws * k);
+  K->Z = take((size_t)ncols * k);
+  K->Bt = take((size_t)ncols * k);
+  K->Ub = take((size_t)ncols * k);
+  K->R = take((size_t)k * k);
+  K->V = take((size_t)k * k);
+  K->U = take((size_t)k * k);
+  K->Vs = take((size_t)k * k);
+  K->S = take(k);
+  K->P = take((size_t)K->nseg * k * ncols);
+  K->part = take((size_t)K->nseg * K->colblocks);
+  K->scal = take(2);
+  K->sweeps = reinterpret_cast<int*>(take(1));
+  return p;
+}
+
+// Randomized SVDs of the nz centred matrices of a batch (nz = nb: the first kind
+// alone) with k columns and `power` power iterations, then coefficients and modes
+// of all of them.  The caller checks the certificates (rr_certified) from scal
+// and S.
+e2e_status randomized_svds(const RrBatch& b, int nz, int power, double* Om, cudaStream_t st) {
+  const bool both = nz > b.nb;
+  const int ncols = both ? std::max(b.kind[0].ncols, b.kind[1].ncols) : b.kind[0].ncols;
+  const int k = both ? std::max(b.kind[0].k, b.kind[1].k) : b.kind[0].k;
+  const int nseg = both ? std::max(b.kind[0].nseg, b.kind[1].nseg) : b.kind[0].nseg;
+  const unsigned z = (unsigned)nz;
+  const dim3 cols((unsigned)((ncols + 127) / 128), (unsigned)nseg, z);
+  const dim3 per_col((unsigned)(((int64_t)ncols * k + 255) / 256), 1, z);
+  const dim3 per_row((unsigned)(((int64_t)b.nws * k + 255) / 256), 1, z);
+  const dim3 one(1, 1, z);
+  const int64_t no = (int64_t)ncols * k;
+  k_env_test_matrix<<<(unsigned)((no + 255) / 256), 256, 0, st>>>(Om, no);
+  rr_bucket(k, [&](auto bucket) {
+    constexpr int K = decltype(bucket)::value, kRows = K == 16 ? 4 : 1;
+    const dim3 rows((unsigned)((b.nws + 4 * kRows - 1) / (4 * kRows)), 1, z);  // 4 warps a CTA
+    auto xtb = [&](bool to_bt) {
+      k_rr_xtb<K><<<cols, 128, 0, st>>>(b);
+      k_rr_sum_segments<<<per_col, 256, 0, st>>>(b, to_bt);
+    };
+    k_rr_xb<K, kRows><<<rows, 128, 0, st>>>(b, true);  // Q = X Om
+    k_rr_cgs2<K><<<one, 256, 0, st>>>(b, RR_Q);
+    for (int it = 0; it < power; ++it) {  // Q <- orth(X orth(X^T Q))
+      xtb(false);
+      k_rr_cgs2<K><<<one, 256, 0, st>>>(b, RR_Z);
+      k_rr_xb<K, kRows><<<rows, 128, 0, st>>>(b, false);
+      k_rr_cgs2<K><<<one, 256, 0, st>>>(b, RR_Q);
+    }
+    xtb(true);  // Bt = X^T Q
+    k_rr_resid<K><<<cols, 128, 0, st>>>(b);
+    k_rr_sum_serial<<<one, 32, 0, st>>>(b);
+    k_rr_sumsq<<<one, 256, 0, st>>>(b);
+    // Bt = Qb R (Bt becomes Qb), R = U_R S V_R^T, Ub = Qb U_R, L = Q V_R
+    k_rr_cgs2<K><<<one, 256, 0, st>>>(b, RR_BT);
+  });
+  k_rr_jacobi<<<one, 256, 0, st>>>(b);
+  k_rr_small<<<per_col, 256, 0, st>>>(b, false);
+  k_rr_small<<<per_row, 256, 0, st>>>(b, true);
+  k_env_modes<<<dim3((unsigned)b.r, 1, z), 256, 0, st>>>(b);
   CK(cudaGetLastError());
   return E2E_OK;
 }
 
-// C (nws x k, ld nws) = X B (B ncols x k, ld ncols)
-e2e_status rr_xb(const double* X, int nws, int ncols, const double* B, int k, double* C, cudaStream_t st) {
-  const unsigned blocks = (unsigned)(((int64_t)nws * 32 + 255) / 256);
-  switch (rr_bucket(k)) {
-    case 16: k_rr_xb<16><<<blocks, 256, 0, st>>>(X, nws, ncols, B, ncols, k, C, nws); break;
-    case 32: k_rr_xb<32><<<blocks, 256, 0, st>>>(X, nws, ncols, B, ncols, k, C, nws); break;
-    default: k_rr_xb<64><<<blocks, 256, 0, st>>>(X, nws, ncols, B, ncols, k, C, nws); break;
-  }
-  CK(cudaGetLastError());
-  return E2E_OK;
-}
-
-e2e_status rr_orth(double* A, int rows, int k, double* R, cudaStream_t st) {
-  switch (rr_bucket(k)) {
-    case 16: k_rr_cgs2<16><<<1, 256, 0, st>>>(A, rows, k, rows, R); break;
-    case 32: k_rr_cgs2<32><<<1, 256, 0, st>>>(A, rows, k, rows, R); break;
-    default: k_rr_cgs2<64><<<1, 256, 0, st>>>(A, rows, k, rows, R); break;
-  }
-  CK(cudaGetLastError());
-  return E2E_OK;
-}
-
-// |X - Q Bt^T|_F^2 into w.scal[0]
-e2e_status rr_residual(SvdWork& w, const double* X, int nws, int ncols, int k, cudaStream_t st) {
-  int nseg, seg_rows;
-  rr_segments(nws, ncols, &nseg, &seg_rows);
-  const dim3 grid((unsigned)((ncols + 127) / 128), (unsigned)nseg);
-  const int np = (int)(grid.x * grid.y);
-  if (np > w.part_cap) return fail(E2E_ERR_INVALID, "residual partials above capacity");
-  switch (rr_bucket(k)) {
-    case 16: k_rr_resid<16><<<grid, 128, 0, st>>>(X, nws, ncols, w.Q, w.Bt, k, seg_rows, w.part); break;
-    case 32: k_rr_resid<32><<<grid, 128, 0, st>>>(X, nws, ncols, w.Q, w.Bt, k, seg_rows, w.part); break;
-    default: k_rr_resid<64><<<grid, 128, 0, st>>>(X, nws, ncols, w.Q, w.Bt, k, seg_rows, w.part); break;
-  }
-  CK(cudaGetLastError());
-  k_rr_sum_serial<<<1, 32, 0, st>>>(w.part, np, w.scal, 0);
-  CK(cudaGetLastError());
-  return E2E_OK;
-}
-
-// Randomized SVD of the centred X (row-major nws x ncols) with k columns and
-// `power` power iterations; *ok when certified:
+// A reduction stands when
 //  * |X - Q Q^T X|_F <= 1e-10 s_1 (then each kept singular value is exact to
 //    about |R|^2 / s_k, machine precision relative to s_1), or
 //  * s_1 <= 1e-10 sqrt(nws) |mean|: the centred matrix is below the rounding of
 //    the data it was centred from (every realisation alike, as at t = 0), so
 //    its singular vectors are not determined by the data and the computed ones
 //    stand, as LAPACK's do for the reference.
-e2e_status randomized_svd(SvdWork& w, const double* X, int nws, int ncols, int r, int k, int power,
-                          const double* mean, double* C, double* M, double* svals, bool* ok, cudaStream_t st) {
-  *ok = false;
-  const int64_t no = (int64_t)ncols * k;
-  k_env_test_matrix<<<(unsigned)((no + 255) / 256), 256, 0, st>>>(w.Om, no);
-  CK(cudaGetLastError());
-  e2e_status s;
-  if ((s = rr_xb(X, nws, ncols, w.Om, k, w.Q, st)) != E2E_OK) return s;     // Q = X Om
-  if ((s = rr_orth(w.Q, nws, k, nullptr, st)) != E2E_OK) return s;
-  for (int it = 0; it < power; ++it) {                                        // Q <- orth(X orth(X^T Q))
-    if ((s = rr_xtb(w, X, nws, ncols, w.Q, k, w.Z, st)) != E2E_OK) return s;
-    if ((s = rr_orth(w.Z, ncols, k, nullptr, st)) != E2E_OK) return s;
-    if ((s = rr_xb(X, nws, ncols, w.Z, k, w.Q, st)) != E2E_OK) return s;
-    if ((s = rr_orth(w.Q, nws, k, nullptr, st)) != E2E_OK) return s;
-  }
-  if ((s = rr_xtb(w, X, nws, ncols, w.Q, k, w.Bt, st)) != E2E_OK) return s;  // Bt = X^T Q
-  if ((s = rr_residual(w, X, nws, ncols, k, st)) != E2E_OK) return s;
-  k_rr_sumsq<<<1, 256, 0, st>>>(mean, ncols, w.scal, 1);
-  CK(cudaGetLastError());
-  // Bt = Qb R (Bt becomes Qb), R = U_R S V_R^T, Ub = Qb U_R, L = Q V_R
-  if ((s = rr_orth(w.Bt, ncols, k, w.R, st)) != E2E_OK) return s;
-  k_rr_jacobi<<<1, 256, 0, st>>>(w.R, w.V, k, w.S, w.U, w.Vs, w.sweeps);
-  CK(cudaGetLastError());
-  const int64_t nu = (int64_t)ncols * k, nl = (int64_t)nws * k;
-  k_rr_small<<<(unsigned)((nu + 255) / 256), 256, 0, st>>>(w.Bt, ncols, ncols, k, w.U, w.Ub, ncols);
-  k_rr_small<<<(unsigned)((nl + 255) / 256), 256, 0, st>>>(w.Q, nws, nws, k, w.Vs, w.L, nws);
-  CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(w.hscal, w.scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(w.hscal + 2, w.S, sizeof(double), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  const double rnorm = sqrt(w.hscal[0]), mnorm = sqrt(w.hscal[1]), s1 = w.hscal[2];
-  const bool certified = (s1 > 0.0 && rnorm <= 1e-10 * s1) || !(s1 > 1e-10 * sqrt((double)nws) * mnorm);
-  if (!certified || !std::isfinite(rnorm) || !std::isfinite(s1)) return E2E_OK;
-  ModeArgs a;
-  a.nws = nws;
-  a.ncols = ncols;
-  a.r = r;
-  a.S = w.S;
-  a.Us = w.L;
-  a.ldu = nws;
-  a.Vs = w.Ub;
-  a.ldv = ncols;
-  a.C = C;
-  a.M = M;
-  a.svals = svals;
-  k_env_modes<<<r, 256, 0, st>>>(a);
-  CK(cudaGetLastError());
-  *ok = true;
-  return E2E_OK;
+bool rr_certified(const double* scal, double s1, int nws) {
+  const double rnorm = sqrt(scal[0]), mnorm = sqrt(scal[1]);
+  const bool ok = (s1 > 0.0 && rnorm <= 1e-10 * s1) || !(s1 > 1e-10 * sqrt((double)nws) * mnorm);
+  return ok && std::isfinite(rnorm) && std::isfinite(s1);
 }
 
-// The leading r triplets: k = n_modes + 10 columns and two power iterations;
-// if that is not certified, twice the columns (up to 64 and the matrix's
-// smaller side) and four power iterations until it is.  When the columns span
-// the whole smaller side the residual is rounding only, so only n_modes above
-// 54 on a matrix wider than 64 can end uncertified: then an error.
-e2e_status truncated_svd(SvdWork& w, const double* X, int nws, int ncols, int r, const double* mean, double* C,
-                         double* M, double* svals, cudaStream_t st, int* enlarged) {
-  const int nsmall = std::min(nws, ncols);
-  int k = std::min(std::min(r + 10, kRrMaxK), nsmall), power = 2;
-  if (k < r) return fail(E2E_ERR_UNSUPPORTED, "n_modes above the range finder's 64 columns");
-  for (;;) {
-    bool ok = false;
-    e2e_status s = randomized_svd(w, X, nws, ncols, r, k, power, mean, C, M, svals, &ok, st);
-    if (s != E2E_OK) return s;
-    if (ok) return E2E_OK;
+// One matrix (X, mean, outputs as in `one.kind[0]`) whose first reduction did not
+// stand: twice the columns (up to 64 and the matrix's smaller side) and four
+// power iterations until it does.  When the columns span the whole smaller side
+// the residual is rounding only, so only n_modes above 54 on a matrix wider than
+// 64 can end uncertified: then an error.
+e2e_status enlarge_svd(RrBatch one, int k, double* Om, cudaStream_t st, int* enlarged) {
+  const int nws = one.nws, ncols = one.kind[0].ncols, nsmall = std::min(nws, ncols);
+  one.nb = 1;
+  for (bool first = true;; first = false) {
     const int k2 = std::min(std::min(2 * k, kRrMaxK), nsmall);
-    if (k2 == k && power >= 4)
+    if (k2 == k && !first)
       return fail(E2E_ERR_DEVICE, "rank reduction not certified with " + std::to_string(k) +
                                       " columns (|X - QQ^T X| above 1e-10 s_1)");
     ++*enlarged;
     k = k2;
-    power = 4;
+    DeviceScratch scratch(st);
+    double* work = nullptr;
+    CK(dalloc((void**)&work, sizeof(double) * rr_work_doubles(nws, ncols, k), st));
+    scratch.add(work);
+    rr_carve(&one.kind[0], nws, ncols, k, 1, work);
+    e2e_status s = randomized_svds(one, 1, 4, Om, st);
+    if (s != E2E_OK) return s;
+    double h[3];
+    CK(cudaMemcpyAsync(h, one.kind[0].scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(h + 2, one.kind[0].S, sizeof(double), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (rr_certified(h, h[2], nws)) return E2E_OK;
   }
 }
 
@@ -844,27 +936,21 @@ extern "C" e2e_status e2e_env_generate(const e2e_env_params* p, const int32_t* i
   CK(cudaMemcpyAsync(dvert, interp_vertices, sizeof(int32_t) * 3 * (size_t)G2, cudaMemcpyDefault, st));
   CK(cudaMemcpyAsync(dwgt, interp_weights, sizeof(double) * 3 * (size_t)G2, cudaMemcpyDefault, st));
 
-  // per-step matrices and the results of all steps
-  double *Xv, *Xp, *mv, *mp, *Cv, *Cp, *Mv, *Mp, *sv;
-  double* coarse;
-  float *yi, *phi_yi;
-  const int nb = 3 + 3 * r;
-  CK(dalloc((void**)&Xv, sizeof(double) * (size_t)nws * 2 * n, st));
-  scratch.add(Xv);
-  CK(dalloc((void**)&Xp, sizeof(double) * (size_t)nws * n, st));
-  scratch.add(Xp);
-  CK(dalloc((void**)&mv, sizeof(double) * 2 * (size_t)n, st));
-  scratch.add(mv);
-  CK(dalloc((void**)&mp, sizeof(double) * (size_t)n, st));
-  scratch.add(mp);
-  CK(dalloc((void**)&Cv, sizeof(double) * (size_t)nws * r, st));
-  scratch.add(Cv);
-  CK(dalloc((void**)&Cp, sizeof(double) * (size_t)nws * r, st));
-  scratch.add(Cp);
-  CK(dalloc((void**)&Mv, sizeof(double) * (size_t)r * 2 * n, st));
-  scratch.add(Mv);
-  CK(dalloc((void**)&Mp, sizeof(double) * (size_t)r * n, st));
-  scratch.add(Mp);
+  // a batch of steps: matrices, reductions' work, coefficients and modes
+  const int nb = 3 + 3 * r, nc2[2] = {2 * n, n};
+  int kk[2];
+  size_t step_doubles = 0;
+  for (int q = 0; q < 2; ++q) {
+    kk[q] = std::min(std::min(r + 10, kRrMaxK), std::min(nws, nc2[q]));
+    if (kk[q] < r) return fail(E2E_ERR_UNSUPPORTED, "n_modes above the range finder's 64 columns");
+    step_doubles += (size_t)nws * nc2[q] + nc2[q] + (size_t)nws * r + (size_t)r * nc2[q] + rr_work_doubles(nws, nc2[q], kk[q]);
+  }
+  const int batch = (int)std::min<size_t>((size_t)nt, std::max<size_t>(1, (size_t(2) << 30) / (8 * step_doubles)));
+  double *work, *Om, *sv, *coarse;
+  CK(dalloc((void**)&work, sizeof(double) * step_doubles * batch, st));
+  scratch.add(work);
+  CK(dalloc((void**)&Om, sizeof(double) * (size_t)2 * n * kRrMaxK, st));
+  scratch.add(Om);
   CK(dalloc((void**)&sv, sizeof(double) * 2 * (size_t)nt * r, st));
   scratch.add(sv);
   CK(dalloc((void**)&coarse, sizeof(double) * (size_t)nt * nb * n, st));
@@ -883,62 +969,65 @@ extern "C" e2e_status e2e_env_generate(const e2e_env_params* p, const int32_t* i
     CK(dalloc((void**)&o.mask, sizeof(int32_t) * (size_t)nt * G2, st));
     scratch.add(o.mask);
   }
-  yi = o.yi;
-  phi_yi = o.phi_yi;
-
-  // rank-reduction work space, sized for the wider (velocity) matrix and the
-  // largest range finder
-  SvdWork w;
-  {
-    w.kmax = kRrMaxK;
-    w.ncols_max = 2 * n;
-    const size_t kc = (size_t)w.ncols_max * w.kmax, ks = (size_t)nws * w.kmax, kk = (size_t)w.kmax * w.kmax;
-    double** wide[] = {&w.Om, &w.Z, &w.Bt, &w.Ub};
-    for (double** b : wide) {
-      CK(dalloc((void**)b, sizeof(double) * kc, st));
-      scratch.add(*b);
-    }
-    double** tall[] = {&w.Q, &w.L};
-    for (double** b : tall) {
-      CK(dalloc((void**)b, sizeof(double) * ks, st));
-      scratch.add(*b);
-    }
-    double** sq[] = {&w.R, &w.V, &w.U, &w.Vs};
-    for (double** b : sq) {
-      CK(dalloc((void**)b, sizeof(double) * kk, st));
-      scratch.add(*b);
-    }
-    CK(dalloc((void**)&w.S, sizeof(double) * w.kmax, st));
-    scratch.add(w.S);
-    CK(dalloc((void**)&w.P, sizeof(double) * kRrSegs * kc, st));
-    scratch.add(w.P);
-    w.part_cap = ((w.ncols_max + 127) / 128) * kRrSegs;
-    CK(dalloc((void**)&w.part, sizeof(double) * w.part_cap, st));
-    scratch.add(w.part);
-    CK(dalloc((void**)&w.scal, sizeof(double) * 2, st));
-    scratch.add(w.scal);
-    CK(dalloc((void**)&w.sweeps, sizeof(int), st));
-    scratch.add(w.sweeps);
-  }
   int enlarged = 0;
-
-  for (int t = 0; t < nt; ++t) {
-    RealArgs ra{g, nws, t, (double)t * p->dt, p->dxy, p->A, p->eps, p->w_lo, p->w_hi, p->wx, 0.5 * kPi, Xv, Xp};
+  for (int t0 = 0; t0 < nt; t0 += batch) {
+    const int nbt = std::min(batch, nt - t0);
+    RrBatch b{};
+    b.nb = nbt;
+    b.nws = nws;
+    b.r = r;
+    b.Om = Om;
+    double* p2 = work;
+    for (int q = 0; q < 2; ++q) {
+      RrKind& K = b.kind[q];
+      auto take = [&](size_t each) {
+        double* at = p2;
+        p2 += each * nbt;
+        return at;
+      };
+      K.X = take((size_t)nws * nc2[q]);
+      K.mean = take(nc2[q]);
+      K.C = take((size_t)nws * r);
+      K.M = take((size_t)r * nc2[q]);
+      p2 = rr_carve(&K, nws, nc2[q], kk[q], nbt, p2);
+      K.svals = sv + (size_t)(q * nt + t0) * r;
+    }
+    RealArgs ra{g, nws, t0, p->dt, p->dxy, p->A, p->eps, p->w_lo, p->w_hi, p->wx, 0.5 * kPi, b.kind[0].X, b.kind[1].X};
     const int64_t nr = (int64_t)nws * n;
-    k_env_realisations<<<(unsigned)((nr + 255) / 256), 256, 0, st>>>(ra);
+    k_env_realisations<<<dim3((unsigned)((nr + 255) / 256), (unsigned)nbt), 256, 0, st>>>(ra);
+    const unsigned cb = (unsigned)((2 * n + 127) / 128);
+    k_env_means<<<dim3(cb, 1, 2 * nbt), 128, 0, st>>>(b);
+    k_env_subtract<<<dim3(cb, (unsigned)std::min(nws, 64), 2 * nbt), 128, 0, st>>>(b);
     CK(cudaGetLastError());
-    k_env_center<<<(2 * n + 127) / 128, 128, 0, st>>>(Xv, nws, 2 * n, mv);
-    k_env_center<<<(n + 127) / 128, 128, 0, st>>>(Xp, nws, n, mp);
-    CK(cudaGetLastError());
-    e2e_status s = truncated_svd(w, Xv, nws, 2 * n, r, mv, Cv, Mv, sv + (int64_t)t * r, st, &enlarged);
+    e2e_status s = randomized_svds(b, 2 * nbt, 2, Om, st);
     if (s != E2E_OK) return s;
-    s = truncated_svd(w, Xp, nws, n, r, mp, Cp, Mp, sv + (int64_t)(nt + t) * r, st, &enlarged);
-    if (s != E2E_OK) return s;
+    // certificates of the batch: residual and mean norms, largest singular value
+    std::vector<double> scal[2], S[2];
+    for (int q = 0; q < 2; ++q) {
+      scal[q].resize(2 * (size_t)nbt);
+      S[q].resize((size_t)kk[q] * nbt);
+      CK(cudaMemcpyAsync(scal[q].data(), b.kind[q].scal, sizeof(double) * scal[q].size(), cudaMemcpyDeviceToHost, st));
+      CK(cudaMemcpyAsync(S[q].data(), b.kind[q].S, sizeof(double) * S[q].size(), cudaMemcpyDeviceToHost, st));
+    }
+    CK(cudaStreamSynchronize(st));
+    for (int q = 0; q < 2; ++q) {
+      for (int m = 0; m < nbt; ++m) {
+        if (rr_certified(&scal[q][2 * m], S[q][(size_t)kk[q] * m], nws)) continue;
+        RrBatch one = b;
+        RrKind& K = one.kind[0];
+        K = b.kind[q];
+        K.X += (int64_t)m * nws * nc2[q];
+        K.mean += (int64_t)m * nc2[q];
+        K.C += (int64_t)m * nws * r;
+        K.M += (int64_t)m * r * nc2[q];
+        K.svals += (int64_t)m * r;
+        s = enlarge_svd(one, kk[q], Om, st, &enlarged);
+        if (s != E2E_OK) return s;
+      }
+    }
     const int64_t ns = std::max<int64_t>((int64_t)nb * n, (int64_t)nws * r);
-    k_env_store<<<(unsigned)((ns + 255) / 256), 256, 0, st>>>(n, nws, r, mv, mp, Mv, Mp, Cv, Cp,
-                                                                coarse + (int64_t)t * nb * n,
-                                                                yi + (int64_t)t * nws * r,
-                                                                phi_yi + (int64_t)t * nws * r);
+    k_env_store<<<dim3((unsigned)((ns + 255) / 256), (unsigned)nbt), 256, 0, st>>>(
+        b, n, coarse + (int64_t)t0 * nb * n, o.yi + (int64_t)t0 * nws * r, o.phi_yi + (int64_t)t0 * nws * r);
     CK(cudaGetLastError());
   }
   unsigned int* derr = nullptr;
