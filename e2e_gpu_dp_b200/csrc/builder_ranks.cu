@@ -55,6 +55,7 @@ constexpr int kObsR = 10;         // obstacle bitmap radius around a cell
 constexpr int kObsRows = 2 * kObsR + 1;
 constexpr int kMaxCells = 32;     // cells of a CTA
 constexpr int kMaxTiles = 4;      // emission tiles of a CTA, one a warp
+constexpr int kRewardR = 6;       // reach of k_rank_rewards' tables around a cell
 
 // A cell of the CTA and its table
 struct __align__(16) CellTab {
@@ -198,6 +199,51 @@ __device__ __forceinline__ void land_any(const DevProblem& P, float F, float cs,
   else land_general(P, F, cs, sn, vx, vy, x, y, i2, j2);
 }
 
+// obstacle bits of the rows around the CTA's cells c0 .. c0 + n - 1 of layer T
+__device__ __forceinline__ void stage_obstacles(const RankArgs& K, int T, int g, int nc, int c0, int n, int i0, int j0,
+                                                uint32_t* orow) {
+  for (int e = threadIdx.x; e < n * kObsRows; e += kThreads) {
+    const int c = e / kObsRows, a = e - c * kObsRows - kObsR;
+    uint32_t bits = 0;
+    if (c0 + c < nc) {
+      int i = i0 + a, j = j0 + c;
+      for (; j >= g; j -= g) ++i;
+      if (i >= 0 && i < g) {
+        const uint32_t* row = K.obits + ((int64_t)T * g + i) * K.owords;
+        const int b = j - kObsR, w = b >> 5;
+        const uint32_t lo = w >= 0 ? __ldg(row + w) : 0u, hi = w + 1 < K.owords ? __ldg(row + w + 1) : 0u;
+        bits = __funnelshift_r(lo, hi, b & 31) & ((1u << kObsRows) - 1u);
+        if (a == 0) bits &= ~(1u << kObsR);  // the cell itself does not count
+      }
+    }
+    orow[e] = bits;
+  }
+}
+
+// reward of a sample of `cell` (speed F) that lands in (i2, j2) after k domain
+// clamps, no obstacle on its way: move() and transition_calc
+// (src/build_model.cu:291-354, :533), the additions in their order
+__device__ __forceinline__ float landing_reward(const BuildArgs& A, int T, bool late, bool rad, float F, int cell, int i2,
+                                                int j2, int k) {
+  const DevProblem& P = A.P;
+  const int64_t nc = (int64_t)P.g * P.g;
+  float r = 0.f;
+  for (; k > 0; --k) r += P.r_out;
+  if (i2 == 0 || i2 == P.g - 1 || j2 == 0 || j2 == P.g - 1) r += P.r_out;
+  if (is_terminal(P, i2, j2)) {
+    r += P.r_term;
+  } else {
+    if (late) r += 0.05 * P.r_out;
+  }
+  float rad1 = 0.f, rad2 = 0.f;
+  if (rad) {
+    rad1 = __ldg(A.F.s + (int64_t)T * nc + cell);
+    rad2 = __ldg(A.F.s + (int64_t)(T + 1) * nc + (int64_t)i2 * P.g + j2);
+  }
+  const float r_step = step_reward(P, F, rad1, rad2);
+  return r + r_step;
+}
+
 struct Smem {
   uint32_t* lut;     // the plan's words
   float* tab;        // 32 x 8 landing rewards
@@ -329,6 +375,12 @@ __device__ __forceinline__ void finish_tile(const BuildArgs& A, const RankArgs& 
       for (uint64_t m = nz; m; m &= m - 1) {
         const int b = __ffsll((long long)m) - 1;
         const int i2 = wi0 + (b >> 3), j2 = wj0 + (b & 7);
+        // k_rank_rewards: landings within its tables, none that the general
+        // builder takes out of the samples' order
+        if (K.seq_rewards) {
+          const int reach = min(P.del, kRewardR);
+          ok = ok && abs(i2 - i1) <= reach && abs(j2 - j1) <= reach;
+        }
         if (passes_obstacle(P, A.F.mask, T, S.orow + cl * kObsRows, i1, j1, i2 - i1, j2 - j1)) ovr |= 1ull << b;
       }
       // domain clamps of the samples in bins that no obstacle overrides: each adds
@@ -577,22 +629,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_build_ranks(BuildArgs A, RankAr
       S.md[c * NM + k] = make_float4(ui, ui, vi, vi);
     }
     const int i0 = c0 / g, j0 = c0 - i0 * g;
-    for (int e = tid; e < CT * kObsRows; e += kThreads) {
-      const int c = e / kObsRows, a = e - c * kObsRows - kObsR;
-      uint32_t bits = 0;
-      if (c0 + c < nc) {
-        int i = i0 + a, j = j0 + c;
-        for (; j >= g; j -= g) ++i;
-        if (i >= 0 && i < g) {
-          const uint32_t* row = K.obits + ((int64_t)T * g + i) * K.owords;
-          const int b = j - kObsR, w = b >> 5;
-          const uint32_t lo = w >= 0 ? __ldg(row + w) : 0u, hi = w + 1 < K.owords ? __ldg(row + w + 1) : 0u;
-          bits = __funnelshift_r(lo, hi, b & 31) & ((1u << kObsRows) - 1u);
-          if (a == 0) bits &= ~(1u << kObsR);  // the cell itself does not count
-        }
-      }
-      S.orow[e] = bits;
-    }
+    stage_obstacles(K, T, g, nc, c0, CT, i0, j0, S.orow);
     if (tid < CT) {
       CellTab& ct = S.cells[tid];
       int state = 1, i = i0, j = j0 + tid;
@@ -728,6 +765,209 @@ __global__ void __launch_bounds__(kThreads, 4) k_build_ranks(BuildArgs A, RankAr
   }
 }
 
+// Reward sums of the window rows in the order of their samples (K.seq_rewards):
+// for spacings other than one the general builder adds a row's rewards sample by
+// sample, which for rewards that are no small integers is not the sum of count x
+// reward.  Same tasks as k_build_ranks, after it: per chunk of realisations the
+// velocities of the CTA's cells, then a lane per row walks them: landing (the
+// packed snapping chain of k_build_tiles, its rounding constants scaled by the
+// spacing, a power of two, so it rounds as the reference's remainderf snapping),
+// reward by the landing's place (and number of clamps) in the cell's table, one
+// addition.  Bound by issue: 35 instructions a sample and row of 32 lanes, half of
+// them the walk itself.  120x120x40, 8 actions, 500 realisations, radiation
+// reward: 58.5 ms a call with the general builder (remainderf twice a sample and
+// the full expression again), 5.7 ms now (this kernel 3.3, k_build_ranks 1.4;
+// without tables for clamped samples 10.2).
+constexpr int kRewardSide = 2 * kRewardR + 1;
+constexpr int kRewardPlaces = kRewardSide * kRewardSide;
+constexpr int kRewardTable = 3 * kRewardPlaces;  // after 0, 1, 2 domain clamps
+constexpr int kRewardChunk = 64;
+constexpr int kVelStride = kRewardChunk + 2;
+constexpr uint32_t kNoReward = 0xffffffffu;  // table place not taken yet (no reward has these bits)
+
+// Reward of the landing at place `at` around cell (i1, j1) after k clamps (each adds
+// r_outbound first, unless an obstacle on the way overrides the reward).  Out of
+// line: taken once per place and cell, and inlined into the sample loop it costs
+// the loop its registers.
+__device__ __noinline__ float reward_at(const BuildArgs& A, int T, float F, const uint32_t* obs, int i1, int j1,
+                                        uint32_t at, int k) {
+  const DevProblem& P = A.P;
+  const int i2 = i1 + (int)(at / kRewardSide) - kRewardR, j2 = j1 + (int)(at % kRewardSide) - kRewardR;
+  if (i2 < 0 || i2 >= P.g || j2 < 0 || j2 >= P.g) return 0.f;  // (a row that is left to the general builder)
+  if (passes_obstacle(P, A.F.mask, T, obs, i1, j1, i2 - i1, j2 - j1)) return P.r_out;
+  return landing_reward(A, T, T > P.nt - 20, P.reward_type == 2 || P.reward_type == 3, F, i1 * P.g + j1, i2, j2, k);
+}
+
+template <int NM>
+__global__ void __launch_bounds__(kThreads, 6) k_rank_rewards(const __grid_constant__ BuildArgs A,
+                                                              const __grid_constant__ RankArgs K) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const DevProblem& P = A.P;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = P.g, nrz = P.nrzns, CT = 1 << K.cells_log2, nc = g * g;
+  const int cpw_log2 = 5 - A.lanes_log2;
+  float2* const vel = reinterpret_cast<float2*>(smem);               // CT x kVelStride
+  float2* const md = vel + CT * kVelStride;                          // CT x NM: (ui, vi)
+  float2* const uv = md + CT * NM;                                   // CT
+  float* const rew = reinterpret_cast<float*>(uv + CT);              // CT x speeds x kRewardTable
+  uint32_t* const orow = reinterpret_cast<uint32_t*>(rew + CT * K.nspeeds * kRewardTable);
+  const int tasks_per_layer = (nc + CT - 1) >> K.cells_log2;
+  int T = K.t0, chunk = (int)blockIdx.x;
+  for (;; chunk += (int)gridDim.x) {
+    while (chunk >= tasks_per_layer) {
+      chunk -= tasks_per_layer;
+      ++T;
+    }
+    if (T >= K.t1) break;
+    const int c0 = chunk << K.cells_log2, i0 = c0 / g, j0 = c0 - i0 * g;
+    __syncthreads();
+    for (int e = tid; e < CT * NM; e += kThreads) {
+      const int k = e >> K.cells_log2, c = e & (CT - 1);
+      float2 m = make_float2(0.f, 0.f);
+      if (k < P.nm && c0 + c < nc) {
+        m.x = __ldg(A.F.ui + ((int64_t)T * P.nm + k) * nc + c0 + c);
+        m.y = __ldg(A.F.vi + ((int64_t)T * P.nm + k) * nc + c0 + c);
+      }
+      md[c * NM + k] = m;
+    }
+    if (tid < CT && c0 + tid < nc)
+      uv[tid] = make_float2(__ldg(A.F.u + (int64_t)T * nc + c0 + tid), __ldg(A.F.v + (int64_t)T * nc + c0 + tid));
+    stage_obstacles(K, T, g, nc, c0, CT, i0, j0, orow);
+    __syncthreads();
+    // ---- rewards of unclamped landings around a cell -----------------------------
+    // A warp's own cells: the box that nearly every sample lands in is taken at
+    // once (lanes over its places), other places at their first use.
+    const int per_cell = K.nspeeds * kRewardTable;
+    for (int q = 0; q < (1 << cpw_log2); ++q) {
+      const int c = (warp << cpw_log2) + q;
+      if (c >= CT || c0 + c >= nc) break;  // whole warps
+      float* const t = rew + c * per_cell;
+      for (int e = lane; e < per_cell; e += 32) t[e] = __uint_as_float(kNoReward);
+      int i1 = i0, j1 = j0 + c;
+      for (; j1 >= g; j1 -= g) ++i1;
+      int lo[2], hi[2];
+#pragma unroll
+      for (int ax = 0; ax < 2; ++ax) {
+        float m = ax ? uv[c].y : uv[c].x, var = 0.f;
+#pragma unroll
+        for (int k = 0; k < NM; ++k) {
+          const float w = ax ? md[c * NM + k].y : md[c * NM + k].x;
+          const float2 st = __ldg(reinterpret_cast<const float2*>(K.ystat + (int64_t)T * 2 * NM) + k);
+          m = fmaf(w, st.x, m);
+          var = fmaf(w * w, st.y, var);
+        }
+        const float s = (ax ? K.sy : K.sx) * (1.0f / (1 << kRankFrac)), h = 3.0f * sqrtf(var) * fabsf(s);
+        lo[ax] = (int)floorf(fminf(fmaxf(K.a_min[ax] + m * s - h + 0.5f, -(float)kRewardR), (float)kRewardR));
+        hi[ax] = (int)floorf(fminf(fmaxf(K.a_max[ax] + m * s + h + 0.5f, -(float)kRewardR), (float)kRewardR));
+      }
+      const int w = hi[0] - lo[0] + 1, places = w * (hi[1] - lo[1] + 1);
+      __syncwarp();
+      for (int e = lane; e < places * K.nspeeds; e += 32) {
+        const int f = e / places, o = e - f * places, di = lo[1] + o / w, dj = lo[0] + o % w;
+        const uint32_t at = (uint32_t)((di + kRewardR) * kRewardSide + dj + kRewardR);
+        t[f * kRewardTable + at] = reward_at(A, T, P.ac_speed[f * K.nangles], orow + c * kObsRows, i1, j1, at, 0);
+      }
+    }
+    // ---- this lane's row --------------------------------------------------------
+    const int tile = warp, cl = (tile << cpw_log2) + (lane >> A.lanes_log2);
+    const int a = lane & ((1 << A.lanes_log2) - 1), aa = a < P.na ? a : 0;
+    const int cell = c0 + cl;
+    int i1 = i0, j1 = j0 + (cl < CT ? cl : 0);
+    for (; j1 >= g; j1 -= g) ++i1;
+    bool row = cl < CT && cell < nc && a < P.na;
+    row = row && !is_terminal(P, i1, j1) && __ldg(A.F.mask + (int64_t)T * nc + cell) != 1;
+    const float F = P.ac_speed[aa];
+    const float2 FF = make_float2(F, F), csn = make_float2(P.ac_cos[aa], P.ac_sin[aa]), dt2 = make_float2(P.dt, P.dt);
+    const float2 xy1 = make_float2(P.xs[row ? j1 : 0], P.ys[row ? g - 1 - i1 : 0]);
+    const float2 sgn = make_float2(1.0f, -1.0f), org = make_float2(-P.xs0, P.ysn);
+    const float2 half = make_float2(0.5f * P.Dj, 0.5f * P.Di);
+    const float2 big = make_float2(12582912.0f * P.Dj, 12582912.0f * P.Di);  // 1.5 * 2^23 cells
+    const float2 magic = make_float2(big.x - (float)(j1 - kRewardR) * P.Dj, big.y - (float)(i1 - kRewardR) * P.Di);
+    const uint32_t mx = __float_as_uint(big.x), my = __float_as_uint(big.y);
+    float* const rt = rew + (row ? cl * per_cell + (aa / K.nangles) * kRewardTable : 0);
+    const uint32_t rt_addr = (uint32_t)__cvta_generic_to_shared(rt);
+    // cells whose samples can reach the domain's clamps (a landing beyond the
+    // tables' reach is not this kernel's)
+    const bool edge = __any_sync(0xffffffffu, row && (i1 <= kRewardR + 1 || j1 <= kRewardR + 1 || i1 >= g - 2 - kRewardR ||
+                                                      j1 >= g - 2 - kRewardR));
+    float sum = 0.f;
+    auto place = [&](float2 d) -> uint32_t {
+      const float2 t = __fadd2_rd(__fadd2_rd(d, half), magic);
+      const uint32_t at = (__float_as_uint(t.y) - my) * (uint32_t)kRewardSide + (__float_as_uint(t.x) - mx);
+      return min(at, (uint32_t)(kRewardPlaces - 1));  // (rows that are left to the general builder land anywhere)
+    };
+    const uint32_t* const obs = orow + cl * kObsRows;
+    // the rewards of up to four landings (at: clamps * kRewardPlaces + place), in
+    // order, onto the sum
+    auto take = [&](const uint32_t (&at)[4], int n) {
+      float r[4];
+      bool all = true;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(r[i]) : "r"(rt_addr + (at[i] << 2)) : "memory");
+        all = all && __float_as_uint(r[i]) != kNoReward;
+      }
+      if (!all) {
+        for (int i = 0; i < 4; ++i) {
+          if (__float_as_uint(r[i]) != kNoReward) continue;
+          r[i] = reward_at(A, T, F, obs, i1, j1, at[i] % kRewardPlaces, (int)(at[i] / kRewardPlaces));
+          rt[at[i]] = r[i];  // (lanes that meet here write the same value)
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i < n) sum += r[i];
+    };
+    const float* yt = K.yt + (int64_t)T * NM * K.nrp;
+    for (int base = 0; base < nrz; base += kRewardChunk) {
+      const int clen = min(kRewardChunk, nrz - base);
+      __syncthreads();  // tables in place; the chunk before is consumed
+      {
+        const int q = tid & (kRewardChunk - 1);
+        float y[NM];
+#pragma unroll
+        for (int k = 0; k < NM; ++k) y[k] = __ldg(yt + (int64_t)k * K.nrp + base + q);  // (rows are padded)
+        for (int c = tid / kRewardChunk; c < CT; c += kThreads / kRewardChunk) {
+          float2 s = md[c * NM];
+          s = make_float2(s.x * y[0], s.y * y[0]);
+#pragma unroll
+          for (int k = 1; k < NM; ++k) s = __ffma2_rn(md[c * NM + k], make_float2(y[k], y[k]), s);
+          vel[c * kVelStride + q] = make_float2(uv[c].x + s.x, uv[c].y + s.y);
+        }
+      }
+      __syncthreads();
+      if (row) {
+        const float2* v = vel + cl * kVelStride;
+        for (int q = 0; q < clen; q += 4) {  // (a velocity row holds two more than a chunk, and clen's rest is not added)
+          const float4 w0 = *reinterpret_cast<const float4*>(v + q), w1 = *reinterpret_cast<const float4*>(v + q + 2);
+          const float2 vv[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y),
+                                make_float2(w1.z, w1.w)};
+          uint32_t at[4];
+          if (!edge) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) at[i] = place(__ffma2_rn(advect2(FF, csn, vv[i], dt2, xy1), sgn, org));
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float2 xy = advect2(FF, csn, vv[i], dt2, xy1);
+              const float2 d = __ffma2_rn(xy, sgn, org);
+              at[i] = place(make_float2(fminf(fmaxf(d.x, 0.0f), P.axmax), fminf(fmaxf(d.y, 0.0f), P.aymax)));
+              at[i] += (xy.x > P.xsn || xy.x < P.xs0) ? kRewardPlaces : 0;
+              at[i] += (xy.y > P.ysn || xy.y < P.ys0) ? kRewardPlaces : 0;
+            }
+          }
+          take(at, clen - q);
+        }
+      }
+    }
+    if (row) {
+      const int64_t grow = ((int64_t)T * nc + cell) * P.na + a;
+      A.R[grow] = sum / P.nrzns;
+      if (A.sumR) A.sumR[grow] = sum;
+    }
+  }
+}
+
 // Per layer [t0, t1): the coefficients mode-major with rows padded to nrp (so a
 // lane reads four realisations at once), their mean and variance per mode (the
 // tables' ranges), and a bit per cell for the obstacles at T or T + 1.
@@ -806,6 +1046,14 @@ cudaError_t dispatch_nm(int nmp, F&& f) {
 
 constexpr size_t kSmemPerCta = 55 * 1024;  // four CTAs an SM
 
+constexpr size_t kRewardSmem = 48 * 1024;  // k_rank_rewards: no opt-in needed
+
+size_t reward_smem_bytes(const RankArgs& K, int nmp) {
+  const size_t ct = (size_t)1 << K.cells_log2;
+  return ct * (sizeof(float2) * (kVelStride + nmp + 1) + sizeof(float) * K.nspeeds * kRewardTable +
+               sizeof(uint32_t) * kObsRows);
+}
+
 }  // namespace
 
 int rank_padded_modes(int nm) { return nm <= 2 ? 2 : (nm + 1) & ~1; }
@@ -820,6 +1068,7 @@ bool rank_shape(int nm, int slots_log2, int lanes_log2, int nrzns, RankArgs* K) 
   const size_t fixed = smem_fixed_bytes(slots_log2, nmp, cells);
   if (fixed + 16 * 1024 > kSmemPerCta) return false;
   K->pool_words = (int)((kSmemPerCta - fixed) / 4) & ~3;
+  if (K->seq_rewards && reward_smem_bytes(*K, nmp) > kRewardSmem) return false;
   K->nrp = (nrzns + 127) / 128 * 128;
   K->nblocks = K->nrp / 128;
   // subsets of the cells: a warp's work item is 128 realisations x one subset.
@@ -868,6 +1117,10 @@ cudaError_t launch_build_ranks(const BuildArgs& A, const RankArgs& K, cudaStream
       }
     }
     kern<<<grid, kThreads, sm, st>>>(A, K);
+    cudaError_t e2 = cudaGetLastError();
+    if (e2 != cudaSuccess || !K.seq_rewards) return e2;
+    const size_t rb = reward_smem_bytes(K, nmp);  // (at most kRewardSmem: rank_shape)
+    k_rank_rewards<decltype(nm)::value><<<(unsigned)std::min<int64_t>(tasks, 8 * (int64_t)sms), kThreads, rb, st>>>(A, K);
     return cudaGetLastError();
   });
 }

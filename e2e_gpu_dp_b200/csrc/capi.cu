@@ -710,11 +710,13 @@ e2e_status plan_build(const e2e_problem* p, int count_bits, int64_t stage_hint, 
     host_actions(p, speed, angle);
     RankPlan rp;
     // Unit spacing: the general builder folds its rewards from the counts too.
-    // Other spacings: it adds them sample by sample, so only sums that do not
-    // depend on the order come from the counts.
+    // Other spacings: it adds them sample by sample, so sums that depend on the
+    // order are taken sample by sample here too.
     const bool unit_step = std::fabs(xs[1] - xs[0]) == 1.0f && std::fabs(ys[1] - ys[0]) == 1.0f;
-    if ((unit_step || order_free_rewards(p)) &&
-        make_rank_plan(p->gsize, pl->na, p->dt, speed, angle, xs, ys, &rp) &&
+    pl->rank.seq_rewards = !unit_step && !order_free_rewards(p);
+    pl->rank.nspeeds = p->num_ac_speeds;
+    pl->rank.nangles = p->num_ac_angles;
+    if (make_rank_plan(p->gsize, pl->na, p->dt, speed, angle, xs, ys, &rp) &&
         rank_shape(p->nmodes, rp.slots_log2, build_lanes_log2(pl->na), p->nrzns, &pl->rank)) {
       pl->ranked = true;
       pl->rank_words.swap(rp.words);
