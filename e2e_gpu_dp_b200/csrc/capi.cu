@@ -761,6 +761,8 @@ e2e_status plan_build(const e2e_problem* p, int count_bits, int64_t stage_hint, 
   }
   if (pl->tiles_per_layer > 0x7fffffff || p->nt - 1 > 65535)
     return fail(E2E_ERR_UNSUPPORTED, "grid too large for one launch");
+  // about a millisecond of the ranked builder, and more of the general one
+  pl->long_build = (double)pl->n_rows * p->nrzns > 4e9;
   pl->stage_cap = stage_hint > 0 ? stage_hint : pl->n_rows * 4 + 4096;
   pl->pool_units = std::min<int64_t>(std::max<int64_t>(pl->n_rows / 64, 256), 8192);
   return E2E_OK;
@@ -818,6 +820,9 @@ e2e_status copy_field_steps(const FieldsOnDevice& fd, int t0, int t1, cudaStream
   }
   return E2E_OK;
 }
+
+// host fields below this many bytes are uploaded before the builder starts
+constexpr size_t kUploadAtOnce = size_t(16) << 20;
 
 e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, cudaStream_t st, DeviceScratch* scratch,
                                LayerBuild* L) {
@@ -953,12 +958,17 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
     };
     CK(cudaEventRecord(ev[0], st));
     trace_mark("buffers");
-    if (attempt == 0 && fd.n_deferred) {
-      // host fields: copy the first layers' steps, then build them while the
-      // rest is copied on a second stream, then build the remaining layers
-      const int la = std::max(1, std::min(p->nt - 1, (p->nt - 1) / 16));
-      e2e_status cs = copy_field_steps(fd, 0, la + 1, st);
+    if (attempt == 0 && fd.n_deferred && fd.h2d_bytes < kUploadAtOnce) {
+      // small host fields: one copy and one launch (50x50x30, 4 MB: a second
+      // stream and launch cost 0.2 of 1.5 ms and hid nothing)
+      e2e_status cs = copy_field_steps(fd, 0, p->nt, st);
       if (cs != E2E_OK) return cs;
+      trace_mark("copies");
+      CK(build_layers(0, p->nt - 1));
+    } else if (attempt == 0 && fd.n_deferred) {
+      // host fields: a range of layers is built while the steps of the next one
+      // are copied on a second stream (1/16, 1/4, 1/2 and the whole of the layers:
+      // the copy of a range takes less than the build of the one before)
       cudaStream_t cps = nullptr;
       cudaEvent_t evs[2] = {nullptr, nullptr};
       struct CopyFree {
@@ -970,24 +980,26 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
           if (*s) cudaStreamDestroy(*s);
         }
       } cpfree{&cps, evs};
-      if (la < p->nt - 1) {
-        CK(cudaStreamCreateWithFlags(&cps, cudaStreamNonBlocking));
-        for (int k = 0; k < 2; ++k) CK(cudaEventCreateWithFlags(&evs[k], cudaEventDisableTiming));
-        // after the buffers exist (stream-ordered allocations) and the first
-        // steps are in, before the first launch, so the copy runs beside it
-        CK(cudaEventRecord(evs[0], st));
-        CK(cudaStreamWaitEvent(cps, evs[0], 0));
-        trace_mark("copy_stream");
-        cs = copy_field_steps(fd, la + 1, p->nt, cps);
+      const int layers = p->nt - 1, ends[4] = {std::max(1, layers / 16), layers / 4, layers / 2, layers};
+      int done = 0;
+      for (int k = 0; k < 4; ++k) {
+        const int end = ends[k];
+        if (end <= done) continue;
+        e2e_status cs = copy_field_steps(fd, done ? done + 1 : 0, end + 1, done ? cps : st);
         if (cs != E2E_OK) return cs;
-        CK(cudaEventRecord(evs[1], cps));
-        trace_mark("copies");
-      }
-      CK(build_layers(0, la));
-      trace_mark("first_layers");
-      if (la < p->nt - 1) {
-        CK(cudaStreamWaitEvent(st, evs[1], 0));
-        CK(build_layers(la, p->nt - 1));
+        if (done) {
+          CK(cudaEventRecord(evs[1], cps));
+          CK(cudaStreamWaitEvent(st, evs[1], 0));
+        } else {
+          CK(cudaStreamCreateWithFlags(&cps, cudaStreamNonBlocking));
+          for (int q = 0; q < 2; ++q) CK(cudaEventCreateWithFlags(&evs[q], cudaEventDisableTiming));
+          // after the buffers exist (stream-ordered allocations) and the first
+          // steps are in, before the first launch, so the copies run beside it
+          CK(cudaEventRecord(evs[0], st));
+          CK(cudaStreamWaitEvent(cps, evs[0], 0));
+        }
+        CK(build_layers(done, end));
+        done = end;
       }
     } else {
       CK(build_layers(0, p->nt - 1));
@@ -996,9 +1008,10 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
     trace_mark("launch");
     CK(cudaEventRecord(ev[1], st));
     trace_mark("record");
-    // sleep through the builder; the counters' copy into host (stack) memory
-    // would otherwise spin until it finishes
-    CK(sleep_sync(st));
+    // sleep through a long builder launch; the counters' copy into host (stack)
+    // memory would otherwise spin until it finishes.  A short one is spun
+    // through: being woken takes longer than it runs.
+    if (pl.long_build) CK(sleep_sync(st));
     trace_mark("build");
     CK(cudaMemcpyAsync(hc, ctr, sizeof(hc), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -1041,6 +1054,7 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
   m->misbinned = hc[CTR_MISBIN];
   m->overflow_rows = hc[CTR_OVERFLOW_ROWS];
   m->layered = true;
+  m->built = true;
   m->prob = *p;
   m->has_prob = true;
   const int pb = m->index_bits == 32 ? 4 : 8;
@@ -1162,7 +1176,7 @@ extern "C" e2e_status e2e_model_copy_to_host(const e2e_model* m, int64_t* row_pt
 namespace e2e {
 
 // The sliced copy of the model that the sweeps stream (built once per model).
-e2e_status ensure_pack(const e2e_model* m, double* pack_ms, cudaStream_t st) {
+e2e_status ensure_pack(const e2e_model* m, double* pack_ms, cudaStream_t st, PackTimer* timer) {
   *pack_ms = 0.0;
   if (m->pack) return E2E_OK;
   const ViModel M = vi_model(m);
@@ -1171,26 +1185,21 @@ e2e_status ensure_pack(const e2e_model* m, double* pack_ms, cudaStream_t st) {
   const int g = geo ? m->prob.gsize : 0;
   const int del = geo ? (m->prob.neighb_gsize - 1) / 2 : 0;
   const int64_t nc = m->layered ? m->ncells : 0;
-  cudaEvent_t e0, e1;
-  CK(cudaEventCreate(&e0));
-  CK(cudaEventCreate(&e1));
-  struct EvGuard {
-    cudaEvent_t a, b;
-    ~EvGuard() { cudaEventDestroy(a); cudaEventDestroy(b); }
-  } evg{e0, e1};
+  PackTimer own, *tm = timer ? timer : &own;
+  for (cudaEvent_t& e : tm->ev) CK(cudaEventCreate(&e));
   auto* ps = new PackStore();
-  CK(cudaEventRecord(e0, st));
-  cudaError_t e = build_pack(M, nc, g, del, ps, st);
+  CK(cudaEventRecord(tm->ev[0], st));
+  cudaError_t e = build_pack(M, nc, g, del, m->built, ps, st);
   if (e != cudaSuccess) {
     free_pack(ps);
     delete ps;
     return cuda_fail(e, "build_pack");
   }
-  CK(cudaEventRecord(e1, st));
-  CK(cudaEventSynchronize(e1));
-  float ms = 0.f;
-  CK(cudaEventElapsedTime(&ms, e0, e1));
-  *pack_ms = ms;
+  CK(cudaEventRecord(tm->ev[1], st));
+  if (!timer) {  // else the caller reads the time behind its own synchronisation
+    CK(cudaEventSynchronize(tm->ev[1]));
+    CK(tm->read(pack_ms));
+  }
   m->pack = ps;
   return E2E_OK;
 }
@@ -1327,8 +1336,9 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
     if (done || js != E2E_OK) return js;
   }
   double pack_ms = 0.0;
+  PackTimer pack_timer;
   {
-    e2e_status ps = ensure_pack(m, &pack_ms, st);
+    e2e_status ps = ensure_pack(m, &pack_ms, st, &pack_timer);
     if (ps != E2E_OK) return ps;
   }
   trace_mark("pack");
@@ -1342,8 +1352,10 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
   CK(dalloc((void**)&resid, sizeof(unsigned long long) * (size_t)(max_iter + 3), st));
   scratch.add(resid);
   CK(cudaMemsetAsync(resid, 0, sizeof(unsigned long long) * (size_t)(max_iter + 3), st));
-  // last slot: barrier count and error bits of the persistent layered sweep
-  unsigned int* syncw = reinterpret_cast<unsigned int*>(resid + max_iter + 2);
+  // first slot: barrier count and error bits of the persistent layered sweep
+  unsigned int* syncw = reinterpret_cast<unsigned int*>(resid);
+  ++resid;
+  unsigned int herr = 0;
   cudaEvent_t e0, e1, e2;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -1359,8 +1371,10 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
   const int64_t sweep_bytes = csr_sweep_bytes(m);
   CK(cudaEventRecord(e0, st));
   if (o.method == 1) {
-    if (!m->layered || m->ncells <= 0 || m->nt <= 0 || P.nlayers < 2)
+    if (!m->layered || m->ncells <= 0 || m->nt <= 0 || P.nlayers < 2) {
+      CK(cudaStreamSynchronize(st));  // the sliced copy, which stays with the model, is complete
       return fail(E2E_ERR_UNSUPPORTED, "layered solve needs a time-layered model (nt, ncells known)");
+    }
     // all layers, last first, in one cooperative launch
     CK(launch_vi_layered(P, dV, dpi, syncw, gsel, st, tune_layered));
     CK(cudaEventRecord(e2, st));
@@ -1370,11 +1384,12 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
     CK(dalloc((void**)&pi2, sizeof(int32_t) * (size_t)ns, st));
     scratch.add(pi2);
     CK(launch_vi_chunks(P, 0, P.nchunks, dV, W, pi2, resid, st, tune_jacobi, syncw + 1));
-    unsigned long long h = 0;
-    CK(cudaMemcpyAsync(&h, resid, sizeof(h), cudaMemcpyDeviceToHost, st));
+    unsigned long long h[2] = {0, 0};  // the error bits, the residual
     CK(cudaEventRecord(e1, st));
+    CK(cudaMemcpyAsync(h, resid - 1, sizeof(h), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    std::memcpy(&last_res, &h, sizeof(double));
+    herr = (unsigned int)(h[0] >> 32);
+    std::memcpy(&last_res, &h[1], sizeof(double));
     iters = 2;
   } else {
     float* a = dV;
@@ -1412,12 +1427,12 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
       return fail(E2E_ERR_NOT_CONVERGED, "max_iter reached before the threshold");
     }
   }
-  {
-    unsigned int herr = 0;
+  if (o.method == 0) {
     CK(cudaMemcpyAsync(&herr, syncw + 1, sizeof(herr), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (herr) return fail(E2E_ERR_DEVICE, "a bounded device-side wait of the sweep gave up");
   }
+  if (herr) return fail(E2E_ERR_DEVICE, "a bounded device-side wait of the sweep gave up");
+  CK(pack_timer.read(&pack_ms));
   float ms = 0.f, ms_pass = 0.f;
   CK(cudaEventElapsedTime(&ms, e0, e1));
   if (layered_pass) CK(cudaEventElapsedTime(&ms_pass, e0, e2));

@@ -237,9 +237,9 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
       CK(launch_layers(A, pl, L, t0, t1, st));
       CK(launch_leftover(A, pl, L, t0, t1, st));
       ++launches;
-      // sleep through the block, then read its counters and the error word of the
+      // sleep through a long block, then read its counters and the error word of the
       // backup before it
-      CK(sleep_sync(st));
+      if (pl.long_build) CK(sleep_sync(st));
       CK(cudaMemcpyAsync(hc, b ? bc - 1 : bc, sizeof(unsigned long long) * (CTR_COUNT + (b ? 1 : 0)),
                          cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));

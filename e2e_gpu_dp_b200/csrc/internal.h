@@ -26,6 +26,7 @@ struct e2e_model {
   uint64_t dropped = 0, misbinned = 0, overflow_rows = 0;
   double build_kernel_ms = 0, assemble_ms = 0;
   int32_t build_launches = 0;
+  bool built = false;        // by this library: every next state lies in its row's m x m window
   bool layered = false;      // every transition of a layer-t state leads into layer t+1
   e2e_problem prob{};
   bool has_prob = false;
@@ -92,6 +93,7 @@ struct BuildPlan {
   bool ranked = false;     // the builder by velocity ranks takes the problem
   RankArgs rank{};         // its launch shape (pointers set by run_build)
   std::vector<uint32_t> rank_words;
+  bool long_build = true;  // worth sleeping through
   bool keep_sums = false;  // keep per-row reward sums (e2e_build_opts.keep_reward_parts)
 };
 
@@ -140,8 +142,27 @@ void free_model_buffers(e2e_model* m);
 int64_t model_bytes(const e2e_model* m);
 e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, int32_t* dpi,
                            e2e_vi_stats* stats, cudaStream_t st);
-// build the model's sliced copy for the sweeps if it has none yet
-e2e_status ensure_pack(const e2e_model* m, double* pack_ms, cudaStream_t st);
+// Device time between two events of a call that ran, once the stream is done
+struct PackTimer {
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  PackTimer() = default;
+  PackTimer(const PackTimer&) = delete;
+  PackTimer& operator=(const PackTimer&) = delete;
+  ~PackTimer() {
+    for (cudaEvent_t e : ev)
+      if (e) cudaEventDestroy(e);
+  }
+  cudaError_t read(double* out) const {
+    if (!ev[1]) return cudaSuccess;
+    float v = 0.f;
+    cudaError_t e = cudaEventElapsedTime(&v, ev[0], ev[1]);
+    if (e == cudaSuccess) *out = v;
+    return e;
+  }
+};
+// Build the model's sliced copy for the sweeps if it has none yet.  With a timer
+// the call does not wait for the copy: the caller reads the time later.
+e2e_status ensure_pack(const e2e_model* m, double* pack_ms, cudaStream_t st, PackTimer* timer = nullptr);
 
 // One layered solve of a batch: a model, its outputs and, for a served
 // request, the re-targeted R around its target (ViJob fields).

@@ -176,8 +176,9 @@ struct PackStore {
 
 // Build the sliced copy of a state-major CSR model.  nc = states per layer
 // (0: none); g, del = grid side and window half-width of a layered model built
-// on a g x g grid (0: unknown, int32 columns).
-cudaError_t build_pack(const ViModel& M, int64_t nc, int g, int del, PackStore* out, cudaStream_t st);
+// on a g x g grid (0: unknown, int32 columns).  in_window: every column is known to
+// lie in its row's window (models of the builder), which is then not checked.
+cudaError_t build_pack(const ViModel& M, int64_t nc, int g, int del, bool in_window, PackStore* out, cudaStream_t st);
 void free_pack(PackStore* p);
 // bytes one sweep over the pack moves (entries with padding, R, tables, V)
 int64_t pack_sweep_bytes(const ViPack& P);

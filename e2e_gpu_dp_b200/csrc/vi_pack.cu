@@ -947,7 +947,7 @@ int64_t pack_sweep_bytes(const ViPack& P) {
          P.nchunks * (8 + P.na_pad * 2) + P.ns * 12;
 }
 
-cudaError_t build_pack(const ViModel& M, int64_t nc, int g, int del, PackStore* out, cudaStream_t st) {
+cudaError_t build_pack(const ViModel& M, int64_t nc, int g, int del, bool in_window, PackStore* out, cudaStream_t st) {
   *out = PackStore{};
   ViPack& P = out->v;
   P.ns = M.ns;
@@ -1025,6 +1025,7 @@ cudaError_t build_pack(const ViModel& M, int64_t nc, int g, int del, PackStore* 
       return cudaGetLastError();
     });
     if (e != cudaSuccess) return cleanup(), e;
+    if (in_window || P.ent_mode == ENT_I32) break;
     unsigned int hf = 0;
     if ((e = cudaMemcpyAsync(&hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
       return cleanup(), e;
