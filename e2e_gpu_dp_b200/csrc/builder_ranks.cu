@@ -21,14 +21,14 @@
 // k_build_tiles.
 //
 // Measured on B200 (whole call, counting loops -> ranks): 200x200x120, 16
-// actions, 5000 realisations 330.6 -> 66.2 ms; 300x300x40, 2000 realisations
+// actions, 5000 realisations 330.6 -> 63 ms; 300x300x40, 2000 realisations
 // 102.3 -> 24.4 ms; 137x137x53, 24 actions, 777 realisations 29.7 -> 8.8 ms.
-// Of the 14.3 ms of 200x200x30 the counting takes 10.5 ms (shared-memory
+// Of the 13.8 ms of 200x200x30 the counting takes about 10 ms (shared-memory
 // wavefronts and issue slots both at about half of their peaks), staging 0.9,
-// the prefix sums 0.5, the rows 2.4.  Four CTAs of 4 warps an SM: one CTA's
-// staging and rows run beside the others' counting (two of 8 warps: 16.8 ms);
-// the table reads of a lane's four samples before their increments: 15.5 ->
-// 14.3 ms.
+// the prefix sums 0.5, the rows 2.4.  Four or five CTAs of 4 warps an SM: one
+// CTA's staging and rows run beside the others' counting (two of 8 warps: 16.8
+// ms, four of 4: 14.3); the table reads of a lane's four samples before their
+// increments: 15.5 -> 14.3 ms.
 //
 // A CTA (4 warps) takes a run of cells of one layer, 128 rows where the action
 // count allows it.  A warp holds the coefficients of 128 realisations (4 a
@@ -47,7 +47,7 @@ namespace e2e {
 
 namespace {
 
-constexpr int kThreads = 128;     // 4 CTAs an SM: one CTA's set-up and rows overlap the others' counting
+constexpr int kThreads = 128;     // 4 or 5 CTAs an SM: one CTA's set-up and rows overlap the others' counting
 constexpr int kWarps = kThreads / 32;
 constexpr int kWin = 8;           // window side, as k_build_tiles
 constexpr int kListPool = 384;    // samples on the lists of a CTA's cells
@@ -555,7 +555,7 @@ __device__ __forceinline__ void cell_axis(const RankArgs& K, const uint32_t* pla
 }
 
 template <int NM>
-__global__ void __launch_bounds__(kThreads, 4) k_build_ranks(BuildArgs A, RankArgs K) {
+__global__ void __launch_bounds__(kThreads, 5) k_build_ranks(BuildArgs A, RankArgs K) {
   extern __shared__ __align__(16) unsigned char smem[];
   const DevProblem& P = A.P;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1044,7 +1044,13 @@ cudaError_t dispatch_nm(int nmp, F&& f) {
   return cudaErrorInvalidValue;
 }
 
-constexpr size_t kSmemPerCta = 55 * 1024;  // four CTAs an SM
+// Shared memory of a CTA where four or five of them share an SM.  Five wherever
+// the pool then still holds the widest tables of a tile of inner cells (ranges
+// of 2 x kRankMaxHalfRange cells), else its cells would go to the general
+// builder: 200x200x30, 10 modes, 5000 realisations 14.5 -> 13.8 ms; 8 modes, 2000
+// 7.54 -> 7.30, 1000 5.73 -> 5.77; 8 actions, 4 modes, 1280 3.83 -> 3.56; six
+// CTAs 14.0, 7.70, 6.30, 3.50.
+constexpr size_t kSmem4 = 55 * 1024, kSmem5 = 44 * 1024;
 
 constexpr size_t kRewardSmem = 48 * 1024;  // k_rank_rewards: no opt-in needed
 
@@ -1066,8 +1072,12 @@ bool rank_shape(int nm, int slots_log2, int lanes_log2, int nrzns, RankArgs* K) 
   K->cells_log2 = std::min(5, 7 - lanes_log2);
   const int cells = 1 << K->cells_log2;
   const size_t fixed = smem_fixed_bytes(slots_log2, nmp, cells);
-  if (fixed + 16 * 1024 > kSmemPerCta) return false;
-  K->pool_words = (int)((kSmemPerCta - fixed) / 4) & ~3;
+  if (fixed + 16 * 1024 > kSmem4) return false;
+  const float width = 2.0f * kRankMaxHalfRange;
+  const int nx = (int)(width * K->groups[RANK_X]) + 3, ny = (int)(width * K->groups[RANK_Y]) + 3;
+  const size_t widest = sizeof(uint32_t) * (((size_t)32 >> lanes_log2) * ((nx + 1) | 1) * (ny + 1) + 8);
+  K->ctas_per_sm = fixed + widest <= kSmem5 ? 5 : 4;
+  K->pool_words = (int)(((K->ctas_per_sm == 5 ? kSmem5 : kSmem4) - fixed) / 4) & ~3;
   if (K->seq_rewards && reward_smem_bytes(*K, nmp) > kRewardSmem) return false;
   K->nrp = (nrzns + 127) / 128 * 128;
   K->nblocks = K->nrp / 128;
@@ -1104,14 +1114,14 @@ cudaError_t launch_build_ranks(const BuildArgs& A, const RankArgs& K, cudaStream
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   const int64_t nc = (int64_t)A.P.g * A.P.g;
   const int64_t tasks = (int64_t)(K.t1 - K.t0) * ((nc + (1 << K.cells_log2) - 1) >> K.cells_log2);
-  const unsigned grid = (unsigned)std::min<int64_t>(tasks, 4 * (int64_t)sms);
+  const unsigned grid = (unsigned)std::min<int64_t>(tasks, K.ctas_per_sm * (int64_t)sms);
   if (grid == 0) return cudaSuccess;
   return dispatch_nm(nmp, [&](auto nm) -> cudaError_t {
     auto kern = k_build_ranks<decltype(nm)::value>;
     {
       std::lock_guard<std::mutex> lk(g_cap_mu);
       if (dev < 0 || dev >= 64 || !g_cap_set[dev][nmp / 2]) {
-        cudaError_t e2 = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemPerCta);
+        cudaError_t e2 = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem4);
         if (e2 != cudaSuccess) return e2;
         if (dev >= 0 && dev < 64) g_cap_set[dev][nmp / 2] = true;
       }

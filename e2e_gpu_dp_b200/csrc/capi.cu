@@ -716,8 +716,9 @@ e2e_status plan_build(const e2e_problem* p, int count_bits, int64_t stage_hint, 
     pl->rank.seq_rewards = !unit_step && !order_free_rewards(p);
     pl->rank.nspeeds = p->num_ac_speeds;
     pl->rank.nangles = p->num_ac_angles;
-    if (make_rank_plan(p->gsize, pl->na, p->dt, speed, angle, xs, ys, &rp) &&
-        rank_shape(p->nmodes, rp.slots_log2, build_lanes_log2(pl->na), p->nrzns, &pl->rank)) {
+    const bool planned = make_rank_plan(p->gsize, pl->na, p->dt, speed, angle, xs, ys, &rp);
+    for (int k = 0; k < 4; ++k) pl->rank.groups[k] = rp.groups[k];
+    if (planned && rank_shape(p->nmodes, rp.slots_log2, build_lanes_log2(pl->na), p->nrzns, &pl->rank)) {
       pl->ranked = true;
       pl->rank_words.swap(rp.words);
       RankArgs& K = pl->rank;
@@ -725,7 +726,6 @@ e2e_status plan_build(const e2e_problem* p, int count_bits, int64_t stage_hint, 
       K.shift = rp.shift;
       K.sx = rp.sx;
       K.sy = rp.sy;
-      for (int k = 0; k < 4; ++k) K.groups[k] = rp.groups[k];
       for (int k = 0; k < 2; ++k) {
         K.a_min[k] = (float)rp.a_min[k];
         K.a_max[k] = (float)rp.a_max[k];

@@ -79,6 +79,7 @@ struct RankArgs {
   int nblocks, nsub_log2;    // 128-realisation blocks; subsets of a CTA's cells
   int cells_log2;            // cells of a CTA
   int pool_words;            // shared words for its rank tables
+  int ctas_per_sm;           // 4 or 5, by the tables' size
   int seq_rewards;           // reward sums sample by sample (k_rank_rewards)
   int nspeeds, nangles;      // actions = nspeeds x nangles
   float stay_sum;            // r_outbound added once per realisation: an obstacle cell's reward sum
@@ -87,7 +88,7 @@ struct RankArgs {
   int64_t etiles_per_layer;
 };
 int rank_padded_modes(int nm);
-// launch shape for nm modes and a plan (K->seq_rewards, nspeeds set); false when
+// launch shape for nm modes and a plan (K->seq_rewards, nspeeds, groups set); false when
 // the kernels do not take it
 bool rank_shape(int nm, int slots_log2, int lanes_log2, int nrzns, RankArgs* K);
 // fills yt, ystat, obits of layers [K.t0, K.t1)
