@@ -1325,10 +1325,10 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
   if ((o.schedule & ~0x1ff) || (gsel != 0 && gsel != 1 && gsel != 2 && gsel != 4 && gsel != 8))
     return fail(E2E_ERR_INVALID,
                 "schedule: bits 0-3 warps per chunk (0, 1, 2, 4, 8), bits 4-7 sweep tuning, bit 8 tuning given");
-  // sweep tuning: given, or the defaults measured on B200 (layered: look-ahead
-  // kernel, next layer's chunks prefetched into L2; Jacobi: lean kernel)
+  // sweep tuning: given, or the defaults measured on B200 (layered: -1, chosen at
+  // the launch; Jacobi: lean kernel)
   const bool tune_given = (o.schedule & 0x100) != 0;
-  const int tune_layered = tune_given ? (o.schedule >> 4) & 15 : VI_TUNE_PF_NEXT;
+  const int tune_layered = tune_given ? (o.schedule >> 4) & 15 : -1;
   const int tune_jacobi = tune_given ? (o.schedule >> 4) & 15 : VI_TUNE_LEAN;
   if (o.method == 0 && !tune_given) {
     bool done = false;

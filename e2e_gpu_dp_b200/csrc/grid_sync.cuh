@@ -42,6 +42,26 @@ __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
   return v;
 }
 
+// orders the CTA's earlier writes (behind a __syncthreads) before the count;
+// against a fence and an addition 0.3 us less a barrier
+__device__ __forceinline__ void add_release(unsigned int* p, unsigned int n) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(n) : "memory");
+}
+
+// The limits of one wait.  The clock is read on every 32nd poll only: the read
+// takes longer than a wait that is about to end.
+struct WaitClock {
+  static constexpr int kEvery = 32;
+  long long polls = 0;
+  unsigned long long t0 = 0;
+  __device__ __forceinline__ bool over(const WaitBound& wb) {
+    if (++polls % kEvery) return false;
+    const unsigned long long now = global_ns();
+    if (t0 == 0) t0 = now;
+    return polls > wb.spins || now - t0 > wb.timeout_ns;
+  }
+};
+
 // Grid-wide barrier of a cooperative launch.  sync[0] counts arrivals (never
 // reset inside a launch); a wait that outlives its limit sets bit 1 of sync[1]
 // and every later barrier returns false at once.
@@ -50,19 +70,15 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* sync, unsigned int ta
   __syncthreads();
   if (threadIdx.x == 0) {
     int good = 1;
-    __threadfence();
-    atomicAdd(sync, 1u);
-    const unsigned long long t0 = global_ns();
-    long long it = 0;
+    add_release(sync, 1u);
+    WaitClock clock;
     while (ld_acquire(sync) < target + wb.extra) {
-      if (ld_acquire(sync + 1) != 0u || ++it > wb.spins || global_ns() - t0 > wb.timeout_ns) {
+      if (clock.over(wb) || (clock.polls % WaitClock::kEvery == 0 && ld_acquire(sync + 1) != 0u)) {
         atomicOr(sync + 1, 2u);
         good = 0;
         break;
       }
-      __nanosleep(32);
     }
-    __threadfence();
     ok = good;
   }
   __syncthreads();

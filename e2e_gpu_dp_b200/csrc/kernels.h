@@ -195,7 +195,8 @@ cudaError_t launch_vi_chunks(const ViPack& P, int64_t c_begin, int64_t c_end, co
                              int tune, unsigned int* err = nullptr);
 // The whole layered schedule in one cooperative launch, in place on V.
 // sync: two zeroed words (barrier count, error bits); groups: warps per chunk
-// (1, 2, 4, 8; 0 picks one).
+// (1, 2, 4, 8; 0 picks one); tune: the bits above, or -1 for the default schedule
+// (k_vi_ahead where it applies).
 cudaError_t launch_vi_layered(const ViPack& P, float* V, int32_t* pi, unsigned int* sync, int groups,
                               cudaStream_t st, int tune);
 

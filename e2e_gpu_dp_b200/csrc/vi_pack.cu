@@ -640,6 +640,199 @@ __global__ void __launch_bounds__(kThreads, MinBlocks<MODE, VAR>::value)
   }
 }
 
+// ---- the layered schedule, loads ahead of the barrier (packed layout) ---------------
+// A layer is a chain: the barrier behind the layer after it, its gathers, its
+// values.  k_vi_layered adds the chunk's slot, lengths, entries and R to that
+// chain, one load behind the other; none of them depends on values.  Here a warp
+// takes a few actions of a chunk and has their R, lengths and first 16 entries
+// in registers when the barrier opens (and has asked for the layer before in
+// L2); it then issues 16 gathers at once whatever the actions' lengths are.  One
+// CTA an SM, so that a barrier counts few arrivals; a CTA owns the same run of
+// chunks in every layer, whose gathers share lines.  The operations on a row are
+// those of k_vi_layered in the same order.
+//
+// Pass on B200, k_vi_layered -> this: 200x200x120, 16 actions, 500 realisations
+// 1203 -> 786 us (243 us of traffic at the copy rate); 300x300x40 633 -> 456;
+// 100x100x40, 32 actions 320 -> 207; 50x50x30, 8 actions 136 -> 97; 16x16x8 33 ->
+// 29.  A layer of one chunk a CTA takes 3.4 us: barrier, gather, sums in turn.
+// Entries staged in shared memory instead (cp.async, or bulk copies into a ring)
+// cost L1 the room that the gathers need: 955 and 1108 us.
+constexpr int kAhActions = 6;  // of a warp, at most
+constexpr int kAhWarps = 32;
+
+struct AheadShape {
+  int grid, teams, groups, rounds;  // a team of `groups` warps a chunk, rounds of `teams` chunks a layer
+  int actions;                      // of a warp
+};
+
+__device__ __forceinline__ void bar_named(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// the values of 8 entries, the first n of them of the warp's rows
+__device__ __forceinline__ void ahead_gather(const uint32_t* e, const float* vb, int n, float (&v)[8]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    v[j] = 0.f;
+    if (j < n) v[j] = ld_value<true>(vb + (e[j] & 0xffffu));
+  }
+}
+
+// ... and their part of the sums; bit j of ends: a row ends with entry j
+__device__ __forceinline__ void ahead_fold(const uint32_t* e, const float (&v)[8], int n, unsigned ends, float*& sum,
+                                           float& acc) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (j < n) acc = fmaf((float)(e[j] >> 16), v[j], acc);
+    if (ends >> j & 1u) {
+      *sum = acc;
+      sum += 32;
+      acc = 0.f;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(32 * kAhWarps, 1)
+    k_vi_ahead(ViPack P, AheadShape S, float* V, int32_t* pi, unsigned int* sync, WaitBound wb) {
+  __shared__ float sums[kAhWarps][kAhActions][32];
+  __shared__ float sq[2][kAhWarps][32];
+  __shared__ int sa[2][kAhWarps][32];
+  __shared__ int s_stop;
+  volatile int* stop = &s_stop;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int G = S.groups, team = wid / G, grp = wid - team * G;
+  const int cpl = (int)P.cpl, nc = (int)P.nc, na = P.na;
+  const int c0 = (int)((int64_t)cpl * blockIdx.x / gridDim.x), c1 = (int)((int64_t)cpl * (blockIdx.x + 1) / gridDim.x);
+  const int a0 = min(na, grp * S.actions), a1 = min(na, a0 + S.actions);
+  const uint32_t* const col = reinterpret_cast<const uint32_t*>(P.col);
+  if (threadIdx.x == 0) s_stop = 0;
+  __syncthreads();
+  unsigned gen = 0;
+  int it = 0;
+  for (int t = P.nlayers - 1; t >= 0; --t) {
+    for (int round = 0; round < S.rounds; ++round, ++it) {
+      const int cc = c0 + round * S.teams + team;
+      const bool active = cc < c1;
+      const int sl = cc * 32 + lane;
+      const bool valid = active && sl < nc;
+      const int64_t s = (int64_t)t * nc + sl;
+      const float* vb = V;
+      int k1 = 0, ml = 0, end = 0;  // slot rows of the warp; per lane: of action `lane`, and where they end
+      const uint32_t* ent = col;
+      uint32_t e[16];
+      float rr[kAhActions];
+      if (active) {
+        const int64_t c = (int64_t)t * cpl + cc;
+        const int64_t slot = __ldg(P.chunk_slot + c);
+        ml = lane < na ? __ldg(P.maxlen + c * P.na_pad + lane) : 0;
+        const float* Rp = P.R + (c * na + a0) * 32 + lane;
+#pragma unroll
+        for (int a = 0; a < kAhActions; ++a) rr[a] = a0 + a < a1 ? ld_stream(Rp + a * 32) : 0.f;
+        end = ml;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, end, o);
+          if (lane >= o) end += v;
+        }
+        if (a0 < a1) {
+          const int k0 = __shfl_sync(0xffffffffu, end - ml, a0);
+          k1 = __shfl_sync(0xffffffffu, end, a1 - 1) - k0;
+          end -= k0;
+          ent = col + (slot + k0) * 32 + lane;
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) e[j] = j < k1 ? ld_stream(ent + j * 32) : 0u;
+        if (valid && s < P.n_row_states && t + 1 < P.nlayers) {
+          const int i = sl / P.g, j = sl - i * P.g;
+          vb += (int64_t)(t + 1) * nc + (int64_t)(i - P.del) * P.g + (j - P.del);
+        }
+        if (grp == 0 && lane == 0 && t > 0) prefetch_chunk(P, (int)(c - cpl), 4, 0);
+      }
+      if (round == 0 && t + 1 < P.nlayers) {
+        // ---- every CTA has written layer t + 1 --------------------------------------
+        if (threadIdx.x == 0) {
+          WaitClock clock;
+          const unsigned target = gen * gridDim.x + wb.extra;
+          while (ld_acquire(sync) < target) {
+            if (*stop || clock.over(wb) || (clock.polls % WaitClock::kEvery == 0 && ld_acquire(sync + 1) != 0u)) {
+              atomicOr(sync + 1, 2u);
+              *stop = 1;
+              break;
+            }
+          }
+        }
+        __syncthreads();
+        if (*stop) return;  // (the whole CTA: written before the barrier only)
+      }
+      float bq = -INFINITY;
+      int ba = 0x7fffffff;
+      if (active) {
+        const bool own = lane >= a0 && lane < a1 && ml > 0;
+        float* sum = &sums[wid][0][lane];
+        float acc = 0.f;
+        for (int k = 0; k < k1; k += 16) {
+          if (k > 0) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) e[j] = k + j < k1 ? ld_stream(ent + (k + j) * 32) : 0u;
+          }
+          const int m = k1 - k;
+          float v0[8], v1[8];
+          ahead_gather(e, vb, m, v0);
+          if (m > 8) ahead_gather(e + 8, vb, m - 8, v1);
+          const int at = end - 1 - k;  // this lane's action ends in the batch
+          const unsigned ends = __reduce_or_sync(0xffffffffu, own && at >= 0 && at < 16 ? 1u << at : 0u);
+          ahead_fold(e, v0, m, ends, sum, acc);
+          if (m > 8) ahead_fold(e + 8, v1, m - 8, ends >> 8, sum, acc);
+        }
+        const unsigned has = __ballot_sync(0xffffffffu, own) >> a0;  // actions with rows
+        sum = &sums[wid][0][lane];
+#pragma unroll
+        for (int a = 0; a < kAhActions; ++a) {
+          if (a0 + a < a1) {
+            float x = 0.f;
+            if (has >> a & 1u) {
+              x = *sum;
+              sum += 32;
+            }
+            const float q = finish_row(rr[a], x, 0.f, P.nrzns, true);
+            if (q > bq) {  // (false for NaN)
+              bq = q;
+              ba = a0 + a;
+            }
+          }
+        }
+      }
+      if (G > 1) {
+        if (grp > 0) {
+          sq[it & 1][wid][lane] = bq;
+          sa[it & 1][wid][lane] = ba;
+        }
+        bar_named(1 + team, G * 32);
+        if (grp == 0) {
+          for (int g2 = 1; g2 < G; ++g2) {
+            const float oq = sq[it & 1][wid + g2][lane];
+            if (oq > bq) {  // later groups hold later actions: strict '>' keeps the first maximum
+              bq = oq;
+              ba = sa[it & 1][wid + g2][lane];
+            }
+          }
+        }
+      }
+      if (valid && grp == 0) {
+        float vout;
+        int32_t pout;
+        finish_state(bq, ba, vout, pout);
+        V[s] = vout;
+        pi[s] = pout;
+      }
+    }
+    if (t > 0) {
+      ++gen;
+      __syncthreads();
+      if (threadIdx.x == 0) add_release(sync, 1u);
+    }
+  }
+}
+
 // Many layered solves in one persistent launch.  Step k covers layer
 // nlayers-1-k of every job that has more than k layers (jobs sorted by layer
 // count, so those are a prefix and their chunks a contiguous item range).
@@ -1084,6 +1277,29 @@ cudaError_t launch_vi_chunks(const ViPack& P, int64_t c_begin, int64_t c_end, co
 
 cudaError_t launch_vi_layered(const ViPack& P, float* V, int32_t* pi, unsigned int* sync, int groups,
                               cudaStream_t st, int tune) {
+  // (the packed layout is the builder's; lengths of up to 32 actions fit a warp)
+  if (groups == 0 && tune < 0 && P.ent_mode == ENT_PACKED && P.na <= 32) {
+    AheadShape S;
+    S.grid = (int)std::min<int64_t>(P.cpl, sm_count_pack());
+    const int per_cta = (int)((P.cpl + S.grid - 1) / S.grid);
+    int most = 0;
+    // The fewest actions a warp that leave a CTA one round of chunks (a second
+    // round's loads start behind the barrier): 200x200, 4 actions and two rounds
+    // 967 us, 6 and one 786; 50x50, 4 actions 119 us, 2 actions 97.
+    for (S.actions = 2;; ++S.actions) {
+      S.groups = (P.na + S.actions - 1) / S.actions;
+      most = std::min(15, kAhWarps / S.groups);  // (named barriers 1 to 15)
+      if (per_cta <= most || S.actions == kAhActions) break;
+    }
+    S.rounds = (per_cta + most - 1) / most;
+    S.teams = (per_cta + S.rounds - 1) / S.rounds;
+    ViPack Pc = P;
+    WaitBound wb = wait_bound_from_env();
+    void* args[] = {(void*)&Pc, (void*)&S, (void*)&V, (void*)&pi, (void*)&sync, (void*)&wb};
+    return cudaLaunchCooperativeKernel((const void*)k_vi_ahead, dim3((unsigned)S.grid),
+                                       dim3((unsigned)(32 * S.teams * S.groups)), args, 0, st);
+  }
+  if (tune < 0) tune = PF_NEXT;
   const int prefetch = tune & (PF_NEXT | PF_CURRENT);
   return dispatch_pack(P, [&](auto mode, auto* cntt) -> cudaError_t {
     using CntT = std::remove_pointer_t<decltype(cntt)>;
