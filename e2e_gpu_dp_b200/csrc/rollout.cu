@@ -69,9 +69,17 @@ struct RolloutArgs {
 
 // NumPy's float32 divmod (fmod, exact correction of the quotient, floor with
 // the 0.5 guard); returns floor(a / b) and sets rem.
+// (With b = 1 the remainder is a less its integer part, exactly, and nothing is
+// divided: the same results without the two long sequences.)
 __device__ __forceinline__ float divmod32(float a, float b, float& rem) {
-  float mod = fmodf(a, b);
-  float div = __fdiv_rn(__fsub_rn(a, mod), b);
+  float mod, div;
+  if (b == 1.0f) {
+    mod = __fsub_rn(a, truncf(a));
+    div = __fsub_rn(a, mod);
+  } else {
+    mod = fmodf(a, b);
+    div = __fdiv_rn(__fsub_rn(a, mod), b);
+  }
   if (mod != 0.f) {
     if ((b < 0.f) != (mod < 0.f)) {
       mod = __fadd_rn(mod, b);
@@ -225,7 +233,41 @@ __device__ Interp interp_action(const RolloutArgs& A, int t, int i, int j, float
   return r;
 }
 
-__global__ void __launch_bounds__(128) k_rollout(RolloutArgs A) {
+// What a step reads at its cell (t, i, j).  Its values are the last that the step
+// before reads (scalar field, mask, policy), so all of them are loaded together
+// as soon as the cell is known: one trip to memory a step.
+constexpr int kAheadModes = 12;  // modes loaded ahead; later ones are read in the step
+struct CellLoads {
+  float u, v, s;
+  int mask, a;
+  float ui[kAheadModes], vi[kAheadModes];
+};
+
+__device__ __forceinline__ void load_cell(const RolloutArgs& A, int64_t nc, int t, int i, int j, CellLoads& C) {
+  const int64_t ij = (int64_t)i * A.g + j, cell = (int64_t)t * nc + ij;
+  C.s = A.F.s[cell];
+  C.mask = A.F.mask[cell];
+  C.a = A.policy[cell];
+  C.u = A.F.u[cell];
+  C.v = A.F.v[cell];
+  const int64_t m0 = (int64_t)t * A.nm * nc + ij;
+#pragma unroll
+  for (int k = 0; k < kAheadModes; ++k)
+    if (k < A.nm) {
+      C.ui[k] = A.F.ui[m0 + k * nc];
+      C.vi[k] = A.F.vi[m0 + k * nc];
+    }
+}
+
+// A thread's steps are one chain: the cell, what is read there, the next cell.
+// 5000 vehicles are 157 warps, about one an SM, which lets nothing hide a load:
+// the step's reads in one trip (they were three, the modes in batches) and CTAs
+// of one warp took 200x200x120, 10 modes, 5000 realisations from 299 to 167 us,
+// 137x137x53, 20 modes, 777 realisations from 164 to 109.  Prefetching the lines
+// of the layer after next costs the warp more issue slots (212 us) than it hides.
+constexpr int kRolloutThreads = 32;
+
+__global__ void __launch_bounds__(kRolloutThreads) k_rollout(RolloutArgs A) {
   const int rzn = blockIdx.x * blockDim.x + threadIdx.x;
   if (rzn >= A.nrzns) return;
   const int g = A.g, nt = A.nt, nm = A.nm;
@@ -241,7 +283,14 @@ __global__ void __launch_bounds__(128) k_rollout(RolloutArgs A) {
   float thr = 0.f, cth = 0.f, sth = 0.f;
   double thr_d = 0.0, cth_d = 0.0, sth_d = 0.0;
   const float xs0 = A.xs[0], xsn = A.xs[g - 1], ys0 = A.ys[0], ysn = A.ys[g - 1];
-  int a = A.policy[(int64_t)t * nc + (int64_t)i * g + j];
+  CellLoads C;
+  load_cell(A, nc, t, i, j, C);
+  float y_[kAheadModes];  // the step's coefficients
+  const float* yk = A.F.Y + (int64_t)rzn * nm;
+#pragma unroll
+  for (int k = 0; k < kAheadModes; ++k)
+    if (k < nm) y_[k] = yk[k];
+  int a = C.a;
   if (a >= 0 && a < A.na) {
     thr = A.speed[a];
     cth = A.cosv[a];
@@ -256,17 +305,21 @@ __global__ void __launch_bounds__(128) k_rollout(RolloutArgs A) {
         success = -2;
         break;
       }
-      const int64_t cell = (int64_t)t * nc + (int64_t)i * g + j;
       float dx_ = 0.f, dy_ = 0.f;
-      const float* yk = A.F.Y + ((int64_t)t * A.nrzns_field + rzn) * nm;
-      for (int k = 0; k < nm; ++k) {
+#pragma unroll
+      for (int k = 0; k < kAheadModes; ++k)
+        if (k < nm) {
+          dx_ = fmaf(C.ui[k], y_[k], dx_);
+          dy_ = fmaf(C.vi[k], y_[k], dy_);
+        }
+      for (int k = kAheadModes; k < nm; ++k) {
         const float w = yk[k];
         dx_ = fmaf(A.F.ui[((int64_t)t * nm + k) * nc + (int64_t)i * g + j], w, dx_);
         dy_ = fmaf(A.F.vi[((int64_t)t * nm + k) * nc + (int64_t)i * g + j], w, dy_);
       }
-      const float vx = __fadd_rn(A.F.u[cell], dx_);
-      const float vy = __fadd_rn(A.F.v[cell], dy_);
-      const float rad1 = A.F.s[cell];
+      const float vx = __fadd_rn(C.u, dx_);
+      const float vy = __fadd_rn(C.v, dy_);
+      const float rad1 = C.s;
       if (!term(i, j) && t < nt - 1 && !act_d) {  // move_exact
         const float thrust = thr;
         const float vnx = __fadd_rn(__fmul_rn(thrust, cth), vx);
@@ -314,7 +367,12 @@ __global__ void __launch_bounds__(128) k_rollout(RolloutArgs A) {
         }
         t += 1;
       }
-      const float rad2 = A.F.s[(int64_t)t * nc + (int64_t)i * g + j];
+      load_cell(A, nc, t, i, j, C);
+      yk = A.F.Y + ((int64_t)t * A.nrzns_field + rzn) * nm;
+#pragma unroll
+      for (int k = 0; k < kAheadModes; ++k)
+        if (k < nm) y_[k] = yk[k];
+      const float rad2 = C.s;
       travel += 1;
       const float sp = act_d ? (float)thr_d : thr;
       const float sp2 = __fmul_rn(sp, sp);
@@ -323,7 +381,7 @@ __global__ void __launch_bounds__(128) k_rollout(RolloutArgs A) {
       e_col = __fadd_rn(e_col, half);
       e_net = __fadd_rn(e_net, __fsub_rn(sp2, half));
     }
-    if (i == 0 || i == g - 1 || j == 0 || j == g - 1 || A.F.mask[(int64_t)t * nc + (int64_t)i * g + j] == 1)
+    if (i == 0 || i == g - 1 || j == 0 || j == g - 1 || C.mask == 1)
       success = 0;
     if (!term(i, j) && t < nt - 1 && success == -1) {
       if (A.interp) {
@@ -340,7 +398,7 @@ __global__ void __launch_bounds__(128) k_rollout(RolloutArgs A) {
         cth_d = cos(r.angle);
         sth_d = sin(r.angle);
       } else {
-        a = A.policy[(int64_t)t * nc + (int64_t)i * g + j];
+        a = C.a;
         if (a >= 0 && a < A.na) {
           thr = A.speed[a];
           cth = A.cosv[a];
@@ -350,6 +408,7 @@ __global__ void __launch_bounds__(128) k_rollout(RolloutArgs A) {
     }
     else if (term(i, j)) success = 1;
     else success = 0;
+    if (success != -1) break;  // (the remaining steps of a decided run change nothing)
   }
   A.success[rzn] = (int8_t)success;
   A.ttime[rzn] = travel;
@@ -469,7 +528,7 @@ extern "C" e2e_status e2e_rollout(const e2e_problem* p, const e2e_fields* f, int
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   CK(cudaEventRecord(e0, st));
-  k_rollout<<<(n + 127) / 128, 128, 0, st>>>(A);
+  k_rollout<<<(n + kRolloutThreads - 1) / kRolloutThreads, kRolloutThreads, 0, st>>>(A);
   CK(cudaGetLastError());
   CK(cudaEventRecord(e1, st));
   std::vector<int8_t> hs((size_t)n);
