@@ -1018,33 +1018,51 @@ __global__ void k_scan_finish(const int32_t* __restrict__ len, int64_t n,
 }
 
 // K3: one warp per tile (the rows of one builder warp): move the tile's
-// entries from staging to their canonical position and write row_ptr.
+// entries from staging to their canonical position and write row_ptr.  Bound by
+// its loads' latency rather than by bandwidth: a tile is about a hundred
+// entries, so a lane has four of them (and its row's offset) on the way before it
+// stores any: 200x200x120, 16 actions 1.23 -> 0.94 ms (4.0 TB/s), 300x300x40 0.92 -> 0.71.
 template <typename CntT, typename PtrT>
-__global__ void k_assemble(AssembleArgs A) {
+__global__ void __launch_bounds__(256) k_assemble(AssembleArgs A) {
   const int lane = threadIdx.x & 31;
   const int64_t tile = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (tile >= A.n_tiles) return;
-  const int64_t src = A.tile_base[tile];
-  const int64_t dst = A.canon[tile];
-  const int len = A.tile_len[tile];
+  const int64_t src = __ldg(A.tile_base + tile);
+  const int64_t dst = __ldg(A.canon + tile);
+  const int len = __ldg(A.tile_len + tile);
+  const int64_t layer = A.n_tiles <= UINT32_MAX ? (int64_t)((uint32_t)tile / (uint32_t)A.tiles_per_layer)
+                                                : tile / A.tiles_per_layer;
+  const int64_t cb = (tile - layer * A.tiles_per_layer) * A.cells_per_tile;
+  const int64_t ce = min(cb + A.cells_per_tile, A.ncells);
+  const int rows = (int)max(ce - cb, (int64_t)0) * A.na;
+  const int64_t r0 = (layer * A.ncells + cb) * A.na;
+  const uint32_t off = lane < rows ? __ldg(A.row_off + r0 + lane) : 0u;
   const int32_t* __restrict__ scol = A.stage_col + src;
   const CntT* __restrict__ scnt = reinterpret_cast<const CntT*>(A.stage_cnt) + src;
   int32_t* __restrict__ dcol = A.col + dst;
   CntT* __restrict__ dcnt = reinterpret_cast<CntT*>(A.cnt) + dst;
-  for (int k = lane; k < len; k += 32) {
-    dcol[k] = scol[k];
-    dcnt[k] = scnt[k];
+  constexpr int B = 4;
+  for (int k0 = lane; k0 < len; k0 += 32 * B) {
+    int32_t c[B];
+    CntT w[B];
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      const int k = k0 + 32 * b;
+      c[b] = k < len ? __ldcs(scol + k) : 0;
+      w[b] = k < len ? __ldcs(scnt + k) : (CntT)0;
+    }
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      const int k = k0 + 32 * b;
+      if (k < len) {
+        dcol[k] = c[b];
+        dcnt[k] = w[b];
+      }
+    }
   }
-  const int64_t layer = tile / A.tiles_per_layer;
-  const int64_t tl = tile - layer * A.tiles_per_layer;
-  const int64_t cb = tl * A.cells_per_tile;
-  const int64_t ce = min(cb + A.cells_per_tile, A.ncells);
   PtrT* rp = reinterpret_cast<PtrT*>(A.row_ptr);
-  if (cb < ce) {
-    const int64_t r0 = (layer * A.ncells + cb) * A.na;
-    const int64_t r1 = (layer * A.ncells + ce) * A.na;
-    for (int64_t r = r0 + lane; r < r1; r += 32) rp[r] = (PtrT)(dst + A.row_off[r]);
-  }
+  if (lane < rows) rp[r0 + lane] = (PtrT)(dst + off);
+  for (int r = lane + 32; r < rows; r += 32) rp[r0 + r] = (PtrT)(dst + A.row_off[r0 + r]);
   if (tile == A.n_tiles - 1 && lane == 0) rp[A.n_rows] = (PtrT)A.total_nnz;
 }
 
