@@ -254,7 +254,7 @@ def k1_issue_roofline(samples: int, k1_s: float, sm_mhz: float, n_sm: int):
     SM clock measured during the timed steps)."""
     path = os.path.join(ROOT, "profiles", "traffic.json")
     try:
-        per_sample = float(json.load(open(path))[f"k_build_tiles/{WORKLOAD}/warp_inst_per_sample"])
+        per_sample = float(json.load(open(path))[f"k_build_ranks/{WORKLOAD}/warp_inst_per_sample"])
     except Exception:
         return None
     inst = per_sample * samples
@@ -560,7 +560,7 @@ def run_ours(args, ws, rank, local):
     tpath = os.path.join(ROOT, "profiles", "traffic.json")
     if os.path.exists(tpath):
         try:
-            traffic = json.load(open(tpath)).get(f"k_build_tiles/{WORKLOAD}/dram_bytes")
+            traffic = json.load(open(tpath)).get(f"k_build_ranks/{WORKLOAD}/dram_bytes")
         except Exception:
             traffic = None
     samples = (prob.nt - 1) * prob.ncells * prob.num_actions * prob.nrzns
@@ -572,16 +572,16 @@ def run_ours(args, ws, rank, local):
     hbm_part = {"achieved": round(k1_gbs, 2), "peak": hbm, "unit": "GB/s", "frac": round(k1_gbs / hbm, 5),
                 "traffic": traffic, "peak_source": f"{peak_kind} hbm_gbs", "algorithmic_bytes": k1_bytes}
     if issue is not None:
-        roof = {"kernel": "k_build_tiles", "bound": "issue", "achieved": round(issue["achieved"], 1),
+        roof = {"kernel": "k_build_ranks", "bound": "issue", "achieved": round(issue["achieved"], 1),
                 "peak": round(issue["peak"], 1), "unit": "warp-inst/s",
                 "frac": round(issue["achieved"] / issue["peak"], 4), "traffic": traffic,
                 "warp_inst_per_sample": issue["warp_inst_per_sample"], "sm_mhz": sm_mhz, "sms": n_sm,
                 "note": "issue-bound Monte-Carlo kernel: warp instructions (per-sample count of the ncu "
-                        "capture in profiles/k_build_tiles_c2nt30.md x samples) / K1 time, against 4 warp "
+                        "capture in profiles/k_build_ranks_c2nt30.md x samples) / K1 time, against 4 warp "
                         "instructions per cycle per SM at the measured SM clock; its HBM figure below",
                 "hbm": hbm_part}
     else:
-        roof = {"kernel": "k_build_tiles", "bound": "hbm", **hbm_part}
+        roof = {"kernel": "k_build_ranks", "bound": "hbm", **hbm_part}
     asm_bytes = assembly_bytes(info["nnz"], info["n_rows"], cb, info["index_bits"])
     asm_gbs = asm_bytes / (asm_ms * 1e-3) / 1e9 if asm_ms > 0 else None
     asm_roof = {"kernels": "k_scan_* (K2) + k_assemble (K3)", "bound": "hbm", "ms": round(asm_ms, 3),

@@ -21,10 +21,10 @@
 // k_build_tiles.
 //
 // Measured on B200 (whole call, counting loops -> ranks): 200x200x120, 16
-// actions, 5000 realisations 330.6 -> 63 ms; 300x300x40, 2000 realisations
-// 102.3 -> 24.4 ms; 137x137x53, 24 actions, 777 realisations 29.7 -> 8.8 ms.
-// Of the 13.8 ms of 200x200x30 the counting takes about 10 ms (shared-memory
-// wavefronts and issue slots both at about half of their peaks), staging 0.9,
+// actions, 5000 realisations 330.6 -> 61.5 ms; 300x300x40, 2000 realisations
+// 102.3 -> 23.6 ms; 137x137x53, 24 actions, 777 realisations 29.7 -> 8.7 ms.
+// Of the 13.8 ms of 200x200x30 the counting takes about 10 ms (the shared-memory
+// pipe at 60 % of its peak, issue slots at 62 %), staging 0.9,
 // the prefix sums 0.5, the rows 2.4.  Four or five CTAs of 4 warps an SM: one
 // CTA's staging and rows run beside the others' counting (two of 8 warps: 16.8
 // ms, four of 4: 14.3); the table reads of a lane's four samples before their

@@ -144,7 +144,10 @@ typedef struct {
                             sweep (0 = auto, 1, 2, 4, 8).  Bit 8 set: bits 4-7 give the sweep
                             tuning (4: L2 prefetch of the chunk a warp takes next, 5: of the chunk
                             it starts, 6: lean kernel without entry look-ahead, 7: Jacobi sweeps
-                            staged through shared memory by TMA bulk copies). */
+                            staged through shared memory by TMA bulk copies).  Automatic: the
+                            layered pass with loads ahead of its barriers, and Jacobi with all
+                            sweeps of a layer at once (time-layered models); a tuning or a warp
+                            count selects one of the other kernels, with the same results. */
 } e2e_vi_opts;
 
 typedef struct {
@@ -363,9 +366,11 @@ e2e_status e2e_rollout(const e2e_problem* p, const e2e_fields* f, int fields_whe
  * fields, V and policy).  Value and policy are bit-identical to
  * e2e_build_model + e2e_spvi_solve with the layered method (whose fixed point
  * is the Jacobi one); last layer: value 0, action 0.  policy_out / value_out:
- * ns entries each in out_where memory (either may be NULL).  One cooperative
- * launch: a tile's backup waits (bounded by E2E_WAIT_LIMIT_MS, default 5000)
- * for the next layer's completion; a wait that runs out gives E2E_ERR_DEVICE. */
+ * ns entries each in out_where memory (either may be NULL).  Layers are built in
+ * blocks, last first, into a bounded staging area, and each block is backed up
+ * by one cooperative launch whose layers are separated by a grid barrier
+ * (bounded by E2E_WAIT_LIMIT_MS, default 2000); a wait that runs out gives
+ * E2E_ERR_DEVICE. */
 typedef struct {
   double seconds;          /* device time of the pass (CUDA events) */
   int64_t n_rows;          /* rows built and backed up */
@@ -373,7 +378,7 @@ typedef struct {
   uint64_t dropped;        /* as e2e_model_info */
   uint64_t misbinned;
   uint64_t overflow_rows;
-  int32_t launches;        /* kernel launches (one cooperative launch per pass; a pass is re-run when rows needed more dense histograms) */
+  int32_t launches;        /* builder and backup launches (per block of layers; a build is re-run when rows needed more dense histograms) */
   int32_t reserved;
   int64_t h2d_bytes;       /* field bytes copied from host memory */
 } e2e_fused_stats;
