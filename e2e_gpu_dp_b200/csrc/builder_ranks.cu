@@ -1052,7 +1052,11 @@ cudaError_t dispatch_nm(int nmp, F&& f) {
 // CTAs 14.0, 7.70, 6.30, 3.50.
 constexpr size_t kSmem4 = 55 * 1024, kSmem5 = 44 * 1024;
 
-constexpr size_t kRewardSmem = 48 * 1024;  // k_rank_rewards: no opt-in needed
+// k_rank_rewards: two CTAs an SM at least.  (Few actions a cell, or several speeds,
+// make the tables of the 32 or 16 cells of a CTA need
+// more than 48 KB: with the general builder 90x90x40, 300 realisations, 4 actions
+// took 14.8 ms, here 1.9; 2 speeds x 4 headings 21.4 -> 2.2; 4 x 4 33.1 -> 3.7.)
+constexpr size_t kRewardSmem = 110 * 1024;
 
 size_t reward_smem_bytes(const RankArgs& K, int nmp) {
   const size_t ct = (size_t)1 << K.cells_log2;
@@ -1130,7 +1134,15 @@ cudaError_t launch_build_ranks(const BuildArgs& A, const RankArgs& K, cudaStream
     cudaError_t e2 = cudaGetLastError();
     if (e2 != cudaSuccess || !K.seq_rewards) return e2;
     const size_t rb = reward_smem_bytes(K, nmp);  // (at most kRewardSmem: rank_shape)
-    k_rank_rewards<decltype(nm)::value><<<(unsigned)std::min<int64_t>(tasks, 8 * (int64_t)sms), kThreads, rb, st>>>(A, K);
+    // as many CTAs as are resident: each takes the same number of tasks
+    int per_sm = 0;
+    e2 = cudaFuncSetAttribute(k_rank_rewards<decltype(nm)::value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)kRewardSmem);
+    if (e2 != cudaSuccess) return e2;
+    e2 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rank_rewards<decltype(nm)::value>, kThreads, rb);
+    if (e2 != cudaSuccess) return e2;
+    k_rank_rewards<decltype(nm)::value>
+        <<<(unsigned)std::min<int64_t>(tasks, std::max(per_sm, 1) * (int64_t)sms), kThreads, rb, st>>>(A, K);
     return cudaGetLastError();
   });
 }

@@ -81,6 +81,12 @@ def test_rewards_and_spacings(kind, dx, dy, dt):
     _check(p, make_fields(p, s))
 
 
+@pytest.mark.parametrize("speeds,angles", [(1, 2), (1, 4), (2, 2), (2, 4), (3, 4), (4, 4), (4, 8), (16, 2)])
+def test_sequential_sums_of_small_and_many_speed_action_sets(speeds, angles):  # large tables of rewards a CTA
+    p = _prob(g=26, nt=5, nrzns=130, nm=4, speeds=speeds, angles=angles, dx=0.5, dy=0.5, dt=0.5, F=1.1, prob_type="energy2")
+    _check(p, make_fields(p, FieldSpec(A=0.5, sigma0=0.2, obstacle_frac=0.05, scalar=0.3, scalar_wave=0.4, seed=speeds + angles)))
+
+
 @pytest.mark.parametrize("m", [1, 3, 5, 9])
 def test_small_neighbourhoods(m):  # counted bins outside the m x m neighbourhood
     for dx in (1.0, 0.5):
