@@ -15,10 +15,9 @@
 // one ordinary sweep gives the result.
 //
 // The model is read once instead of once per sweep (sweeps: 0.35 ms each at the
-// copy bandwidth).  What bounds it is issue: about 1400 warp instructions per
-// state of 16 rows and 64 sweeps (a quarter the rows' loop and branches, a
-// quarter their exact quotients).  200x200x120, 500 realisations: 120 sweeps
-// 42.9 -> 11.3 ms; 137x137x53, 12 actions 4.1 -> 2.0 ms; 50x50x30 0.84 -> 0.40 ms.
+// copy bandwidth).  What bounds it is issue: the reads and multiply-adds, the
+// exact quotients, the set-up of a state.  200x200x120, 500 realisations: 120 sweeps
+// 42.9 -> 8.8 ms; 137x137x53, 12 actions 4.1 -> 1.7 ms; 50x50x30 0.84 -> 0.34 ms.
 #include <math.h>
 
 #include <algorithm>
@@ -54,22 +53,48 @@ __device__ __forceinline__ float quotient(float acc, float n, float rn) {
 // values (its flag is set) is divided with the operator itself.
 constexpr float kPlainMin = 1e-10f, kPlainMax = 1e25f;
 
-// One row's sums of N entries: every read of the history, then the multiply-adds
-// in entry order
-template <int N, int NB>
-__device__ __forceinline__ void row_sums(const uint2* ent, const char* hn, float (&acc)[NB]) {
-  float v[N][NB], w[N];
+// The rows of a state that are staged in ent[0 .. cnt): a batch of entries at a
+// time, every read of the history, then the multiply-adds in entry order; bit k of
+// ends says that entry k is its row's last, whose Q is then formed with the next
+// of the rewards r.  (One pass over the entries whatever the rows' lengths: with a
+// switch on each row's length 200x200x120 took 11.3 ms, now 8.8; batches of 8 for all
+// counts of sweeps 10.0, of 4 9.0.)
+template <int NB, bool PLAIN>
+__device__ __forceinline__ void take_rows(const uint2* ent, int cnt, const unsigned (&ends)[kStage / 32], const char* hn,
+                                          bool counts, float n, float rn, const float*& r, float (&acc)[NB],
+                                          float (&bq)[NB]) {
+  constexpr int B = NB > 2 ? 4 : 8;
 #pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const uint2 x = ent[i];
-    w[i] = __uint_as_float(x.y);
+  for (int w = 0; w < kStage / 32; ++w) {
+    if (32 * w >= cnt) break;
+    unsigned m = ends[w];
+    const uint2* p = ent + 32 * w;
+    const int todo = min(cnt - 32 * w, 32);
+    for (int k = 0; k < todo; k += B, p += B, m >>= B) {
+      float v[B][NB], f[B];
 #pragma unroll
-    for (int b = 0; b < NB; ++b) v[i][b] = __ldg(reinterpret_cast<const float*>(hn + (size_t)x.x) + 32 * b);
+      for (int i = 0; i < B; ++i) {
+        const uint2 x = p[i];
+        f[i] = __uint_as_float(x.y);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) v[i][b] = __ldg(reinterpret_cast<const float*>(hn + (size_t)x.x) + 32 * b);
+      }
+#pragma unroll
+      for (int i = 0; i < B; ++i) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) acc[b] = fmaf(f[i], v[i][b], acc[b]);
+        if (m >> i & 1u) {
+          const float rr = *r++;
+#pragma unroll
+          for (int b = 0; b < NB; ++b) {
+            const float q = PLAIN ? (counts ? quotient(acc[b], n, rn) : acc[b]) : divide(acc[b], n);
+            bq[b] = fmaxf(bq[b], rr + q);  // (NaN is never taken)
+            acc[b] = 0.f;
+          }
+        }
+      }
+    }
   }
-#pragma unroll
-  for (int i = 0; i < N; ++i)
-#pragma unroll
-    for (int b = 0; b < NB; ++b) acc[b] = fmaf(w[i], v[i][b], acc[b]);
 }
 
 // Sweeps j0 + 1 .. j0 + 32 NB (up to J) of the layer of states [s0, s0 + nc).
@@ -81,7 +106,8 @@ __global__ void __launch_bounds__(kThreads) k_jacobi_layer(ViModel M, int64_t s0
                                                            const unsigned int* odd_next, unsigned int* odd) {
   __shared__ double red[kWarps][NB * 32];
   // entries of a warp's state: (offset of the next state's history, weight)
-  __shared__ uint2 ents[kWarps][kStage];
+  __shared__ __align__(16) uint2 ents[kWarps][kStage];
+  __shared__ float rews[kWarps][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool counts = M.count_type != VAL_F32;
   const float n = (float)M.nrzns, rn = 1.0f / n;
@@ -112,58 +138,43 @@ __global__ void __launch_bounds__(kThreads) k_jacobi_layer(ViModel M, int64_t s0
       // lane a: end of row a, relative to the state's first entry
       const int ends = (int)((int64_t)__ldg(rp + r0 + min(lane + 1, M.na)) - e0);
       const int last = __shfl_sync(0xffffffffu, ends, M.na - 1);
+      const int begin = __shfl_up_sync(0xffffffffu, ends, 1);
+      const bool some = lane < M.na && ends > (lane ? begin : 0);
+      const unsigned filled = __ballot_sync(0xffffffffu, some);
       uint2* const ent = ents[warp];
-      int staged = 0, at = 0;  // entries [at, staged) wait in ent[0 ..]
-      int begin = 0;
-      for (int a = 0; a < M.na; ++a) {
-        const int end = __shfl_sync(0xffffffffu, ends, a);
-        if (end > staged) {
-          // as many of the next entries as fit (a row longer than that takes several)
-          at = begin;
-          staged = min(last, at + kStage);
-          __syncwarp();
-          for (int k = at + lane; k < staged; k += 32) {
-            const uint32_t col = (uint32_t)((int64_t)__ldg(M.col + e0 + k) - next0);
-            ent[k - at] = make_uint2(col * sn * 4u, __float_as_uint(to_f(__ldg(cnt + e0 + k))));
+      // rows without entries: Q = R + 0 / n
+      for (unsigned none = ~filled & (M.na == 32 ? ~0u : (1u << M.na) - 1u); none; none &= none - 1) {
+        const float r = __shfl_sync(0xffffffffu, rv, __ffs(none) - 1);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) bq[b] = fmaxf(bq[b], r + 0.f);
+      }
+      __syncwarp();
+      if (some) rews[warp][__popc(filled & ((1u << lane) - 1u))] = rv;  // of the others, in order
+      const float* r = rews[warp];
+      float acc[NB];
+#pragma unroll
+      for (int b = 0; b < NB; ++b) acc[b] = 0.f;
+      for (int at = 0; at < last; at += kStage) {
+        const int staged = min(last - at, kStage);
+        __syncwarp();
+        for (int k = lane; k < ((staged + 7) & ~7); k += 32) {
+          // (behind the last row of the state the sums are not used)
+          uint2 x = make_uint2(0u, 0u);
+          if (k < staged) {
+            const uint32_t col = (uint32_t)((int64_t)__ldg(M.col + e0 + at + k) - next0);
+            x = make_uint2(col * sn * 4u, __float_as_uint(to_f(__ldg(cnt + e0 + at + k))));
           }
-          __syncwarp();
+          ent[k] = x;
         }
-        const float r = __shfl_sync(0xffffffffu, rv, a);
-        float acc[NB];
+        unsigned marks[kStage / 32];
 #pragma unroll
-        for (int b = 0; b < NB; ++b) acc[b] = 0.f;
-        const uint2* p = ent + (begin - at);
-        switch (end - begin) {
-          case 0: break;
-          case 1: row_sums<1, NB>(p, hn, acc); break;
-          case 2: row_sums<2, NB>(p, hn, acc); break;
-          case 3: row_sums<3, NB>(p, hn, acc); break;
-          case 4: row_sums<4, NB>(p, hn, acc); break;
-          case 5: row_sums<5, NB>(p, hn, acc); break;
-          case 6: row_sums<6, NB>(p, hn, acc); break;
-          default:
-            for (int k = begin; k < end; ++k) {
-              if (k >= staged) {  // a row longer than the staging area
-                at = k;
-                staged = min(last, at + kStage);
-                __syncwarp();
-                for (int q = at + lane; q < staged; q += 32) {
-                  const uint32_t col = (uint32_t)((int64_t)__ldg(M.col + e0 + q) - next0);
-                  ent[q - at] = make_uint2(col * sn * 4u, __float_as_uint(to_f(__ldg(cnt + e0 + q))));
-                }
-                __syncwarp();
-              }
-              row_sums<1, NB>(ent + (k - at), hn, acc);
-            }
+        for (int w = 0; w < kStage / 32; ++w) {
+          const int k = ends - 1 - at - 32 * w;
+          marks[w] = __reduce_or_sync(0xffffffffu, some && k >= 0 && k < 32 ? 1u << k : 0u);
         }
-        begin = end;
-        if (plain) {
-#pragma unroll
-          for (int b = 0; b < NB; ++b) bq[b] = fmaxf(bq[b], r + (counts ? quotient(acc[b], n, rn) : acc[b]));
-        } else {
-#pragma unroll
-          for (int b = 0; b < NB; ++b) bq[b] = fmaxf(bq[b], r + divide(acc[b], n));
-        }
+        __syncwarp();
+        if (plain) take_rows<NB, true>(ent, staged, marks, hn, counts, n, rn, r, acc, bq);
+        else take_rows<NB, false>(ent, staged, marks, hn, counts, n, rn, r, acc, bq);
       }
     }
     float* h = H + (int64_t)c * s;
