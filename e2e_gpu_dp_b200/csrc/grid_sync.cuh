@@ -62,15 +62,19 @@ struct WaitClock {
   }
 };
 
-// Grid-wide barrier of a cooperative launch.  sync[0] counts arrivals (never
-// reset inside a launch); a wait that outlives its limit sets bit 1 of sync[1]
-// and every later barrier returns false at once.
-__device__ __forceinline__ bool grid_barrier(unsigned int* sync, unsigned int target, const WaitBound& wb) {
-  __shared__ int ok;
+// Grid-wide barrier of a cooperative launch, in two halves so that work which needs
+// no other CTA can stand between them.  sync[0] counts arrivals (never reset inside
+// a launch); a wait that outlives its limit sets bit 1 of sync[1] and every later
+// wait returns false at once.
+__device__ __forceinline__ void grid_arrive(unsigned int* sync) {
   __syncthreads();
+  if (threadIdx.x == 0) add_release(sync, 1u);
+}
+
+__device__ __forceinline__ bool grid_wait(unsigned int* sync, unsigned int target, const WaitBound& wb) {
+  __shared__ int ok;
   if (threadIdx.x == 0) {
     int good = 1;
-    add_release(sync, 1u);
     WaitClock clock;
     while (ld_acquire(sync) < target + wb.extra) {
       if (clock.over(wb) || (clock.polls % WaitClock::kEvery == 0 && ld_acquire(sync + 1) != 0u)) {
@@ -83,6 +87,11 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* sync, unsigned int ta
   }
   __syncthreads();
   return ok != 0;
+}
+
+__device__ __forceinline__ bool grid_barrier(unsigned int* sync, unsigned int target, const WaitBound& wb) {
+  grid_arrive(sync);
+  return grid_wait(sync, target, wb);
 }
 
 }  // namespace e2e
