@@ -138,10 +138,19 @@ void drop_cached(int dev, cudaStream_t st) {
 }  // namespace
 
 namespace e2e {
+// Test hook: E2E_TEST_ALLOC_FAIL=lo:hi refuses every request of lo to hi bytes, as
+// a device without that much memory would.
+static bool refused_by_test(size_t bytes) {
+  const char* v = std::getenv("E2E_TEST_ALLOC_FAIL");
+  unsigned long long lo = 0, hi = 0;
+  return v && std::sscanf(v, "%llu:%llu", &lo, &hi) == 2 && bytes >= lo && bytes <= hi;
+}
+
 cudaError_t dalloc(void** p, size_t bytes, cudaStream_t st) {
   cudaMemPool_t pool;
   cudaError_t e = device_pool(&pool);
   if (e != cudaSuccess) return e;
+  if (refused_by_test(bytes)) return cudaErrorMemoryAllocation;
   if (bytes < kCacheMinBytes) return cudaMallocFromPoolAsync(p, bytes ? bytes : 16, pool, st);
   const int dev = current_device();
   if (dev < 0) return cudaErrorInvalidDevice;
@@ -1191,16 +1200,17 @@ e2e_status ensure_pack(const e2e_model* m, double* pack_ms, cudaStream_t st, Pac
   CK(cudaEventRecord(tm->ev[0], st));
   cudaError_t e = build_pack(M, nc, g, del, m->built, ps, st);
   if (e != cudaSuccess) {
+    cudaStreamSynchronize(st);  // (free_pack releases on another stream)
     free_pack(ps);
     delete ps;
     return cuda_fail(e, "build_pack");
   }
+  m->pack = ps;
   CK(cudaEventRecord(tm->ev[1], st));
   if (!timer) {  // else the caller reads the time behind its own synchronisation
     CK(cudaEventSynchronize(tm->ev[1]));
     CK(tm->read(pack_ms));
   }
-  m->pack = ps;
   return E2E_OK;
 }
 
@@ -1337,6 +1347,15 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
   }
   double pack_ms = 0.0;
   PackTimer pack_timer;
+  // The sliced copy stays with the model, which a later call may use or free on
+  // another stream: no exit leaves its fill, or a sweep over it, in flight.
+  struct SyncOnExit {
+    cudaStream_t st;
+    bool done = false;
+    ~SyncOnExit() {
+      if (!done) cudaStreamSynchronize(st);
+    }
+  } settle{st};
   {
     e2e_status ps = ensure_pack(m, &pack_ms, st, &pack_timer);
     if (ps != E2E_OK) return ps;
@@ -1371,10 +1390,8 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
   const int64_t sweep_bytes = csr_sweep_bytes(m);
   CK(cudaEventRecord(e0, st));
   if (o.method == 1) {
-    if (!m->layered || m->ncells <= 0 || m->nt <= 0 || P.nlayers < 2) {
-      CK(cudaStreamSynchronize(st));  // the sliced copy, which stays with the model, is complete
+    if (!m->layered || m->ncells <= 0 || m->nt <= 0 || P.nlayers < 2)
       return fail(E2E_ERR_UNSUPPORTED, "layered solve needs a time-layered model (nt, ncells known)");
-    }
     // all layers, last first, in one cooperative launch
     CK(launch_vi_layered(P, dV, dpi, syncw, gsel, st, tune_layered));
     CK(cudaEventRecord(e2, st));
@@ -1431,6 +1448,7 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
     CK(cudaMemcpyAsync(&herr, syncw + 1, sizeof(herr), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
   }
+  settle.done = true;
   if (herr) return fail(E2E_ERR_DEVICE, "a bounded device-side wait of the sweep gave up");
   CK(pack_timer.read(&pack_ms));
   float ms = 0.f, ms_pass = 0.f;
