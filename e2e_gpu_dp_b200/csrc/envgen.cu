@@ -743,6 +743,7 @@ __global__ void __launch_bounds__(256) k_rr_sumsq(RrBatch b) {
   if (threadIdx.x == 0) t.K->scal[2 * t.m + 1] = s;
 }
 
+constexpr int kMaxBatch = 65535 / 2;  // steps of a batch at most
 constexpr int kRrSegs = 16;  // row segments of the X^T B products at most
 
 // row segments for X^T B / the residual: enough CTAs to cover the SMs for one
@@ -945,7 +946,8 @@ extern "C" e2e_status e2e_env_generate(const e2e_env_params* p, const int32_t* i
     if (kk[q] < r) return fail(E2E_ERR_UNSUPPORTED, "n_modes above the range finder's 64 columns");
     step_doubles += (size_t)nws * nc2[q] + nc2[q] + (size_t)nws * r + (size_t)r * nc2[q] + rr_work_doubles(nws, nc2[q], kk[q]);
   }
-  const int batch = (int)std::min<size_t>((size_t)nt, std::max<size_t>(1, (size_t(2) << 30) / (8 * step_doubles)));
+  // (both fields' matrices of a step are a launch's z index, of which there are 65535)
+  const int batch = (int)std::min<size_t>(std::min(nt, kMaxBatch), std::max<size_t>(1, (size_t(2) << 30) / (8 * step_doubles)));
   double *work, *Om, *sv, *coarse;
   CK(dalloc((void**)&work, sizeof(double) * step_doubles * batch, st));
   scratch.add(work);

@@ -1,0 +1,23 @@
+"""The generator's batches of time steps: a step's fields do not depend on the batch it is in."""
+import numpy as np
+import pytest
+
+from e2e_gpu_dp_b200 import envgen
+
+pytestmark = pytest.mark.gpu
+BY_STEP = [k for k in envgen.FILES if k not in ("all_s_mat", "obstacle_mask")]
+
+
+def _generate(nt, dt):
+    return envgen.build_environment_DG_with_westward_clouds(
+        init_gsize=4, nt=nt, dt=dt, dxy=0.5, A=0.5, A_sc=3.0, eps=0.1, op_nrzns=10, n_wsamples=16,
+        w_range=(np.pi / 10, 8 * np.pi / 10), wx=np.pi, interpolate_degree=2, n_modes=2, dyn_obstacle_data=("None",))
+
+
+def test_more_steps_than_a_launch_dimension_holds():
+    # the times k * 3000 * 2^-10 are exact in both runs
+    many, few = _generate(33001, 2.0 ** -10), _generate(12, 3000 * 2.0 ** -10)
+    for k in BY_STEP:
+        assert np.array_equal(many[k][::3000], few[k]), k
+    for k in ("svals_vel", "svals_phi"):
+        assert np.array_equal(many[k][::3000], few[k]), k
