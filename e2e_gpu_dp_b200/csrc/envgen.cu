@@ -947,9 +947,14 @@ extern "C" e2e_status e2e_env_generate(const e2e_env_params* p, const int32_t* i
     step_doubles += (size_t)nws * nc2[q] + nc2[q] + (size_t)nws * r + (size_t)r * nc2[q] + rr_work_doubles(nws, nc2[q], kk[q]);
   }
   // (both fields' matrices of a step are a launch's z index, of which there are 65535)
-  const int batch = (int)std::min<size_t>(std::min(nt, kMaxBatch), std::max<size_t>(1, (size_t(2) << 30) / (8 * step_doubles)));
+  int batch = (int)std::min<size_t>(std::min(nt, kMaxBatch), std::max<size_t>(1, (size_t(2) << 30) / (8 * step_doubles)));
   double *work, *Om, *sv, *coarse;
-  CK(dalloc((void**)&work, sizeof(double) * step_doubles * batch, st));
+  for (;; batch = (batch + 1) / 2) {  // a device with less free memory takes smaller batches
+    const cudaError_t e = dalloc((void**)&work, sizeof(double) * step_doubles * batch, st);
+    if (e == cudaSuccess) break;
+    if (e != cudaErrorMemoryAllocation || batch == 1) return cuda_fail(e, "work arrays of the rank reductions");
+    cudaGetLastError();
+  }
   scratch.add(work);
   CK(dalloc((void**)&Om, sizeof(double) * (size_t)2 * n * kRrMaxK, st));
   scratch.add(Om);

@@ -1,4 +1,6 @@
 """The generator's batches of time steps: a step's fields do not depend on the batch it is in."""
+import os
+
 import numpy as np
 import pytest
 
@@ -21,3 +23,15 @@ def test_more_steps_than_a_launch_dimension_holds():
         assert np.array_equal(many[k][::3000], few[k]), k
     for k in ("svals_vel", "svals_phi"):
         assert np.array_equal(many[k][::3000], few[k]), k
+
+
+def test_less_memory_than_one_batch_needs():
+    # requests of 1 MB and more are refused: four batches instead of one of 2.5 MB
+    whole = _generate(61, 0.25)
+    os.environ["E2E_TEST_ALLOC_FAIL"] = f"{1 << 20}:{1 << 40}"
+    try:
+        parts = _generate(61, 0.25)
+    finally:
+        os.environ.pop("E2E_TEST_ALLOC_FAIL", None)
+    for k in envgen.FILES + ("svals_vel", "svals_phi"):
+        assert np.array_equal(whole[k], parts[k]), k
