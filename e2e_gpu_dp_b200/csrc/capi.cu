@@ -1267,21 +1267,21 @@ static e2e_status jacobi_by_layers(const e2e_model* m, const e2e_vi_opts& o, flo
   const size_t hist_bytes = sizeof(float) * jacobi_history_floats(nc, L, J);
   // (a layer's history is indexed with 32 bits)
   if (hist_bytes > (size_t(8) << 30) || nc * (int64_t)(J + 32) >= ((int64_t)1 << 31)) return E2E_OK;
+  // one request: the history (whole lines), the residuals of the sweeps and a flag word
+  // per layer, V of the last but one sweep.  Refused, the sweeps still fit.
+  const size_t words = (size_t)J + 2 + (size_t)L, word_bytes = sizeof(unsigned long long) * words;
   DeviceScratch scratch(st);
   float* hist = nullptr;
-  if (dalloc((void**)&hist, hist_bytes, st) != cudaSuccess) {
+  const cudaError_t me = dalloc((void**)&hist, hist_bytes + word_bytes + sizeof(float) * (size_t)ns, st);
+  if (me == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     return E2E_OK;
   }
+  CK(me);
   scratch.add(hist);
-  float* prev = nullptr;
-  unsigned long long* resid = nullptr;
-  CK(dalloc((void**)&prev, sizeof(float) * (size_t)ns, st));
-  scratch.add(prev);
-  const size_t words = (size_t)J + 2 + (size_t)L;  // residuals, then a flag word per layer
-  CK(dalloc((void**)&resid, sizeof(unsigned long long) * words, st));
-  scratch.add(resid);
-  CK(cudaMemsetAsync(resid, 0, sizeof(unsigned long long) * words, st));
+  auto* resid = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(hist) + hist_bytes);
+  float* prev = reinterpret_cast<float*>(resid + words);
+  CK(cudaMemsetAsync(resid, 0, word_bytes, st));
   int dev = 0, sms = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

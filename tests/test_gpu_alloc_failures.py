@@ -12,6 +12,7 @@ import pytest
 
 from e2e_gpu_dp_b200 import api
 from e2e_gpu_dp_b200._lib import E2EError
+from e2e_gpu_dp_b200.problem import FieldSpec, Problem, make_fields
 from tests.helpers import problem
 
 pytestmark = pytest.mark.gpu
@@ -45,4 +46,21 @@ def test_solve_that_fails_after_the_sliced_copy_leaves_it_complete(what):
     assert s1.query()  # nothing of the failed call is still running
     m.solve(method="layered", value=V, policy=pi, stream=s2)
     assert np.array_equal(V.cpu().numpy(), V0) and np.array_equal(pi.cpu().numpy(), pi0)
+    m.free()
+
+
+def test_jacobi_without_memory_for_the_history_sweeps():
+    torch = pytest.importorskip("torch")
+    prob = Problem(gsize=9, nt=130, nrzns=40, nmodes=2, num_ac_angles=4, i_term=6, j_term=3, neighb_gsize=9)
+    m = api.build_model(prob, make_fields(prob, FieldSpec(obstacle_frac=0.05, seed=2)))
+    V = torch.empty(prob.ns, dtype=torch.float32, device="cuda")
+    pi = torch.empty(prob.ns, dtype=torch.int32, device="cuda")
+    V0, pi0, st0 = m.solve(method="jacobi")
+    # everything of the size of the history; then the sizes of one array of values and of the residuals alone
+    for lo, hi in ((1 << 20, 1 << 40), (4 * prob.ns, 4 * prob.ns), (8 * (130 + 2 + 130), 8 * (130 + 2 + 130))):
+        V.fill_(0), pi.fill_(-5)
+        with refuse(lo, hi):
+            _, _, st = m.solve(method="jacobi", value=V, policy=pi)
+        assert np.array_equal(V.cpu().numpy(), V0) and np.array_equal(pi.cpu().numpy(), pi0)
+        assert (st["iterations"], st["residual"]) == (st0["iterations"], st0["residual"])
     m.free()
