@@ -1252,17 +1252,53 @@ static e2e_status fp64_check(const e2e_model* m, const float* dV, e2e_vi_stats* 
   return E2E_OK;
 }
 
-// The Jacobi iteration of a layered model without one sweep after another
-// (jacobi.cu).  *done false: not taken (no layers, a wall-clock limit, which is
-// checked between sweeps, or no memory for the history), nothing changed.
+static int jacobi_max_iter(const e2e_model* m, const e2e_vi_opts& o) {
+  return o.max_iter > 0 ? o.max_iter : (m->nt > 0 ? m->nt + 2 : 100000);
+}
+
+// How a Jacobi solve goes on a model: sweep after sweep for `first` sweeps, then
+// every sweep of a layer at once (jacobi.cu) if `layers`.
+struct JacobiWay {
+  bool layers = false;
+  int first = 0;
+};
+
+// All sweeps of a layer at once cost about the same however early the iteration
+// ends; sweeps cost by their number.  Both measured on B200, in microseconds with
+// the host's part (3e4 to 1.8e8 entries, 3 to 300 layers, 1 to all sweeps): a
+// layer 10 and 36 per million entries, a sweep 25 and 1.8 per million, the sliced
+// copy that the sweeps need 7 per million.  They meet at 20 of 120 sweeps on
+// 200x200x120 with 16 actions (6.4 ms), 18 of 40 on 100x100x40 (0.74 ms), 12 of 30
+// on 50x50x30 (0.35 ms).  Fewer sweeps than that (max_iter; few large layers)
+// are taken one after another.  A threshold can end the iteration
+// anywhere; one that is small beside the rewards ends it when the last layers'
+// values have come through all others, and others, at the first sweep as a rule
+// (200x200x120: a threshold of 50 or 2 takes 120 sweeps, one of 101 a single one),
+// get a tenth of that number of sweeps first (or all, where the layers are few).
+static JacobiWay jacobi_way(const e2e_model* m, const e2e_vi_opts& o) {
+  JacobiWay w;
+  const int64_t ns = m->ns, nc = m->ncells;
+  // (a wall-clock limit is checked between sweeps)
+  if (!m->layered || nc <= 0 || ns % nc != 0 || m->na > 32 || o.timeout_s > 0) return w;
+  const int64_t L = ns / nc;
+  if (L < 3 || L > 4096 || m->n_row_states > ns - nc) return w;
+  const double entries = 1e-6 * (double)m->nnz;
+  const double meet = (10.0 * (double)L + (m->pack ? 36.0 : 29.0) * entries) / (25.0 + 1.8 * entries);
+  if ((double)std::min<int64_t>(jacobi_max_iter(m, o), L) < meet) return w;
+  w.layers = true;
+  const double reward = m->has_prob ? std::max(std::fabs(m->prob.r_outbound), std::fabs(m->prob.r_terminal)) : 10.0;
+  if (!(o.threshold <= 0.01 * reward)) w.first = std::max(1, (int)(0.1 * meet));
+  if (3 * w.first >= L) w.layers = false;
+  return w;
+}
+
+// The Jacobi iteration of a layered model (jacobi_way) without one sweep after
+// another.  *done false: no memory for the history, nothing changed.
 static e2e_status jacobi_by_layers(const e2e_model* m, const e2e_vi_opts& o, float* dV, int32_t* dpi,
                                    e2e_vi_stats* stats, cudaStream_t st, bool* done) {
   *done = false;
   const int64_t ns = m->ns, nc = m->ncells;
-  if (!m->layered || nc <= 0 || ns % nc != 0 || m->na > 32 || o.timeout_s > 0) return E2E_OK;
-  const int64_t L64 = ns / nc;
-  if (L64 < 3 || L64 > 4096 || m->n_row_states > ns - nc) return E2E_OK;
-  const int L = (int)L64, max_iter = o.max_iter > 0 ? o.max_iter : (m->nt > 0 ? m->nt + 2 : 100000);
+  const int L = (int)(ns / nc), max_iter = jacobi_max_iter(m, o);
   const int J = std::min(max_iter, L);
   const size_t hist_bytes = sizeof(float) * jacobi_history_floats(nc, L, J);
   // (a layer's history is indexed with 32 bits)
@@ -1340,7 +1376,10 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
   const bool tune_given = (o.schedule & 0x100) != 0;
   const int tune_layered = tune_given ? (o.schedule >> 4) & 15 : -1;
   const int tune_jacobi = tune_given ? (o.schedule >> 4) & 15 : VI_TUNE_LEAN;
-  if (o.method == 0 && !tune_given) {
+  JacobiWay way;
+  if (o.method == 0 && !tune_given) way = jacobi_way(m, o);
+  if (way.layers && way.first == 0) {
+    way.layers = false;
     bool done = false;
     e2e_status js = jacobi_by_layers(m, o, dV, dpi, stats, st, &done);
     if (done || js != E2E_OK) return js;
@@ -1365,7 +1404,7 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
   DeviceScratch scratch(st);
   float* W = nullptr;
   unsigned long long* resid = nullptr;
-  const int max_iter = o.max_iter > 0 ? o.max_iter : (m->nt > 0 ? m->nt + 2 : 100000);
+  const int max_iter = jacobi_max_iter(m, o);
   CK(dalloc((void**)&W, sizeof(float) * (size_t)ns, st));
   scratch.add(W);
   CK(dalloc((void**)&resid, sizeof(unsigned long long) * (size_t)(max_iter + 3), st));
@@ -1415,6 +1454,25 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
     bool done = false;
     while (!done) {
       if (iters >= max_iter) break;
+      if (way.layers && iters == way.first) {
+        way.layers = false;
+        bool by_layers = false;
+        e2e_status js = jacobi_by_layers(m, o, dV, dpi, stats, st, &by_layers);
+        if (js != E2E_OK) return js;
+        if (by_layers) {
+          CK(cudaEventRecord(e1, st));
+          CK(cudaStreamSynchronize(st));
+          settle.done = true;
+          float ms = 0.f;
+          CK(cudaEventElapsedTime(&ms, e0, e1));
+          CK(pack_timer.read(&pack_ms));
+          if (stats) {
+            stats->seconds = ms * 1e-3;
+            stats->pack_ms = pack_ms;
+          }
+          return E2E_OK;
+        }
+      }
       ++iters;
       CK(launch_vi_chunks(P, 0, P.nchunks, a, b, dpi, resid + iters, st, tune_jacobi, syncw + 1));
       unsigned long long h = 0;
