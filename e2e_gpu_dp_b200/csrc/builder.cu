@@ -174,10 +174,11 @@ __device__ __forceinline__ void vel_pairs4(const float2* md, const float* y0, in
   }
 }
 
-// K1 on one tile (32 cells of layer T and all their actions) by one CTA.
-template <typename CntT, bool UNIT>
+// K1 on one tile (32 cells of layer T and all their actions) by one CTA; LISTED:
+// the warps' groups are slots tile * warps ... of the layer's n_listed listed ones.
+template <typename CntT, bool UNIT, bool LISTED>
 __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* smem, const int T, const int tile,
-                                           const int n_listed = -1) {
+                                           const int n_listed) {
   const DevProblem& P = A.P;
   const int nthr = blockDim.x;
   const int tid = threadIdx.x;
@@ -198,7 +199,7 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
       const int cpw_log2 = 5 - lanes_log2;
       const int slot = tile * nwarps + (tid >> cpw_log2);
       int64_t grp = A.etiles_per_layer;  // a listed launch's unused warp: cells beyond the layer
-      if (n_listed < 0) grp = group_of_slot(slot, g, 1 << cpw_log2);
+      if (!LISTED) grp = group_of_slot(slot, g, 1 << cpw_log2);
       else if (slot < n_listed) grp = A.defer_list[(int64_t)T * A.etiles_per_layer + slot];
       cell_tab[tid] = (int)((grp << cpw_log2) + (tid & ((1 << cpw_log2) - 1)));
     }
@@ -918,30 +919,46 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
   }
 }
 
-// K1 over a grid of (tile, layer - t0) CTAs; or, with a list from the ranked
-// builder, resident CTAs striding over the listed tiles, a CTA's warps taking
-// tiles of one layer.
+// K1 over a grid of (tile, layer - t0) CTAs.
 template <typename CntT, bool UNIT>
 __global__ void __launch_bounds__(1024) k_build_tiles(BuildArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const bool listed = A.defer_count != nullptr;
-  int T = A.t0 + (int)blockIdx.y, tile = (int)blockIdx.x, n = -1;
-  if (listed && A.counters[CTR_DEFERRED] == 0ull) return;
-  int64_t before = 0;  // items of the layers before T
-  const int nwarps = blockDim.x >> 5;
-  for (int64_t item = blockIdx.x;; item += gridDim.x) {
-    if (listed) {
-      for (; T < A.t1; ++T) {
-        n = (int)A.defer_count[T];
-        const int items = (n + nwarps - 1) / nwarps;
-        if (item < before + items) break;
-        before += items;
+  build_tile<CntT, UNIT, false>(A, smem, A.t0 + (int)blockIdx.y, (int)blockIdx.x, 0);
+}
+
+// K1 over the tiles that the ranked builder listed: resident CTAs striding over
+// them, a CTA's warps taking tiles of one layer.  A kernel of its own, with the
+// position in the list in shared memory: in one kernel with the grid above, the
+// position cost that one registers (120x120x24, 12 modes, 16 actions: 7.35 ms in
+// one, 7.2 apart).
+template <typename CntT, bool UNIT>
+__global__ void __launch_bounds__(1024) k_build_listed(BuildArgs A) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ struct {
+    int T, tile, n;
+    int64_t item, before;  // items: the CTA's next one, those of the layers before T
+  } at;
+  if (A.counters[CTR_DEFERRED] == 0ull) return;
+  if (threadIdx.x == 0) {
+    at.T = A.t0;
+    at.item = blockIdx.x;
+    at.before = 0;
+  }
+  for (;;) {
+    if (threadIdx.x == 0) {
+      const int nwarps = blockDim.x >> 5;
+      for (; at.T < A.t1; ++at.T) {
+        at.n = (int)A.defer_count[at.T];
+        const int items = (at.n + nwarps - 1) / nwarps;
+        if (at.item < at.before + items) break;
+        at.before += items;
       }
-      if (T >= A.t1) return;
-      tile = (int)(item - before);
+      at.tile = (int)(at.item - at.before);
+      at.item += gridDim.x;
     }
-    build_tile<CntT, UNIT>(A, smem, T, tile, n);
-    if (!listed) return;
+    __syncthreads();
+    if (at.T >= A.t1) return;
+    build_tile<CntT, UNIT, true>(A, smem, at.T, at.tile, at.n);
     __syncthreads();  // the shared memory is free for the next tile
   }
 }
@@ -1141,18 +1158,20 @@ static cudaError_t raise_smem_cap(K kern, size_t sm, int* cap_set, std::mutex& m
 
 template <typename CntT, bool UNIT>
 static cudaError_t launch_one(const BuildArgs& A, int n_layers, cudaStream_t st) {
+  const bool listed = A.defer_count != nullptr;
+  auto kern = listed ? k_build_listed<CntT, UNIT> : k_build_tiles<CntT, UNIT>;
   dim3 grid((unsigned)A.tiles_per_layer, (unsigned)n_layers);
-  if (A.defer_count) {  // resident CTAs: about two an SM
+  if (listed) {  // resident CTAs: about two an SM
     const int64_t most = (int64_t)A.tiles_per_layer * n_layers;
     grid = dim3((unsigned)std::min<int64_t>(most, 296));
   }
   dim3 block((unsigned)(32u << A.lanes_log2));
   const size_t sm = build_smem_bytes(A.P.na, A.P.nm, A.rc, UNIT, A.ybufs);
   static std::mutex mu;
-  static int cap_set[64] = {};
-  cudaError_t e = raise_smem_cap(k_build_tiles<CntT, UNIT>, sm, cap_set, mu);
+  static int cap_set[2][64] = {};
+  cudaError_t e = raise_smem_cap(kern, sm, cap_set[listed], mu);
   if (e != cudaSuccess) return e;
-  k_build_tiles<CntT, UNIT><<<grid, block, sm, st>>>(A);
+  kern<<<grid, block, sm, st>>>(A);
   return cudaGetLastError();
 }
 
