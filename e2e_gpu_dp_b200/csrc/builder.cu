@@ -175,10 +175,11 @@ __device__ __forceinline__ void vel_pairs4(const float2* md, const float* y0, in
 }
 
 // K1 on one tile (32 cells of layer T and all their actions) by one CTA; LISTED:
-// the warps' groups are slots tile * warps ... of the layer's n_listed listed ones.
+// the warps' groups are slots tile * warps ... of the layer's listed ones, n_edge near
+// the edge and n_listed in all, in the order of group_of_slot: near the edge first.
 template <typename CntT, bool UNIT, bool LISTED>
 __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* smem, const int T, const int tile,
-                                           const int n_listed) {
+                                           const int n_edge, const int n_listed) {
   const DevProblem& P = A.P;
   const int nthr = blockDim.x;
   const int tid = threadIdx.x;
@@ -200,7 +201,8 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
       const int slot = tile * nwarps + (tid >> cpw_log2);
       int64_t grp = A.etiles_per_layer;  // a listed launch's unused warp: cells beyond the layer
       if (!LISTED) grp = group_of_slot(slot, g, 1 << cpw_log2);
-      else if (slot < n_listed) grp = A.defer_list[(int64_t)T * A.etiles_per_layer + slot];
+      else if (slot < n_listed)
+        grp = A.defer_list[(T + (slot < n_edge ? 0 : 1)) * A.etiles_per_layer + (slot < n_edge ? slot : n_edge - 1 - slot)];
       cell_tab[tid] = (int)((grp << cpw_log2) + (tid & ((1 << cpw_log2) - 1)));
     }
     __syncthreads();
@@ -923,42 +925,42 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
 template <typename CntT, bool UNIT>
 __global__ void __launch_bounds__(1024) k_build_tiles(BuildArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  build_tile<CntT, UNIT, false>(A, smem, A.t0 + (int)blockIdx.y, (int)blockIdx.x, 0);
+  build_tile<CntT, UNIT, false>(A, smem, A.t0 + (int)blockIdx.y, (int)blockIdx.x, 0, 0);
 }
 
-// K1 over the tiles that the ranked builder listed: resident CTAs striding over
-// them, a CTA's warps taking tiles of one layer.  A kernel of its own, with the
-// position in the list in shared memory: in one kernel with the grid above, the
-// position cost that one registers (120x120x24, 12 modes, 16 actions: 7.35 ms in
-// one, 7.2 apart).
+// K1 over the tiles that the ranked builder listed: as many CTAs as are resident, each
+// taking a CTA's worth of one layer's list at a time from a counter.  A kernel of
+// its own, with the position in the list in shared memory: in one kernel with the
+// grid above, the position cost that one registers (120x120x24, 12 modes, 16
+// actions: 7.35 ms in one, 7.2 apart).
 template <typename CntT, bool UNIT>
 __global__ void __launch_bounds__(1024) k_build_listed(BuildArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ struct {
-    int T, tile, n;
-    int64_t item, before;  // items: the CTA's next one, those of the layers before T
+    int T, tile, n_edge, n;
+    int64_t before;  // items of the layers before T
   } at;
   if (A.counters[CTR_DEFERRED] == 0ull) return;
   if (threadIdx.x == 0) {
     at.T = A.t0;
-    at.item = blockIdx.x;
     at.before = 0;
   }
   for (;;) {
     if (threadIdx.x == 0) {
       const int nwarps = blockDim.x >> 5;
+      const int64_t item = (int64_t)atomicAdd(A.counters + CTR_NEXT, 1ull);  // (grows from one turn to the next)
       for (; at.T < A.t1; ++at.T) {
-        at.n = (int)A.defer_count[at.T];
+        at.n_edge = (int)A.defer_count[2 * at.T];
+        at.n = at.n_edge + (int)A.defer_count[2 * at.T + 1];
         const int items = (at.n + nwarps - 1) / nwarps;
-        if (at.item < at.before + items) break;
+        if (item < at.before + items) break;
         at.before += items;
       }
-      at.tile = (int)(at.item - at.before);
-      at.item += gridDim.x;
+      at.tile = (int)(item - at.before);
     }
     __syncthreads();
     if (at.T >= A.t1) return;
-    build_tile<CntT, UNIT, true>(A, smem, at.T, at.tile, at.n);
+    build_tile<CntT, UNIT, true>(A, smem, at.T, at.tile, at.n_edge, at.n);
     __syncthreads();  // the shared memory is free for the next tile
   }
 }
@@ -1161,9 +1163,12 @@ static cudaError_t launch_one(const BuildArgs& A, int n_layers, cudaStream_t st)
   const bool listed = A.defer_count != nullptr;
   auto kern = listed ? k_build_listed<CntT, UNIT> : k_build_tiles<CntT, UNIT>;
   dim3 grid((unsigned)A.tiles_per_layer, (unsigned)n_layers);
-  if (listed) {  // resident CTAs: about two an SM
-    const int64_t most = (int64_t)A.tiles_per_layer * n_layers;
-    grid = dim3((unsigned)std::min<int64_t>(most, 296));
+  if (listed) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    grid = dim3((unsigned)std::min<int64_t>((int64_t)A.tiles_per_layer * n_layers, (int64_t)A.ctas_per_sm * sms));
   }
   dim3 block((unsigned)(32u << A.lanes_log2));
   const size_t sm = build_smem_bytes(A.P.na, A.P.nm, A.rc, UNIT, A.ybufs);

@@ -42,6 +42,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "rank_plan.h"
+#include "tile_order.h"
 
 namespace e2e {
 
@@ -428,9 +429,11 @@ __device__ __forceinline__ void finish_tile(const BuildArgs& A, const RankArgs& 
     }
   }
   if (__any_sync(0xffffffffu, !ok)) {  // the tile goes to the general builder
+    const bool inner = !__any_sync(0xffffffffu, valid && in_edge_band(i1, j1, g));
     if (lane == 0) {
-      const unsigned at = atomicAdd(A.defer_count + T, 1u);
-      A.defer_list[(int64_t)T * K.etiles_per_layer + at] = (int32_t)et;
+      const int64_t at = atomicAdd(A.defer_count + 2 * T + inner, 1u);
+      const int64_t first = (int64_t)T * K.etiles_per_layer;
+      A.defer_list[inner ? first + K.etiles_per_layer - 1 - at : first + at] = (int32_t)et;
       atomicAdd(A.counters + CTR_DEFERRED, 1ull);
     }
     return;

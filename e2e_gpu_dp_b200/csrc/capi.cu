@@ -763,10 +763,9 @@ e2e_status plan_build(const e2e_problem* p, int count_bits, int64_t stage_hint, 
   pl->ybufs = 1;
   {
     const size_t sm2 = build_smem_bytes(pl->na, p->nmodes, pl->rc, unit, 2);
-    if (sm2 <= 220 * 1024) {
-      const int c1 = build_ctas_per_sm(pl->na, sm, unit);
-      if (c1 > 0 && build_ctas_per_sm(pl->na, sm2, unit) >= c1) pl->ybufs = 2;
-    }
+    const int c1 = build_ctas_per_sm(pl->na, sm, unit);
+    if (sm2 <= 220 * 1024 && c1 > 0 && build_ctas_per_sm(pl->na, sm2, unit) >= c1) pl->ybufs = 2;
+    pl->ctas_per_sm = std::max(1, c1);
   }
   if (pl->tiles_per_layer > 0x7fffffff || p->nt - 1 > 65535)
     return fail(E2E_ERR_UNSUPPORTED, "grid too large for one launch");
@@ -851,7 +850,7 @@ e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, cudaSt
   CK(take(sizeof(float) * layers * nmp * (size_t)K.nrp, &yt));
   CK(take(sizeof(float) * layers * nmp * 2, &ystat));
   CK(take(sizeof(uint32_t) * layers * (size_t)p->gsize * (size_t)K.owords, &obits));
-  CK(take(sizeof(unsigned int) * layers, &count));
+  CK(take(sizeof(unsigned int) * 2 * layers, &count));
   CK(take(sizeof(int32_t) * (size_t)pl.n_tiles, &list));
   K.plan = static_cast<const uint32_t*>(plan);
   K.yt = static_cast<const float*>(yt);
@@ -872,7 +871,7 @@ cudaError_t launch_layers(const BuildArgs& A, const BuildPlan& pl, const LayerBu
   RankArgs R = L.K;
   R.t0 = t0;
   R.t1 = t1;
-  cudaError_t e = cudaMemsetAsync(L.defer_count + t0, 0, sizeof(unsigned int) * (size_t)(t1 - t0), st);
+  cudaError_t e = cudaMemsetAsync(L.defer_count + 2 * t0, 0, sizeof(unsigned int) * 2 * (size_t)(t1 - t0), st);
   if (e == cudaSuccess) e = launch_rank_prepare(A.P, A.F, R, st);
   return e != cudaSuccess ? e : launch_build_ranks(B, R, st);
 }
@@ -885,6 +884,7 @@ cudaError_t launch_leftover(const BuildArgs& A, const BuildPlan& pl, const Layer
   B.t1 = t1;
   B.defer_count = L.defer_count;
   B.defer_list = L.defer_list;
+  B.ctas_per_sm = pl.ctas_per_sm;
   return launch_build_tiles(B, pl.count_bits, t1 - t0, st);
 }
 

@@ -18,6 +18,7 @@ enum : int {
   CTR_POOL = 4,           // dense-histogram pool slots requested
   CTR_FLAGS = 5,          // error flags
   CTR_DEFERRED = 6,       // emission tiles the ranked builder left to the general one
+  CTR_NEXT = 7,           // those the general builder has taken (in CTAs' worth)
   CTR_COUNT = 8
 };
 enum : unsigned int { FLAG_POOL_EXHAUSTED = 1u };
@@ -27,10 +28,13 @@ struct BuildArgs {
   DevFields F;
   int t0, t1;           // layers of this launch: t0 + blockIdx.y (t1: end, for listed tiles)
   int64_t etiles_per_layer;      // emission tiles (warps' groups of cells) per layer
-  // null, or the emission tiles left by the ranked builder: per layer their
-  // number and, from T * etiles_per_layer on, their indices in the layer
+  // null, or the emission tiles left by the ranked builder: per layer the numbers of
+  // those near the grid's edge (in_edge_band) and of the others, and from
+  // T * etiles_per_layer on their indices in the layer, the first from the front and
+  // the second from the back
   unsigned int* defer_count;
   int32_t* defer_list;
+  int ctas_per_sm;      // general builder CTAs that an SM holds
   int tiles_per_layer;  // CTAs per layer = ceil(ncells / 32); emission tiles are warps
   int rc;               // realisations per warp-private velocity chunk
   int ybufs;            // chunk coefficient buffers in shared memory: 1, or 2 (one CTA barrier a chunk)

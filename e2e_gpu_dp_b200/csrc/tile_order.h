@@ -24,6 +24,10 @@ namespace e2e {
 // grid has no interior.
 static constexpr int kEdgeBand = 7;  // window reach (kWin / 2 + 1) plus a mean-flow drift of two cells
 
+E2E_TILE_ORDER_FN bool in_edge_band(int i, int j, int g) {
+  return i < kEdgeBand || j < kEdgeBand || i >= g - kEdgeBand || j >= g - kEdgeBand;
+}
+
 E2E_TILE_ORDER_FN int64_t group_of_slot(int64_t s, int g, int cpw) {
   const int64_t gq = g / cpw, ngroups = (int64_t)g * gq;
   const int qlo = (kEdgeBand + cpw - 1) / cpw, qhi = (g - kEdgeBand) / cpw - 1;
