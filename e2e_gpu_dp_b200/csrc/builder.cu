@@ -535,7 +535,9 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
           mode = MODE_LOST;
         }
       }
-      if (mode == MODE_DENSE) dense[di * P.m + dj] += 1u;
+      // (the row's own, but as a reduction the lane need not wait for the old count:
+      // 120x120x24, wide noise, 16 actions 97 -> 77 ms a build)
+      if (mode == MODE_DENSE) atomicAdd(dense + di * P.m + dj, 1u);
     } else {
       n_drop++;
       if (di < P.m && dj < P.m) n_misbin++;
