@@ -175,11 +175,10 @@ __device__ __forceinline__ void vel_pairs4(const float2* md, const float* y0, in
 }
 
 // K1 on one tile (32 cells of layer T and all their actions) by one CTA; LISTED:
-// the warps' groups are slots tile * warps ... of the layer's listed ones, n_edge near
-// the edge and n_listed in all, in the order of group_of_slot: near the edge first.
+// the warps' groups are listed[warp].
 template <typename CntT, bool UNIT, bool LISTED>
 __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* smem, const int T, const int tile,
-                                           const int n_edge, const int n_listed) {
+                                           const int* listed) {
   const DevProblem& P = A.P;
   const int nthr = blockDim.x;
   const int tid = threadIdx.x;
@@ -192,17 +191,14 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
   const int cl = warp * (32 >> lanes_log2) + cw; // cell within tile (0..31)
   const int g = P.g;
   const int64_t nc = (int64_t)g * g;
-  // the cells of the tile's warps' groups (group_of_slot, or the list), local
+  // the cells of the tile's warps' groups (group_of_slot, or listed), local
   // cell l at cell_tab[l]
   __shared__ int cell_tab[32];
   {
     if (tid < 32) {
       const int cpw_log2 = 5 - lanes_log2;
-      const int slot = tile * nwarps + (tid >> cpw_log2);
-      int64_t grp = A.etiles_per_layer;  // a listed launch's unused warp: cells beyond the layer
-      if (!LISTED) grp = group_of_slot(slot, g, 1 << cpw_log2);
-      else if (slot < n_listed)
-        grp = A.defer_list[(T + (slot < n_edge ? 0 : 1)) * A.etiles_per_layer + (slot < n_edge ? slot : n_edge - 1 - slot)];
+      const int64_t grp = LISTED ? listed[tid >> cpw_log2]
+                                 : group_of_slot(tile * nwarps + (tid >> cpw_log2), g, 1 << cpw_log2);
       cell_tab[tid] = (int)((grp << cpw_log2) + (tid & ((1 << cpw_log2) - 1)));
     }
     __syncthreads();
@@ -927,34 +923,88 @@ __device__ __forceinline__ void build_tile(const BuildArgs& A, unsigned char* sm
 template <typename CntT, bool UNIT>
 __global__ void __launch_bounds__(1024) k_build_tiles(BuildArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  build_tile<CntT, UNIT, false>(A, smem, A.t0 + (int)blockIdx.y, (int)blockIdx.x, 0, 0);
+  build_tile<CntT, UNIT, false>(A, smem, A.t0 + (int)blockIdx.y, (int)blockIdx.x, nullptr);
 }
 
-// K1 over the tiles that the ranked builder listed: as many CTAs as are resident, each
-// taking a CTA's worth of one layer's list at a time from a counter.  A kernel of
-// its own, with the position in the list in shared memory: in one kernel with the
-// grid above, the position cost that one registers (120x120x24, 12 modes, 16
+// The nwarps left-over tiles of layer T from the lo-th on, in the order of
+// group_of_slot (near the edge first, n_edge of them, each kind by index), to
+// groups[]; etiles_per_layer where there are no more.  By the whole CTA: a thread
+// counts the marks of a run of tiles, and its tiles' places follow from the counts
+// before it.
+__device__ __forceinline__ void left_over_groups(const BuildArgs& A, int T, int lo, int n_edge, int* groups) {
+  __shared__ int2 sums[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int n = (int)A.etiles_per_layer, run = ((n + (int)blockDim.x - 1) / (int)blockDim.x + 3) & ~3;
+  const uint8_t* marks = A.defer_flag + T * defer_stride(n);
+  auto word = [&](int k) -> uint32_t {  // of tiles k .. k + 3
+    if (k >= n) return 0u;
+    const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(marks + k));
+    return k + 4 <= n ? w : w & ((1u << (8 * (n - k))) - 1u);
+  };
+  int2 c = make_int2(0, 0);
+  for (int k = tid * run; k < (tid + 1) * run; k += 4) {
+    const uint32_t w = word(k);
+    c.x += __popc(w & 0x01010101u);
+    c.y += __popc(w & 0x02020202u);
+  }
+  int2 end = c;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, end.x, o), y = __shfl_up_sync(0xffffffffu, end.y, o);
+    if (lane >= o) {
+      end.x += x;
+      end.y += y;
+    }
+  }
+  if (lane == 31) sums[warp] = end;
+  if (tid < nwarps) groups[tid] = n;
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) {
+    end.x += sums[w].x;
+    end.y += sums[w].y;
+  }
+  int edge = end.x - c.x, inner = n_edge + end.y - c.y;
+  if ((edge < lo + nwarps && end.x > lo) || (inner < lo + nwarps && n_edge + end.y > lo)) {
+    for (int k = tid * run; k < (tid + 1) * run; k += 4) {
+      uint32_t w = word(k);
+      for (int b = 0; w; ++b, w >>= 8) {
+        const uint32_t m = w & 255u;
+        if (m == TILE_BUILT) continue;
+        const int at = (m == TILE_EDGE ? edge++ : inner++) - lo;
+        if (at >= 0 && at < nwarps) groups[at] = k + b;
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// K1 over the tiles that the ranked builder left over: as many CTAs as are resident,
+// each taking a CTA's worth of one layer's tiles at a time from a counter, in the
+// order of the grid above: neighbours, which need about the same time, fill a CTA,
+// whose warps wait for each other at every chunk (120x120x24, 1000 realisations, wide
+// noise: in the order they were left over 77 ms a build with 16 actions and 141 with
+// 24, so 64 and 108).  A kernel of its own, with its position in shared memory: in
+// one kernel with the grid above, the position cost that one registers (12 modes, 16
 // actions: 7.35 ms in one, 7.2 apart).
 template <typename CntT, bool UNIT>
 __global__ void __launch_bounds__(1024) k_build_listed(BuildArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ struct {
-    int T, tile, n_edge, n;
+    int T, tile, n_edge;
     int64_t before;  // items of the layers before T
+    int groups[32];
   } at;
   if (A.counters[CTR_DEFERRED] == 0ull) return;
   if (threadIdx.x == 0) {
     at.T = A.t0;
     at.before = 0;
   }
+  const int nwarps = blockDim.x >> 5;
   for (;;) {
     if (threadIdx.x == 0) {
-      const int nwarps = blockDim.x >> 5;
       const int64_t item = (int64_t)atomicAdd(A.counters + CTR_NEXT, 1ull);  // (grows from one turn to the next)
       for (; at.T < A.t1; ++at.T) {
         at.n_edge = (int)A.defer_count[2 * at.T];
-        at.n = at.n_edge + (int)A.defer_count[2 * at.T + 1];
-        const int items = (at.n + nwarps - 1) / nwarps;
+        const int items = (at.n_edge + (int)A.defer_count[2 * at.T + 1] + nwarps - 1) / nwarps;
         if (item < at.before + items) break;
         at.before += items;
       }
@@ -962,7 +1012,8 @@ __global__ void __launch_bounds__(1024) k_build_listed(BuildArgs A) {
     }
     __syncthreads();
     if (at.T >= A.t1) return;
-    build_tile<CntT, UNIT, true>(A, smem, at.T, at.tile, at.n_edge, at.n);
+    left_over_groups(A, at.T, at.tile * nwarps, at.n_edge, at.groups);
+    build_tile<CntT, UNIT, true>(A, smem, at.T, at.tile, at.groups);
     __syncthreads();  // the shared memory is free for the next tile
   }
 }

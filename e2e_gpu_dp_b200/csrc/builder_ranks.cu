@@ -428,16 +428,17 @@ __device__ __forceinline__ void finish_tile(const BuildArgs& A, const RankArgs& 
       }
     }
   }
+  uint8_t* const left = A.defer_flag + T * defer_stride(K.etiles_per_layer) + et;
   if (__any_sync(0xffffffffu, !ok)) {  // the tile goes to the general builder
     const bool inner = !__any_sync(0xffffffffu, valid && in_edge_band(i1, j1, g));
     if (lane == 0) {
-      const int64_t at = atomicAdd(A.defer_count + 2 * T + inner, 1u);
-      const int64_t first = (int64_t)T * K.etiles_per_layer;
-      A.defer_list[inner ? first + K.etiles_per_layer - 1 - at : first + at] = (int32_t)et;
+      *left = inner ? TILE_INNER : TILE_EDGE;
+      atomicAdd(A.defer_count + 2 * T + inner, 1u);
       atomicAdd(A.counters + CTR_DEFERRED, 1ull);
     }
     return;
   }
+  if (lane == 0) *left = TILE_BUILT;
   float sumR = 0.f;
   uint32_t n_drop = 0, n_misbin = 0;
   if (window) {

@@ -843,7 +843,7 @@ e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, cudaSt
     if (e == cudaSuccess) scratch->add(*q);
     return e;
   };
-  void *plan, *yt, *ystat, *obits, *count, *list;
+  void *plan, *yt, *ystat, *obits, *count, *flag;
   const size_t pb = sizeof(uint32_t) * pl.rank_words.size();
   CK(take(pb, &plan));
   CK(cudaMemcpyAsync(plan, pl.rank_words.data(), pb, cudaMemcpyHostToDevice, st));
@@ -851,13 +851,13 @@ e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, cudaSt
   CK(take(sizeof(float) * layers * nmp * 2, &ystat));
   CK(take(sizeof(uint32_t) * layers * (size_t)p->gsize * (size_t)K.owords, &obits));
   CK(take(sizeof(unsigned int) * 2 * layers, &count));
-  CK(take(sizeof(int32_t) * (size_t)pl.n_tiles, &list));
+  CK(take(layers * (size_t)defer_stride(pl.etiles_per_layer), &flag));
   K.plan = static_cast<const uint32_t*>(plan);
   K.yt = static_cast<const float*>(yt);
   K.ystat = static_cast<const float*>(ystat);
   K.obits = static_cast<const uint32_t*>(obits);
   L->defer_count = static_cast<unsigned int*>(count);
-  L->defer_list = static_cast<int32_t*>(list);
+  L->defer_flag = static_cast<uint8_t*>(flag);
   return E2E_OK;
 }
 
@@ -867,7 +867,7 @@ cudaError_t launch_layers(const BuildArgs& A, const BuildPlan& pl, const LayerBu
   B.t1 = t1;
   if (!pl.ranked) return launch_build_tiles(B, pl.count_bits, t1 - t0, st);
   B.defer_count = L.defer_count;
-  B.defer_list = L.defer_list;
+  B.defer_flag = L.defer_flag;
   RankArgs R = L.K;
   R.t0 = t0;
   R.t1 = t1;
@@ -883,7 +883,7 @@ cudaError_t launch_leftover(const BuildArgs& A, const BuildPlan& pl, const Layer
   B.t0 = t0;
   B.t1 = t1;
   B.defer_count = L.defer_count;
-  B.defer_list = L.defer_list;
+  B.defer_flag = L.defer_flag;
   B.ctas_per_sm = pl.ctas_per_sm;
   return launch_build_tiles(B, pl.count_bits, t1 - t0, st);
 }

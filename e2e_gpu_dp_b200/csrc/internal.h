@@ -131,7 +131,7 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
 struct LayerBuild {
   RankArgs K{};
   unsigned int* defer_count = nullptr;
-  int32_t* defer_list = nullptr;
+  uint8_t* defer_flag = nullptr;
 };
 e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, cudaStream_t st, DeviceScratch* scratch,
                                LayerBuild* L);
