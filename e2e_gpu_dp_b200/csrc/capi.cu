@@ -920,9 +920,7 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
   if (s != E2E_OK) return s;
 
   int64_t cap = pl.stage_cap, pool_units = pl.pool_units;
-  int32_t* stage_col = nullptr;
-  void* stage_cnt = nullptr;
-  uint32_t* pool = nullptr;
+  BuildStaging buf(st);
   unsigned long long hc[CTR_COUNT];
   const int mm = p->neighb_gsize * p->neighb_gsize;
   cudaEvent_t ev[4];
@@ -934,11 +932,7 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
   } evfree{ev};
   trace_mark("setup");
   for (int attempt = 0; attempt < 3; ++attempt) {
-    if (!stage_col) {
-      CK(dalloc((void**)&stage_col, sizeof(int32_t) * (size_t)cap, st));
-      CK(dalloc((void**)&stage_cnt, (size_t)cbytes * (size_t)cap, st));
-    }
-    if (!pool) CK(dalloc((void**)&pool, sizeof(uint32_t) * (size_t)mm * (size_t)pool_units, st));
+    CK(buf.provide(cap, (size_t)cbytes, pool_units, p->neighb_gsize));
     CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * CTR_COUNT, st));
     BuildArgs A{};
     A.P = D;
@@ -950,8 +944,8 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
     A.rc = pl.rc;
     A.ybufs = pl.ybufs;
     A.lanes_log2 = build_lanes_log2(pl.na);
-    A.stage_col = stage_col;
-    A.stage_cnt = stage_cnt;
+    A.stage_col = static_cast<int32_t*>(buf.col);
+    A.stage_cnt = buf.cnt;
     A.stage_cap = cap;
     A.counters = ctr;
     A.row_off = row_off;
@@ -959,7 +953,7 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
     A.tile_len = tile_len;
     A.R = m->R;
     A.sumR = m->sumR;
-    A.pool = pool;
+    A.pool = static_cast<uint32_t*>(buf.pool);
     A.pool_units = pool_units;
     auto build_layers = [&](int t0, int t1) -> cudaError_t {
       m->build_launches++;
@@ -1027,27 +1021,20 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
     trace_mark("counters");
     bool again = false;
     if (hc[CTR_FLAGS] & FLAG_POOL_EXHAUSTED) {
-      dfree(pool, st);
-      pool = nullptr;
+      buf.drop_pool();
       pool_units = (int64_t)hc[CTR_POOL];
       if ((double)pool_units * mm * 4 > 32.0 * (1ull << 30))
         return fail(E2E_ERR_UNSUPPORTED, "transition spread too wide: dense-histogram pool above 32 GiB");
       again = true;
     }
     if ((int64_t)hc[CTR_STAGE] > cap) {
-      dfree(stage_col, st);
-      dfree(stage_cnt, st);
-      stage_col = nullptr;
-      stage_cnt = nullptr;
+      buf.drop_stage();
       cap = (int64_t)hc[CTR_STAGE];
       again = true;
     }
     if (!again) break;
     if (attempt == 2) return fail(E2E_ERR_DEVICE, "builder did not settle after re-runs");
   }
-  scratch->add(stage_col);
-  scratch->add(stage_cnt);
-  scratch->add(pool);
   const int64_t nnz = (int64_t)hc[CTR_STAGE];
   m->ns = pl.ns;
   m->n_rows = pl.n_rows;
@@ -1096,8 +1083,8 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
   S.tile_len = tile_len;
   S.canon = canon;
   S.row_off = row_off;
-  S.stage_col = stage_col;
-  S.stage_cnt = stage_cnt;
+  S.stage_col = static_cast<const int32_t*>(buf.col);
+  S.stage_cnt = buf.cnt;
   S.row_ptr = m->row_ptr;
   S.col = m->col;
   S.cnt = m->cnt;

@@ -221,16 +221,7 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
   CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * ctr_words * nblocks, st));
   const int mm = p->neighb_gsize * p->neighb_gsize;
   int64_t pool_units = pl.pool_units, cap = rows * bl * 4 + 4096;
-  struct Growing {  // buffers that a re-run may replace
-    cudaStream_t st;
-    void *pool = nullptr, *col = nullptr, *cnt = nullptr;
-    ~Growing() {
-      dfree(pool, st);
-      dfree(col, st);
-      dfree(cnt, st);
-    }
-  } buf{st};
-  auto take = [&](void** q, size_t bytes) { return *q ? cudaSuccess : dalloc(q, bytes, st); };
+  BuildStaging buf(st);
 
   int dev = 0, sms = 0, per_sm = 0;
   CK(cudaGetDevice(&dev));
@@ -252,9 +243,7 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
     bc = ctr + ctr_words * b;
     unsigned long long hc[CTR_COUNT + 1];
     for (int attempt = 0;; ++attempt) {
-      CK(take(&buf.col, sizeof(int32_t) * (size_t)cap));
-      CK(take(&buf.cnt, sizeof(uint16_t) * (size_t)cap));
-      CK(take(&buf.pool, sizeof(uint32_t) * (size_t)mm * (size_t)pool_units));
+      CK(buf.provide(cap, sizeof(uint16_t), pool_units, p->neighb_gsize));
       if (attempt) CK(cudaMemsetAsync(bc, 0, sizeof(unsigned long long) * CTR_COUNT, st));
       BuildArgs A{};
       A.P = D;
@@ -292,17 +281,14 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
       }
       bool again = false;
       if (hc[CTR_FLAGS] & FLAG_POOL_EXHAUSTED) {
-        dfree(buf.pool, st);
-        buf.pool = nullptr;
+        buf.drop_pool();
         pool_units = (int64_t)hc[CTR_POOL];
         if ((double)pool_units * mm * 4 > 32.0 * (1ull << 30))
           return fail(E2E_ERR_UNSUPPORTED, "transition spread too wide: dense-histogram pool above 32 GiB");
         again = true;
       }
       if ((int64_t)hc[CTR_STAGE] > cap) {
-        dfree(buf.col, st);
-        dfree(buf.cnt, st);
-        buf.col = buf.cnt = nullptr;
+        buf.drop_stage();
         cap = (int64_t)hc[CTR_STAGE] + (int64_t)hc[CTR_STAGE] / 8;  // (later blocks differ a little)
         again = true;
       }

@@ -138,6 +138,35 @@ e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, cudaSt
 cudaError_t launch_layers(const BuildArgs& A, const BuildPlan& pl, const LayerBuild& L, int t0, int t1, cudaStream_t st);
 cudaError_t launch_leftover(const BuildArgs& A, const BuildPlan& pl, const LayerBuild& L, int t0, int t1,
                             cudaStream_t st);
+// A build's staging and dense pool, which a re-run may replace
+struct BuildStaging {
+  cudaStream_t st;
+  void *pool = nullptr, *col = nullptr, *cnt = nullptr;
+  explicit BuildStaging(cudaStream_t s) : st(s) {}
+  BuildStaging(const BuildStaging&) = delete;
+  BuildStaging& operator=(const BuildStaging&) = delete;
+  ~BuildStaging() {
+    drop_stage();
+    drop_pool();
+  }
+  void drop_stage() {
+    dfree(col, st);
+    dfree(cnt, st);
+    col = cnt = nullptr;
+  }
+  void drop_pool() {
+    dfree(pool, st);
+    pool = nullptr;
+  }
+  // what is missing of cap entries and pool_units histograms of m x m
+  cudaError_t provide(int64_t cap, size_t count_bytes, int64_t pool_units, int m) {
+    cudaError_t e = cudaSuccess;
+    if (!col) e = dalloc(&col, sizeof(int32_t) * (size_t)cap, st);
+    if (e == cudaSuccess && !cnt) e = dalloc(&cnt, count_bytes * (size_t)cap, st);
+    if (e == cudaSuccess && !pool) e = dalloc(&pool, sizeof(uint32_t) * (size_t)m * (size_t)m * (size_t)pool_units, st);
+    return e;
+  }
+};
 ViModel vi_model(const e2e_model* m);
 void free_model_buffers(e2e_model* m);
 int64_t model_bytes(const e2e_model* m);

@@ -10,7 +10,7 @@ import os
 import numpy as np
 import pytest
 
-from e2e_gpu_dp_b200 import api
+from e2e_gpu_dp_b200 import _lib, api
 from e2e_gpu_dp_b200._lib import E2EError
 from e2e_gpu_dp_b200.problem import FieldSpec, Problem, make_fields
 from tests.helpers import problem
@@ -64,3 +64,21 @@ def test_jacobi_without_memory_for_the_history_sweeps():
         assert np.array_equal(V.cpu().numpy(), V0) and np.array_equal(pi.cpu().numpy(), pi0)
         assert (st["iterations"], st["residual"]) == (st0["iterations"], st0["residual"])
     m.free()
+
+
+def test_build_that_fails_keeps_no_memory():
+    torch = pytest.importorskip("torch")
+    prob, fields = problem("c1")
+    staged = prob.num_actions * prob.ncells * (prob.nt - 1) * 4 + 4096  # entries of a first attempt
+    api.build_model(prob, fields).free()
+
+    def free_bytes():
+        _lib.check(_lib.lib().e2e_memory_trim())
+        return torch.cuda.mem_get_info()[0]
+
+    before = free_bytes()
+    for _ in range(8):
+        with refuse(2 * staged):  # the staged counts, behind the staged columns
+            with pytest.raises(E2EError):
+                api.build_model(prob, fields)
+    assert free_bytes() >= before
