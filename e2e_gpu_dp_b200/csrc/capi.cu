@@ -658,6 +658,7 @@ extern "C" e2e_status e2e_build_model(const e2e_problem* p, const e2e_fields* f,
   plan.keep_sums = o.keep_reward_parts != 0;
 
   HostTrace trace("build_model");
+  SettleOnExit settle(st);
   DeviceScratch scratch(st);
   FieldsOnDevice fd;
   s = fields_to_device(p, f, where, st, &fd, &scratch, /*defer=*/true);
@@ -667,12 +668,14 @@ extern "C" e2e_status e2e_build_model(const e2e_problem* p, const e2e_fields* f,
   e2e_model* m = new (std::nothrow) e2e_model();
   if (!m) return fail(E2E_ERR_NOMEM, "host allocation");
   s = run_build(p, fd, plan, st, &scratch, m);
+  const cudaError_t se = cudaStreamSynchronize(st);  // (a failed build's buffers too: they are freed on another stream)
+  settle.done = true;
+  if (s == E2E_OK && se != cudaSuccess) s = cuda_fail(se, "cudaStreamSynchronize");
   if (s != E2E_OK) {
     free_model_buffers(m);
     delete m;
     return s;
   }
-  CK(cudaStreamSynchronize(st));
   trace.mark("done");
   *out = m;
   return E2E_OK;
@@ -977,9 +980,11 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
       struct CopyFree {
         cudaStream_t* s;
         cudaEvent_t* e;
+        bool copying = false;  // copies queued that st does not wait for yet
         ~CopyFree() {
           for (int k = 0; k < 2; ++k)
             if (e[k]) cudaEventDestroy(e[k]);
+          if (copying) cudaStreamSynchronize(*s);
           if (*s) cudaStreamDestroy(*s);
         }
       } cpfree{&cps, evs};
@@ -988,11 +993,13 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
       for (int k = 0; k < 4; ++k) {
         const int end = ends[k];
         if (end <= done) continue;
+        cpfree.copying = done > 0;
         e2e_status cs = copy_field_steps(fd, done ? done + 1 : 0, end + 1, done ? cps : st);
         if (cs != E2E_OK) return cs;
         if (done) {
           CK(cudaEventRecord(evs[1], cps));
           CK(cudaStreamWaitEvent(st, evs[1], 0));
+          cpfree.copying = false;
         } else {
           CK(cudaStreamCreateWithFlags(&cps, cudaStreamNonBlocking));
           for (int q = 0; q < 2; ++q) CK(cudaEventCreateWithFlags(&evs[q], cudaEventDisableTiming));
@@ -1375,13 +1382,7 @@ e2e_status solve_on_device(const e2e_model* m, const e2e_vi_opts& o, float* dV, 
   PackTimer pack_timer;
   // The sliced copy stays with the model, which a later call may use or free on
   // another stream: no exit leaves its fill, or a sweep over it, in flight.
-  struct SyncOnExit {
-    cudaStream_t st;
-    bool done = false;
-    ~SyncOnExit() {
-      if (!done) cudaStreamSynchronize(st);
-    }
-  } settle{st};
+  SettleOnExit settle(st);
   {
     e2e_status ps = ensure_pack(m, &pack_ms, st, &pack_timer);
     if (ps != E2E_OK) return ps;

@@ -163,6 +163,7 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
   BuildPlan pl;
   e2e_status s = plan_build(p, 16, 0, &pl);
   if (s != E2E_OK) return s;
+  SettleOnExit settle(st);
   DeviceScratch scratch(st);
   FieldsOnDevice fd;
   s = fields_to_device(p, f, where, st, &fd, &scratch);
@@ -329,6 +330,7 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
   unsigned long long err = 0;
   CK(cudaMemcpyAsync(&err, bc + CTR_COUNT, sizeof(err), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  settle.done = true;
   if (err >> 32) return fail(E2E_ERR_DEVICE, "build+solve: a wait for a layer's completion ran out of its bound");
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, ev[0], ev[1]));

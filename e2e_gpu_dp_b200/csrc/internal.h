@@ -138,6 +138,20 @@ e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, cudaSt
 cudaError_t launch_layers(const BuildArgs& A, const BuildPlan& pl, const LayerBuild& L, int t0, int t1, cudaStream_t st);
 cudaError_t launch_leftover(const BuildArgs& A, const BuildPlan& pl, const LayerBuild& L, int t0, int t1,
                             cudaStream_t st);
+// Waits for the stream on every way out of a call that has not waited (done): what
+// the call queued reads its caller's arrays or writes buffers that are freed, or used
+// next, on other streams.
+struct SettleOnExit {
+  cudaStream_t st;
+  bool done = false;
+  explicit SettleOnExit(cudaStream_t s) : st(s) {}
+  SettleOnExit(const SettleOnExit&) = delete;
+  SettleOnExit& operator=(const SettleOnExit&) = delete;
+  ~SettleOnExit() {
+    if (!done) cudaStreamSynchronize(st);
+  }
+};
+
 // A build's staging and dense pool, which a re-run may replace
 struct BuildStaging {
   cudaStream_t st;

@@ -82,3 +82,18 @@ def test_build_that_fails_keeps_no_memory():
             with pytest.raises(E2EError):
                 api.build_model(prob, fields)
     assert free_bytes() >= before
+
+
+@pytest.mark.parametrize("call", ["build_model", "build_solve"])
+def test_failed_build_leaves_nothing_in_flight(call):
+    torch = pytest.importorskip("torch")
+    prob, fields = problem("c1")
+    s = torch.cuda.Stream()
+    dense = 4 * prob.neighb_gsize ** 2 * min(max(prob.num_actions * prob.ncells * (prob.nt - 1) // 64, 256), 8192)
+    with refuse(dense):  # the dense pool: the last buffer before the first launch
+        with pytest.raises(E2EError):
+            getattr(api, call)(prob, fields, stream=s)
+    assert s.query()
+    want = api.build_model(prob, fields).to_host()
+    got = api.build_model(prob, fields, stream=s).to_host()
+    assert all(np.array_equal(want[k], got[k]) for k in ("row_ptr", "col", "cnt", "R"))
