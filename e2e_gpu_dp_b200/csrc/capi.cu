@@ -922,7 +922,7 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
   s = layer_build_buffers(p, pl, st, scratch, &L);
   if (s != E2E_OK) return s;
 
-  int64_t cap = pl.stage_cap, pool_units = pl.pool_units;
+  int64_t cap = pl.stage_cap, least = cap, pool_units = pl.pool_units;
   BuildStaging buf(st);
   unsigned long long hc[CTR_COUNT];
   const int mm = p->neighb_gsize * p->neighb_gsize;
@@ -935,7 +935,7 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
   } evfree{ev};
   trace_mark("setup");
   for (int attempt = 0; attempt < 3; ++attempt) {
-    CK(buf.provide(cap, (size_t)cbytes, pool_units, p->neighb_gsize));
+    CK(buf.provide(&cap, least, (size_t)cbytes, pool_units, p->neighb_gsize));
     CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * CTR_COUNT, st));
     BuildArgs A{};
     A.P = D;
@@ -1027,16 +1027,20 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
     CK(cudaStreamSynchronize(st));
     trace_mark("counters");
     bool again = false;
+    int64_t lost = 0;  // rows without a histogram
     if (hc[CTR_FLAGS] & FLAG_POOL_EXHAUSTED) {
       buf.drop_pool();
+      lost = (int64_t)hc[CTR_POOL] - pool_units;
       pool_units = (int64_t)hc[CTR_POOL];
       if ((double)pool_units * mm * 4 > 32.0 * (1ull << 30))
         return fail(E2E_ERR_UNSUPPORTED, "transition spread too wide: dense-histogram pool above 32 GiB");
       again = true;
     }
-    if ((int64_t)hc[CTR_STAGE] > cap) {
+    const int64_t staged = (int64_t)hc[CTR_STAGE];
+    if (staged + lost * BuildStaging::kLostRowEntries > cap) {
       buf.drop_stage();
-      cap = (int64_t)hc[CTR_STAGE];
+      least = std::max(cap, staged);
+      cap = std::max(least, staged + lost * BuildStaging::kLostRowEntries);
       again = true;
     }
     if (!again) break;

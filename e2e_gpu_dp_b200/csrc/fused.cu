@@ -221,7 +221,7 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
   scratch.add(ctr);
   CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * ctr_words * nblocks, st));
   const int mm = p->neighb_gsize * p->neighb_gsize;
-  int64_t pool_units = pl.pool_units, cap = rows * bl * 4 + 4096;
+  int64_t pool_units = pl.pool_units, cap = rows * bl * 4 + 4096, least = cap;
   BuildStaging buf(st);
 
   int dev = 0, sms = 0, per_sm = 0;
@@ -244,7 +244,7 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
     bc = ctr + ctr_words * b;
     unsigned long long hc[CTR_COUNT + 1];
     for (int attempt = 0;; ++attempt) {
-      CK(buf.provide(cap, sizeof(uint16_t), pool_units, p->neighb_gsize));
+      CK(buf.provide(&cap, least, sizeof(uint16_t), pool_units, p->neighb_gsize));
       if (attempt) CK(cudaMemsetAsync(bc, 0, sizeof(unsigned long long) * CTR_COUNT, st));
       BuildArgs A{};
       A.P = D;
@@ -281,16 +281,20 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
         std::copy(hc + 1, hc + 1 + CTR_COUNT, hc);
       }
       bool again = false;
+      int64_t lost = 0;  // rows without a histogram
       if (hc[CTR_FLAGS] & FLAG_POOL_EXHAUSTED) {
         buf.drop_pool();
+        lost = (int64_t)hc[CTR_POOL] - pool_units;
         pool_units = (int64_t)hc[CTR_POOL];
         if ((double)pool_units * mm * 4 > 32.0 * (1ull << 30))
           return fail(E2E_ERR_UNSUPPORTED, "transition spread too wide: dense-histogram pool above 32 GiB");
         again = true;
       }
-      if ((int64_t)hc[CTR_STAGE] > cap) {
+      const int64_t staged = (int64_t)hc[CTR_STAGE];
+      if (staged + lost * BuildStaging::kLostRowEntries > cap) {
         buf.drop_stage();
-        cap = (int64_t)hc[CTR_STAGE] + (int64_t)hc[CTR_STAGE] / 8;  // (later blocks differ a little)
+        least = std::max(cap, staged + staged / 8);  // (later blocks differ a little)
+        cap = std::max(least, staged + lost * BuildStaging::kLostRowEntries);
         again = true;
       }
       if (!again) break;

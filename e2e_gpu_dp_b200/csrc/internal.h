@@ -152,8 +152,12 @@ struct SettleOnExit {
   }
 };
 
-// A build's staging and dense pool, which a re-run may replace
+// A build's staging and dense pool, which a re-run may replace.  A run whose pool was
+// too small did not stage the rows that found no histogram; the next one is given
+// room for them too, so that it is the last (120x120x24, 1000 realisations, wide
+// noise, 24 actions: build+solve 109 -> 61 ms).  Dense rows have 40 entries there.
 struct BuildStaging {
+  static constexpr int64_t kLostRowEntries = 128;
   cudaStream_t st;
   void *pool = nullptr, *col = nullptr, *cnt = nullptr;
   explicit BuildStaging(cudaStream_t s) : st(s) {}
@@ -172,13 +176,19 @@ struct BuildStaging {
     dfree(pool, st);
     pool = nullptr;
   }
-  // what is missing of cap entries and pool_units histograms of m x m
-  cudaError_t provide(int64_t cap, size_t count_bytes, int64_t pool_units, int m) {
+  // What is missing of *cap entries, or of `least` of them where memory for more is
+  // missing, and of pool_units histograms of m x m
+  cudaError_t provide(int64_t* cap, int64_t least, size_t count_bytes, int64_t pool_units, int m) {
     cudaError_t e = cudaSuccess;
-    if (!col) e = dalloc(&col, sizeof(int32_t) * (size_t)cap, st);
-    if (e == cudaSuccess && !cnt) e = dalloc(&cnt, count_bytes * (size_t)cap, st);
-    if (e == cudaSuccess && !pool) e = dalloc(&pool, sizeof(uint32_t) * (size_t)m * (size_t)m * (size_t)pool_units, st);
-    return e;
+    if (!pool) e = dalloc(&pool, sizeof(uint32_t) * (size_t)m * (size_t)m * (size_t)pool_units, st);
+    if (e != cudaSuccess || col) return e;
+    for (;; *cap = least) {
+      e = dalloc(&col, sizeof(int32_t) * (size_t)*cap, st);
+      if (e == cudaSuccess) e = dalloc(&cnt, count_bytes * (size_t)*cap, st);
+      if (e != cudaErrorMemoryAllocation || *cap == least) return e;
+      cudaGetLastError();
+      drop_stage();
+    }
   }
 };
 ViModel vi_model(const e2e_model* m);
