@@ -141,9 +141,71 @@ inline bool pow2(double v) {
   return v > 0 && frexp(v, &e) == 0.5;
 }
 
-struct Brk {
-  double z;  // breakpoint in p' for b = j = n0 = 0
-  int action, edge;
+// The breakpoints of one kind of table, z = their places in p' for b = j = n0 = 0 and
+// a shift of 0, and their groups for a shift: zones [lo, hi] in fixed point
+struct Breakpoints {
+  int n = 0;
+  double z[2 * kRankMaxActions];
+  int order[2 * kRankMaxActions];  // by place within a unit; kept from one shift to the next, which rotates it
+  int group[2 * kRankMaxActions];  // of breakpoint i
+  int whole[2 * kRankMaxActions];  // its units
+  int64_t lo[2 * kRankMaxActions], hi[2 * kRankMaxActions];
+  int groups = 0;
+
+  void add(double at) {
+    order[n] = n;
+    z[n++] = at;
+  }
+
+  // zones of h on each side of a breakpoint, those within tau of each other merged
+  void make_groups(double shift, int h, int64_t tau) {
+    const double one = ldexp(1.0, kRankFrac);
+    double in[2 * kRankMaxActions];
+    for (int i = 0; i < n; ++i) {
+      const double at = z[i] + shift, w = floor(at);
+      whole[i] = (int)w;
+      in[i] = at - w;
+    }
+    for (int i = 1; i < n; ++i) {
+      const int k = order[i];
+      int to = i;
+      for (; to > 0 && in[order[to - 1]] > in[k]; --to) order[to] = order[to - 1];
+      order[to] = k;
+    }
+    groups = 0;
+    for (int i = 0; i < n; ++i) {
+      const int k = order[i];
+      const int64_t q = (int64_t)floor(in[k] * one), l = q - h, r = q + 1 + h;
+      if (groups && l <= hi[groups - 1] + tau) {
+        hi[groups - 1] = std::max(hi[groups - 1], r);
+      } else {
+        lo[groups] = l;
+        hi[groups++] = r;
+      }
+      group[k] = groups - 1;
+    }
+  }
+
+  // whether some neighbouring zones lie between `from` and `to` apart: else both merge the same
+  bool merges_differ(int h, int64_t from, int64_t to) {
+    make_groups(0.0, h, from);
+    for (int k = 0; k < groups; ++k) {
+      const int64_t next = k + 1 < groups ? lo[k + 1] : lo[0] + ((int64_t)1 << kRankFrac);
+      if (next - hi[k] <= to + 4) return true;  // (a shift moves a place by a unit)
+    }
+    return false;
+  }
+
+  // every group inside a slot of its own
+  bool fits(int64_t slot_w) const {
+    if (groups > kRankMaxGroups) return false;
+    for (int k = 0; k < groups; ++k) {
+      const int64_t s = lo[k] >= 0 ? lo[k] / slot_w : -1;
+      if (lo[k] < 0 || hi[k] >= ((int64_t)1 << kRankFrac) || hi[k] / slot_w != s) return false;
+      if (k && lo[k - 1] / slot_w == s) return false;
+    }
+    return true;
+  }
 };
 
 }  // namespace rank_detail
@@ -202,65 +264,58 @@ inline bool make_rank_plan(int g, int na, double dt, const std::vector<float>& s
   // merge distance (close breakpoints of different actions share a group with a
   // wider zone), slots a unit, and the phase of the slots: the first that gives
   // every group a slot of its own with its zone inside
-  // (edge cells without tables, groups[..] = 0, when only the boundaries fit)
+  // (edge cells without tables, groups[..] = 0, when only the boundaries fit).
+  // The search is part of every build: up to 0.1 ms where it fails (16 headings at
+  // speed 1.3 took 0.21 ms and 32 headings 0.36 when every trial made its tables).
+  Breakpoints kinds[RANK_KINDS];
+  for (int kind = 0; kind < RANK_KINDS; ++kind) {
+    for (int a = 0; a < na; ++a) kinds[kind].add(-0.5 - disp[kind / 2][a]);
+    if (kind & 1)
+      for (int a = 0; a < na; ++a) kinds[kind].add(-disp[kind / 2][a]);
+  }
   for (int with_edge = 1; with_edge >= 0; --with_edge) {
+    // with the clamps' breakpoints the tables that hold them are the fullest: tried first
+    const int tables[4] = {RANK_X_EDGE, RANK_Y_EDGE, RANK_X, RANK_Y};
+    const int skip = with_edge ? 0 : 2;
+    int64_t tau_before = -1;
     for (int tau : {0, 64, 256, 1024}) {
+      bool differs = tau_before < 0;
+      for (int t = skip; t < 4 && !differs; ++t) differs = kinds[tables[t]].merges_differ(hq[tables[t] / 2], tau_before, tau);
+      tau_before = tau;
+      if (!differs) continue;
       for (int sl = 5; sl <= 8; ++sl) {
         for (int ph = 0; ph < 8; ++ph) {
           const double shift = (ph + 0.5) / (8.0 * (1 << sl));
           const int64_t slot_w = unit >> sl;
-          std::vector<uint32_t> words((size_t)rank_plan_words(sl), 0u);
-          int groups[RANK_KINDS] = {0, 0, 0, 0};
           int64_t widest = 1;
           bool ok = true;
-          std::vector<int64_t> glo[RANK_KINDS];
-          for (int kind = 0; kind < RANK_KINDS && ok; ++kind) {
-            const int ax = kind / 2;
-            if ((kind & 1) && !with_edge) continue;
-            std::vector<Brk> br;
-            for (int a = 0; a < na; ++a) br.push_back({-0.5 - disp[ax][a] + shift, a, 0});
-            if (kind & 1)
-              for (int a = 0; a < na; ++a) br.push_back({-disp[ax][a] + shift, a, 1});
-            std::sort(br.begin(), br.end(),
-                      [](const Brk& l, const Brk& r) { return l.z - floor(l.z) < r.z - floor(r.z); });
-            int* off = reinterpret_cast<int*>(words.data() + rank_off_at(sl) + kind * 2 * kRankMaxActions);
-            std::vector<int64_t>& lo = glo[kind];
-            std::vector<int64_t> hi;
-            std::vector<int> of(br.size());
-            for (size_t i = 0; i < br.size(); ++i) {
-              const int64_t q = (int64_t)floor((br[i].z - floor(br[i].z)) * one);
-              const int64_t l = q - hq[ax], h = q + 1 + hq[ax];
-              if (!lo.empty() && l <= hi.back() + tau) hi.back() = std::max(hi.back(), h);
-              else lo.push_back(l), hi.push_back(h);
-              of[i] = (int)lo.size() - 1;
-            }
-            const int G = groups[kind] = (int)lo.size();
-            if (G > kRankMaxGroups) ok = false;
-            for (int k = 0; k < G && ok; ++k) {
-              widest = std::max(widest, hi[k] - lo[k] + 1);
-              const int64_t s = lo[k] >= 0 ? lo[k] / slot_w : -1;
-              if (lo[k] < 0 || hi[k] >= unit || hi[k] / slot_w != s) ok = false;
-              if (k && ok && lo[k - 1] / slot_w == s) ok = false;
-            }
-            if (!ok) break;
-            for (size_t i = 0; i < br.size(); ++i)
-              off[br[i].edge * kRankMaxActions + br[i].action] = (int)floor(br[i].z) * G + of[i];
-            for (int k = 0; k < G; ++k) words[rank_gq_at(sl) + kind * kRankMaxGroups + k] = (uint32_t)lo[k];
+          for (int t = skip; t < 4 && ok; ++t) {
+            Breakpoints& b = kinds[tables[t]];
+            b.make_groups(shift, hq[tables[t] / 2], tau);
+            ok = b.fits(slot_w);
+            for (int k = 0; k < b.groups && ok; ++k) widest = std::max(widest, b.hi[k] - b.lo[k] + 1);
           }
           if (!ok) continue;
           int64_t W = 1;
           while (W < widest) W *= 2;
           if (W > slot_w / 4) continue;
+          out->words.assign((size_t)rank_plan_words(sl), 0u);
+          uint32_t* const words = out->words.data();
           for (int kind = 0; kind < RANK_KINDS; ++kind) {
-            const std::vector<int64_t>& lo = glo[kind];
-            const int G = groups[kind], per = 1 << sl;
+            const Breakpoints& b = kinds[kind];
+            const bool have = with_edge || !(kind & 1);
+            const int G = out->groups[kind] = have ? b.groups : 0, per = 1 << sl;
+            int* off = reinterpret_cast<int*>(words + rank_off_at(sl) + kind * 2 * kRankMaxActions);
+            for (int i = 0; i < b.n && have; ++i)  // breakpoint i: cell boundaries, then clamps, of action i % na
+              off[(i / na) * kRankMaxActions + i % na] = b.whole[i] * G + b.group[i];
+            for (int k = 0; k < G; ++k) words[rank_gq_at(sl) + kind * kRankMaxGroups + k] = (uint32_t)b.lo[k];
             for (int u = 0; u < kRankUnits; ++u) {
               int k = 0;
               for (int s = 0; s < per; ++s) {
                 const int64_t start = (int64_t)u * unit + s * slot_w;
                 uint32_t w = (uint32_t)(u * G + k) << 16;
-                if (k < G && lo[k] / slot_w == s) {
-                  w += 0x10000u - (uint32_t)(lo[k] - s * slot_w);
+                if (k < G && b.lo[k] / slot_w == s) {
+                  w += 0x10000u - (uint32_t)(b.lo[k] - s * slot_w);
                   ++k;
                 } else {
                   w += (uint32_t)W;
@@ -272,8 +327,6 @@ inline bool make_rank_plan(int g, int na, double dt, const std::vector<float>& s
           out->slots_log2 = sl;
           out->zone_mask = 0xffffu & ~((uint32_t)W - 1u);
           out->shift = shift;
-          for (int kind = 0; kind < RANK_KINDS; ++kind) out->groups[kind] = groups[kind];
-          out->words.swap(words);
           return true;
         }
       }
