@@ -848,19 +848,29 @@ e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, cudaSt
   };
   void *plan, *yt, *ystat, *obits, *count, *flag;
   const size_t pb = sizeof(uint32_t) * pl.rank_words.size();
-  CK(take(pb, &plan));
+  const std::pair<size_t, void**> need[] = {
+      {pb, &plan},
+      {sizeof(float) * layers * nmp * (size_t)K.nrp, &yt},
+      {sizeof(float) * layers * nmp * 2, &ystat},
+      {sizeof(uint32_t) * layers * (size_t)p->gsize * (size_t)K.owords, &obits},
+      {sizeof(unsigned int) * 2 * layers, &count},
+      {layers * (size_t)defer_stride(pl.etiles_per_layer), &flag}};
+  for (const auto& [bytes, q] : need) {
+    const cudaError_t e = take(bytes, q);
+    if (e == cudaErrorMemoryAllocation) {  // (the coefficients again, above all): the general builder needs none of it
+      cudaGetLastError();
+      return E2E_OK;
+    }
+    CK(e);
+  }
   CK(cudaMemcpyAsync(plan, pl.rank_words.data(), pb, cudaMemcpyHostToDevice, st));
-  CK(take(sizeof(float) * layers * nmp * (size_t)K.nrp, &yt));
-  CK(take(sizeof(float) * layers * nmp * 2, &ystat));
-  CK(take(sizeof(uint32_t) * layers * (size_t)p->gsize * (size_t)K.owords, &obits));
-  CK(take(sizeof(unsigned int) * 2 * layers, &count));
-  CK(take(layers * (size_t)defer_stride(pl.etiles_per_layer), &flag));
   K.plan = static_cast<const uint32_t*>(plan);
   K.yt = static_cast<const float*>(yt);
   K.ystat = static_cast<const float*>(ystat);
   K.obits = static_cast<const uint32_t*>(obits);
   L->defer_count = static_cast<unsigned int*>(count);
   L->defer_flag = static_cast<uint8_t*>(flag);
+  L->ranked = true;
   return E2E_OK;
 }
 
@@ -868,7 +878,7 @@ cudaError_t launch_layers(const BuildArgs& A, const BuildPlan& pl, const LayerBu
   BuildArgs B = A;
   B.t0 = t0;
   B.t1 = t1;
-  if (!pl.ranked) return launch_build_tiles(B, pl.count_bits, t1 - t0, st);
+  if (!L.ranked) return launch_build_tiles(B, pl.count_bits, t1 - t0, st);
   B.defer_count = L.defer_count;
   B.defer_flag = L.defer_flag;
   RankArgs R = L.K;
@@ -881,7 +891,7 @@ cudaError_t launch_layers(const BuildArgs& A, const BuildPlan& pl, const LayerBu
 
 cudaError_t launch_leftover(const BuildArgs& A, const BuildPlan& pl, const LayerBuild& L, int t0, int t1,
                             cudaStream_t st) {
-  if (!pl.ranked) return cudaSuccess;
+  if (!L.ranked) return cudaSuccess;
   BuildArgs B = A;
   B.t0 = t0;
   B.t1 = t1;

@@ -129,6 +129,7 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
 // launch_layers queues the builder for layers [t0, t1); launch_leftover the
 // general builder for the tiles of [t0, t1) that the ranked one listed.
 struct LayerBuild {
+  bool ranked = false;  // the plan's choice, unless memory for the ranked builder is missing
   RankArgs K{};
   unsigned int* defer_count = nullptr;
   uint8_t* defer_flag = nullptr;

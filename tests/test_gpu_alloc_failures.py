@@ -97,3 +97,20 @@ def test_failed_build_leaves_nothing_in_flight(call):
     want = api.build_model(prob, fields).to_host()
     got = api.build_model(prob, fields, stream=s).to_host()
     assert all(np.array_equal(want[k], got[k]) for k in ("row_ptr", "col", "cnt", "R"))
+
+
+@pytest.mark.parametrize("call", ["build_model", "build_solve"])
+def test_build_without_memory_for_the_rank_tables(call):
+    prob, fields = problem("c1")
+    coeffs = 4 * (prob.nt - 1) * (prob.nmodes + prob.nmodes % 2) * (-(-prob.nrzns // 128) * 128)
+
+    def results():
+        if call == "build_solve":
+            return api.build_solve(prob, fields)[:2]
+        h = api.build_model(prob, fields).to_host()
+        return [h[k] for k in ("row_ptr", "col", "cnt", "R")]
+
+    want = results()
+    with refuse(coeffs):
+        got = results()
+    assert all(np.array_equal(a, b) for a, b in zip(want, got))
