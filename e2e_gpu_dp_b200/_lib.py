@@ -58,7 +58,7 @@ class ModelInfo(C.Structure):
         ("index_bits", C.c_int32), ("row_ptr", C.c_void_p), ("col", C.c_void_p),
         ("cnt", C.c_void_p), ("R", C.c_void_p), ("dropped", C.c_uint64),
         ("overflow_units", C.c_uint64), ("build_kernel_ms", C.c_double),
-        ("assemble_ms", C.c_double), ("build_launches", C.c_int32), ("reserved", C.c_int32),
+        ("assemble_ms", C.c_double), ("build_launches", C.c_int32), ("general_tiles", C.c_int32),
     ]
 
 
@@ -122,7 +122,7 @@ class RolloutStats(C.Structure):
 class FusedStats(C.Structure):
     _fields_ = [("seconds", C.c_double), ("n_rows", C.c_int64), ("nnz", C.c_int64), ("dropped", C.c_uint64),
                 ("misbinned", C.c_uint64), ("overflow_rows", C.c_uint64), ("launches", C.c_int32),
-                ("reserved", C.c_int32), ("h2d_bytes", C.c_int64)]
+                ("general_tiles", C.c_int32), ("h2d_bytes", C.c_int64)]
 
 
 E2E_OBST_NONE, E2E_OBST_STATIC, E2E_OBST_DYNAMIC = 0, 1, 2

@@ -1070,6 +1070,7 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
   m->dropped = hc[CTR_DROPPED];
   m->misbinned = hc[CTR_MISBIN];
   m->overflow_rows = hc[CTR_OVERFLOW_ROWS];
+  m->general_tiles = (int32_t)std::min<int64_t>(L.ranked ? (int64_t)hc[CTR_DEFERRED] : pl.n_tiles, INT32_MAX);
   m->layered = true;
   m->built = true;
   m->prob = *p;
@@ -1152,6 +1153,7 @@ extern "C" e2e_status e2e_model_get_info(const e2e_model* m, e2e_model_info* inf
   info->build_kernel_ms = m->build_kernel_ms;
   info->assemble_ms = m->assemble_ms;
   info->build_launches = m->build_launches;
+  info->general_tiles = m->general_tiles;
   return E2E_OK;
 }
 

@@ -346,6 +346,7 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
     stats->misbinned = sum[CTR_MISBIN];
     stats->overflow_rows = sum[CTR_OVERFLOW_ROWS];
     stats->launches = launches;
+    stats->general_tiles = (int32_t)std::min<int64_t>(L.ranked ? (int64_t)sum[CTR_DEFERRED] : pl.n_tiles, INT32_MAX);
     stats->h2d_bytes = (int64_t)fd.h2d_bytes;
   }
   return E2E_OK;

@@ -25,7 +25,7 @@ struct e2e_model {
   float* sumR = nullptr;     // device, ns * na: reward sums (keep_reward_parts), or null
   uint64_t dropped = 0, misbinned = 0, overflow_rows = 0;
   double build_kernel_ms = 0, assemble_ms = 0;
-  int32_t build_launches = 0;
+  int32_t build_launches = 0, general_tiles = 0;
   bool built = false;        // by this library: every next state lies in its row's m x m window
   bool layered = false;      // every transition of a layer-t state leads into layer t+1
   e2e_problem prob{};

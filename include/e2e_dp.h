@@ -128,7 +128,9 @@ typedef struct {
   double build_kernel_ms;  /* device time of the last builder launch (CUDA events on the build stream) */
   double assemble_ms;      /* device time of the CSR assembly (tile scan + copy) */
   int32_t build_launches;  /* builder launches (1, or 2 after a re-run with larger buffers) */
-  int32_t reserved;
+  int32_t general_tiles;   /* of the (nt-1) * ceil(ncells / c) groups of c = 32 / P cells, P the power of two
+                              that holds num_actions, those that the general builder built: none or few where
+                              the ranked builder takes the problem, else all (0: a model read from files) */
 } e2e_model_info;
 
 typedef struct e2e_model e2e_model;
@@ -379,7 +381,7 @@ typedef struct {
   uint64_t misbinned;
   uint64_t overflow_rows;
   int32_t launches;        /* builder and backup launches (per block of layers; a build is re-run when rows needed more dense histograms) */
-  int32_t reserved;
+  int32_t general_tiles;   /* as e2e_model_info */
   int64_t h2d_bytes;       /* field bytes copied from host memory */
 } e2e_fused_stats;
 
