@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdlib>
 
 #include "e2e_dp.h"
 #include "grid_sync.cuh"
@@ -31,7 +32,11 @@ using namespace e2e;
 namespace {
 
 constexpr int kThreads = 256;
-constexpr size_t kStageBudget = size_t(256) << 20;  // bytes of a block of layers' staging
+// bytes of a block of layers' staging (tests: E2E_TEST_STAGE_BYTES)
+size_t stage_budget() {
+  const char* v = std::getenv("E2E_TEST_STAGE_BYTES");
+  return v ? (size_t)std::strtoull(v, nullptr, 10) : size_t(256) << 20;
+}
 
 struct BackupArgs {
   int t0, t1, na, lanes_log2, cells_log2, nrzns;  // 1 << cells_log2 cells per emission tile
@@ -200,7 +205,7 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
   const int layers = p->nt - 1;
   const int64_t rows = nc * pl.na;
   const size_t per_layer = (size_t)rows * (sizeof(uint32_t) + sizeof(float) + 4 * 6);
-  const int most = (int)std::max<size_t>(1, std::min<size_t>((size_t)layers, kStageBudget / per_layer));
+  const int most = (int)std::max<size_t>(1, std::min<size_t>((size_t)layers, stage_budget() / per_layer));
   const int nblocks = (layers + most - 1) / most, bl = (layers + nblocks - 1) / nblocks;
   uint32_t* row_off = nullptr;
   int64_t* tile_base = nullptr;
