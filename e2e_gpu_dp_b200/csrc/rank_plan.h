@@ -211,8 +211,9 @@ struct Breakpoints {
 }  // namespace rank_detail
 
 // The tables of a problem, or false when the general builder has to take it:
-// spacings that are no power of two (the reference's division then rounds, and
-// its cells are no step function), breakpoints too dense for a table.
+// spacings that are no power of two (the grid's ticks and the reference's quotient
+// then round, and some cells' numbers come out one lower: a step function too, but
+// not the one of these tables), breakpoints too dense for a table.
 //   speed, angle: the actions (float values); xs, ys: grid ticks
 inline bool make_rank_plan(int g, int na, double dt, const std::vector<float>& speed, const std::vector<float>& angle,
                            const std::vector<float>& xs, const std::vector<float>& ys, RankPlan* out) {

@@ -148,8 +148,10 @@ typedef struct {
                             it starts, 6: lean kernel without entry look-ahead, 7: Jacobi sweeps
                             staged through shared memory by TMA bulk copies).  Automatic: the
                             layered pass with loads ahead of its barriers, and Jacobi with all
-                            sweeps of a layer at once (time-layered models); a tuning or a warp
-                            count selects one of the other kernels, with the same results. */
+                            sweeps of a layer at once (time-layered models, where that is cheaper
+                            than the sweeps that max_iter and threshold leave).  A tuning selects
+                            one of the other kernels, a warp count that of the layered sweep, with
+                            the same results. */
 } e2e_vi_opts;
 
 typedef struct {
@@ -159,7 +161,8 @@ typedef struct {
   double fp64_max_abs_err; /* fp64_check: max |V32 - V64| */
   double fp64_max_rel_err; /* fp64_check: max |V32 - V64| / max |V64| */
   int64_t bytes_per_sweep; /* algorithmic bytes of one sweep (CSR form: row_ptr, col, count, R, V) */
-  int64_t stream_bytes_per_sweep; /* bytes a sweep over the sliced copy moves (padding included) */
+  int64_t stream_bytes_per_sweep; /* bytes a sweep over the sliced copy moves (padding included);
+                              bytes_per_sweep if the solve needed no sliced copy and the model has none */
   double pack_ms;          /* device time spent building the sliced copy in this call (0 if cached) */
   double sweep_seconds;    /* layered: device time of the backward pass alone */
 } e2e_vi_stats;
