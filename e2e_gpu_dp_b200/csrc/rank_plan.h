@@ -237,8 +237,14 @@ inline bool make_rank_plan(int g, int na, double dt, const std::vector<float>& s
   // Distance between a breakpoint's place in exact arithmetic and where the
   // float chain has it, in units of p: half an ulp of the velocity sum and of
   // the net velocity (times dt), of the new position, and of the snapping
-  // coordinate unless that subtraction is exact; the ticks' own deviation from
-  // multiples of D; and the device's cosine and sine (2 ulp) against the host's.
+  // coordinate; the ticks' own deviation from multiples of D; and the device's
+  // cosine and sine (2 ulp) against the host's.
+  //
+  // The snapping coordinate is the position's distance from an end of the axis
+  // (org).  It is finer than a float where the position is closer to 0 than the
+  // distance is long: never on an x axis of positive coordinates (org the lower
+  // end); on such a y axis (org the upper end) only where the position's own half
+  // ulp is at most half the distance's, so 1.5 of the largest half ulp bound both.
   for (int ax = 0; ax < 2; ++ax) {
     const std::vector<float>& t = ax == 0 ? xs : ys;
     const double t0 = t[0], tn = t[g - 1], d = D[ax];
@@ -250,10 +256,11 @@ inline bool make_rank_plan(int g, int na, double dt, const std::vector<float>& s
       dev = std::max(dev, fabs(got - i * d));
     }
     const double org = ax == 0 ? t0 : tn, ulp = 2 * half_ulp(top);
-    const bool exact = fmod(org, ulp) == 0;
-    const double drift = kRankMaxDrift + kRankUnits;
-    double e = half_ulp(drift * d / dt) * dt + half_ulp((drift + amax) * d / dt) * dt + half_ulp(top) +
-               (exact ? 0.0 : half_ulp(top)) + dev + 5e-7 * amax * d;
+    const bool positive = t0 >= 0 && fmod(org, ulp) == 0;
+    const double snap = !positive ? half_ulp(std::max(top, tn - t0 + d)) : ax == 0 ? 0.0 : 0.5 * half_ulp(top);
+    const double drift = kRankMaxDrift + kRankMaxHalfRange + 1.1;  // of a sample in a range, with its last step's unit
+    double e = half_ulp(drift * d / dt) * dt + half_ulp((drift + amax) * d / dt) * dt + half_ulp(top) + snap + dev +
+               5e-7 * amax * d;
     out->err[ax] = 1.05 * e / d;
   }
   const double one = ldexp(1.0, kRankFrac);

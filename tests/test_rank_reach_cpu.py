@@ -48,10 +48,10 @@ REACH = [
     "1x8 none 0 plain 1 large 14",
     "1x12 none 0 plain 1 large 35",
     "1x16 none 4 plain 6 large 51",
-    "1x24 none 4 plain 8 large 118",
+    "1x24 none 4 plain 9 large 117",
     "1x32 none 14 plain 13 large 139",
-    "2x8 none 1 plain 2 large 66",
-    "2x16 none 9 plain 9 large 149",
+    "2x8 none 1 plain 3 large 65",
+    "2x16 none 9 plain 10 large 148",
 ]
 
 
