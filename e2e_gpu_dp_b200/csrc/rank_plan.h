@@ -74,7 +74,8 @@ struct RankRange {
 // mean_v: the cell's mean velocity (added to the mode sums); centre, var: mean
 // and variance of the whole velocity (they choose the range only, no result
 // depends on them); idx: the cell's index on the axis.  False: left to the
-// general builder (spread or drift too wide for a table, or edge cells without one).
+// general builder (spread or drift too wide for a table, a mean velocity of more than
+// 56 cells that the modes cancel, or edge cells without one).
 E2E_RANK_FN bool rank_range(const uint32_t* plan, int slots_log2, const int* groups, int axis, float s, double shift,
                             float a_min, float a_max, float mean_v, float centre, float var, int idx, int g,
                             RankRange* r) {
@@ -83,6 +84,9 @@ E2E_RANK_FN bool rank_range(const uint32_t* plan, int slots_log2, const int* gro
   const float h = kRankSigmas * sqrtf(var) * fabsf(s) * (1.0f / unit) + 1e-3f;
   if (!(fabsf(c) <= (float)kRankMaxDrift) || !(h <= kRankMaxHalfRange)) return false;
   const int n0 = (int)floorf(c - 0.5f) - 3;
+  // (a float of less than 2^26 is within two units of the bias: the zones have three to spare)
+  const double bias = (double)kRankMagic + ((double)mean_v * ((double)s / unit) + shift - n0) * unit;
+  if (!(fabs(bias) < 67108864.0)) return false;
   const float pc = c - (float)n0;  // 3.5 .. 4.5
   const int ql = (int)((pc - h) * unit), qh = (int)((pc + h) * unit);
   for (int kind = 2 * axis; kind < 2 * axis + 2; ++kind) {
@@ -105,7 +109,7 @@ E2E_RANK_FN bool rank_range(const uint32_t* plan, int slots_log2, const int* gro
       const float at = (float)(idx + n0) - (float)shift;
       if (!(at + a_min + (float)qa / unit > 0.01f && at + a_max + (float)qb / unit < (float)(g - 1) - 0.01f)) continue;
     }
-    r->bias = (float)((double)kRankMagic + ((double)mean_v * ((double)s / unit) + shift - n0) * unit);
+    r->bias = (float)bias;
     r->qa = (int)kRankBits + qa;
     r->qb = (int)kRankBits + qb;
     r->lut = kind * rank_lut_words(slots_log2) - (int)(kRankBits >> (kRankFrac - slots_log2));

@@ -104,3 +104,9 @@ def zones(tmp_path_factory):
 def test_samples_outside_the_zones(zones, g, na, dx, x0):
     r = subprocess.run([zones, str(g), str(na), str(dx), str(x0), "0"], capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stdout
+
+
+@pytest.mark.parametrize("mean", [20, 50, -50, 60, 120, -120, 1000, -1000])
+def test_mean_velocities_that_the_modes_cancel(zones, mean):
+    r = subprocess.run([zones, "200", "16", "1", "0.5", str(mean)], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout
