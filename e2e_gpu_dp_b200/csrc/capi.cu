@@ -138,12 +138,19 @@ void drop_cached(int dev, cudaStream_t st) {
 }  // namespace
 
 namespace e2e {
-// Test hook: E2E_TEST_ALLOC_FAIL=lo:hi refuses every request of lo to hi bytes, as
-// a device without that much memory would.
+// Test hooks: E2E_TEST_ALLOC_FAIL=lo:hi refuses every request of lo to hi bytes,
+// E2E_TEST_ALLOC_TOTAL=n every request of a large block with which more than n bytes
+// of them would be handed out, as a device without that much memory would.
 static bool refused_by_test(size_t bytes) {
   const char* v = std::getenv("E2E_TEST_ALLOC_FAIL");
   unsigned long long lo = 0, hi = 0;
-  return v && std::sscanf(v, "%llu:%llu", &lo, &hi) == 2 && bytes >= lo && bytes <= hi;
+  if (v && std::sscanf(v, "%llu:%llu", &lo, &hi) == 2 && bytes >= lo && bytes <= hi) return true;
+  const char* most = std::getenv("E2E_TEST_ALLOC_TOTAL");
+  if (!most || bytes < kCacheMinBytes) return false;
+  std::lock_guard<std::mutex> lk(g_live_mu);
+  size_t held = bytes;
+  for (const auto& b : g_live) held += b.second.first;
+  return held > std::strtoull(most, nullptr, 10);
 }
 
 cudaError_t dalloc(void** p, size_t bytes, cudaStream_t st) {

@@ -949,13 +949,6 @@ extern "C" e2e_status e2e_env_generate(const e2e_env_params* p, const int32_t* i
   // (both fields' matrices of a step are a launch's z index, of which there are 65535)
   int batch = (int)std::min<size_t>(std::min(nt, kMaxBatch), std::max<size_t>(1, (size_t(2) << 30) / (8 * step_doubles)));
   double *work, *Om, *sv, *coarse;
-  for (;; batch = (batch + 1) / 2) {  // a device with less free memory takes smaller batches
-    const cudaError_t e = dalloc((void**)&work, sizeof(double) * step_doubles * batch, st);
-    if (e == cudaSuccess) break;
-    if (e != cudaErrorMemoryAllocation || batch == 1) return cuda_fail(e, "work arrays of the rank reductions");
-    cudaGetLastError();
-  }
-  scratch.add(work);
   CK(dalloc((void**)&Om, sizeof(double) * (size_t)2 * n * kRrMaxK, st));
   scratch.add(Om);
   CK(dalloc((void**)&sv, sizeof(double) * 2 * (size_t)nt * r, st));
@@ -976,6 +969,21 @@ extern "C" e2e_status e2e_env_generate(const e2e_env_params* p, const int32_t* i
     CK(dalloc((void**)&o.mask, sizeof(int32_t) * (size_t)nt * G2, st));
     scratch.add(o.mask);
   }
+  // the last of the buffers: a device with less free memory takes smaller batches, which
+  // leave room for a reduction of more columns (enlarge_svd)
+  void* room = nullptr;
+  for (;; batch = (batch + 1) / 2) {
+    const cudaError_t e = dalloc((void**)&work, sizeof(double) * step_doubles * batch, st);
+    if (e == cudaSuccess) break;
+    if (e != cudaErrorMemoryAllocation || batch == 1) {
+      dfree(room, st);
+      return cuda_fail(e, "work arrays of the rank reductions");
+    }
+    cudaGetLastError();
+    if (!room) CK(dalloc(&room, sizeof(double) * rr_work_doubles(nws, 2 * n, std::min(kRrMaxK, std::min(nws, 2 * n))), st));
+  }
+  dfree(room, st);
+  scratch.add(work);
   int enlarged = 0;
   for (int t0 = 0; t0 < nt; t0 += batch) {
     const int nbt = std::min(batch, nt - t0);

@@ -35,3 +35,19 @@ def test_less_memory_than_one_batch_needs():
         os.environ.pop("E2E_TEST_ALLOC_FAIL", None)
     for k in envgen.FILES + ("svals_vel", "svals_phi"):
         assert np.array_equal(whole[k], parts[k]), k
+
+
+def test_batches_leave_room_for_every_other_buffer():
+    # 39 MB of outputs and 126 MB of work arrays: with less memory than that, smaller batches
+    make = lambda: envgen.build_environment_DG_with_westward_clouds(
+        init_gsize=8, nt=200, dt=0.25, dxy=0.25, A=0.5, A_sc=3.0, eps=0.1, op_nrzns=10, n_wsamples=200,
+        w_range=(np.pi / 10, 8 * np.pi / 10), wx=np.pi, interpolate_degree=8, n_modes=4, dyn_obstacle_data=("None",))
+    whole = make()
+    for mb in range(70, 301, 10):
+        os.environ["E2E_TEST_ALLOC_TOTAL"] = str(mb << 20)
+        try:
+            parts = make()
+        finally:
+            os.environ.pop("E2E_TEST_ALLOC_TOTAL", None)
+        for k in envgen.FILES + ("svals_vel", "svals_phi"):
+            assert np.array_equal(whole[k], parts[k]), (mb, k)
