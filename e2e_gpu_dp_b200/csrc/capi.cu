@@ -845,15 +845,14 @@ e2e_status copy_field_steps(const FieldsOnDevice& fd, int t0, int t1, cudaStream
 // host fields below this many bytes are uploaded before the builder starts
 constexpr size_t kUploadAtOnce = size_t(16) << 20;
 
-e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, cudaStream_t st, DeviceScratch* scratch,
-                               LayerBuild* L) {
+e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, LayerBuild* L) {
   if (!pl.ranked) return E2E_OK;
   const size_t nmp = (size_t)rank_padded_modes(p->nmodes), layers = (size_t)(p->nt - 1);
   RankArgs& K = L->K;
   K = pl.rank;
   auto take = [&](size_t bytes, void** q) -> cudaError_t {
-    cudaError_t e = dalloc(q, bytes, st);
-    if (e == cudaSuccess) scratch->add(*q);
+    cudaError_t e = dalloc(q, bytes, L->st);
+    if (e == cudaSuccess) L->bufs.push_back(*q);
     return e;
   };
   void *plan, *yt, *ystat, *obits, *count, *flag;
@@ -869,11 +868,12 @@ e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, cudaSt
     const cudaError_t e = take(bytes, q);
     if (e == cudaErrorMemoryAllocation) {  // (the coefficients again, above all): the general builder needs none of it
       cudaGetLastError();
+      L->drop();
       return E2E_OK;
     }
     CK(e);
   }
-  CK(cudaMemcpyAsync(plan, pl.rank_words.data(), pb, cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(plan, pl.rank_words.data(), pb, cudaMemcpyHostToDevice, L->st));
   K.plan = static_cast<const uint32_t*>(plan);
   K.yt = static_cast<const float*>(yt);
   K.ystat = static_cast<const float*>(ystat);
@@ -938,8 +938,8 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
   CK(dalloc((void**)&ctr, sizeof(unsigned long long) * CTR_COUNT, st));
   scratch->add(ctr);
 
-  LayerBuild L;
-  s = layer_build_buffers(p, pl, st, scratch, &L);
+  LayerBuild L(st);
+  s = layer_build_buffers(p, pl, &L);
   if (s != E2E_OK) return s;
 
   int64_t cap = pl.stage_cap, least = cap, pool_units = pl.pool_units;
@@ -955,7 +955,7 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
   } evfree{ev};
   trace_mark("setup");
   for (int attempt = 0; attempt < 3; ++attempt) {
-    CK(buf.provide(&cap, least, (size_t)cbytes, pool_units, p->neighb_gsize));
+    CK(buf.provide(&cap, least, (size_t)cbytes, pool_units, p->neighb_gsize, &L));
     CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * CTR_COUNT, st));
     BuildArgs A{};
     A.P = D;
@@ -1081,6 +1081,7 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
   m->misbinned = hc[CTR_MISBIN];
   m->overflow_rows = hc[CTR_OVERFLOW_ROWS];
   m->general_tiles = (int32_t)std::min<int64_t>(L.ranked ? (int64_t)hc[CTR_DEFERRED] : pl.n_tiles, INT32_MAX);
+  L.drop();  // the model takes its place
   m->layered = true;
   m->built = true;
   m->prob = *p;

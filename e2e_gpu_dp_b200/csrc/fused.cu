@@ -176,10 +176,6 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
   DevProblem D;
   s = make_dev_problem(p, st, &D, &scratch);
   if (s != E2E_OK) return s;
-  LayerBuild L;
-  s = layer_build_buffers(p, pl, st, &scratch, &L);
-  if (s != E2E_OK) return s;
-
   const int64_t ns = pl.ns, nc = pl.ncells;
   float* dV = nullptr;
   int32_t* dpi = nullptr;
@@ -227,6 +223,9 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
   CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * ctr_words * nblocks, st));
   const int mm = p->neighb_gsize * p->neighb_gsize;
   int64_t pool_units = pl.pool_units, cap = rows * bl * 4 + 4096, least = cap;
+  LayerBuild L(st);
+  s = layer_build_buffers(p, pl, &L);
+  if (s != E2E_OK) return s;
   BuildStaging buf(st);
 
   int dev = 0, sms = 0, per_sm = 0;
@@ -249,7 +248,7 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
     bc = ctr + ctr_words * b;
     unsigned long long hc[CTR_COUNT + 1];
     for (int attempt = 0;; ++attempt) {
-      CK(buf.provide(&cap, least, sizeof(uint16_t), pool_units, p->neighb_gsize));
+      CK(buf.provide(&cap, least, sizeof(uint16_t), pool_units, p->neighb_gsize, &L));
       if (attempt) CK(cudaMemsetAsync(bc, 0, sizeof(unsigned long long) * CTR_COUNT, st));
       BuildArgs A{};
       A.P = D;

@@ -125,17 +125,28 @@ e2e_status copy_field_steps(const FieldsOnDevice& fd, int t0, int t1, cudaStream
 e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const BuildPlan& pl,
                      cudaStream_t st, DeviceScratch* scratch, e2e_model* m);
 // Builder launches over ranges of layers.  layer_build_buffers allocates what the
-// ranked builder needs beside the fields (nothing for other problems);
-// launch_layers queues the builder for layers [t0, t1); launch_leftover the
-// general builder for the tiles of [t0, t1) that the ranked one listed.
+// ranked builder needs beside the fields (nothing for other problems), drop gives it
+// back: the general builder then takes whole layers; launch_layers queues the builder
+// for layers [t0, t1); launch_leftover the general builder for the tiles of [t0, t1)
+// that the ranked one listed.
 struct LayerBuild {
+  cudaStream_t st;
   bool ranked = false;  // the plan's choice, unless memory for the ranked builder is missing
   RankArgs K{};
   unsigned int* defer_count = nullptr;
   uint8_t* defer_flag = nullptr;
+  std::vector<void*> bufs;
+  explicit LayerBuild(cudaStream_t s) : st(s) {}
+  LayerBuild(const LayerBuild&) = delete;
+  LayerBuild& operator=(const LayerBuild&) = delete;
+  ~LayerBuild() { drop(); }
+  void drop() {
+    for (void* p : bufs) dfree(p, st);
+    bufs.clear();
+    ranked = false;
+  }
 };
-e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, cudaStream_t st, DeviceScratch* scratch,
-                               LayerBuild* L);
+e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, LayerBuild* L);
 cudaError_t launch_layers(const BuildArgs& A, const BuildPlan& pl, const LayerBuild& L, int t0, int t1, cudaStream_t st);
 cudaError_t launch_leftover(const BuildArgs& A, const BuildPlan& pl, const LayerBuild& L, int t0, int t1,
                             cudaStream_t st);
@@ -178,17 +189,25 @@ struct BuildStaging {
     pool = nullptr;
   }
   // What is missing of *cap entries, or of `least` of them where memory for more is
-  // missing, and of pool_units histograms of m x m
-  cudaError_t provide(int64_t* cap, int64_t least, size_t count_bytes, int64_t pool_units, int m) {
-    cudaError_t e = cudaSuccess;
-    if (!pool) e = dalloc(&pool, sizeof(uint32_t) * (size_t)m * (size_t)m * (size_t)pool_units, st);
-    if (e != cudaSuccess || col) return e;
+  // missing, and of pool_units histograms of m x m; where even that cannot be had, what
+  // the ranked builder holds is given back first.
+  cudaError_t provide(int64_t* cap, int64_t least, size_t count_bytes, int64_t pool_units, int m, LayerBuild* L) {
     for (;; *cap = least) {
-      e = dalloc(&col, sizeof(int32_t) * (size_t)*cap, st);
-      if (e == cudaSuccess) e = dalloc(&cnt, count_bytes * (size_t)*cap, st);
-      if (e != cudaErrorMemoryAllocation || *cap == least) return e;
+      cudaError_t e = cudaSuccess;
+      if (!pool) e = dalloc(&pool, sizeof(uint32_t) * (size_t)m * (size_t)m * (size_t)pool_units, st);
+      if (e != cudaSuccess) pool = nullptr;
+      if (e == cudaSuccess && !col) {
+        e = dalloc(&col, sizeof(int32_t) * (size_t)*cap, st);
+        if (e == cudaSuccess) e = dalloc(&cnt, count_bytes * (size_t)*cap, st);
+        else col = nullptr;
+        if (e != cudaSuccess) {
+          cnt = nullptr;
+          drop_stage();
+        }
+      }
+      if (e != cudaErrorMemoryAllocation || (*cap == least && !L->ranked)) return e;
       cudaGetLastError();
-      drop_stage();
+      if (*cap == least) L->drop();
     }
   }
 };

@@ -114,3 +114,31 @@ def test_build_without_memory_for_the_rank_tables(call):
     with refuse(coeffs):
         got = results()
     assert all(np.array_equal(a, b) for a, b in zip(want, got))
+
+
+@pytest.mark.parametrize("call", ["build_model", "build_solve"])
+def test_build_gives_the_rank_tables_back_for_the_other_buffers(call):
+    torch = pytest.importorskip("torch")
+    prob = Problem(gsize=44, nt=40, nrzns=12000, nmodes=10, num_ac_angles=8, i_term=25, j_term=9, neighb_gsize=15)
+    spec = FieldSpec(sigma0=0.1, obstacle_frac=0.04, seed=6)
+    fields = {k: torch.as_tensor(v).cuda() for k, v in make_fields(prob, spec).items()}
+
+    def results():
+        if call == "build_solve":
+            *r, st = api.build_solve(prob, fields)
+            return [np.asarray(torch.as_tensor(x).cpu()) for x in r], st["general_tiles"]
+        m = api.build_model(prob, fields)
+        h, tiles = m.to_host(), m.info()["general_tiles"]
+        m.free()
+        return [h[k] for k in ("row_ptr", "col", "cnt", "R")], tiles
+
+    want, tiles = results()
+    assert tiles < prob.ncells * (prob.nt - 1) // 4
+    # 10 MB of staged columns, then a model of less, beside 19 MB of coefficients
+    os.environ["E2E_TEST_ALLOC_TOTAL"] = str(24 << 20)
+    try:
+        got, tiles = results()
+    finally:
+        os.environ.pop("E2E_TEST_ALLOC_TOTAL", None)
+    assert call == "build_solve" or tiles == prob.ncells * (prob.nt - 1) // 4  # (groups of 4 cells)
+    assert all(np.array_equal(a, b) for a, b in zip(want, got))
