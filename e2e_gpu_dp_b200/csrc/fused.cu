@@ -197,24 +197,48 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
   CK(cudaMemsetAsync(dV + last, 0, sizeof(float) * (size_t)nc, st));
   CK(cudaMemsetAsync(dpi + last, 0, sizeof(int32_t) * (size_t)nc, st));
 
-  // blocks of layers, of about equal size within the staging budget
+  // blocks of layers, of about equal size within the staging budget, or of fewer layers
+  // where memory for that is missing
+  LayerBuild L(st);
+  s = layer_build_buffers(p, pl, &L);
+  if (s != E2E_OK) return s;
+  BuildStaging buf(st);
+  struct {
+    uint32_t* row_off;
+    float* R;
+    int64_t* tile_base;
+    int32_t* tile_len;
+  } blk;
   const int layers = p->nt - 1;
   const int64_t rows = nc * pl.na;
   const size_t per_layer = (size_t)rows * (sizeof(uint32_t) + sizeof(float) + 4 * 6);
-  const int most = (int)std::max<size_t>(1, std::min<size_t>((size_t)layers, stage_budget() / per_layer));
-  const int nblocks = (layers + most - 1) / most, bl = (layers + nblocks - 1) / nblocks;
-  uint32_t* row_off = nullptr;
-  int64_t* tile_base = nullptr;
-  int32_t* tile_len = nullptr;
-  float* R = nullptr;
-  CK(dalloc((void**)&row_off, sizeof(uint32_t) * (size_t)rows * bl, st));
-  scratch.add(row_off);
-  CK(dalloc((void**)&R, sizeof(float) * (size_t)rows * bl, st));
-  scratch.add(R);
-  CK(dalloc((void**)&tile_base, sizeof(int64_t) * (size_t)pl.etiles_per_layer * bl, st));
-  scratch.add(tile_base);
-  CK(dalloc((void**)&tile_len, sizeof(int32_t) * (size_t)pl.etiles_per_layer * bl, st));
-  scratch.add(tile_len);
+  int64_t pool_units = pl.pool_units, cap = 0, least = 0;
+  int most = (int)std::max<size_t>(1, std::min<size_t>((size_t)layers, stage_budget() / per_layer));
+  int nblocks = 0, bl = 0;
+  for (;;) {
+    nblocks = (layers + most - 1) / most;
+    bl = (layers + nblocks - 1) / nblocks;
+    cap = least = rows * bl * 4 + 4096;
+    const size_t n = (size_t)rows * bl, nt = (size_t)pl.etiles_per_layer * bl;
+    char* at = nullptr;
+    cudaError_t e = dalloc((void**)&at, sizeof(int64_t) * nt + sizeof(int32_t) * nt + (sizeof(uint32_t) + sizeof(float)) * n, st);
+    if (e == cudaSuccess) {
+      e = buf.provide(&cap, least, sizeof(uint16_t), pool_units, p->neighb_gsize, nullptr);
+      if (e == cudaSuccess) {
+        scratch.add(at);
+        blk.tile_base = reinterpret_cast<int64_t*>(at);
+        blk.row_off = reinterpret_cast<uint32_t*>(blk.tile_base + nt);
+        blk.R = reinterpret_cast<float*>(blk.row_off + n);
+        blk.tile_len = reinterpret_cast<int32_t*>(blk.R + n);
+        break;
+      }
+      dfree(at, st);
+    }
+    if (e != cudaErrorMemoryAllocation || (most == 1 && !L.ranked)) return cuda_fail(e, "buffers of a block of layers");
+    cudaGetLastError();
+    if (most > 1) most /= 2;
+    else L.drop();
+  }
   // per block: the builder's counters, then the barrier words of its backup
   unsigned long long* ctr = nullptr;
   const size_t ctr_words = CTR_COUNT + 1;
@@ -222,11 +246,6 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
   scratch.add(ctr);
   CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * ctr_words * nblocks, st));
   const int mm = p->neighb_gsize * p->neighb_gsize;
-  int64_t pool_units = pl.pool_units, cap = rows * bl * 4 + 4096, least = cap;
-  LayerBuild L(st);
-  s = layer_build_buffers(p, pl, &L);
-  if (s != E2E_OK) return s;
-  BuildStaging buf(st);
 
   int dev = 0, sms = 0, per_sm = 0;
   CK(cudaGetDevice(&dev));
@@ -267,10 +286,10 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
       A.stage_cnt = buf.cnt;
       A.stage_cap = cap;
       // the builder indexes by layer: the block's first one at the buffers' start
-      A.row_off = row_off - rows * t0;
-      A.R = R - rows * t0;
-      A.tile_base = tile_base - pl.etiles_per_layer * t0;
-      A.tile_len = tile_len - pl.etiles_per_layer * t0;
+      A.row_off = blk.row_off - rows * t0;
+      A.R = blk.R - rows * t0;
+      A.tile_base = blk.tile_base - pl.etiles_per_layer * t0;
+      A.tile_len = blk.tile_len - pl.etiles_per_layer * t0;
       CK(launch_layers(A, pl, L, t0, t1, st));
       CK(launch_leftover(A, pl, L, t0, t1, st));
       ++launches;
@@ -314,10 +333,10 @@ extern "C" e2e_status e2e_build_solve(const e2e_problem* p, const e2e_fields* f,
     B.nrzns = p->nrzns;
     B.nc = (int)nc;
     B.etiles_per_layer = pl.etiles_per_layer;
-    B.row_off = row_off;
-    B.tile_base = tile_base;
-    B.tile_len = tile_len;
-    B.R = R;
+    B.row_off = blk.row_off;
+    B.tile_base = blk.tile_base;
+    B.tile_len = blk.tile_len;
+    B.R = blk.R;
     B.stage_col = static_cast<const int32_t*>(buf.col);
     B.stage_cnt = static_cast<const uint16_t*>(buf.cnt);
     B.V = dV;

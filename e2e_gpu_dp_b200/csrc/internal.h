@@ -190,7 +190,7 @@ struct BuildStaging {
   }
   // What is missing of *cap entries, or of `least` of them where memory for more is
   // missing, and of pool_units histograms of m x m; where even that cannot be had, what
-  // the ranked builder holds is given back first.
+  // the ranked builder L (or none) holds is given back first.
   cudaError_t provide(int64_t* cap, int64_t least, size_t count_bytes, int64_t pool_units, int m, LayerBuild* L) {
     for (;; *cap = least) {
       cudaError_t e = cudaSuccess;
@@ -205,7 +205,7 @@ struct BuildStaging {
           drop_stage();
         }
       }
-      if (e != cudaErrorMemoryAllocation || (*cap == least && !L->ranked)) return e;
+      if (e != cudaErrorMemoryAllocation || (*cap == least && !(L && L->ranked))) return e;
       cudaGetLastError();
       if (*cap == least) L->drop();
     }

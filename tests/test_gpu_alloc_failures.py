@@ -142,3 +142,17 @@ def test_build_gives_the_rank_tables_back_for_the_other_buffers(call):
         os.environ.pop("E2E_TEST_ALLOC_TOTAL", None)
     assert call == "build_solve" or tiles == prob.ncells * (prob.nt - 1) // 4  # (groups of 4 cells)
     assert all(np.array_equal(a, b) for a, b in zip(want, got))
+
+
+def test_build_solve_without_memory_for_a_block_of_layers():
+    torch = pytest.importorskip("torch")
+    prob = Problem(gsize=44, nt=40, nrzns=200, nmodes=2, num_ac_angles=8, i_term=25, j_term=9, neighb_gsize=15)
+    fields = make_fields(prob, FieldSpec(sigma0=0.1, obstacle_frac=0.04, seed=6))
+    *want, st = api.build_solve(prob, fields)
+    assert st["launches"] == 2
+    # 10 MB of staged columns; with the first range refused three blocks, with the second (not the dense pool's 7.4 MB) five
+    for lo, hi, blocks in ((9000000, 1 << 40, 3), (3000000, 7300000, 5)):
+        with refuse(lo, hi):
+            *got, st = api.build_solve(prob, fields)
+        assert st["launches"] == 2 * blocks
+        assert all(np.array_equal(a, b) for a, b in zip(want, got))
