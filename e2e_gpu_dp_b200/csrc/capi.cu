@@ -842,8 +842,17 @@ e2e_status copy_field_steps(const FieldsOnDevice& fd, int t0, int t1, cudaStream
   return E2E_OK;
 }
 
-// host fields below this many bytes are uploaded before the builder starts
-constexpr size_t kUploadAtOnce = size_t(16) << 20;
+// Host fields below this many bytes are uploaded before the builder starts.  A second
+// stream and four launches cost 0.05 to 0.2 ms, so they have to hide that much copying
+// behind that much building.  Measured (upload first, overlapped; 10 modes and the
+// ranked builder): 4.8 MB 0.66, 0.70 ms; 11 MB and 1.8e8 samples 1.02, 1.19; 15.7 MB and
+// 2.6e8 1.38, 1.44; 16 MB and 2.4e9 1.87, 1.74; 6.3 MB and 5.6e9 1.57, 1.73; 7.3 MB and
+// 3.2e9 1.44, 1.34; 8.5 MB and 4.5e9 1.78, 1.34.  The general builder: 6.4 MB 1.20, 1.26
+// ms; 9.1 MB 2.32, 2.48; 12.5 MB 1.76, 1.51; 18.4 MB 8.99, 8.59.
+static size_t upload_at_once(const BuildPlan& pl, int nrzns) {
+  if (!pl.ranked) return size_t(10) << 20;
+  return (double)pl.n_rows * nrzns < 2e9 ? size_t(16) << 20 : size_t(7) << 20;
+}
 
 e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, LayerBuild* L) {
   if (!pl.ranked) return E2E_OK;
@@ -984,9 +993,8 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
     };
     CK(cudaEventRecord(ev[0], st));
     trace_mark("buffers");
-    if (attempt == 0 && fd.n_deferred && fd.h2d_bytes < kUploadAtOnce) {
-      // small host fields: one copy and one launch (50x50x30, 4 MB: a second
-      // stream and launch cost 0.2 of 1.5 ms and hid nothing)
+    if (attempt == 0 && fd.n_deferred && fd.h2d_bytes < upload_at_once(pl, p->nrzns)) {
+      // small host fields: one copy and one launch
       e2e_status cs = copy_field_steps(fd, 0, p->nt, st);
       if (cs != E2E_OK) return cs;
       trace_mark("copies");
