@@ -16,6 +16,7 @@ from e2e_gpu_dp_b200.problem import FieldSpec, Problem, make_fields
 from tests.helpers import problem
 
 pytestmark = pytest.mark.gpu
+os.environ["E2E_TEST_HOOKS"] = "1"  # read at the library's first allocation
 
 
 class refuse:

@@ -7,6 +7,7 @@ import pytest
 from e2e_gpu_dp_b200 import envgen
 
 pytestmark = pytest.mark.gpu
+os.environ["E2E_TEST_HOOKS"] = "1"  # read at the library's first allocation
 BY_STEP = [k for k in envgen.FILES if k not in ("all_s_mat", "obstacle_mask")]
 
 

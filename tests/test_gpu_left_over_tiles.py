@@ -16,6 +16,7 @@ from e2e_gpu_dp_b200.problem import FieldSpec, make_fields
 from .test_gpu_ranks import _check, _prob
 
 pytestmark = pytest.mark.gpu
+os.environ["E2E_TEST_HOOKS"] = "1"  # read at the library's first allocation
 
 
 @pytest.mark.parametrize("angles", [2, 3, 4, 8, 16, 32])
