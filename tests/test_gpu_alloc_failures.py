@@ -157,3 +157,24 @@ def test_build_solve_without_memory_for_a_block_of_layers():
             *got, st = api.build_solve(prob, fields)
         assert st["launches"] == 2 * blocks
         assert all(np.array_equal(a, b) for a, b in zip(want, got))
+
+
+def test_model_takes_the_place_of_the_rank_tables():
+    torch = pytest.importorskip("torch")
+    prob = Problem(gsize=44, nt=40, nrzns=12000, nmodes=10, num_ac_angles=8, i_term=25, j_term=9, neighb_gsize=15)
+    spec = FieldSpec(sigma0=0.38, obstacle_frac=0.04, seed=6)
+    fields = {k: torch.as_tensor(v).cuda() for k, v in make_fields(prob, spec).items()}
+    m = api.build_model(prob, fields)
+    want, nnz = m.to_host(), m.info()["nnz"]
+    m.free()
+    assert 4 * nnz > 8 << 20
+    # 19 MB of coefficients, the staged columns and the model's
+    for over in (0, 4 << 20, 8 << 20):
+        os.environ["E2E_TEST_ALLOC_TOTAL"] = str((30 << 20) + over)
+        try:
+            m = api.build_model(prob, fields)
+        finally:
+            os.environ.pop("E2E_TEST_ALLOC_TOTAL", None)
+        got = m.to_host()
+        m.free()
+        assert all(np.array_equal(want[k], got[k]) for k in ("row_ptr", "col", "cnt", "R"))
