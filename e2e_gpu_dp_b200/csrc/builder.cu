@@ -13,7 +13,7 @@
 //    i.e. a contiguous range of model rows.  Which cell groups a CTA takes is
 //    chosen by group_of_slot (warps that reach the grid edge in CTAs of their
 //    own).  Problems that the ranked builder takes (builder_ranks.cu) come here
-//    only for the groups of cells it lists;
+//    only for the groups of cells it leaves over;
 //  * the velocity of every (cell, realisation) is computed once per chunk of
 //    realisations (u + sum_k ui_k*Y_k, reference order) into warp-private
 //    shared memory and reused by all actions (the reference recomputes it per
@@ -935,7 +935,7 @@ __device__ __forceinline__ void left_over_groups(const BuildArgs& A, int T, int 
   __shared__ int2 sums[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const int n = (int)A.etiles_per_layer, run = ((n + (int)blockDim.x - 1) / (int)blockDim.x + 3) & ~3;
-  const uint8_t* marks = A.defer_flag + T * defer_stride(n);
+  const uint8_t* marks = A.defer + T * defer_bytes(n) + kDeferCounts;
   auto word = [&](int k) -> uint32_t {  // of tiles k .. k + 3
     if (k >= n) return 0u;
     const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(marks + k));
@@ -1003,8 +1003,9 @@ __global__ void __launch_bounds__(1024) k_build_listed(BuildArgs A) {
     if (threadIdx.x == 0) {
       const int64_t item = (int64_t)atomicAdd(A.counters + CTR_NEXT, 1ull);  // (grows from one turn to the next)
       for (; at.T < A.t1; ++at.T) {
-        at.n_edge = (int)A.defer_count[2 * at.T];
-        const int items = (at.n_edge + (int)A.defer_count[2 * at.T + 1] + nwarps - 1) / nwarps;
+        const int* counts = reinterpret_cast<const int*>(A.defer + at.T * defer_bytes(A.etiles_per_layer));
+        at.n_edge = counts[0];
+        const int items = (counts[0] + counts[1] + nwarps - 1) / nwarps;
         if (item < at.before + items) break;
         at.before += items;
       }
@@ -1213,7 +1214,7 @@ static cudaError_t raise_smem_cap(K kern, size_t sm, int* cap_set, std::mutex& m
 
 template <typename CntT, bool UNIT>
 static cudaError_t launch_one(const BuildArgs& A, int n_layers, cudaStream_t st) {
-  const bool listed = A.defer_count != nullptr;
+  const bool listed = A.defer != nullptr;
   auto kern = listed ? k_build_listed<CntT, UNIT> : k_build_tiles<CntT, UNIT>;
   dim3 grid((unsigned)A.tiles_per_layer, (unsigned)n_layers);
   if (listed) {

@@ -1,7 +1,7 @@
 // K1 by velocity ranks: the Monte-Carlo transition builder for grids whose
 // spacing is a power of two, up to ten modes and 2 to 32 actions; groups of
 // cells it cannot take (velocities spread too widely for a table, rows with
-// samples outside their 8x8 window) are listed and left to k_build_tiles.
+// samples outside their 8x8 window) are marked and left to k_build_listed.
 //
 // transition_calc (src/build_model.cu:483-559) moves every sample of every
 // action.  But along one axis the landing cell is a step function of the
@@ -15,7 +15,7 @@
 //     together, against 11-14 per action of the counting loops;
 //   per (cell, action): at most 81 table reads.
 // A sample within the zone of a step (where the reference's float rounding
-// decides) or outside the table's range, about 1 in 2000, goes to the cell's
+// decides) or outside the table's range, about 1 in 2000 (1 in 1000 on a thousand cells a side), goes to the cell's
 // list and takes the reference's full expression for each action.  Counts are
 // the reference's exactly; rewards are folded from the counts as in
 // k_build_tiles.
@@ -428,17 +428,16 @@ __device__ __forceinline__ void finish_tile(const BuildArgs& A, const RankArgs& 
       }
     }
   }
-  uint8_t* const left = A.defer_flag + T * defer_stride(K.etiles_per_layer) + et;
   if (__any_sync(0xffffffffu, !ok)) {  // the tile goes to the general builder
     const bool inner = !__any_sync(0xffffffffu, valid && in_edge_band(i1, j1, g));
     if (lane == 0) {
-      *left = inner ? TILE_INNER : TILE_EDGE;
-      atomicAdd(A.defer_count + 2 * T + inner, 1u);
+      uint8_t* const left = A.defer + T * defer_bytes(K.etiles_per_layer);
+      left[kDeferCounts + et] = inner ? TILE_INNER : TILE_EDGE;
+      atomicAdd(reinterpret_cast<unsigned int*>(left) + inner, 1u);
       atomicAdd(A.counters + CTR_DEFERRED, 1ull);
     }
     return;
   }
-  if (lane == 0) *left = TILE_BUILT;
   float sumR = 0.f;
   uint32_t n_drop = 0, n_misbin = 0;
   if (window) {

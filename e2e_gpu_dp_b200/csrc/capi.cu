@@ -868,15 +868,14 @@ e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, LayerB
     if (e == cudaSuccess) L->bufs.push_back(*q);
     return e;
   };
-  void *plan, *yt, *ystat, *obits, *count, *flag;
+  void *plan, *yt, *ystat, *obits, *defer;
   const size_t pb = sizeof(uint32_t) * pl.rank_words.size();
   const std::pair<size_t, void**> need[] = {
       {pb, &plan},
       {sizeof(float) * layers * nmp * (size_t)K.nrp, &yt},
       {sizeof(float) * layers * nmp * 2, &ystat},
       {sizeof(uint32_t) * layers * (size_t)p->gsize * (size_t)K.owords, &obits},
-      {sizeof(unsigned int) * 2 * layers, &count},
-      {layers * (size_t)defer_stride(pl.etiles_per_layer), &flag}};
+      {layers * (size_t)defer_bytes(pl.etiles_per_layer), &defer}};
   for (const auto& [bytes, q] : need) {
     const cudaError_t e = take(bytes, q);
     if (e == cudaErrorMemoryAllocation) {  // (the coefficients again, above all): the general builder needs none of it
@@ -891,8 +890,7 @@ e2e_status layer_build_buffers(const e2e_problem* p, const BuildPlan& pl, LayerB
   K.yt = static_cast<const float*>(yt);
   K.ystat = static_cast<const float*>(ystat);
   K.obits = static_cast<const uint32_t*>(obits);
-  L->defer_count = static_cast<unsigned int*>(count);
-  L->defer_flag = static_cast<uint8_t*>(flag);
+  L->defer = static_cast<uint8_t*>(defer);
   L->ranked = true;
   return E2E_OK;
 }
@@ -902,12 +900,12 @@ cudaError_t launch_layers(const BuildArgs& A, const BuildPlan& pl, const LayerBu
   B.t0 = t0;
   B.t1 = t1;
   if (!L.ranked) return launch_build_tiles(B, pl.count_bits, t1 - t0, st);
-  B.defer_count = L.defer_count;
-  B.defer_flag = L.defer_flag;
+  B.defer = L.defer;
   RankArgs R = L.K;
   R.t0 = t0;
   R.t1 = t1;
-  cudaError_t e = cudaMemsetAsync(L.defer_count + 2 * t0, 0, sizeof(unsigned int) * 2 * (size_t)(t1 - t0), st);
+  const size_t db = (size_t)defer_bytes(pl.etiles_per_layer);
+  cudaError_t e = cudaMemsetAsync(L.defer + t0 * db, 0, (t1 - t0) * db, st);
   if (e == cudaSuccess) e = launch_rank_prepare(A.P, A.F, R, st);
   return e != cudaSuccess ? e : launch_build_ranks(B, R, st);
 }
@@ -918,8 +916,7 @@ cudaError_t launch_leftover(const BuildArgs& A, const BuildPlan& pl, const Layer
   BuildArgs B = A;
   B.t0 = t0;
   B.t1 = t1;
-  B.defer_count = L.defer_count;
-  B.defer_flag = L.defer_flag;
+  B.defer = L.defer;
   B.ctas_per_sm = pl.ctas_per_sm;
   return launch_build_tiles(B, pl.count_bits, t1 - t0, st);
 }

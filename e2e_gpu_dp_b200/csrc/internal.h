@@ -128,13 +128,12 @@ e2e_status run_build(const e2e_problem* p, const FieldsOnDevice& fd, const Build
 // ranked builder needs beside the fields (nothing for other problems), drop gives it
 // back: the general builder then takes whole layers; launch_layers queues the builder
 // for layers [t0, t1); launch_leftover the general builder for the tiles of [t0, t1)
-// that the ranked one listed.
+// that the ranked one left over.
 struct LayerBuild {
   cudaStream_t st;
   bool ranked = false;  // the plan's choice, unless memory for the ranked builder is missing
   RankArgs K{};
-  unsigned int* defer_count = nullptr;
-  uint8_t* defer_flag = nullptr;
+  uint8_t* defer = nullptr;  // (BuildArgs)
   std::vector<void*> bufs;
   explicit LayerBuild(cudaStream_t s) : st(s) {}
   LayerBuild(const LayerBuild&) = delete;

@@ -26,13 +26,12 @@ enum : unsigned int { FLAG_POOL_EXHAUSTED = 1u };
 struct BuildArgs {
   DevProblem P;
   DevFields F;
-  int t0, t1;           // layers of this launch: t0 + blockIdx.y (t1: end, for listed tiles)
+  int t0, t1;           // layers of this launch: t0 + blockIdx.y (t1: end, for left-over tiles)
   int64_t etiles_per_layer;      // emission tiles (warps' groups of cells) per layer
-  // null, or what the ranked builder left over: per layer the number of emission tiles
-  // near the grid's edge (in_edge_band) and of others, and from T * defer_stride on a
-  // byte a tile: 0 built, or TILE_EDGE, TILE_INNER
-  unsigned int* defer_count;
-  uint8_t* defer_flag;
+  // null, or what the ranked builder left over, defer_bytes a layer: the numbers of
+  // emission tiles near the grid's edge (in_edge_band) and of others, then a byte a tile:
+  // 0 built, or TILE_EDGE, TILE_INNER
+  uint8_t* defer;
   int ctas_per_sm;      // general builder CTAs that an SM holds
   int tiles_per_layer;  // CTAs per layer = ceil(ncells / 32); emission tiles are warps
   int rc;               // realisations per warp-private velocity chunk
@@ -96,11 +95,14 @@ int rank_padded_modes(int nm);
 bool rank_shape(int nm, int slots_log2, int lanes_log2, int nrzns, RankArgs* K);
 // fills yt, ystat, obits of layers [K.t0, K.t1)
 cudaError_t launch_rank_prepare(const DevProblem& P, const DevFields& F, const RankArgs& K, cudaStream_t st);
-// builds layers [K.t0, K.t1); tiles it does not take are marked in A.defer_flag
+// builds layers [K.t0, K.t1); tiles it does not take are marked in A.defer
 cudaError_t launch_build_ranks(const BuildArgs& A, const RankArgs& K, cudaStream_t st);
 
 enum : uint8_t { TILE_BUILT = 0, TILE_EDGE = 1, TILE_INNER = 2 };
-__host__ __device__ inline int64_t defer_stride(int64_t etiles_per_layer) { return (etiles_per_layer + 15) & ~int64_t(15); }
+constexpr int kDeferCounts = 16;  // bytes of a layer's two counts, padded
+__host__ __device__ inline int64_t defer_bytes(int64_t etiles_per_layer) {
+  return kDeferCounts + ((etiles_per_layer + 15) & ~int64_t(15));
+}
 
 int build_lanes_log2(int na);
 size_t build_smem_bytes(int na, int nm, int rc, bool unit, int ybufs);
@@ -108,7 +110,7 @@ size_t build_smem_bytes(int na, int nm, int rc, bool unit, int ybufs);
 // the kernels with 16- and 32-bit counts), from the
 // kernels' registers and static shared memory and the device's limits
 int build_ctas_per_sm(int na, size_t smem, bool unit);
-// n_layers layers from A.t0 on, every tile; with A.defer_count the marked tiles of
+// n_layers layers from A.t0 on, every tile; with A.defer the marked tiles of
 // [A.t0, A.t1) only
 cudaError_t launch_build_tiles(const BuildArgs& A, int count_bits, int n_layers, cudaStream_t st);
 cudaError_t launch_scan_tiles(const int32_t* tile_len, int64_t n_tiles, int64_t* canon,
