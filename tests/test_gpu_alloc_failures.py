@@ -178,3 +178,21 @@ def test_model_takes_the_place_of_the_rank_tables():
         got = m.to_host()
         m.free()
         assert all(np.array_equal(want[k], got[k]) for k in ("row_ptr", "col", "cnt", "R"))
+
+
+def test_build_solve_without_memory_for_one_layer_beside_the_rank_tables():
+    torch = pytest.importorskip("torch")
+    prob = Problem(gsize=256, nt=21, nrzns=10600, nmodes=10, num_ac_angles=8, i_term=25, j_term=9, neighb_gsize=15)
+    spec = FieldSpec(sigma0=0.1, obstacle_frac=0.04, seed=6)
+    fields = {k: torch.as_tensor(v).cuda() for k, v in make_fields(prob, spec).items()}
+    *want, st = api.build_solve(prob, fields)
+    assert st["general_tiles"] < prob.ncells * (prob.nt - 1) // 4
+    # a layer's staged columns and all coefficients, 8.4 and 8.5 MB, in 12 MB
+    os.environ.update(E2E_TEST_ALLOC_TOTAL=str(12 << 20), E2E_TEST_STAGE_BYTES="1")
+    try:
+        *got, st = api.build_solve(prob, fields)
+    finally:
+        os.environ.pop("E2E_TEST_ALLOC_TOTAL", None)
+        os.environ.pop("E2E_TEST_STAGE_BYTES", None)
+    assert st["general_tiles"] == prob.ncells * (prob.nt - 1) // 4  # (groups of 4 cells)
+    assert all(np.array_equal(a, b) for a, b in zip(want, got))
